@@ -123,8 +123,7 @@ struct StoreF32SU3 {
 #pragma unroll
     for (int j = 0; j < 3; j++) {
       const int a1 = (j + 1) % 3, b1 = (j + 2) % 3;
-      cx<CT> t = csub(cmul(u.e[0][a1], u.e[1][b1]), cmul(u.e[0][b1], u.e[1][a1]));
-      u.e[2][j] = {t.re, -t.im};
+      u.e[2][j] = cross_conj(u.e[0][a1], u.e[1][b1], u.e[0][b1], u.e[1][a1]);
     }
     return u;
   }

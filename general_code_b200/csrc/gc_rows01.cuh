@@ -15,8 +15,7 @@ __device__ __forceinline__ void rebuild_row2(SU3<float> &u) {
 #pragma unroll
   for (int j = 0; j < 3; j++) {
     const int a1 = (j + 1) % 3, b1 = (j + 2) % 3;
-    cx<float> t = csub(cmul(u.e[0][a1], u.e[1][b1]), cmul(u.e[0][b1], u.e[1][a1]));
-    u.e[2][j] = {t.re, -t.im};
+    u.e[2][j] = cross_conj(u.e[0][a1], u.e[1][b1], u.e[0][b1], u.e[1][a1]);
   }
 }
 // rows 0 and 1 of A B (A: rows 0, 1; B: all rows)

@@ -13,9 +13,9 @@
 //      levels of three consecutive slices (hyp_slices_kernel), with the
 //      decorated links in rings of slices that stay in L2.
 // The staple sums use the compute type CT (FP64 for the plain form, FP32 for
-// the mixed form). The projection: FP64 SU(3) runs the reference's
-// Newton-Schulz iteration in FP64; mixed SU(3) runs FP32 steps and a last
-// FP64 step (proj_store); SU(2) normalises with |a|^2 and 1/|a| in FP64.
+// the mixed form). The projection (proj_store): SU(3) by a polynomial in the
+// sum's Gram matrix, FP64 or FP32 with a last FP64 correction; SU(2) normalises
+// with |a|^2 and 1/|a| in FP64.
 #include "gc_internal.cuh"
 #include "gc_kernels.h"
 #include "gc_rows01.cuh"
@@ -51,55 +51,63 @@ __device__ __forceinline__ void add_staples(M &S, const void *fmu,
   add_staples2<Store, CT>(S, fmu, fnu, V, x, x_pnu, x_pmu, x_mnu, x_mnu, x_mnu_pmu, c);
 }
 
-// Projection tolerance of the FP64 iteration: an update below it ends the
-// iteration early (see proj in gc_algebra.cuh); 1e-14, so the result equals
-// the full six-step iteration to rounding. (SU(2) projection is a single
-// normalisation and FP32-stored SU(3) uses proj_store's split iteration.)
-template <class Store> struct ProjTol {
-  static constexpr double value = 1e-14;
-};
 // HYP's decorated links of the mixed form are kept in FP32 with all 18 reals
 // (InterStore): the reference's six-step projection of a level-1 or level-2
 // sum need not reach SU(3) (e.g. 0.4 U + 0.3 x staples can be nearly
 // singular), and the 12-real form would replace such a matrix's third row.
 
-// FP32-stored SU(3) (the mixed form): Newton-Schulz steps in FP32 while the
-// unitarity defect exceeds 2e-5 (at most five), then one FP64 step, whose
-// result is stored (ns_until). Other storage: the reference's iteration in
-// FP64 with the early exit of proj(A, tol).
-template <class Store> struct SplitProj {
+// FP32-stored SU(3): the 12-real links or HYP's 18-real decorated links.
+template <class Store> struct MixedSU3 {
   static constexpr bool value = Store::NC == 3 && (Store::kBytes == 48 || Store::kBytes == 72);
 };
 
+// Projection of a sum and its store. SU(3): polar_su3 (gc_algebra.cuh), and
+// outside its region the reference's matrix steps (out of line: one sum in a
+// hundred of HYP's level 1, none of APE's). What bounds it: the FP64 pipe in
+// the FP64 form, the FMA pipe's operand bandwidth in the mixed form, so what
+// counts is the number of multiply-adds. Against the matrix iteration for
+// every sum (3 to 6 steps): HYP at SU(3) 32^4 3.18 -> 2.05 ms FP64 and 1.60
+// -> 1.25 ms mixed, an APE step 0.498 -> 0.384 ms FP64; a mixed APE step
+// 0.251 -> 0.236 ms on the first ten after HYP and unchanged (0.215 ms) on a
+// field so smooth that one FP32 matrix step had been enough.
+//
+// Steps: FP64 the iteration with the early exit of proj(A, tol); FP32 steps
+// while the unitarity defect exceeds 2e-5 (at most five), then one FP64 step.
 // NORM (APE): the FP32 iteration starts from S scaled to sum_ij |S_ij|^2 = 3
-// (mean squared singular value 1). A Newton-Schulz step and the determinant
-// phase fix commute with a positive real factor, so a converging iteration
-// ends at the same SU(3) matrix; it gets there in fewer steps (APE sums of a
-// smeared field are close to a multiple of a unitary matrix: about one FP32
-// step instead of one to two). HYP's level-1 and level-2 sums, which need
-// not converge, keep the reference's trajectory (NORM false).
-template <class Store, class CT, bool NORM = false, class M>
-__device__ __forceinline__ void proj_store(void *out, size_t V, int site,
-                                           const M &S) {
-  using MD = typename Store::template M<double>;
-  if constexpr (SplitProj<Store>::value) {
-    using MF = typename Store::template M<float>;
-    int n;
-    MF a = convert(S, (MF *)nullptr);
-    if constexpr (NORM) {
-      float f2 = 0.f;
+// (a step commutes with a positive factor, so a converging iteration ends at
+// the same matrix); HYP's level-1 and level-2 sums, which need not converge,
+// keep the reference's trajectory.
+template <bool NORM> __device__ __noinline__ void proj_steps(SU3<double> &U) {
+  U = proj(U, 1e-14);
+}
+template <bool NORM> __device__ __noinline__ void proj_steps(SU3<float> &U) {
+  if (NORM) {
+    float f2 = 0.f;
 #pragma unroll
-      for (int i = 0; i < 3; i++)
-#pragma unroll
-        for (int j = 0; j < 3; j++) {
-          f2 = fmaf(a.e[i][j].re, a.e[i][j].re, f2);
-          f2 = fmaf(a.e[i][j].im, a.e[i][j].im, f2);
-        }
-      if (f2 > 0.f)
-        a = scale(a, rsqrtf(f2 * (1.f / 3.f)));
+    for (int k = 0; k < 9; k++) {
+      f2 = fmaf(U.e[k / 3][k % 3].re, U.e[k / 3][k % 3].re, f2);
+      f2 = fmaf(U.e[k / 3][k % 3].im, U.e[k / 3][k % 3].im, f2);
     }
-    const MF f = ns_until(a, 2e-5f, 5, &n);
-    Store::template store<double>(out, V, site, ns_step(convert(f, (MD *)nullptr)));
+    if (f2 > 0.f)
+      U = scale(U, rsqrtf(f2 * (1.f / 3.f)));
+  }
+  int n;
+  const SU3<float> f = ns_until(U, 2e-5f, 5, &n);
+  U = convert(ns_step(convert(f, (SU3<double> *)nullptr)), (SU3<float> *)nullptr);
+}
+
+template <class Store, bool NORM = false, class M>
+__device__ __forceinline__ void proj_store(void *out, size_t V, int site, const M &S) {
+  using MD = typename Store::template M<double>;
+  if constexpr (MixedSU3<Store>::value) {
+    SU3<float> U;
+    if (polar_su3(S, U)) {
+      U = polar_finish<Store::kBytes == 72>(U);
+    } else {
+      U = S;
+      proj_steps<NORM>(U);
+    }
+    Store::template store<float>(out, V, site, U);
   } else if constexpr (Store::NC == 2 && Store::kBytes == 16) {
     // FP32-stored SU(2): a / |a| with |a|^2 and 1/|a| in FP64 (one
     // reciprocal square root instead of a square root and four divisions),
@@ -109,9 +117,15 @@ __device__ __forceinline__ void proj_store(void *out, size_t V, int site,
     const SU2<double> a = convert(S, (SU2<double> *)nullptr);
     const double r = rsqrt(dot4(a.a0, a.a0, a.a1, a.a1, a.a2, a.a2, a.a3, a.a3));
     Store::template store<double>(out, V, site, SU2<double>{a.a0 * r, a.a1 * r, a.a2 * r, a.a3 * r});
+  } else if constexpr (Store::NC == 2) {
+    Store::template store<double>(out, V, site, proj(S));
   } else {
-    MD d = convert(S, (MD *)nullptr);
-    Store::template store<double>(out, V, site, proj(d, ProjTol<Store>::value));
+    MD U;
+    if (!polar_su3(S, U)) {
+      U = S;
+      proj_steps<NORM>(U);
+    }
+    Store::template store<double>(out, V, site, U);
   }
 }
 
@@ -235,7 +249,7 @@ __device__ __forceinline__ void ape_site_mixed_su3(const Geom &g, const Fields4 
                  StoreF32SU3::load<float>(in.f[mu], V, n.mnu));
     add_staple01(S, mul01(a, StoreF32SU3::load<float>(in.f[nu], V, n.mnu_pmu)), c);
   }
-  proj_store<StoreF32SU3, float, true>(out.f[mu], V, site, S);
+  proj_store<StoreF32SU3, true>(out.f[mu], V, site, S);
 }
 
 // One (site, mu) of an APE step (smearing.h:121-155).
@@ -261,7 +275,7 @@ __device__ __forceinline__ void ape_site(const Geom &g, const Fields4 &in,
     add_staples<Store, CT>(S, in.f[mu], in.f[nu], V, site, n.pnu, n.pmu,
                            n.mnu, n.mnu_pmu, c);
   }
-  proj_store<Store, CT, true>(out.f[mu], V, site, S);
+  proj_store<Store, true>(out.f[mu], V, site, S);
 }
 
 // Level-1 decorated links. Field index f:
@@ -305,7 +319,7 @@ __device__ __forceinline__ void hyp_l1_site(const Geom &g, const Fields4 &U,
     a = mul_da01(StoreF32SU3::load<float>(U.f[eta], V, n.mnu),
                  StoreF32SU3::load<float>(U.f[mu], V, n.mnu));
     add_staple01(S, mul01(a, StoreF32SU3::load<float>(U.f[eta], V, n.mnu_pmu)), c);
-    proj_store<StoreF32SU3Full, float>(out.f[f], d.VR, oi, S);
+    proj_store<StoreF32SU3Full>(out.f[f], d.VR, oi, S);
     return;
   }
   using M = typename Store::template M<CT>;
@@ -317,7 +331,7 @@ __device__ __forceinline__ void hyp_l1_site(const Geom &g, const Fields4 &U,
   Nbr n = neighbours(g, site, x, mu, eta);
   add_staples<Store, CT>(S, U.f[mu], U.f[eta], V, site, n.pnu, n.pmu, n.mnu,
                          n.mnu_pmu, CT(alpha3 / 2));
-  proj_store<typename InterStore<Store>::type, CT>(out.f[f], d.VR, oi, S);
+  proj_store<typename InterStore<Store>::type>(out.f[f], d.VR, oi, S);
 }
 
 // Level-1 field holding Vbar_{mu; nu, t} for spatial mu != nu.
@@ -363,7 +377,7 @@ __device__ __forceinline__ void hyp_l2_site(const Geom &g, const Fields4 &U,
     add_staples2<I, CT>(S, fmu, fnu, d.VR, site + d.o0, n.pnu + om, n.pmu + on1,
                         n.mnu + d.o0, n.mnu + om, n.mnu_pmu + on1, c);
   }
-  proj_store<I, CT>(out.f[f], d.VR, site + (temporal ? d.q0 : d.o0), S);
+  proj_store<I>(out.f[f], d.VR, site + (temporal ? d.q0 : d.o0), S);
 }
 
 // Level 3: the new temporal link (smearing.h:484-503). Reads the level-2
@@ -386,7 +400,7 @@ __device__ __forceinline__ void hyp_l3_site(const Geom &g, const void *Ut,
         S, l2.f[nu], l2.f[3 + nu], d.VR, site + d.o0, n.pnu + d.q0, n.pmu + d.o1,
         n.mnu + d.o0, n.mnu + d.q0, n.mnu_pmu + d.o1, c);
   }
-  proj_store<Store, CT>(out_t, V, site, S);
+  proj_store<Store>(out_t, V, site, S);
 }
 
 // One APE step of SU(2) at a site, all three spatial links: the staples of
@@ -435,7 +449,7 @@ __device__ __forceinline__ void ape_site_su2(const Geom &g, const Fields4 &in,
                          Store::template load<CT>(in.f[mu], V, mnu));
       S = add(S, mul(scale(b, c), Store::template load<CT>(in.f[nu], V, mnu_pmu)));
     }
-    proj_store<Store, CT, true>(out.f[mu], V, site, S);
+    proj_store<Store>(out.f[mu], V, site, S);
   }
 }
 
@@ -661,8 +675,8 @@ __global__ void __launch_bounds__(128, 4)
   S1 = add(S1, scale(mul(l1, Store::template load<CT>(f2, V, mb_pa)), c));
   const M l2 = mul_da(Store::template load<CT>(f1, V, ma), Store::template load<CT>(f2, V, ma));
   S2 = add(S2, scale(mul(l2, Store::template load<CT>(f1, V, ma_pb)), c));
-  proj_store<Store, CT>(o1, V, site, S1);
-  proj_store<Store, CT>(o2, V, site, S2);
+  proj_store<Store>(o1, V, site, S1);
+  proj_store<Store>(o2, V, site, S2);
 }
 
 } // namespace

@@ -351,6 +351,27 @@ template <class T> GC_HD SU3<T> ns_finish(const SU3<T> &A, const cx<T> H[3][3]) 
   return B;
 }
 
+// One polar step without the determinant, 3/2 A - 1/2 A A^dag A: a matrix
+// with unitarity defect d becomes unitary to O(d^2), its phase unchanged.
+template <class T> GC_HD SU3<T> polar_step(const SU3<T> &A) {
+  cx<T> H[3][3];
+  ns_gram(A, H);
+  SU3<T> B;
+#pragma unroll
+  for (int i = 0; i < 3; i++)
+#pragma unroll
+    for (int j = 0; j < 3; j++) {
+      // A + (1/2 - A A^dag / 2) A: the small part is added last
+      const T h = H[i][i].re + T(0.5);
+      cx<T> s = {h * A.e[i][j].re, h * A.e[i][j].im};
+#pragma unroll
+      for (int k = 0; k < 3; k++)
+        if (i != k)
+          s = cmadd(s, H[i][k], A.e[k][j]);
+      B.e[i][j] = cadd(A.e[i][j], s);
+    }
+  return B;
+}
 template <class T> GC_HD SU3<T> ns_step(const SU3<T> &A) {
   cx<T> H[3][3];
   ns_gram(A, H);

@@ -704,10 +704,19 @@ int gc_hyp(gc_lattice *h, double a1, double a2, double a3, int steps) {
 // Prepares the temporal-gauge form of W: the gauge time lines of both cuts
 // and the transformed spatial links, in the HYP decorated-link scratch (which
 // holds them: per site at most 2 x 144 + 6 x 144 bytes against 15 x 144 for
-// FP64 SU(3)), and the device's unitarity check of the temporal links into
-// h->flag_dev. *use is cleared when the scratch cannot hold them.
-static int gauge_prepare(gc_lattice *h, Fields4 *UA, Fields4 *UB, bool *use) {
+// FP64 SU(3)), and the device's unitarity check of the links into *flag, a
+// word of h->flag_dev. *use is cleared when the scratch cannot hold them, or,
+// with `optional`, when it cannot be allocated (the caller has a form that
+// does without it).
+enum { kFlagOnaxis = 0, kFlagOther = 1 }; // words of h->flag_dev
+static int gauge_prepare(gc_lattice *h, Fields4 *UA, Fields4 *UB, bool *use, int **flag,
+                         int word = kFlagOnaxis, bool optional = false) {
   int rc = ensure_hyp(h);
+  if (rc == GC_ERR_NOMEM && optional) {
+    cudaGetLastError(); // (the failed allocation is not the next launch's error)
+    *use = false;
+    return GC_OK;
+  }
   if (rc)
     return rc;
   if (!h->flag_dev) {
@@ -722,6 +731,7 @@ static int gauge_prepare(gc_lattice *h, Fields4 *UA, Fields4 *UB, bool *use) {
     *use = false;
     return GC_OK;
   }
+  *flag = h->flag_dev + word;
   char *base = (char *)h->hyp;
   void *GA = base, *GB = base + lb;
   for (int d = 0; d < 3; d++) {
@@ -729,7 +739,7 @@ static int gauge_prepare(gc_lattice *h, Fields4 *UA, Fields4 *UB, bool *use) {
     UB->f[d] = base + 2 * lb + (3 + d) * h->field_bytes;
   }
   UA->f[3] = UB->f[3] = nullptr;
-  rc = GC_DISPATCH(h, launch_wilson_gauge_prep, h->g, h->cur, GA, GB, *UA, *UB, h->flag_dev,
+  rc = GC_DISPATCH(h, launch_wilson_gauge_prep, h->g, h->cur, GA, GB, *UA, *UB, *flag,
                    h->stream);
   if (rc)
     return launch_fail(h, rc);
@@ -806,8 +816,9 @@ static int wilson_impl(gc_lattice *h, int rmin, int rmax, int tmin, int tmax,
   bool gauge = h->wilson_method == GC_WILSON_AUTO && !second &&
                wilson_gauge_applies(h->g, tmax, nt, h->nc, ct_bytes, tstarts);
   Fields4 UA{}, UB{};
+  int *flag = nullptr;
   if (gauge) {
-    rc = gauge_prepare(h, &UA, &UB, &gauge);
+    rc = gauge_prepare(h, &UA, &UB, &gauge, &flag);
     if (rc)
       return rc;
   }
@@ -823,7 +834,7 @@ static int wilson_impl(gc_lattice *h, int rmin, int rmax, int tmin, int tmax,
     const int ncr = r1 - r0 + 1;
     if (gauge)
       rc = GC_DISPATCH(h, launch_wilson_auto, h->g, h->cur, UA, UB, r0, r1, tmin, tmax,
-                       adjoint, h->flag_dev, h->partials, chunk_out, h->stream, 0, tstarts);
+                       adjoint, flag, h->partials, chunk_out, h->stream, 0, tstarts);
     else
       rc = GC_DISPATCH(h, launch_wilson, h->g, h->cur, r0, r1, tmin, tmax,
                        h->partials, chunk_out, h->stream, adjoint, u2, tstarts);
@@ -976,8 +987,8 @@ int gc_plaquette_time(gc_lattice *h, double *out) {
   return GC_OK;
 }
 
-// Off-axis loops: one space-line field and one loop launch per line of the
-// plan, all loop averages copied back once, then averaged per (direction,
+// Off-axis loops of every line of the plan, all loop averages copied back
+// once, then averaged per (direction,
 // multiplier, T) in the plan's order (a left-to-right sum from 0, as
 // std::accumulate).
 static int offaxis_impl(gc_lattice *h, const std::vector<std::array<int, 3>> &dirs,
@@ -1002,10 +1013,40 @@ static int offaxis_impl(gc_lattice *h, const std::vector<std::array<int, 3>> &di
   if (plan.lines.empty())
     return GC_OK;
   std::lock_guard<std::mutex> lk(h->mu);
-  // the lines as a device table (steps and end displacement as residues)
-  std::vector<OffaxisLineDesc> table(plan.lines.size());
-  for (size_t i = 0; i < table.size(); i++) {
-    const OffaxisLine &line = plan.lines[i];
+  const int ct_bytes = h->prec == GC_PREC_FP64 ? 8 : 4;
+  // Lines with equal steps are computed once. In the temporal gauge (T <=
+  // Lt/2, links unitary by the device's check) the distinct lines are walked
+  // as a tree; the exact product, gated on the device's flag, runs otherwise.
+  int gauge_blocks = h->wilson_method == GC_WILSON_AUTO
+                         ? offaxis_gauge_blocks(h->g, h->nc, ct_bytes, tmin, tmax, adjoint)
+                         : 0;
+  const int exact_blocks = offaxis_fused_blocks(h->g, h->nc, ct_bytes);
+  // Partials, [block][line][T], stay within 32 MB per launch.
+  const size_t per_line = (size_t)std::max(exact_blocks, gauge_blocks) * nt;
+  const size_t most = std::max<size_t>(1, ((size_t)4 << 20) / per_line);
+  // lines per block of the tree walk: up to 48 (a block recomputes the steps
+  // it shares with its neighbours' lines: 5% of the nodes at r <= 6), fewer
+  // where the columns alone give the SMs less than a dozen blocks each
+  const size_t fill = std::max<size_t>(1, 12 * 148 / (size_t)std::max(1, gauge_blocks));
+  const OffaxisTree tree = offaxis_tree(
+      h->g, plan,
+      (int)std::min(most, std::max<size_t>(8, std::min<size_t>(48, plan.lines.size() / fill))));
+  const size_t nlines = tree.first.size();
+  if (tree.nodes.empty())
+    gauge_blocks = 0;
+  bool gauge = gauge_blocks > 0;
+  Fields4 UA{}, UB{};
+  int *flag = nullptr;
+  if (gauge) {
+    rc = gauge_prepare(h, &UA, &UB, &gauge, &flag, kFlagOther, true);
+    if (rc)
+      return rc;
+  }
+  // the lines as a device table (steps and end displacement as residues), and
+  // the tree
+  std::vector<OffaxisLineDesc> table(nlines);
+  for (size_t i = 0; i < nlines; i++) {
+    const OffaxisLine &line = plan.lines[tree.first[i]];
     OffaxisLineDesc &d = table[i];
     std::memset(&d, 0, sizeof d);
     d.n = (int)line.pattern.size();
@@ -1014,39 +1055,58 @@ static int offaxis_impl(gc_lattice *h, const std::vector<std::array<int, 3>> &di
     for (int q = 0; q < d.n; q++)
       d.s[q] = (signed char)line.pattern[q];
   }
-  rc = ensure_aux(h, table.size() * sizeof(OffaxisLineDesc));
+  const size_t node_bytes = gauge ? tree.nodes.size() * sizeof(OffaxisNode) : 0;
+  const size_t chunk_bytes = gauge ? tree.chunk_nodes.size() * sizeof(int) : 0;
+  const size_t table_off = (node_bytes + chunk_bytes + 15) / 16 * 16;
+  std::vector<unsigned char> host(table_off + nlines * sizeof(OffaxisLineDesc));
+  if (gauge) {
+    std::memcpy(host.data(), tree.nodes.data(), node_bytes);
+    std::memcpy(host.data() + node_bytes, tree.chunk_nodes.data(), chunk_bytes);
+  }
+  std::memcpy(host.data() + table_off, table.data(), nlines * sizeof(OffaxisLineDesc));
+  rc = ensure_aux(h, host.size());
   if (rc)
     return rc;
-  // (from pageable memory: returns once the table is staged, so `table` may go)
-  cudaError_t ce = cudaMemcpyAsync(h->aux, table.data(), table.size() * sizeof(OffaxisLineDesc),
-                                   cudaMemcpyHostToDevice, h->stream);
+  // (from pageable memory: returns once the table is staged, so `host` may go)
+  cudaError_t ce = cudaMemcpyAsync(h->aux, host.data(), host.size(), cudaMemcpyHostToDevice,
+                                   h->stream);
   if (ce != cudaSuccess)
     return cuda_fail(h, "cudaMemcpyAsync(off-axis lines)", ce);
-  // Lines go in chunks whose partials, [block][line][T], stay within 32 MB,
-  // one fused launch and one reduction per chunk.
-  const int blocks = offaxis_fused_blocks(h->g, h->nc, h->prec == GC_PREC_FP64 ? 8 : 4);
-  const size_t per_line = (size_t)blocks * nt;
-  const size_t chunk =
-      std::max<size_t>(1, std::min(plan.lines.size(), ((size_t)4 << 20) / per_line));
-  rc = ensure_partials(h, per_line * chunk);
+  rc = ensure_partials(h, per_line * std::min(most, nlines));
   if (rc)
     return rc;
-  rc = ensure_dev_out(h, plan.lines.size() * (size_t)nt);
+  rc = ensure_dev_out(h, nlines * (size_t)nt);
   if (rc)
     return rc;
-  const OffaxisLineDesc *dev_lines = static_cast<const OffaxisLineDesc *>(h->aux);
-  for (size_t c0 = 0; c0 < plan.lines.size(); c0 += chunk) {
-    const int n = (int)std::min(chunk, plan.lines.size() - c0);
+  const unsigned char *aux = static_cast<const unsigned char *>(h->aux);
+  const OffaxisNode *dev_nodes = reinterpret_cast<const OffaxisNode *>(aux);
+  const int *dev_chunks = reinterpret_cast<const int *>(aux + node_bytes);
+  const OffaxisLineDesc *dev_lines = reinterpret_cast<const OffaxisLineDesc *>(aux + table_off);
+  const double scale = line_loop_scale(h->g, h->nc, adjoint);
+  // one launch of each form and one reduction per run of whole chunks
+  const int nchunks = (int)tree.chunk_lines.size() - 1;
+  for (int k0 = 0; k0 < nchunks;) {
+    const int c0 = tree.chunk_lines[k0];
+    int k1 = k0 + 1;
+    while (k1 < nchunks && (size_t)(tree.chunk_lines[k1 + 1] - c0) <= most)
+      k1++;
+    const int n = tree.chunk_lines[k1] - c0;
     int b = 0;
     rc = GC_DISPATCH(h, launch_offaxis_fused, h->g, h->cur, dev_lines + c0, n, tmin, tmax,
-                     adjoint, h->partials, &b, h->stream);
+                     adjoint, h->partials, &b, h->stream, flag);
+    if (!rc && gauge)
+      rc = GC_DISPATCH(h, launch_offaxis_gauge, h->g, UA, UB, dev_nodes, dev_chunks, k0, k1 - k0,
+                       c0, n, tmin, tmax, adjoint, h->partials, flag, h->stream);
     if (!rc)
-      rc = launch_reduce_rows(h->partials, b, n * nt, line_loop_scale(h->g, h->nc, adjoint),
-                              h->dev_out + c0 * nt, h->stream);
+      rc = gauge ? launch_reduce_select(h->partials, b, gauge_blocks, flag, 1, n * nt, scale,
+                                        h->dev_out + (size_t)c0 * nt, h->stream)
+                 : launch_reduce_rows(h->partials, b, n * nt, scale,
+                                      h->dev_out + (size_t)c0 * nt, h->stream);
     if (rc)
       return launch_fail(h, rc);
+    k0 = k1;
   }
-  std::vector<double> vals(plan.lines.size() * (size_t)nt);
+  std::vector<double> vals(nlines * (size_t)nt);
   cudaError_t e = cudaMemcpyAsync(vals.data(), h->dev_out, vals.size() * sizeof(double),
                                   cudaMemcpyDeviceToHost, h->stream);
   if (e == cudaSuccess)
@@ -1057,7 +1117,7 @@ static int offaxis_impl(gc_lattice *h, const std::vector<std::array<int, 3>> &di
     for (int T = tmin; T <= tmax; T++) {
       double sum = 0.0;
       for (int li : grp.lines)
-        sum += vals[(size_t)li * nt + (T - tmin)];
+        sum += vals[(size_t)tree.distinct[li] * nt + (T - tmin)];
       gc_wilson_result r;
       r.statistics_size = (int)grp.lines.size();
       r.wilson_loop = sum / r.statistics_size;

@@ -199,6 +199,11 @@ int launch_wilson_auto(const Geom &g, const Fields4 &U, const Fields4 &UA, const
                        int rmin, int rmax, int tmin, int tmax, bool adjoint, const int *flag,
                        double *partials, double *out_dev, cudaStream_t s, int units = 0,
                        int tstarts = 0);
+// out_dev[it * nr + ir] = scale * (fixed-order sum of the partials
+// [block][ir * nt + it]) over the blocks of the method that ran (*flag).
+int launch_reduce_select(const double *partials, int blocks_exact, int blocks_gauge,
+                         const int *flag, int nr, int nt, double scale, double *out_dev,
+                         cudaStream_t s);
 size_t wilson_auto_partials_count(const Geom &g, int nr, int nt, int nc, int units = 0);
 template <class Store, class CT>
 int time_wilson_gauge(const Geom &g, const Fields4 &UA, const Fields4 &UB, int rmin, int rmax,
@@ -282,12 +287,48 @@ double line_loop_scale(const Geom &g, int nc, bool adjoint);
 // links sit in shared memory and the T walk reads only those. Per-block
 // partial sums at partials[(block * nlines + line) * nt + (T - tmin)];
 // returns the number of blocks (rows of partials) in *blocks.
+// gate: the temporal-gauge form's flag; nothing is computed when *gate == 0.
 template <class Store, class CT>
 int launch_offaxis_fused(const Geom &g, const Fields4 &U, const OffaxisLineDesc *lines,
                          int nlines, int tmin, int tmax, bool adjoint, double *partials,
-                         int *blocks, cudaStream_t s);
+                         int *blocks, cudaStream_t s, const int *gate = nullptr);
 // Column blocks of the fused launch (rows of its partials) for a lattice.
 int offaxis_fused_blocks(const Geom &g, int nc, int ct_bytes);
+
+// The same loops in the temporal gauge (gc_offaxis_gauge.cu). The lines with
+// equal step patterns are one line, and lines that begin alike share the
+// product of the common steps: the patterns form a tree, one node per step.
+struct OffaxisNode {
+  int d[3];          // site of the node's link, as a residue displacement from the start
+  int line;          // distinct line that ends here, or -1
+  signed char axis;  // the link's axis
+  signed char back;  // 1: a step back (the link's adjoint)
+  signed char from;  // product extended: -1 the previous node's, >= 0 that stack level's,
+                     // -2 none (first step)
+  signed char push;  // stack level that keeps this node's product, or -1
+  int pad[3];
+};
+struct OffaxisTree {
+  std::vector<int> distinct;       // plan line -> distinct line
+  std::vector<int> first;          // distinct line -> a plan line
+  std::vector<OffaxisNode> nodes;  // chunk after chunk
+  std::vector<int> chunk_nodes;    // first node of each chunk, and the end
+  std::vector<int> chunk_lines;    // first distinct line of each chunk, and the end
+};
+// Distinct lines are numbered in tree order; each chunk of at most
+// lines_per_chunk of them walks its own part of the tree. Empty nodes: a line
+// needs more stack levels than the kernel keeps.
+OffaxisTree offaxis_tree(const Geom &g, const OffaxisPlan &plan, int lines_per_chunk);
+// Blocks of columns (rows of partials) of the gauge launch, 0 when its block
+// does not fit (long time extents).
+int offaxis_gauge_blocks(const Geom &g, int nc, int ct_bytes, int tmin, int tmax, bool adjoint);
+// Distinct lines [line0, line0 + nlines) of whole chunks; partials
+// [block][line - line0][T - tmin]. Runs when *flag == 0.
+template <class Store, class CT>
+int launch_offaxis_gauge(const Geom &g, const Fields4 &UA, const Fields4 &UB,
+                         const OffaxisNode *nodes, const int *chunk_nodes,
+                         int chunk0, int nchunks, int line0, int nlines, int tmin, int tmax,
+                         bool adjoint, double *partials, const int *flag, cudaStream_t s);
 
 // Loops of a line field S (decorated-link storage) whose end is displaced
 // by disp (disp[ax] = 0) with "time" axis ax and time links Ut:

@@ -29,6 +29,7 @@
 #include "gc_kernels.h"
 
 #include <algorithm>
+#include <climits>
 #include <cmath>
 
 namespace gc {
@@ -272,7 +273,8 @@ template <class Store, class CT, bool ADJ>
 __device__ __forceinline__ void offaxis_fused_body(const Geom &g, const Fields4 &U,
                                                    const OffaxisLineDesc *__restrict__ lines,
                                                    int nlines, int tmin, int tmax, int cols,
-                                                   int rows, double *partials) {
+                                                   int rows, double *partials, int colblock,
+                                                   int linegroup) {
   using M = typename Store::template M<CT>;
   constexpr int NREAL = Store::NC == 3 ? 18 : 4;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -286,7 +288,7 @@ __device__ __forceinline__ void offaxis_fused_body(const Geom &g, const Fields4 
   CT *scol = ncol + NREAL * nslots;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int c = tid % cols, row = tid / cols;
-  const int s = blockIdx.x * cols + c;
+  const int s = colblock * cols + c;
   const bool active = row < rows && s < g.Vs;
   const int kt = Lt / rows;
   const size_t V = g.V;
@@ -298,7 +300,7 @@ __device__ __forceinline__ void offaxis_fused_body(const Geom &g, const Fields4 
       sm_store(ucol, nslots, t * cols + c, Store::template load<CT>(U.f[3], V, s + t * g.Vs));
     }
   }
-  const int l0 = blockIdx.y * kOffaxisLinesPerBlock;
+  const int l0 = linegroup * kOffaxisLinesPerBlock;
   const int l1 = min(nlines, l0 + kOffaxisLinesPerBlock);
 #pragma unroll 1
   for (int l = l0; l < l1; l++) {
@@ -364,7 +366,7 @@ __device__ __forceinline__ void offaxis_fused_body(const Geom &g, const Fields4 
       double sum = 0.0;
       for (int w = 0; w < nwarps; w++)
         sum += wacc[w * nt + e];
-      partials[((size_t)blockIdx.x * nlines + l) * nt + e] = sum;
+      partials[((size_t)colblock * nlines + l) * nt + e] = sum;
     }
     __syncthreads();
   }
@@ -379,15 +381,25 @@ template <class Store, class CT, bool ADJ>
 __global__ void __launch_bounds__(256, 3)
     offaxis_fused_kernel_f32(const __grid_constant__ Geom g, const __grid_constant__ Fields4 U,
                              const OffaxisLineDesc *__restrict__ lines, int nlines, int tmin,
-                             int tmax, int cols, int rows, double *partials) {
-  offaxis_fused_body<Store, CT, ADJ>(g, U, lines, nlines, tmin, tmax, cols, rows, partials);
+                             int tmax, int cols, int rows, double *partials, int colblocks,
+                             int items, const int *gate) {
+  if (gate && *gate == 0)
+    return;
+  for (int i = blockIdx.x; i < items; i += gridDim.x)
+    offaxis_fused_body<Store, CT, ADJ>(g, U, lines, nlines, tmin, tmax, cols, rows, partials,
+                                       i % colblocks, i / colblocks);
 }
 template <class Store, class CT, bool ADJ>
 __global__ void __launch_bounds__(256)
     offaxis_fused_kernel(const __grid_constant__ Geom g, const __grid_constant__ Fields4 U,
                          const OffaxisLineDesc *__restrict__ lines, int nlines, int tmin,
-                         int tmax, int cols, int rows, double *partials) {
-  offaxis_fused_body<Store, CT, ADJ>(g, U, lines, nlines, tmin, tmax, cols, rows, partials);
+                         int tmax, int cols, int rows, double *partials, int colblocks,
+                             int items, const int *gate) {
+  if (gate && *gate == 0)
+    return;
+  for (int i = blockIdx.x; i < items; i += gridDim.x)
+    offaxis_fused_body<Store, CT, ADJ>(g, U, lines, nlines, tmin, tmax, cols, rows, partials,
+                                       i % colblocks, i / colblocks);
 }
 
 } // namespace
@@ -404,7 +416,7 @@ int offaxis_fused_blocks(const Geom &g, int nc, int ct_bytes) {
 template <class Store, class CT>
 int launch_offaxis_fused(const Geom &g, const Fields4 &U, const OffaxisLineDesc *lines,
                          int nlines, int tmin, int tmax, bool adjoint, double *partials,
-                         int *blocks, cudaStream_t s) {
+                         int *blocks, cudaStream_t s, const int *gate) {
   const int nt = tmax - tmin + 1;
   if (nt < 1 || nt > kWilsonMaxEntries || nlines < 1)
     return plan_error("offaxis_fused_kernel: time range or line count");
@@ -412,12 +424,18 @@ int launch_offaxis_fused(const Geom &g, const Fields4 &U, const OffaxisLineDesc 
   if (f.smem > 227 * 1024)
     return plan_error("offaxis_fused_kernel: time extent too large for shared memory");
   const int colblocks = (g.Vs + f.cols - 1) / f.cols;
-  const dim3 grid(colblocks, (nlines + kOffaxisLinesPerBlock - 1) / kOffaxisLinesPerBlock);
+  const long long items =
+      (long long)colblocks * ((nlines + kOffaxisLinesPerBlock - 1) / kOffaxisLinesPerBlock);
+  if (items > INT_MAX)
+    return plan_error("offaxis_fused_kernel: too many blocks");
+  // (as the gated fallback of the temporal-gauge form a block takes several
+  // work items, so that launching blocks that return at once stays cheap)
+  const int grid = gate ? (int)std::min<long long>(items, 4096) : (int)items;
   auto launch = [&](auto kernel) {
     int rc = allow_large_smem(kernel, f.smem);
     if (!rc)
       kernel<<<grid, f.threads, f.smem, s>>>(g, U, lines, nlines, tmin, tmax, f.cols, f.rows,
-                                             partials);
+                                             partials, colblocks, (int)items, gate);
     return rc;
   };
   int rc;
@@ -490,7 +508,8 @@ int launch_line_extend(const Geom &g, const void *F, void *S, int ax, int offset
                                              int, bool, cudaStream_t);                     \
   template int launch_offaxis_fused<STORE, CT>(const Geom &, const Fields4 &,              \
                                                const OffaxisLineDesc *, int, int, int,     \
-                                               bool, double *, int *, cudaStream_t);
+                                               bool, double *, int *, cudaStream_t,        \
+                                               const int *);
 
 GC_INSTANTIATE_O(StoreF64SU3, double)
 GC_INSTANTIATE_O(StoreF64SU2, double)

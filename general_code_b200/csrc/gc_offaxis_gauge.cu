@@ -1,0 +1,452 @@
+// Off-axis Wilson loops in the temporal gauge (sm_100a): the loops of
+// gc_offaxis.cu (reference wilson_offaxis / wilson_offaxis_adjoint,
+// lib/cpu/include/wilson_loops.h:313-663) from the transformed links of
+// gc_wilson_gauge.cu.
+//
+// In the gauge of a cut slice a time line that does not pass the cut is 1, so
+// a loop of the space line S' (the product of the transformed links along its
+// steps) is Re Tr[S'(x + T t) S'(x)^dag]: one trace instead of the two
+// products of the exact walk. Cut A (slice 0) serves the loops with
+// t0 + T < Lt, whatever their start slice; the loops that pass slice Lt - 1
+// start on the last tmax slices and end on the first tmax - 1, so cut B (slice
+// Lt/2, T <= Lt/2) needs its lines on those 2 tmax slices only.
+//
+// The lines themselves cost more than their loops then (5 links and 6 loops
+// per line at r, T <= 6). Many are equal step for step (the reference counts
+// an orientation twice, and permutations repeat symmetric patterns), and many
+// begin alike: as a tree with a node per step the 678 lines of r <= 6 (4473
+// links) are 550 distinct lines and 1140 products. A block walks a part of
+// the tree in depth-first order for its columns: a thread owns one line slot
+// (column, slice, cut), keeps the current product in registers and the
+// products that a later branch continues on a short private stack (the
+// largest branch is walked last, so the stack holds at most log2 of the nodes).
+// The link of the next node is loaded while the current one is multiplied
+// and its loops are summed.
+//
+// A finished line goes to shared memory (two buffers, one barrier per line),
+// each thread adds the traces of the loops that start on its slot, and the
+// per-thread values of one line are summed over the block in fixed order
+// behind the next line's barrier; the grid sums the blocks as elsewhere.
+//
+// Bound: instruction issue at 20 warps per SM (57% of the issue slots; 28% of
+// the FMA pipe; 3.3 TB/s from L2 at 16^4). r, T <= 6 at SU(3) 24^4, mixed
+// 31.9 -> 12.3 ms, FP64 55.8 -> 21.4 ms; SU(2) mixed 10.8 -> 4.8 ms against
+// the exact walk of every line (gc_offaxis.cu), which stays for T > Lt/2 and
+// for links off the group.
+#include "gc_internal.cuh"
+#include "gc_kernels.h"
+#include "gc_rows01.cuh"
+#include "gc_wcol.cuh"
+
+#include <algorithm>
+#include <map>
+#include <type_traits>
+
+namespace gc {
+
+namespace {
+
+constexpr int kTreeStack = 12;
+
+// A line slot's matrix in shared memory: planes of 16-byte vectors (and one
+// of 8 bytes for the 18 reals of an FP32 SU(3) matrix) over the block's slots.
+template <class M> struct SlotSet;
+template <> struct SlotSet<SU3<double>> {
+  static constexpr int kBytes = 144;
+  __device__ __forceinline__ static void store(unsigned char *p, int n, int i,
+                                               const SU3<double> &m) {
+    double2 *q = reinterpret_cast<double2 *>(p) + i;
+#pragma unroll
+    for (int k = 0; k < 9; k++)
+      q[k * n] = make_double2(m.e[k / 3][k % 3].re, m.e[k / 3][k % 3].im);
+  }
+  __device__ __forceinline__ static SU3<double> load(const unsigned char *p, int n, int i) {
+    const double2 *q = reinterpret_cast<const double2 *>(p) + i;
+    SU3<double> m;
+#pragma unroll
+    for (int k = 0; k < 9; k++) {
+      const double2 v = q[k * n];
+      m.e[k / 3][k % 3] = {v.x, v.y};
+    }
+    return m;
+  }
+};
+template <> struct SlotSet<SU3<float>> {
+  static constexpr int kBytes = 72;
+  __device__ __forceinline__ static void store(unsigned char *p, int n, int i,
+                                               const SU3<float> &m) {
+    float4 *q = reinterpret_cast<float4 *>(p) + i;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      const cx<float> a = m.e[2 * k / 3][2 * k % 3], b = m.e[(2 * k + 1) / 3][(2 * k + 1) % 3];
+      q[k * n] = make_float4(a.re, a.im, b.re, b.im);
+    }
+    reinterpret_cast<float2 *>(p + 64 * (size_t)n)[i] = make_float2(m.e[2][2].re, m.e[2][2].im);
+  }
+  __device__ __forceinline__ static SU3<float> load(const unsigned char *p, int n, int i) {
+    const float4 *q = reinterpret_cast<const float4 *>(p) + i;
+    SU3<float> m;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      const float4 v = q[k * n];
+      m.e[2 * k / 3][2 * k % 3] = {v.x, v.y};
+      m.e[(2 * k + 1) / 3][(2 * k + 1) % 3] = {v.z, v.w};
+    }
+    const float2 v = reinterpret_cast<const float2 *>(p + 64 * (size_t)n)[i];
+    m.e[2][2] = {v.x, v.y};
+    return m;
+  }
+};
+template <class T> struct SlotSet<SU2<T>> {
+  static constexpr int kBytes = 4 * sizeof(T);
+  using V = typename V2<T>::type;
+  __device__ __forceinline__ static void store(unsigned char *p, int n, int i, const SU2<T> &m) {
+    V *q = reinterpret_cast<V *>(p) + i;
+    q[0] = V{m.a0, m.a1};
+    q[n] = V{m.a2, m.a3};
+  }
+  __device__ __forceinline__ static SU2<T> load(const unsigned char *p, int n, int i) {
+    const V *q = reinterpret_cast<const V *>(p) + i;
+    const V a = q[0], b = q[n];
+    return {a.x, a.y, b.x, b.y};
+  }
+};
+
+// P <- P u or P u^dag, and the first factor. FP32 SU(3) products keep rows 0
+// and 1 (gc_rows01.cuh); finish() rebuilds row 2 for the traces.
+template <class M> struct LineOps {
+  __device__ __forceinline__ static M first(const M &u, bool back) { return back ? adjoint(u) : u; }
+  __device__ __forceinline__ static M extend(const M &P, const M &u, bool back) {
+    return back ? mul_ad(P, u) : mul(P, u);
+  }
+  __device__ __forceinline__ static void finish(M &) {}
+};
+template <> struct LineOps<SU3<float>> {
+  using M = SU3<float>;
+  __device__ __forceinline__ static M first(const M &u, bool back) { return back ? adjoint(u) : u; }
+  __device__ __forceinline__ static M extend(const M &P, const M &u, bool back) {
+    return back ? mul_ad01(P, u) : mul01(P, u);
+  }
+  __device__ __forceinline__ static void finish(M &P) { rebuild_row2(P); }
+};
+
+// Slots of a column and their slices: slot i < Lt is cut A on slice i, slot
+// Lt + j cut B on slice (Lt - tmax + j) mod Lt, j < 2 tmax. The loops of a
+// start slot i end on slot i + T.
+__host__ __device__ inline int gauge_slots(int Lt, int tmax) { return Lt + 2 * tmax; }
+
+struct GaugeShape {
+  int cols, threads;
+  size_t smem;
+};
+GaugeShape gauge_shape(const Geom &g, int nc, int ct_bytes, int tmin, int tmax, bool adjoint) {
+  GaugeShape f{};
+  const int n = gauge_slots(g.L[3], tmax), nt = tmax - tmin + 1;
+  const size_t mat = (nc == 3 ? 18 : 4) * (size_t)ct_bytes;
+  const size_t acc = (!adjoint && ct_bytes == 4) ? 4 : 8;
+  auto set = [&](int cols) {
+    f.cols = cols;
+    f.threads = (n * cols + 31) / 32 * 32;
+    f.smem = 2 * (size_t)f.threads * (mat + nt * acc);
+  };
+  // about 160 threads per block (FP32 about 256), a power of two of columns:
+  // their links share the 32-byte sectors
+  const int want = ct_bytes == 4 ? 320 : 160;
+  int cols = 1;
+  while (2 * cols * n <= want && 2 * cols <= 32)
+    cols *= 2;
+  set(cols);
+  if (f.threads > 512 || f.smem > 200 * 1024)
+    f.cols = 0;
+  return f;
+}
+
+template <class Store, class CT, bool ADJ>
+__global__ void __launch_bounds__(512)
+    offaxis_gauge_kernel(const __grid_constant__ Geom g, const __grid_constant__ Fields4 UA,
+                         const __grid_constant__ Fields4 UB,
+                         const OffaxisNode *__restrict__ nodes,
+                         const int *__restrict__ chunk_nodes, int line0, int nlines, int tmin,
+                         int tmax, int cols, double *partials, const int *flag) {
+  if (*flag != 0)
+    return;
+  using M = typename Store::template M<CT>;
+  using SS = SlotSet<M>;
+  using Acc = GAcc<ADJ, CT>;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int Lt = g.L[3], nt = tmax - tmin + 1;
+  const int nth = blockDim.x, tid = threadIdx.x;
+  const int warp = tid >> 5, lane = tid & 31, nwarps = nth >> 5;
+  unsigned char *lines = smem_raw; // [2][SS::kBytes * nth]
+  Acc *red = reinterpret_cast<Acc *>(smem_raw + 2 * (size_t)SS::kBytes * nth); // [2][nt][nth]
+  const int c = tid % cols, slot = tid / cols;
+  const int s = blockIdx.x * cols + c;
+  const bool active = slot < gauge_slots(Lt, tmax) && s < g.Vs;
+  const bool cut_b = slot >= Lt;
+  const int j = slot - Lt;
+  const int t = cut_b ? (Lt - tmax + j) % Lt : slot;
+  // loops that start on this slot: T in [lo, hi]
+  int lo = cut_b ? max(tmin, tmax - j) : tmin;
+  int hi = cut_b ? (j < tmax ? tmax : 0) : min(tmax, Lt - 1 - slot);
+  if (!active)
+    hi = 0, lo = 1;
+  const int x0 = s % g.L[0], x1 = (s / g.L[0]) % g.L[1], x2 = s / (g.L[0] * g.L[1]);
+  const size_t V = g.V;
+  const int toff = t * g.Vs;
+  const void *f0 = cut_b ? UB.f[0] : UA.f[0], *f1 = cut_b ? UB.f[1] : UA.f[1],
+             *f2 = cut_b ? UB.f[2] : UA.f[2];
+  for (int i = tid; i < 2 * nt * nth; i += nth)
+    red[i] = Acc(0);
+
+  // the link of a node, seen from this slot
+  auto link = [&](const int4 &d) {
+    int y0 = x0 + d.x, y1 = x1 + d.y, y2 = x2 + d.z;
+    y0 -= y0 >= g.L[0] ? g.L[0] : 0;
+    y1 -= y1 >= g.L[1] ? g.L[1] : 0;
+    y2 -= y2 >= g.L[2] ? g.L[2] : 0;
+    return y0 + g.L[0] * (y1 + g.L[1] * y2) + toff;
+  };
+  auto field = [&](int axis) { return axis == 0 ? f0 : axis == 1 ? f1 : f2; };
+
+  const int n0 = chunk_nodes[blockIdx.y], n1 = chunk_nodes[blockIdx.y + 1];
+  const int4 *desc = reinterpret_cast<const int4 *>(nodes);
+  M P, stack[kTreeStack];
+  int done = 0, prev = -1; // lines finished by this block, the last one
+  int4 d = __ldg(desc + 2 * n0);
+  int ops = __ldg(reinterpret_cast<const int *>(desc + 2 * n0 + 1));
+  M u;
+  if (active)
+    u = Store::template load<CT>(field(ops & 0xff), V, link(d));
+#pragma unroll 1
+  for (int n = n0; n < n1; n++) {
+    const int line = d.w;
+    const bool back = (ops >> 8) & 1;
+    const int from = (signed char)(ops >> 16), push = ops >> 24;
+    if (active) {
+      if (from == -2) {
+        P = LineOps<M>::first(u, back);
+      } else {
+        if (from >= 0)
+          P = stack[from];
+        P = LineOps<M>::extend(P, u, back);
+      }
+      if (push >= 0)
+        stack[push] = P;
+    }
+    if (n + 1 < n1) {
+      d = __ldg(desc + 2 * n + 2);
+      ops = __ldg(reinterpret_cast<const int *>(desc + 2 * n + 3));
+      if (active)
+        u = Store::template load<CT>(field(ops & 0xff), V, link(d));
+    }
+    if (line < 0)
+      continue;
+    M a = P;
+    LineOps<M>::finish(a);
+    unsigned char *buf = lines + (done & 1) * (size_t)SS::kBytes * nth;
+    Acc *r = red + (done & 1) * (size_t)nt * nth;
+    if (active)
+      SS::store(buf, nth, tid, a);
+    __syncthreads();
+    // the previous line's sums (its values were written before this barrier)
+    if (prev >= 0) {
+      const Acc *rp = red + ((done & 1) ^ 1) * (size_t)nt * nth;
+#pragma unroll 1
+      for (int T = warp; T < nt; T += nwarps) {
+        double v = 0.0;
+        for (int i = lane; i < nth; i += 32)
+          v += double(rp[(size_t)T * nth + i]);
+        v = warp_sum(v);
+        if (lane == 0)
+          partials[((size_t)blockIdx.x * nlines + prev - line0) * nt + T] = v;
+      }
+    }
+#pragma unroll 2
+    for (int T = lo; T <= hi; T++)
+      r[(size_t)(T - tmin) * nth + tid] =
+          gauge_trace<ADJ>(a, SS::load(buf, nth, tid + T * cols), false);
+    prev = line;
+    done++;
+  }
+  __syncthreads();
+  if (prev >= 0) {
+    const Acc *rp = red + ((done & 1) ^ 1) * (size_t)nt * nth;
+#pragma unroll 1
+    for (int T = warp; T < nt; T += nwarps) {
+      double v = 0.0;
+      for (int i = lane; i < nth; i += 32)
+        v += double(rp[(size_t)T * nth + i]);
+      v = warp_sum(v);
+      if (lane == 0)
+        partials[((size_t)blockIdx.x * nlines + prev - line0) * nt + T] = v;
+    }
+  }
+}
+
+} // namespace
+
+int offaxis_gauge_blocks(const Geom &g, int nc, int ct_bytes, int tmin, int tmax, bool adjoint) {
+  if (g.L[3] < 2 || tmax > g.L[3] / 2)
+    return 0;
+  const GaugeShape f = gauge_shape(g, nc, ct_bytes, tmin, tmax, adjoint);
+  return f.cols ? (g.Vs + f.cols - 1) / f.cols : 0;
+}
+
+template <class Store, class CT>
+int launch_offaxis_gauge(const Geom &g, const Fields4 &UA, const Fields4 &UB,
+                         const OffaxisNode *nodes, const int *chunk_nodes, int chunk0,
+                         int nchunks, int line0, int nlines, int tmin, int tmax, bool adjoint,
+                         double *partials, const int *flag, cudaStream_t s) {
+  const GaugeShape f = gauge_shape(g, Store::NC, (int)sizeof(CT), tmin, tmax, adjoint);
+  if (!f.cols || tmax > g.L[3] / 2)
+    return plan_error("offaxis_gauge_kernel: block shape does not fit");
+  const dim3 grid((g.Vs + f.cols - 1) / f.cols, nchunks);
+  auto go = [&](auto kernel) {
+    const int rc = allow_large_smem(kernel, f.smem);
+    if (!rc)
+      kernel<<<grid, f.threads, f.smem, s>>>(g, UA, UB, nodes, chunk_nodes + chunk0, line0,
+                                             nlines, tmin, tmax, f.cols, partials, flag);
+    return rc;
+  };
+  const int rc = adjoint ? go(offaxis_gauge_kernel<Store, CT, true>)
+                         : go(offaxis_gauge_kernel<Store, CT, false>);
+  return rc ? rc : launch_check("offaxis_gauge_kernel");
+}
+
+#define GC_INSTANTIATE_OG(STORE, CT)                                                         \
+  template int launch_offaxis_gauge<STORE, CT>(                                              \
+      const Geom &, const Fields4 &, const Fields4 &, const OffaxisNode *, const int *, int, \
+      int, int, int, int, int, bool, double *, const int *, cudaStream_t);
+
+GC_INSTANTIATE_OG(StoreF64SU3, double)
+GC_INSTANTIATE_OG(StoreF64SU2, double)
+GC_INSTANTIATE_OG(StoreF32SU3, float)
+GC_INSTANTIATE_OG(StoreF32SU2, float)
+
+// ------------------------------------------------------------------ host tree
+namespace {
+
+struct TreeNode {
+  int step = 0, line = -1, weight = 0; // weight: nodes of the subtree
+  std::vector<int> children;
+};
+
+// Children in walking order: the largest subtree last (its products need no
+// stack level below it), the others by size, equal sizes by step.
+void order_children(std::vector<TreeNode> &t, int n) {
+  t[n].weight = 1;
+  for (int c : t[n].children) {
+    order_children(t, c);
+    t[n].weight += t[c].weight;
+  }
+  std::sort(t[n].children.begin(), t[n].children.end(), [&](int a, int b) {
+    return t[a].weight != t[b].weight ? t[a].weight < t[b].weight : t[a].step < t[b].step;
+  });
+}
+
+int add_line(std::vector<TreeNode> &t, const std::vector<int> &steps) {
+  int n = 0;
+  for (int e : steps) {
+    int next = -1;
+    for (int c : t[n].children)
+      if (t[c].step == e)
+        next = c;
+    if (next < 0) {
+      next = (int)t.size();
+      t[n].children.push_back(next);
+      t.emplace_back();
+      t[next].step = e;
+    }
+    n = next;
+  }
+  return n;
+}
+
+} // namespace
+
+OffaxisTree offaxis_tree(const Geom &g, const OffaxisPlan &plan, int lines_per_chunk) {
+  OffaxisTree out;
+  // all distinct lines, numbered in the order of a walk of their tree
+  std::vector<TreeNode> all(1);
+  std::vector<int> end(plan.lines.size()), first_of;
+  for (size_t i = 0; i < plan.lines.size(); i++) {
+    end[i] = add_line(all, plan.lines[i].pattern);
+    if (all[end[i]].line < 0)
+      all[end[i]].line = (int)i; // (a plan line with this pattern)
+  }
+  order_children(all, 0);
+  std::vector<int> number(all.size(), -1), todo{0};
+  while (!todo.empty()) {
+    const int n = todo.back();
+    todo.pop_back();
+    if (all[n].line >= 0) {
+      number[n] = (int)out.first.size();
+      out.first.push_back(all[n].line);
+    }
+    for (size_t k = all[n].children.size(); k-- > 0;)
+      todo.push_back(all[n].children[k]);
+  }
+  for (size_t i = 0; i < plan.lines.size(); i++)
+    out.distinct.push_back(number[end[i]]);
+  // each chunk of consecutive lines as a walk of its own tree
+  const int total = (int)out.first.size();
+  for (int l0 = 0; l0 < total; l0 += lines_per_chunk) {
+    const int l1 = std::min(total, l0 + lines_per_chunk);
+    std::vector<TreeNode> t(1);
+    for (int l = l0; l < l1; l++)
+      t[add_line(t, plan.lines[out.first[l]].pattern)].line = l;
+    order_children(t, 0);
+    out.chunk_nodes.push_back((int)out.nodes.size());
+    out.chunk_lines.push_back(l0);
+    struct Visit {
+      int node, parent_level; // stack level of the parent's product, -1: in registers
+      int level;              // first free stack level
+      int pos[3];             // displacement of the parent's end
+    };
+    // depth first; a node with several children keeps its product on a level
+    // until the last of them, which continues from the stack as well
+    std::vector<Visit> visits;
+    for (size_t k = t[0].children.size(); k-- > 0;)
+      visits.push_back({t[0].children[k], -2, 0, {0, 0, 0}});
+    while (!visits.empty()) {
+      const Visit v = visits.back();
+      visits.pop_back();
+      const TreeNode &tn = t[v.node];
+      OffaxisNode q{};
+      const int axis = std::abs(tn.step) - 1;
+      int at[3] = {v.pos[0], v.pos[1], v.pos[2]}, to[3] = {v.pos[0], v.pos[1], v.pos[2]};
+      if (tn.step > 0)
+        to[axis] += 1;
+      else
+        at[axis] -= 1, to[axis] -= 1;
+      for (int k = 0; k < 3; k++)
+        q.d[k] = ((at[k] % g.L[k]) + g.L[k]) % g.L[k];
+      q.line = tn.line;
+      q.axis = (signed char)axis;
+      q.back = tn.step < 0;
+      q.from = (signed char)v.parent_level;
+      const size_t nch = tn.children.size();
+      q.push = -1;
+      if (nch > 1) {
+        if (v.level >= kTreeStack) {
+          out.nodes.clear();
+          return out;
+        }
+        q.push = (signed char)v.level;
+      }
+      out.nodes.push_back(q);
+      for (size_t k = nch; k-- > 0;) {
+        // the first child follows at once (registers); the others find the
+        // product on the stack, and the last one frees its level
+        Visit w{tn.children[k], k == 0 ? -1 : (int)q.push, 0, {to[0], to[1], to[2]}};
+        w.level = nch > 1 && k + 1 < nch ? v.level + 1 : v.level;
+        visits.push_back(w);
+      }
+    }
+  }
+  out.chunk_nodes.push_back((int)out.nodes.size());
+  out.chunk_lines.push_back(total);
+  return out;
+}
+
+} // namespace gc

@@ -3,7 +3,7 @@
 // of SU(3) matrices is again in SU(3), so a product whose third row will be
 // rebuilt needs only its first two rows computed (2/3 of the multiply-adds).
 // Used by the mixed APE/HYP staples (gc_smear.cu) and the space lines of the
-// one-column temporal-gauge W kernel (gc_wilson_gauge.cu).
+// temporal-gauge loops (gc_wilson_gauge.cu, gc_offaxis_gauge.cu).
 #pragma once
 
 #include "gc_internal.cuh"
@@ -35,6 +35,28 @@ __device__ __forceinline__ SU3<float> mul01(const SU3<float> &A, const SU3<float
         re = fmaf(-A.e[i][k].im, B.e[k][j].im, re);
         im = fmaf(A.e[i][k].re, B.e[k][j].im, im);
         im = fmaf(A.e[i][k].im, B.e[k][j].re, im);
+      }
+      C.e[i][j] = {re, im};
+    }
+  return C;
+}
+// rows 0 and 1 of A B^dag (A: rows 0, 1; B: all rows)
+__device__ __forceinline__ SU3<float> mul_ad01(const SU3<float> &A, const SU3<float> &B) {
+  SU3<float> C;
+#pragma unroll
+  for (int i = 0; i < 2; i++)
+#pragma unroll
+    for (int j = 0; j < 3; j++) {
+      float re = A.e[i][0].re * B.e[j][0].re;
+      float im = A.e[i][0].im * B.e[j][0].re;
+      re = fmaf(A.e[i][0].im, B.e[j][0].im, re);
+      im = fmaf(-A.e[i][0].re, B.e[j][0].im, im);
+#pragma unroll
+      for (int k = 1; k < 3; k++) {
+        re = fmaf(A.e[i][k].re, B.e[j][k].re, re);
+        re = fmaf(A.e[i][k].im, B.e[j][k].im, re);
+        im = fmaf(A.e[i][k].im, B.e[j][k].re, im);
+        im = fmaf(-A.e[i][k].re, B.e[j][k].im, im);
       }
       C.e[i][j] = {re, im};
     }

@@ -167,28 +167,6 @@ __device__ __forceinline__ SU3<float> load_rows01(const void *f, size_t V, int s
   u.e[1][2] = {c.z, c.w};
   return u;
 }
-// rows 0 and 1 of A B^dag (A: rows 0, 1; B: all rows)
-__device__ __forceinline__ SU3<float> mul_ad01(const SU3<float> &A, const SU3<float> &B) {
-  SU3<float> C;
-#pragma unroll
-  for (int i = 0; i < 2; i++)
-#pragma unroll
-    for (int j = 0; j < 3; j++) {
-      float re = A.e[i][0].re * B.e[j][0].re;
-      float im = A.e[i][0].im * B.e[j][0].re;
-      re = fmaf(A.e[i][0].im, B.e[j][0].im, re);
-      im = fmaf(-A.e[i][0].re, B.e[j][0].im, im);
-#pragma unroll
-      for (int k = 1; k < 3; k++) {
-        re = fmaf(A.e[i][k].re, B.e[j][k].re, re);
-        re = fmaf(A.e[i][k].im, B.e[j][k].im, re);
-        im = fmaf(A.e[i][k].im, B.e[j][k].re, im);
-        im = fmaf(-A.e[i][k].re, B.e[j][k].im, im);
-      }
-      C.e[i][j] = {re, im};
-    }
-  return C;
-}
 // rows 0 and 1 of A^dag B (A, B: all rows)
 __device__ __forceinline__ SU3<float> mul_da01(const SU3<float> &A, const SU3<float> &B) {
   SU3<float> C;

@@ -8,6 +8,8 @@
 #include "gc_kernels.h"
 #include "gc_pair.cuh"
 
+#include <type_traits>
+
 namespace gc {
 
 namespace {
@@ -187,6 +189,87 @@ template <> struct LaneLoad<StoreF32SU3, float, 2> {
   }
 };
 
+// The loop value from Tr[a b^dag] as loop_value (gc_wcol.cuh) computes it,
+// with the sum split into one fused chain per row and the three rows added at
+// the end: three independent chains instead of one of 18 dependent FMAs,
+// which the trace loop below (a few warps per scheduler, shared-memory
+// operands) needs to keep the FMA pipe fed.
+// Per-thread sums of the loop values: FP32 for the fundamental loops of the
+// mixed form (a thread adds at most a few loops; every loop value is an FP32
+// dot product), FP64 otherwise; the block and the grid sum them in FP64.
+template <bool ADJ, class CT>
+using GAcc = typename std::conditional<!ADJ && std::is_same<CT, float>::value, float,
+                                       double>::type;
+
+template <bool ADJ, class T>
+__device__ __forceinline__ GAcc<ADJ, T> gauge_trace(const SU3<T> &a, const SU3<T> &b, bool) {
+  T re[3], im[3];
+#pragma unroll
+  for (int i = 0; i < 3; i++) {
+    re[i] = a.e[i][0].re * b.e[i][0].re;
+    re[i] = GC_FMA(a.e[i][0].im, b.e[i][0].im, re[i]);
+    if (ADJ) {
+      im[i] = a.e[i][0].im * b.e[i][0].re;
+      im[i] = GC_FMA(-a.e[i][0].re, b.e[i][0].im, im[i]);
+    }
+#pragma unroll
+    for (int j = 1; j < 3; j++) {
+      re[i] = GC_FMA(a.e[i][j].re, b.e[i][j].re, re[i]);
+      re[i] = GC_FMA(a.e[i][j].im, b.e[i][j].im, re[i]);
+      if (ADJ) {
+        im[i] = GC_FMA(a.e[i][j].im, b.e[i][j].re, im[i]);
+        im[i] = GC_FMA(-a.e[i][j].re, b.e[i][j].im, im[i]);
+      }
+    }
+  }
+  if (!ADJ)
+    return (re[0] + re[1]) + re[2];
+  const double r = double((re[0] + re[1]) + re[2]);
+  const double m = double((im[0] + im[1]) + im[2]);
+  return fma(r, r, fma(m, m, -1.0));
+}
+template <bool ADJ>
+__device__ __forceinline__ GAcc<ADJ, float> gauge_trace(const SU3<f2> &a, const SU3<f2> &b,
+                                                        bool lane1) {
+  f2 re[3], im[3];
+#pragma unroll
+  for (int i = 0; i < 3; i++) {
+    re[i] = a.e[i][0].re * b.e[i][0].re;
+    re[i] = fma(a.e[i][0].im, b.e[i][0].im, re[i]);
+    if (ADJ) {
+      im[i] = a.e[i][0].im * b.e[i][0].re;
+      im[i] = fma(-a.e[i][0].re, b.e[i][0].im, im[i]);
+    }
+#pragma unroll
+    for (int j = 1; j < 3; j++) {
+      re[i] = fma(a.e[i][j].re, b.e[i][j].re, re[i]);
+      re[i] = fma(a.e[i][j].im, b.e[i][j].im, re[i]);
+      if (ADJ) {
+        im[i] = fma(a.e[i][j].im, b.e[i][j].re, im[i]);
+        im[i] = fma(-a.e[i][j].re, b.e[i][j].im, im[i]);
+      }
+    }
+  }
+  const float2 r = make_float2((re[0].v.x + re[1].v.x) + re[2].v.x,
+                               (re[0].v.y + re[1].v.y) + re[2].v.y);
+  if (!ADJ)
+    return lane1 ? r.x + r.y : r.x;
+  const float2 m = make_float2((im[0].v.x + im[1].v.x) + im[2].v.x,
+                               (im[0].v.y + im[1].v.y) + im[2].v.y);
+  const double r0 = double(r.x), i0 = double(m.x);
+  const double v0 = fma(r0, r0, fma(i0, i0, -1.0));
+  if (!lane1)
+    return v0;
+  const double r1 = double(r.y), i1 = double(m.y);
+  return v0 + fma(r1, r1, fma(i1, i1, -1.0));
+}
+template <bool ADJ, class T>
+__device__ __forceinline__ GAcc<ADJ, T> gauge_trace(const SU2<T> &a, const SU2<T> &b,
+                                                    bool lane1) {
+  if (!ADJ)
+    return dot4(a.a0, b.a0, a.a1, b.a1, a.a2, b.a2, a.a3, b.a3);
+  return loop_value<ADJ>(a, b, lane1);
+}
 
 } // namespace
 

@@ -25,7 +25,8 @@
 // The identity needs unitary temporal links. The lines kernel measures the
 // largest unitarity defect max |U_t U_t^dag - 1| of the lattice's temporal
 // links and raises a flag above the form's tolerance (FP64: 1e-14, a few
-// roundings; mixed: 1e-6, FP32 rounding of the 12-real links is 2.6e-7).
+// roundings; mixed: 1e-6, FP32 rounding of the 12-real links is 2.6e-7); for
+// 12-real links the transform kernel checks the spatial links as well.
 // Both W kernels are launched and read the flag on the device: the exact
 // product (gc_wilson.cu) computes when it is raised, this form when it is
 // not, and the reduction sums the partials of the one that ran; no host
@@ -121,6 +122,12 @@ __device__ __forceinline__ typename Store::template M<double> gauge_time_link(
     return u;
 }
 
+// The stored SU(3) lines are made unitary once more: G^dag stands for G^-1,
+// and over a long time extent the links' and the products' rounding adds up
+// (1e-14 at Lt = 40, in the loops' values as well; W's error against 64 bits
+// at 24^4 FP64 9e-15 -> 9e-16). A quaternion's norm does not drift that way.
+__device__ __forceinline__ SU3<double> stored_line(const SU3<double> &G) { return polar_step(G); }
+__device__ __forceinline__ SU2<double> stored_line(const SU2<double> &G) { return G; }
 template <class Store>
 __global__ void __launch_bounds__(128)
     gauge_lines_kernel(const __grid_constant__ Geom g, const void *Ut, void *GA, void *GB,
@@ -138,7 +145,7 @@ __global__ void __launch_bounds__(128)
     MD G = unit(MD());
 #pragma unroll 1
     for (int t = 0; t < Lt; t++) {
-      GS::template store<double>(GA, V, s + t * g.Vs, G);
+      GS::template store<double>(GA, V, s + t * g.Vs, stored_line(G));
       const MD u = Store::template load<double>(Ut, V, s + t * g.Vs);
       dmax = fmax(dmax, unitarity_defect(u));
       if (t + 1 < Lt)
@@ -153,7 +160,7 @@ __global__ void __launch_bounds__(128)
   int t = h;
 #pragma unroll 1
   for (int k = 0; k < Lt; k++) {
-    GS::template store<double>(GB, V, s + t * g.Vs, G);
+    GS::template store<double>(GB, V, s + t * g.Vs, stored_line(G));
     if (k + 1 < Lt)
       G = mul(G, gauge_time_link<Store>(Store::template load<double>(Ut, V, s + t * g.Vs)));
     t = (t + 1 == Lt) ? 0 : t + 1;
@@ -165,7 +172,7 @@ template <class Store>
 __global__ void __launch_bounds__(128)
     gauge_transform_kernel(const __grid_constant__ Geom g, const __grid_constant__ Fields4 U,
                            const void *GA, const void *GB, const __grid_constant__ Fields4 UA,
-                           const __grid_constant__ Fields4 UB) {
+                           const __grid_constant__ Fields4 UB, double tol, int *flag) {
   using GS = typename F64Store<Store::NC>::type;
   using MD = typename Store::template M<double>;
   const int site = blockIdx.x * blockDim.x + threadIdx.x;
@@ -177,6 +184,10 @@ __global__ void __launch_bounds__(128)
   const int sn = site + step_off(g, sel4(x, nu), nu, +1);
   const size_t V = g.V;
   const MD u = Store::template load<double>(U.f[nu], V, site);
+  // 12-real links: the transformed link's third row is rebuilt from its first
+  // two, which holds for links in SU(3) only
+  if (Store::kBytes == 48 && !(unitarity_defect(u) <= tol))
+    *flag = 1;
   Store::template store<double>(
       UA.f[nu], V, site,
       mul_ad(mul(GS::template load<double>(GA, V, site), u),
@@ -185,88 +196,6 @@ __global__ void __launch_bounds__(128)
       UB.f[nu], V, site,
       mul_ad(mul(GS::template load<double>(GB, V, site), u),
              GS::template load<double>(GB, V, sn)));
-}
-
-// The loop value from Tr[a b^dag] as loop_value (gc_wcol.cuh) computes it,
-// with the sum split into one fused chain per row and the three rows added at
-// the end: three independent chains instead of one of 18 dependent FMAs,
-// which the trace loop below (a few warps per scheduler, shared-memory
-// operands) needs to keep the FMA pipe fed.
-// Per-thread sums of the loop values: FP32 for the fundamental loops of the
-// mixed form (a thread adds at most a few loops; every loop value is an FP32
-// dot product), FP64 otherwise; the block and the grid sum them in FP64.
-template <bool ADJ, class CT>
-using GAcc = typename std::conditional<!ADJ && std::is_same<CT, float>::value, float,
-                                       double>::type;
-
-template <bool ADJ, class T>
-__device__ __forceinline__ GAcc<ADJ, T> gauge_trace(const SU3<T> &a, const SU3<T> &b, bool) {
-  T re[3], im[3];
-#pragma unroll
-  for (int i = 0; i < 3; i++) {
-    re[i] = a.e[i][0].re * b.e[i][0].re;
-    re[i] = GC_FMA(a.e[i][0].im, b.e[i][0].im, re[i]);
-    if (ADJ) {
-      im[i] = a.e[i][0].im * b.e[i][0].re;
-      im[i] = GC_FMA(-a.e[i][0].re, b.e[i][0].im, im[i]);
-    }
-#pragma unroll
-    for (int j = 1; j < 3; j++) {
-      re[i] = GC_FMA(a.e[i][j].re, b.e[i][j].re, re[i]);
-      re[i] = GC_FMA(a.e[i][j].im, b.e[i][j].im, re[i]);
-      if (ADJ) {
-        im[i] = GC_FMA(a.e[i][j].im, b.e[i][j].re, im[i]);
-        im[i] = GC_FMA(-a.e[i][j].re, b.e[i][j].im, im[i]);
-      }
-    }
-  }
-  if (!ADJ)
-    return (re[0] + re[1]) + re[2];
-  const double r = double((re[0] + re[1]) + re[2]);
-  const double m = double((im[0] + im[1]) + im[2]);
-  return fma(r, r, fma(m, m, -1.0));
-}
-template <bool ADJ>
-__device__ __forceinline__ GAcc<ADJ, float> gauge_trace(const SU3<f2> &a, const SU3<f2> &b,
-                                                        bool lane1) {
-  f2 re[3], im[3];
-#pragma unroll
-  for (int i = 0; i < 3; i++) {
-    re[i] = a.e[i][0].re * b.e[i][0].re;
-    re[i] = fma(a.e[i][0].im, b.e[i][0].im, re[i]);
-    if (ADJ) {
-      im[i] = a.e[i][0].im * b.e[i][0].re;
-      im[i] = fma(-a.e[i][0].re, b.e[i][0].im, im[i]);
-    }
-#pragma unroll
-    for (int j = 1; j < 3; j++) {
-      re[i] = fma(a.e[i][j].re, b.e[i][j].re, re[i]);
-      re[i] = fma(a.e[i][j].im, b.e[i][j].im, re[i]);
-      if (ADJ) {
-        im[i] = fma(a.e[i][j].im, b.e[i][j].re, im[i]);
-        im[i] = fma(-a.e[i][j].re, b.e[i][j].im, im[i]);
-      }
-    }
-  }
-  const float2 r = make_float2((re[0].v.x + re[1].v.x) + re[2].v.x,
-                               (re[0].v.y + re[1].v.y) + re[2].v.y);
-  if (!ADJ)
-    return lane1 ? r.x + r.y : r.x;
-  const float2 m = make_float2((im[0].v.x + im[1].v.x) + im[2].v.x,
-                               (im[0].v.y + im[1].v.y) + im[2].v.y);
-  const double r0 = double(r.x), i0 = double(m.x);
-  const double v0 = fma(r0, r0, fma(i0, i0, -1.0));
-  if (!lane1)
-    return v0;
-  const double r1 = double(r.y), i1 = double(m.y);
-  return v0 + fma(r1, r1, fma(i1, i1, -1.0));
-}
-template <bool ADJ, class T>
-__device__ __forceinline__ GAcc<ADJ, T> gauge_trace(const SU2<T> &a, const SU2<T> &b,
-                                                    bool lane1) {
-  if (!ADJ)
-    return dot4(a.a0, b.a0, a.a1, b.a1, a.a2, b.a2, a.a3, b.a3);
-  return loop_value<ADJ>(a, b, lane1);
 }
 
 // First spatial site of a column block. When the block's columns tile the x
@@ -940,8 +869,8 @@ int launch_wilson_gauge_prep(const Geom &g, const Fields4 &U, void *GA, void *GB
   int rc = launch_check("gauge_lines_kernel");
   if (rc)
     return rc;
-  gauge_transform_kernel<Store><<<dim3((g.V + 127) / 128, 3), 128, 0, s>>>(g, U, GA, GB, UA,
-                                                                          UB);
+  gauge_transform_kernel<Store><<<dim3((g.V + 127) / 128, 3), 128, 0, s>>>(
+      g, U, GA, GB, UA, UB, wilson_gauge_tolerance((int)sizeof(CT)), flag);
   return launch_check("gauge_transform_kernel");
 }
 
@@ -1035,6 +964,14 @@ int launch_wilson_gauge(const Geom &g, const Fields4 &UA, const Fields4 &UB, int
                               wilson_scale(g.V, Store::NC, adjoint), out_dev, s);
 }
 
+int launch_reduce_select(const double *partials, int blocks_exact, int blocks_gauge,
+                         const int *flag, int nr, int nt, double scale, double *out_dev,
+                         cudaStream_t s) {
+  reduce_select_kernel<<<nr * nt, 256, 0, s>>>(partials, blocks_exact, blocks_gauge, flag, nr,
+                                               nt, scale, out_dev);
+  return launch_check("reduce_select_kernel");
+}
+
 template <class Store, class CT>
 int launch_wilson_auto(const Geom &g, const Fields4 &U, const Fields4 &UA, const Fields4 &UB,
                        int rmin, int rmax, int tmin, int tmax, bool adjoint, const int *flag,
@@ -1053,10 +990,9 @@ int launch_wilson_auto(const Geom &g, const Fields4 &U, const Fields4 &UA, const
     return rc;
   const int nr = rmax - rmin + 1, nt = tmax - tmin + 1;
   // average over the loops counted: every site, or the tstarts slices
-  reduce_select_kernel<<<nr * nt, 256, 0, s>>>(
-      partials, b_exact, b_gauge, flag, nr, nt,
-      wilson_scale((long long)g.Vs * tstarts, Store::NC, adjoint), out_dev);
-  return launch_check("reduce_select_kernel");
+  return launch_reduce_select(partials, b_exact, b_gauge, flag, nr, nt,
+                              wilson_scale((long long)g.Vs * tstarts, Store::NC, adjoint),
+                              out_dev, s);
 }
 
 size_t wilson_auto_partials_count(const Geom &g, int nr, int nt, int nc, int units) {

@@ -184,7 +184,8 @@ int gc_set_hyp_method(gc_lattice *h, int method);
  * Two methods give the same table: the exact product of links (walked in T
  * for every corner), and, for T <= Lt/2 when the temporal links are unitary
  * (checked on the device for every call: defect max |U U^dag - 1| at most
- * 1e-14 in FP64, 1e-6 in the mixed form), the same loops in the temporal
+ * 1e-14 in FP64, 1e-6 in the mixed form, there for the spatial SU(3) links as
+ * well), the same loops in the temporal
  * gauge (one trace per loop instead of two matrix products); see
  * gc_set_wilson_method. A block keeps one column's lines of all Lt slices in
  * shared memory: GC_ERR_ARG when they do not fit (SU(3): Lt > 246).
@@ -202,9 +203,9 @@ int gc_wilson_onaxis(gc_lattice *h, int r_min, int r_max, int time_min,
 int gc_wilson_adjoint_onaxis(gc_lattice *h, int r_min, int r_max, int time_min,
                              int time_max, double *out);
 
-/* Selects the method of gc_wilson_onaxis and gc_wilson_adjoint_onaxis on this
- * handle: GC_WILSON_AUTO (default) or GC_WILSON_EXACT. No counterpart in the
- * reference (which has one method, the exact product). */
+/* Selects the method of gc_wilson_onaxis, gc_wilson_adjoint_onaxis and the
+ * off-axis loops on this handle: GC_WILSON_AUTO (default) or GC_WILSON_EXACT.
+ * No counterpart in the reference (which has one method, the exact product). */
 int gc_set_wilson_method(gc_lattice *h, int method);
 
 /* The method the last on-axis W call of the handle ran: GC_WILSON_EXACT or

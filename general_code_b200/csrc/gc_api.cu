@@ -701,15 +701,15 @@ int gc_hyp(gc_lattice *h, double a1, double a2, double a3, int steps) {
   return GC_OK;
 }
 
-// Prepares the temporal-gauge form of W: the gauge time lines of both cuts
-// and the transformed spatial links, in the HYP decorated-link scratch (which
-// holds them: per site at most 2 x 144 + 6 x 144 bytes against 15 x 144 for
-// FP64 SU(3)), and the device's unitarity check of the links into *flag, a
-// word of h->flag_dev. *use is cleared when the scratch cannot hold them, or,
-// with `optional`, when it cannot be allocated (the caller has a form that
-// does without it).
+// Prepares the temporal-gauge form: the gauge time lines and the transformed
+// spatial links (with `ext` slices past the last one) in the HYP
+// decorated-link scratch, which holds them (FP64 SU(3): at most 144 (1 + 1/Lt)
+// + 3 x 1.5 x 144 bytes per site against 15 x 144), and the device's unitarity
+// check of the links into *flag, a word of h->flag_dev. *use is cleared when
+// the scratch cannot hold them, or, with `optional`, when it cannot be
+// allocated (the caller has a form that does without it).
 enum { kFlagOnaxis = 0, kFlagOther = 1 }; // words of h->flag_dev
-static int gauge_prepare(gc_lattice *h, Fields4 *UA, Fields4 *UB, bool *use, int **flag,
+static int gauge_prepare(gc_lattice *h, int ext, GaugeLinks *links, bool *use, int **flag,
                          int word = kFlagOnaxis, bool optional = false) {
   int rc = ensure_hyp(h);
   if (rc == GC_ERR_NOMEM && optional) {
@@ -726,21 +726,14 @@ static int gauge_prepare(gc_lattice *h, Fields4 *UA, Fields4 *UB, bool *use, int
       return cuda_fail(h, "cudaMalloc(flag)", e);
     }
   }
-  const size_t lb = wilson_gauge_line_bytes(h->g, h->nc);
-  if (2 * lb + 6 * h->field_bytes > 15 * hyp_field_bytes(h)) {
+  const int link_bytes = (int)bytes_per_link(h->nc, h->prec);
+  if (wilson_gauge_bytes(h->g, h->nc, link_bytes, ext) > 15 * hyp_field_bytes(h)) {
     *use = false;
     return GC_OK;
   }
   *flag = h->flag_dev + word;
-  char *base = (char *)h->hyp;
-  void *GA = base, *GB = base + lb;
-  for (int d = 0; d < 3; d++) {
-    UA->f[d] = base + 2 * lb + d * h->field_bytes;
-    UB->f[d] = base + 2 * lb + (3 + d) * h->field_bytes;
-  }
-  UA->f[3] = UB->f[3] = nullptr;
-  rc = GC_DISPATCH(h, launch_wilson_gauge_prep, h->g, h->cur, GA, GB, *UA, *UB, *flag,
-                   h->stream);
+  *links = wilson_gauge_links(h->hyp, h->g, h->nc, link_bytes, ext);
+  rc = GC_DISPATCH(h, launch_wilson_gauge_prep, h->g, h->cur, *links, *flag, h->stream);
   if (rc)
     return launch_fail(h, rc);
   return GC_OK;
@@ -808,22 +801,23 @@ static int wilson_impl(gc_lattice *h, int rmin, int rmax, int tmin, int tmax,
   double *chunk_out = h->dev_out + (size_t)nr * nt;
   // The temporal-gauge form (gc_wilson_gauge.cu) for one configuration's
   // on-axis or adjoint loops with T <= Lt/2, or, for the t-slab entry's start
-  // slices [0, t_starts), with T <= Lt - t_starts (one cut at slice 0: no
-  // counted loop passes the slab lattice's last slice); it runs only where
+  // slices [0, t_starts), with T <= Lt - t_starts (no counted loop passes the
+  // slab lattice's last slice); it runs only where
   // the device finds the temporal links unitary to the form's tolerance, and
   // the exact recursion otherwise.
   const int ct_bytes = h->prec == GC_PREC_FP64 ? 8 : 4;
   bool gauge = h->wilson_method == GC_WILSON_AUTO && !second &&
-               wilson_gauge_applies(h->g, tmax, nt, h->nc, ct_bytes, tstarts);
-  Fields4 UA{}, UB{};
+               wilson_gauge_applies(h->g, tmin, tmax, h->nc, ct_bytes, adjoint, tstarts);
+  GaugeLinks links{};
   int *flag = nullptr;
   if (gauge) {
-    rc = gauge_prepare(h, &UA, &UB, &gauge, &flag);
+    rc = gauge_prepare(h, wilson_gauge_ext(h->g, tmax, tstarts), &links, &gauge, &flag);
     if (rc)
       return rc;
   }
   if (gauge) {
-    rc = ensure_partials(h, wilson_auto_partials_count(h->g, std::min(rchunk, nr), nt, h->nc));
+    rc = ensure_partials(h, wilson_auto_partials_count(h->g, std::min(rchunk, nr), tmin, tmax, h->nc, 0,
+                                                       tstarts));
     if (rc)
       return rc;
   }
@@ -833,7 +827,7 @@ static int wilson_impl(gc_lattice *h, int rmin, int rmax, int tmin, int tmax,
     const int r1 = std::min(rmax, r0 + rchunk - 1);
     const int ncr = r1 - r0 + 1;
     if (gauge)
-      rc = GC_DISPATCH(h, launch_wilson_auto, h->g, h->cur, UA, UB, r0, r1, tmin, tmax,
+      rc = GC_DISPATCH(h, launch_wilson_auto, h->g, h->cur, links, r0, r1, tmin, tmax,
                        adjoint, flag, h->partials, chunk_out, h->stream, 0, tstarts);
     else
       rc = GC_DISPATCH(h, launch_wilson, h->g, h->cur, r0, r1, tmin, tmax,
@@ -1035,10 +1029,10 @@ static int offaxis_impl(gc_lattice *h, const std::vector<std::array<int, 3>> &di
   if (tree.nodes.empty())
     gauge_blocks = 0;
   bool gauge = gauge_blocks > 0;
-  Fields4 UA{}, UB{};
+  GaugeLinks links{};
   int *flag = nullptr;
   if (gauge) {
-    rc = gauge_prepare(h, &UA, &UB, &gauge, &flag, kFlagOther, true);
+    rc = gauge_prepare(h, tmax, &links, &gauge, &flag, kFlagOther, true);
     if (rc)
       return rc;
   }
@@ -1095,7 +1089,7 @@ static int offaxis_impl(gc_lattice *h, const std::vector<std::array<int, 3>> &di
     rc = GC_DISPATCH(h, launch_offaxis_fused, h->g, h->cur, dev_lines + c0, n, tmin, tmax,
                      adjoint, h->partials, &b, h->stream, flag);
     if (!rc && gauge)
-      rc = GC_DISPATCH(h, launch_offaxis_gauge, h->g, UA, UB, dev_nodes, dev_chunks, k0, k1 - k0,
+      rc = GC_DISPATCH(h, launch_offaxis_gauge, h->g, links, dev_nodes, dev_chunks, k0, k1 - k0,
                        c0, n, tmin, tmax, adjoint, h->partials, flag, h->stream);
     if (!rc)
       rc = gauge ? launch_reduce_select(h->partials, b, gauge_blocks, flag, 1, n * nt, scale,
@@ -1563,7 +1557,7 @@ long long gc_job_device_bytes(const int dims[4], int nc, int precision,
   g.Vs = dims[0] * dims[1] * dims[2];
   const int nr = std::max(1, rmax), nt = std::max(1, tmax);
   const long long partials =
-      (long long)wilson_auto_partials_count(g, std::min(nr, std::max(1, 1024 / nt)), nt, nc) *
+      (long long)wilson_auto_partials_count(g, std::min(nr, std::max(1, 1024 / nt)), 1, nt, nc) *
       8;
   const long long hfield =
       ((long long)inter_link_bytes(nc, precision) * V + 255) / 256 * 256;

@@ -107,8 +107,7 @@ struct JobState {
   int gunits = 0;         // its block shape (column units; 0 = default)
   Fields4 wU{};           // the job's links when its W runs
   int *flag = nullptr;    // the job's unitarity flag (device)
-  void *GA = nullptr, *GB = nullptr; // gauge lines (in the HYP scratch)
-  Fields4 UA{}, UB{};     // transformed spatial links (in the HYP scratch)
+  GaugeLinks glinks{};    // gauge lines and transformed links (in the HYP scratch)
   bool has_input = false;
 };
 
@@ -411,10 +410,10 @@ int enqueue_wauto(gc_batch *b, int cls, const std::vector<int> &jobs, cudaStream
   for (size_t m = 0; m < jobs.size(); m++) {
     JobState &j = b->jobs[jobs[m]];
     cudaStream_t ws = b->wstream[cls][m % ns];
-    int rc = launch_wilson_gauge_prep<Store, CT>(j.g, j.wU, j.GA, j.GB, j.UA, j.UB, j.flag, ws);
+    int rc = launch_wilson_gauge_prep<Store, CT>(j.g, j.wU, j.glinks, j.flag, ws);
     if (rc)
       return rc;
-    rc = launch_wilson_auto<Store, CT>(j.g, j.wU, j.UA, j.UB, j.desc.r_min, j.desc.r_max,
+    rc = launch_wilson_auto<Store, CT>(j.g, j.wU, j.glinks, j.desc.r_min, j.desc.r_max,
                                        j.desc.time_min, j.desc.time_max, false, j.flag,
                                        j.partials, j.out_dev, ws, j.gunits);
     if (rc)
@@ -589,7 +588,8 @@ int tune_job(gc_batch *b, JobState &j, double *scratch, cudaStream_t s, int *row
 // gauge form whichever of the two gated kernels has more blocks.
 size_t partials_doubles(const JobState &j) {
   if (j.gauge)
-    return wilson_auto_partials_count(j.g, j.nr, j.nt, j.desc.nc, j.gunits);
+    return wilson_auto_partials_count(j.g, j.nr, j.desc.time_min, j.desc.time_max, j.desc.nc,
+                                      j.gunits);
   return (size_t)j.w_blocks * j.nr * j.nt;
 }
 
@@ -749,18 +749,14 @@ int gc_batch_create(const gc_job *jobs, int njobs, int precision, gc_batch **out
     o += (size_t)j.nr * j.nt;
     // the temporal-gauge W: its lines and transformed links go into the HYP
     // decorated-link scratch (a job without HYP steps has none)
-    const size_t lb = wilson_gauge_line_bytes(j.g, j.desc.nc);
+    const int lbytes = (int)link_bytes(j.desc.nc, precision);
+    const int ext = wilson_gauge_ext(j.g, j.desc.time_max);
     j.gauge = ok && j.nr > 0 &&
-              wilson_gauge_applies(j.g, j.desc.time_max, j.nt, j.desc.nc, ct_bytes) &&
-              2 * lb + 6 * j.field_bytes <= 15 * j.hyp_bytes;
+              wilson_gauge_applies(j.g, j.desc.time_min, j.desc.time_max, j.desc.nc, ct_bytes,
+                                   false) &&
+              wilson_gauge_bytes(j.g, j.desc.nc, lbytes, ext) <= 15 * j.hyp_bytes;
     if (j.gauge) {
-      char *base = (char *)j.hyp[0];
-      j.GA = base;
-      j.GB = base + lb;
-      for (int d = 0; d < 3; d++) {
-        j.UA.f[d] = base + 2 * lb + d * j.field_bytes;
-        j.UB.f[d] = base + 2 * lb + (3 + d) * j.field_bytes;
-      }
+      j.glinks = wilson_gauge_links(j.hyp[0], j.g, j.desc.nc, lbytes, ext);
       j.flag = b->flags + i;
     }
   }
@@ -885,14 +881,14 @@ int gc_batch_autotune(gc_batch *b) {
   b->tune_report.clear();
   // one tuning per distinct (Lt, nc, nr, nt, Vs)
   std::map<std::tuple<int, int, int, int, int>, std::pair<int, int>> cache;
-  std::map<std::tuple<int, int, int, int, int>, int> gcache;
+  std::map<std::tuple<int, int, int, int, int, int>, int> gcache;
   int rc = GC_OK;
   for (JobState &j : b->jobs) {
     if (j.nr <= 0)
       continue;
     if (j.gauge) {
       // the gauge-form W kernel's columns per block, timed on the job's input
-      auto key = std::make_tuple(j.g.L[3], j.desc.nc, j.nr, j.nt, j.g.Vs);
+      auto key = std::make_tuple(j.g.L[3], j.desc.nc, j.nr, j.nt, j.g.Vs, j.glinks.NE);
       auto it = gcache.find(key);
       if (it != gcache.end()) {
         j.gunits = it->second;
@@ -901,13 +897,13 @@ int gc_batch_autotune(gc_batch *b) {
       Fields4 U;
       for (int d = 0; d < 4; d++)
         U.f[d] = j.input[d];
-      rc = GC_DISPATCH_NC(j.desc.nc, b->prec, launch_wilson_gauge_prep, j.g, U, j.GA, j.GB,
-                          j.UA, j.UB, j.flag, b->main);
+      rc = GC_DISPATCH_NC(j.desc.nc, b->prec, launch_wilson_gauge_prep, j.g, U, j.glinks,
+                          j.flag, b->main);
       if (rc)
         break;
       float best = 1e30f;
       int bu = 0;
-      const WilsonPlan dp = wilson_gauge_plan(j.g, j.nt, j.desc.nc,
+      const WilsonPlan dp = wilson_gauge_plan(j.g, j.desc.time_min, j.desc.time_max, j.desc.nc,
                                               b->prec == GC_PREC_FP64 ? 8 : 4);
       char cls[96];
       std::snprintf(cls, sizeof cls, "SU(%d) %dx%dx%dx%d R<=%d T<=%d", j.desc.nc, j.g.L[0],
@@ -915,7 +911,7 @@ int gc_batch_autotune(gc_batch *b) {
       std::string lines;
       for (int units = 1; units * dp.rows <= 256; units *= 2) {
         float ms = 0;
-        rc = GC_DISPATCH_NC(j.desc.nc, b->prec, time_wilson_gauge, j.g, j.UA, j.UB,
+        rc = GC_DISPATCH_NC(j.desc.nc, b->prec, time_wilson_gauge, j.g, j.glinks,
                             j.desc.r_min, j.desc.r_max, j.desc.time_min, j.desc.time_max,
                             units, scratch, b->main, &ms);
         if (rc == GC_ERR_ARG) {

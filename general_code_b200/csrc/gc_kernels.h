@@ -99,10 +99,7 @@ struct WilsonPlan {
   size_t smem;        // dynamic shared memory bytes
   bool fits;          // false when even one column exceeds the budget
   int starts = 1;     // temporal-gauge form: consecutive start slices per thread
-  // temporal-gauge form: 0 wilson_gauge_kernel; one column per thread with
-  // the lines of its starts in registers: 1 wilson_gauge_reg_kernel (mixed
-  // SU(3)), 2 wilson_gauge_q_kernel (SU(2))
-  int kernel = 0;
+  int kernel = 0;     // temporal-gauge form: 0 wilson_gauge_kernel, 1 wilson_gram_kernel
 };
 // Doubles of a W block's per-warp accumulators in shared memory, rounded up
 // to an even count so the 16-byte arrays placed after them stay aligned.
@@ -159,31 +156,45 @@ int launch_wilson(const Geom &g, const Fields4 &U, int rmin, int rmax,
 // W(R,T) in the temporal gauge (gc_wilson_gauge.cu): applies to one
 // configuration's loops over the whole lattice with T <= Lt/2 when the block
 // shape fits; exact to rounding when the temporal links are unitary.
-// units: column units (threads per time row) per block; 0 = about 128 threads.
-WilsonPlan wilson_gauge_plan(const Geom &g, int nt, int nc, int ct_bytes, int units = 0,
-                             bool adjoint = false);
-// tstarts in (0, Lt): the start slices [0, tstarts) of a time slab, in one
-// cut (time_max <= Lt - tstarts); otherwise every start slice (T <= Lt/2).
-bool wilson_gauge_applies(const Geom &g, int tmax, int nt, int nc, int ct_bytes,
+// units: columns (fundamental) or column units (adjoint: threads per time row)
+// per block; 0 = the default. tstarts in (0, Lt): the start slices
+// [0, tstarts) of a time slab (time_max <= Lt - tstarts); otherwise every
+// start slice (T <= Lt/2).
+WilsonPlan wilson_gauge_plan(const Geom &g, int tmin, int tmax, int nc, int ct_bytes,
+                             int units = 0, bool adjoint = false, int tstarts = 0);
+bool wilson_gauge_applies(const Geom &g, int tmin, int tmax, int nc, int ct_bytes, bool adjoint,
                           int tstarts = 0);
+// Transformed slices the loops need past the last one: tmax, none for a slab.
+int wilson_gauge_ext(const Geom &g, int tmax, int tstarts = 0);
 // Largest unitarity defect max |U U^dag - 1| of a temporal link for which the
 // form is used (FP64: ct_bytes 8; mixed: 4).
 double wilson_gauge_tolerance(int ct_bytes);
-// Bytes of one field of gauge time lines (FP64 matrices, 256-byte aligned).
-size_t wilson_gauge_line_bytes(const Geom &g, int nc);
-// Gauge time lines GA, GB (cuts at slices 0 and Lt/2) and the transformed
-// spatial links UA.f[0..2], UB.f[0..2] (the link storage format); *flag (a
-// device int) is set to 1 when a temporal link's defect exceeds the
-// tolerance, else left 0.
+// The form's scratch: gauge time lines G (V matrices, FP64) and W (the lines
+// over the whole extent, Vs matrices), and the transformed spatial links
+// U.f[0..2] on NE = Lt + ext slices (the link storage format with a plane
+// stride of NE Vs sites).
+struct GaugeLinks {
+  void *G, *W;
+  Fields4 U;
+  int NE;
+};
+size_t wilson_gauge_bytes(const Geom &g, int nc, int link_bytes, int ext);
+GaugeLinks wilson_gauge_links(void *base, const Geom &g, int nc, int link_bytes, int ext);
+// Fills them; *flag (a device int) is set to 1 when a link's defect exceeds
+// the tolerance, else left 0.
 template <class Store, class CT>
-int launch_wilson_gauge_prep(const Geom &g, const Fields4 &U, void *GA, void *GB,
-                             const Fields4 &UA, const Fields4 &UB, int *flag, cudaStream_t s);
-// The W table from the transformed links (partials: blocks of
-// wilson_gauge_plan x nr x nt doubles), reduced into out_dev.
+int launch_wilson_gauge_prep(const Geom &g, const Fields4 &U, const GaugeLinks &l, int *flag,
+                             cudaStream_t s);
+
+// The fundamental loops by FP64 matrix instructions (gc_wilson_gram.cu), or
+// with `second` (transformed links of a second configuration in the same
+// gauge) the GEVP loops: per-block partials [block][R][T], run when flag is
+// null or *flag == 0. tstarts start slices; cols 0 = the default.
+WilsonPlan wilson_gram_plan(const Geom &g, int tstarts, int tmax, int nc, int cols, bool gevp);
 template <class Store, class CT>
-int launch_wilson_gauge(const Geom &g, const Fields4 &UA, const Fields4 &UB, int rmin,
-                        int rmax, int tmin, int tmax, bool adjoint, double *partials,
-                        double *out_dev, cudaStream_t s);
+int launch_wilson_gram(const Geom &g, const GaugeLinks &l, const Fields4 *second, int rmin,
+                       int rmax, int tmin, int tmax, const int *flag, double *partials,
+                       int *blocks, cudaStream_t s, int cols, int tstarts);
 
 // Both methods with the choice made on the device: the exact W kernel runs
 // (and the gauge one returns at once) when *flag != 0, else the other way
@@ -192,23 +203,22 @@ int launch_wilson_gauge(const Geom &g, const Fields4 &UA, const Fields4 &UB, int
 // kernel's shared-memory attribute has been set by an earlier launch).
 // partials: wilson_auto_partials_count doubles. tstarts in (0, Lt): the
 // loops of the start slices [0, tstarts) only (a time slab's lattice of its
-// own slices and the ones above them), in one cut at slice 0; the caller
-// guarantees time_max <= Lt - tstarts (no loop passes the lattice's end).
+// own slices and the ones above them); the caller guarantees time_max <=
+// Lt - tstarts (no loop passes the lattice's end).
 template <class Store, class CT>
-int launch_wilson_auto(const Geom &g, const Fields4 &U, const Fields4 &UA, const Fields4 &UB,
-                       int rmin, int rmax, int tmin, int tmax, bool adjoint, const int *flag,
-                       double *partials, double *out_dev, cudaStream_t s, int units = 0,
-                       int tstarts = 0);
+int launch_wilson_auto(const Geom &g, const Fields4 &U, const GaugeLinks &l, int rmin, int rmax,
+                       int tmin, int tmax, bool adjoint, const int *flag, double *partials,
+                       double *out_dev, cudaStream_t s, int units = 0, int tstarts = 0);
 // out_dev[it * nr + ir] = scale * (fixed-order sum of the partials
 // [block][ir * nt + it]) over the blocks of the method that ran (*flag).
 int launch_reduce_select(const double *partials, int blocks_exact, int blocks_gauge,
                          const int *flag, int nr, int nt, double scale, double *out_dev,
                          cudaStream_t s);
-size_t wilson_auto_partials_count(const Geom &g, int nr, int nt, int nc, int units = 0);
+size_t wilson_auto_partials_count(const Geom &g, int nr, int tmin, int tmax, int nc, int units = 0,
+                                  int tstarts = 0);
 template <class Store, class CT>
-int time_wilson_gauge(const Geom &g, const Fields4 &UA, const Fields4 &UB, int rmin, int rmax,
-                      int tmin, int tmax, int units, double *partials, cudaStream_t s,
-                      float *ms);
+int time_wilson_gauge(const Geom &g, const GaugeLinks &l, int rmin, int rmax, int tmin, int tmax,
+                      int units, double *partials, cudaStream_t s, float *ms);
 // The exact W kernel, gated on *gate != 0, without the reduction; *blocks
 // receives the number of blocks (rows of partials). tstarts as for
 // launch_wilson_auto (0: every start slice).
@@ -325,9 +335,8 @@ int offaxis_gauge_blocks(const Geom &g, int nc, int ct_bytes, int tmin, int tmax
 // Distinct lines [line0, line0 + nlines) of whole chunks; partials
 // [block][line - line0][T - tmin]. Runs when *flag == 0.
 template <class Store, class CT>
-int launch_offaxis_gauge(const Geom &g, const Fields4 &UA, const Fields4 &UB,
-                         const OffaxisNode *nodes, const int *chunk_nodes,
-                         int chunk0, int nchunks, int line0, int nlines, int tmin, int tmax,
+int launch_offaxis_gauge(const Geom &g, const GaugeLinks &l, const OffaxisNode *nodes,
+                         const int *chunk_nodes, int chunk0, int nchunks, int line0, int nlines, int tmin, int tmax,
                          bool adjoint, double *partials, const int *flag, cudaStream_t s);
 
 // Loops of a line field S (decorated-link storage) whose end is displaced

@@ -3,13 +3,11 @@
 // lib/cpu/include/wilson_loops.h:313-663) from the transformed links of
 // gc_wilson_gauge.cu.
 //
-// In the gauge of a cut slice a time line that does not pass the cut is 1, so
-// a loop of the space line S' (the product of the transformed links along its
-// steps) is Re Tr[S'(x + T t) S'(x)^dag]: one trace instead of the two
-// products of the exact walk. Cut A (slice 0) serves the loops with
-// t0 + T < Lt, whatever their start slice; the loops that pass slice Lt - 1
-// start on the last tmax slices and end on the first tmax - 1, so cut B (slice
-// Lt/2, T <= Lt/2) needs its lines on those 2 tmax slices only.
+// In the temporal gauge a time line is 1, so a loop of the space line S' (the
+// product of the transformed links along its steps) is
+// Re Tr[S'(x + T t) S'(x)^dag]: one trace instead of the two products of the
+// exact walk. The lines are needed on the Lt start slices and, for the loops
+// that pass the last one, on tmax further slices.
 //
 // The lines themselves cost more than their loops then (5 links and 6 loops
 // per line at r, T <= 6). Many are equal step for step (the reference counts
@@ -130,10 +128,9 @@ template <> struct LineOps<SU3<float>> {
   __device__ __forceinline__ static void finish(M &P) { rebuild_row2(P); }
 };
 
-// Slots of a column and their slices: slot i < Lt is cut A on slice i, slot
-// Lt + j cut B on slice (Lt - tmax + j) mod Lt, j < 2 tmax. The loops of a
-// start slot i end on slot i + T.
-__host__ __device__ inline int gauge_slots(int Lt, int tmax) { return Lt + 2 * tmax; }
+// Slot i of a column is slice i of the extended lattice; the loops of a start
+// slot i < Lt end on slot i + T.
+__host__ __device__ inline int gauge_slots(int Lt, int tmax) { return Lt + tmax; }
 
 struct GaugeShape {
   int cols, threads;
@@ -163,9 +160,8 @@ GaugeShape gauge_shape(const Geom &g, int nc, int ct_bytes, int tmin, int tmax, 
 
 template <class Store, class CT, bool ADJ>
 __global__ void __launch_bounds__(512)
-    offaxis_gauge_kernel(const __grid_constant__ Geom g, const __grid_constant__ Fields4 UA,
-                         const __grid_constant__ Fields4 UB,
-                         const OffaxisNode *__restrict__ nodes,
+    offaxis_gauge_kernel(const __grid_constant__ Geom g, const __grid_constant__ Fields4 U,
+                         int NE, const OffaxisNode *__restrict__ nodes,
                          const int *__restrict__ chunk_nodes, int line0, int nlines, int tmin,
                          int tmax, int cols, double *partials, const int *flag) {
   if (*flag != 0)
@@ -182,19 +178,10 @@ __global__ void __launch_bounds__(512)
   const int c = tid % cols, slot = tid / cols;
   const int s = blockIdx.x * cols + c;
   const bool active = slot < gauge_slots(Lt, tmax) && s < g.Vs;
-  const bool cut_b = slot >= Lt;
-  const int j = slot - Lt;
-  const int t = cut_b ? (Lt - tmax + j) % Lt : slot;
-  // loops that start on this slot: T in [lo, hi]
-  int lo = cut_b ? max(tmin, tmax - j) : tmin;
-  int hi = cut_b ? (j < tmax ? tmax : 0) : min(tmax, Lt - 1 - slot);
-  if (!active)
-    hi = 0, lo = 1;
+  const bool starts = active && slot < Lt; // loops start on this slot
   const int x0 = s % g.L[0], x1 = (s / g.L[0]) % g.L[1], x2 = s / (g.L[0] * g.L[1]);
-  const size_t V = g.V;
-  const int toff = t * g.Vs;
-  const void *f0 = cut_b ? UB.f[0] : UA.f[0], *f1 = cut_b ? UB.f[1] : UA.f[1],
-             *f2 = cut_b ? UB.f[2] : UA.f[2];
+  const size_t VE = (size_t)NE * g.Vs;
+  const int toff = slot * g.Vs;
   for (int i = tid; i < 2 * nt * nth; i += nth)
     red[i] = Acc(0);
 
@@ -206,7 +193,7 @@ __global__ void __launch_bounds__(512)
     y2 -= y2 >= g.L[2] ? g.L[2] : 0;
     return y0 + g.L[0] * (y1 + g.L[1] * y2) + toff;
   };
-  auto field = [&](int axis) { return axis == 0 ? f0 : axis == 1 ? f1 : f2; };
+  auto field = [&](int axis) { return axis == 0 ? U.f[0] : axis == 1 ? U.f[1] : U.f[2]; };
 
   const int n0 = chunk_nodes[blockIdx.y], n1 = chunk_nodes[blockIdx.y + 1];
   const int4 *desc = reinterpret_cast<const int4 *>(nodes);
@@ -216,7 +203,7 @@ __global__ void __launch_bounds__(512)
   int ops = __ldg(reinterpret_cast<const int *>(desc + 2 * n0 + 1));
   M u;
   if (active)
-    u = Store::template load<CT>(field(ops & 0xff), V, link(d));
+    u = Store::template load<CT>(field(ops & 0xff), VE, link(d));
 #pragma unroll 1
   for (int n = n0; n < n1; n++) {
     const int line = d.w;
@@ -237,7 +224,7 @@ __global__ void __launch_bounds__(512)
       d = __ldg(desc + 2 * n + 2);
       ops = __ldg(reinterpret_cast<const int *>(desc + 2 * n + 3));
       if (active)
-        u = Store::template load<CT>(field(ops & 0xff), V, link(d));
+        u = Store::template load<CT>(field(ops & 0xff), VE, link(d));
     }
     if (line < 0)
       continue;
@@ -261,10 +248,12 @@ __global__ void __launch_bounds__(512)
           partials[((size_t)blockIdx.x * nlines + prev - line0) * nt + T] = v;
       }
     }
+    if (starts) {
 #pragma unroll 2
-    for (int T = lo; T <= hi; T++)
-      r[(size_t)(T - tmin) * nth + tid] =
-          gauge_trace<ADJ>(a, SS::load(buf, nth, tid + T * cols), false);
+      for (int T = tmin; T <= tmax; T++)
+        r[(size_t)(T - tmin) * nth + tid] =
+            gauge_trace<ADJ>(a, SS::load(buf, nth, tid + T * cols), false);
+    }
     prev = line;
     done++;
   }
@@ -293,18 +282,18 @@ int offaxis_gauge_blocks(const Geom &g, int nc, int ct_bytes, int tmin, int tmax
 }
 
 template <class Store, class CT>
-int launch_offaxis_gauge(const Geom &g, const Fields4 &UA, const Fields4 &UB,
-                         const OffaxisNode *nodes, const int *chunk_nodes, int chunk0,
-                         int nchunks, int line0, int nlines, int tmin, int tmax, bool adjoint,
+int launch_offaxis_gauge(const Geom &g, const GaugeLinks &l, const OffaxisNode *nodes,
+                         const int *chunk_nodes, int chunk0, int nchunks,
+                         int line0, int nlines, int tmin, int tmax, bool adjoint,
                          double *partials, const int *flag, cudaStream_t s) {
   const GaugeShape f = gauge_shape(g, Store::NC, (int)sizeof(CT), tmin, tmax, adjoint);
-  if (!f.cols || tmax > g.L[3] / 2)
+  if (!f.cols || tmax > g.L[3] / 2 || l.NE < g.L[3] + tmax)
     return plan_error("offaxis_gauge_kernel: block shape does not fit");
   const dim3 grid((g.Vs + f.cols - 1) / f.cols, nchunks);
   auto go = [&](auto kernel) {
     const int rc = allow_large_smem(kernel, f.smem);
     if (!rc)
-      kernel<<<grid, f.threads, f.smem, s>>>(g, UA, UB, nodes, chunk_nodes + chunk0, line0,
+      kernel<<<grid, f.threads, f.smem, s>>>(g, l.U, l.NE, nodes, chunk_nodes + chunk0, line0,
                                              nlines, tmin, tmax, f.cols, partials, flag);
     return rc;
   };
@@ -315,8 +304,8 @@ int launch_offaxis_gauge(const Geom &g, const Fields4 &UA, const Fields4 &UB,
 
 #define GC_INSTANTIATE_OG(STORE, CT)                                                         \
   template int launch_offaxis_gauge<STORE, CT>(                                              \
-      const Geom &, const Fields4 &, const Fields4 &, const OffaxisNode *, const int *, int, \
-      int, int, int, int, int, bool, double *, const int *, cudaStream_t);
+      const Geom &, const GaugeLinks &, const OffaxisNode *, const int *, int, int, int, int,  \
+      int, int, bool, double *, const int *, cudaStream_t);
 
 GC_INSTANTIATE_OG(StoreF64SU3, double)
 GC_INSTANTIATE_OG(StoreF64SU2, double)

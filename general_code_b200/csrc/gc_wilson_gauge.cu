@@ -6,21 +6,23 @@
 // with time lines L(x,T) = U_t(x) U_t(x+t) ... U_t(x+(T-1)t) and space lines
 // S(x,R) = U_nu(x) ... U_nu(x+(R-1)nu).
 //
-// The loop is gauge invariant. With G_c(s,t) the time line of spatial site s
-// from a cut slice c up to slice t (G_c(s,c) = 1, G_c(s,t+1) = G_c(s,t)
-// U_t(s,t) walking forward from c), a time line that does not pass the cut
-// is L(s;t0,T) = G_c(s,t0)^dag G_c(s,t0+T) when the temporal links are
-// unitary, and the loop becomes
+// The loop is gauge invariant. With G(s,t) the time line of spatial site s
+// from slice 0 up to slice t (G(s,0) = 1, G(s,t+1) = G(s,t) U_t(s,t)),
+// continued past the last slice with the periodic links (G(s,Lt+j) =
+// W(s) G(s,j), W(s) the line over the whole extent), every time line is
+// L(s;t0,T) = G(s,t0)^dag G(s,t0+T) when the temporal links are unitary, and
+// the loop becomes
 //     Re Tr[S'(x,R) S'(x+T t,R)^dag] / N,
-//     S'(s,t,R) = G_c(s,t) S(s,t,R) G_c(s+R nu,t)^dag
+//     S'(s,t,R) = G(s,t) S(s,t,R) G(s+R nu,t)^dag
 //               = U'_nu(s,t) ... U'_nu(s+(R-1)nu,t),
-//     U'_nu(s,t) = G_c(s,t) U_nu(s,t) G_c(s+nu,t)^dag.
-// Two cuts cover every loop with T <= h = floor(Lt/2): cut A at slice 0 for
-// loops starting on slices t0 < h (they end at t0+T <= 2h-1 <= Lt-1), cut B
-// at slice h for loops starting on t0 >= h (t0-h+T <= Lt-1). A loop then
-// costs one 9-element trace instead of two matrix products (the T walk of
-// the exact recursion in gc_wilson.cu), and each space line one product per
-// R and cut.
+//     U'_nu(s,t) = G(s,t) U_nu(s,t) G(s+nu,t)^dag
+// with the transformed links on the slices 0 .. Lt-1 and, for the loops that
+// pass the last slice, on T_max further ones. A loop then costs one 9-element
+// trace instead of two matrix products (the T walk of the exact recursion in
+// gc_wilson.cu), and each space line one product per R. (Two cuts of Lt
+// slices each, with the second for the loops that pass the first, took 2 Lt
+// lines per column instead of Lt + T_max: at SU(3) 32^4 FP64 a third more
+// shared memory and products.)
 //
 // The identity needs unitary temporal links. The lines kernel measures the
 // largest unitarity defect max |U_t U_t^dag - 1| of the lattice's temporal
@@ -36,25 +38,26 @@
 // 2 T d (the two time lines), well inside the parity tolerances at these d.
 //
 // Kernels:
-//   gauge_lines_kernel      thread per (spatial site, cut): G_A(s,t) and the
-//                           defect, or G_B(s,t), for all t (FP64, stored as
-//                           FP64 fields)
-//   gauge_transform_kernel  thread per (site, spatial nu): U'_nu for both
-//                           cuts, computed in FP64, stored in the lattice's
-//                           link format
-//   wilson_gauge_kernel     block = `cols` columns (s, nu) over all t: the
-//                           transformed space lines of both cuts in shared
+//   gauge_lines_kernel      thread per spatial site: G(s,t), W(s) and the
+//                           defect (FP64, stored as FP64 fields)
+//   gauge_transform_kernel  thread per (extended site, spatial nu): U'_nu,
+//                           computed in FP64, stored in the lattice's link
+//                           format
+//   wilson_gram_kernel      (gc_wilson_gram.cu) fundamental loops as FP64
+//                           matrix products
+//   wilson_gauge_reg_kernel mixed SU(3), and
+//   wilson_gauge_q_kernel   SU(2) fundamental loops of shorter T ranges: one
+//                           column per thread, the lines of its four start
+//                           slices in registers (gauge_*_applies has the line)
+//   wilson_gauge_kernel     the adjoint loops (|Tr|^2 is no bilinear form of
+//                           the lines): block = `cols` columns (s, nu) over
+//                           all slices, the transformed space lines in shared
 //                           memory, extended by one link per R; a thread per
-//                           (column unit, 1, 2 or 4 start slices) adds the
-//                           traces of its loops for every T into a per-thread
-//                           slot; a
-//                           fixed-order sum over the block's threads gives
-//                           one partial per (block, R, T), and the fixed-order
-//                           tree over blocks of gc_wilson.cu finishes
-//   wilson_gauge_reg_kernel the mixed SU(3) fundamental loops (8 | Lt), and
-//   wilson_gauge_q_kernel   the SU(2) fundamental loops (8 | Lt): one column
-//                           per thread, the space lines of its 4 start slices
-//                           kept in registers
+//                           (column unit, 1, 2 or 4 start slices) adds its
+//                           loops for every T into a per-thread slot
+// The last three sum their per-thread slots over the block in fixed order; one
+// partial per (block, R, T), and the fixed-order tree over blocks of
+// gc_wilson.cu finishes.
 #include "gc_internal.cuh"
 #include "gc_kernels.h"
 #include "gc_pair.cuh"
@@ -128,10 +131,15 @@ __device__ __forceinline__ typename Store::template M<double> gauge_time_link(
 // at 24^4 FP64 9e-15 -> 9e-16). A quaternion's norm does not drift that way.
 __device__ __forceinline__ SU3<double> stored_line(const SU3<double> &G) { return polar_step(G); }
 __device__ __forceinline__ SU2<double> stored_line(const SU2<double> &G) { return G; }
+//
+// The chain over t is serial, so the next links are loaded two steps ahead of
+// the product that needs them, and blocks are small: a 16^3 slice has 4096
+// threads.
+constexpr int kLinesBlock = 32;
 template <class Store>
-__global__ void __launch_bounds__(128)
-    gauge_lines_kernel(const __grid_constant__ Geom g, const void *Ut, void *GA, void *GB,
-                       int h, double tol, int *flag) {
+__global__ void __launch_bounds__(kLinesBlock)
+    gauge_lines_kernel(const __grid_constant__ Geom g, const void *Ut, void *GL, void *W,
+                       double tol, int *flag) {
   using GS = typename F64Store<Store::NC>::type;
   using MD = typename Store::template M<double>;
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
@@ -139,63 +147,58 @@ __global__ void __launch_bounds__(128)
     return;
   const size_t V = g.V;
   const int Lt = g.L[3];
-  if (blockIdx.y == 0) {
-    // cut A: G_A(s,0) = 1, G_A(s,t+1) = G_A(s,t) U_t(s,t); the defect check
-    double dmax = 0.0;
-    MD G = unit(MD());
-#pragma unroll 1
-    for (int t = 0; t < Lt; t++) {
-      GS::template store<double>(GA, V, s + t * g.Vs, stored_line(G));
-      const MD u = Store::template load<double>(Ut, V, s + t * g.Vs);
-      dmax = fmax(dmax, unitarity_defect(u));
-      if (t + 1 < Lt)
-        G = mul(G, gauge_time_link<Store>(u));
-    }
-    if (!(dmax <= tol)) // (a NaN link counts as not unitary)
-      *flag = 1;
-    return;
-  }
-  // cut B: G_B(s,h) = 1, forward through Lt-1 and around to h-1
+  double dmax = 0.0;
   MD G = unit(MD());
-  int t = h;
+  MD u = Store::template load<double>(Ut, V, s);
+  MD next = Store::template load<double>(Ut, V, s + (Lt > 1 ? g.Vs : 0));
 #pragma unroll 1
-  for (int k = 0; k < Lt; k++) {
-    GS::template store<double>(GB, V, s + t * g.Vs, stored_line(G));
-    if (k + 1 < Lt)
-      G = mul(G, gauge_time_link<Store>(Store::template load<double>(Ut, V, s + t * g.Vs)));
-    t = (t + 1 == Lt) ? 0 : t + 1;
+  for (int t = 0; t < Lt; t++) {
+    const MD after = Store::template load<double>(Ut, V, s + min(t + 2, Lt - 1) * g.Vs);
+    GS::template store<double>(GL, V, s + t * g.Vs, stored_line(G));
+    dmax = fmax(dmax, unitarity_defect(u));
+    G = mul(G, gauge_time_link<Store>(u));
+    u = next;
+    next = after;
   }
+  GS::template store<double>(W, g.Vs, s, stored_line(G));
+  if (!(dmax <= tol)) // (a NaN link counts as not unitary)
+    *flag = 1;
 }
 
-// U'_nu(x) = G(x) U_nu(x) G(x + nu)^dag for both cuts; thread per (site, nu).
+// U'_nu(s,te) = G(s,te) U_nu(s,te mod Lt) G(s+nu,te)^dag on the slices te of
+// the extended lattice (sites [0, NE Vs), plane stride NE Vs); thread per
+// (site, nu).
 template <class Store>
 __global__ void __launch_bounds__(128)
     gauge_transform_kernel(const __grid_constant__ Geom g, const __grid_constant__ Fields4 U,
-                           const void *GA, const void *GB, const __grid_constant__ Fields4 UA,
-                           const __grid_constant__ Fields4 UB, double tol, int *flag) {
+                           const void *GL, const void *W, const __grid_constant__ Fields4 UE,
+                           int NE, double tol, int *flag) {
   using GS = typename F64Store<Store::NC>::type;
   using MD = typename Store::template M<double>;
-  const int site = blockIdx.x * blockDim.x + threadIdx.x;
-  if (site >= g.V)
+  const int esite = blockIdx.x * blockDim.x + threadIdx.x;
+  const int VE = NE * g.Vs;
+  if (esite >= VE)
     return;
   const int nu = blockIdx.y;
+  const bool past = esite >= g.V; // a slice past the last one
+  const int site = past ? esite - g.V : esite;
   int x[4];
   site_coords(g, site, x);
-  const int sn = site + step_off(g, sel4(x, nu), nu, +1);
+  const int off = step_off(g, sel4(x, nu), nu, +1);
   const size_t V = g.V;
   const MD u = Store::template load<double>(U.f[nu], V, site);
   // 12-real links: the transformed link's third row is rebuilt from its first
   // two, which holds for links in SU(3) only
-  if (Store::kBytes == 48 && !(unitarity_defect(u) <= tol))
+  if (Store::kBytes == 48 && !past && !(unitarity_defect(u) <= tol))
     *flag = 1;
-  Store::template store<double>(
-      UA.f[nu], V, site,
-      mul_ad(mul(GS::template load<double>(GA, V, site), u),
-             GS::template load<double>(GA, V, sn)));
-  Store::template store<double>(
-      UB.f[nu], V, site,
-      mul_ad(mul(GS::template load<double>(GB, V, site), u),
-             GS::template load<double>(GB, V, sn)));
+  MD a = mul(GS::template load<double>(GL, V, site), u);
+  MD b = GS::template load<double>(GL, V, site + off);
+  if (past) {
+    const int s = site % g.Vs;
+    a = mul(GS::template load<double>(W, g.Vs, s), a);
+    b = mul(GS::template load<double>(W, g.Vs, s + off), b);
+  }
+  Store::template store<double>(UE.f[nu], VE, esite, mul_ad(a, b));
 }
 
 // First spatial site of a column block. When the block's columns tile the x
@@ -223,22 +226,21 @@ __device__ __forceinline__ int column_base(const Geom &g, int cb, int cols, int 
 }
 
 // Shared memory of one block: per-thread loop sums red[nt][threads] (GAcc),
-// then the space lines of cut A and of cut B, one slot per (t, column unit).
+// then the space lines, one slot per (slice, column unit) over the NE slices.
 // KS > 1: a thread owns KS consecutive start slices t0 = KS row + m, m < KS
-// (all of one cut: KS divides the cut slice h), and one shared-memory load of
+// (KS divides Lt), and one shared-memory load of
 // a top space line S(t) serves the loops of all of them that end on t
 // (T = t - t0 - m): nt + KS - 1 loads for KS nt loops, the sums of the last
 // KS values of T kept in registers. KS = 1: a thread owns the slices
 // row + k rows and loads one line per loop.
-// split = h is the first start slice of cut B: Lt/2, or Lt for a time slab,
-// whose counted starts [0, tstarts) all take cut A. SLAB (the same in the
-// one-column kernels below) compiles in the check that a start is counted;
-// the whole-lattice kernels count every start.
+// SLAB compiles in the check that a start is counted (t0 < tstarts, a time
+// slab). A top line past the last slice belongs to an uncounted loop: its slot
+// is clamped.
 template <class Store, class CT, bool ADJ, int KS, bool SLAB>
 __global__ void __launch_bounds__(256)
-    wilson_gauge_kernel(const __grid_constant__ Geom g, const __grid_constant__ Fields4 UA,
-                        const __grid_constant__ Fields4 UB, int rmin, int rmax, int tmin,
-                        int tmax, int cols, int rows, double *partials, const int *flag, int split, int tstarts) {
+    wilson_gauge_kernel(const __grid_constant__ Geom g, const __grid_constant__ Fields4 U,
+                        int NE, int rmin, int rmax, int tmin, int tmax, int cols, int rows,
+                        double *partials, const int *flag, int tstarts) {
   // the exact product runs instead when a temporal link failed the check
   if (flag && *flag != 0)
     return;
@@ -247,16 +249,15 @@ __global__ void __launch_bounds__(256)
   using LL = LaneLoad<Store, CT, LANES>;
   using M = typename LL::M;
   using CS = ColSet<M>;
-  const int Lt = g.L[3], h = split; // the first slice of cut B
+  const int Lt = g.L[3];
   const int nt = tmax - tmin + 1;
   const int nthreads = blockDim.x;
   const int cs = wilson_col_stride(cols, LANES);
   const int units = cs / LANES;
-  const int nslots = Lt * units;
+  const int nslots = NE * units;
   using Acc = GAcc<ADJ, CT>;
   Acc *red = reinterpret_cast<Acc *>(smem_raw); // [nt][nthreads]
   unsigned char *sa = smem_raw + ((sizeof(Acc) * nt * nthreads + 15) & ~(size_t)15);
-  unsigned char *sb = sa + (size_t)CS::kBytes * nslots;
 
   const int tid = threadIdx.x;
   const int warp = tid >> 5, lane = tid & 31, nwarps = nthreads >> 5;
@@ -270,42 +271,35 @@ __global__ void __launch_bounds__(256)
   const int kt = Lt / rows;
   const int Ln = sel4(g.L, nu), stn = sel4(g.stride, nu);
   const int xn0 = (s0 / stn) % Ln, xn1 = (s1 / stn) % Ln;
-  const size_t V = g.V;
+  const size_t VE = (size_t)NE * g.Vs;
   const int ne = (rmax - rmin + 1) * nt;
   double *part = partials + ((size_t)blockIdx.y * gridDim.x + blockIdx.x) * ne;
 
 #pragma unroll 1
   for (int R = 1; R <= rmax; R++) {
-    // extend the space lines of both cuts by the link at x + (R-1) nu
+    // extend the space lines by the link at x + (R-1) nu: the thread's start
+    // slices, and its share of the slices past the last one
     if (active) {
       const int l0 = s0 + ((xn0 + R - 1) % Ln - xn0) * stn;
       const int l1 = s1 + ((xn1 + R - 1) % Ln - xn1) * stn;
 #pragma unroll 1
-      for (int k = 0; k < kt; k++) {
-        const int t = KS > 1 ? KS * row + k : row + k * rows;
+      for (int k = 0; k < kt + (NE - Lt + rows - 1) / rows; k++) {
+        const int t = k >= kt ? Lt + row + (k - kt) * rows : KS > 1 ? KS * row + k : row + k * rows;
+        if (t >= NE)
+          break;
         const int i = t * units + u;
-        // both cuts' links are loaded before either product needs them
-        const M la = LL::load(UA.f[nu], V, l0 + t * g.Vs, l1 + t * g.Vs);
-        const M lb = LL::load(UB.f[nu], V, l0 + t * g.Vs, l1 + t * g.Vs);
-        if (R == 1) {
-          CS::store(sa, nslots, i, la);
-          CS::store(sb, nslots, i, lb);
-        } else {
-          CS::store(sa, nslots, i, mul(CS::load(sa, nslots, i), la));
-          CS::store(sb, nslots, i, mul(CS::load(sb, nslots, i), lb));
-        }
+        const M la = LL::load(U.f[nu], VE, l0 + t * g.Vs, l1 + t * g.Vs);
+        CS::store(sa, nslots, i, R == 1 ? la : mul(CS::load(sa, nslots, i), la));
       }
     }
     __syncthreads();
     if (R >= rmin && KS > 1) {
       const int t0 = KS * row;
-      const unsigned char *set = (t0 < h) ? sa : sb;
       M a[KS];
 #pragma unroll
       for (int m = 0; m < KS; m++)
-        a[m] = active ? CS::load(set, nslots, (t0 + m) * units + u) : unit(M());
-      int tt = t0 + tmin;
-      tt = (tt >= Lt) ? tt - Lt : tt;
+        a[m] = active ? CS::load(sa, nslots, (t0 + m) * units + u) : unit(M());
+      int tt = min(t0 + tmin, NE - 1);
       Acc acc[KS]; // acc[m]: the sum for T index j - m
 #pragma unroll
       for (int m = 0; m < KS; m++)
@@ -327,22 +321,21 @@ __global__ void __launch_bounds__(256)
         acc[0] = Acc(0);
       };
       // two top lines in flight (b0, b1 alternate): the next line's load is
-      // issued before the current line's traces (a slot past the last step
-      // is still a slot of the column: its load is in bounds and unused;
-      // inactive threads use no line)
+      // issued before the current line's traces (past the last step the
+      // clamped slot's line is unused; inactive threads use no line)
       const int nsteps = nt + KS - 1;
       M b0, b1;
       if (active)
-        b0 = CS::load(set, nslots, tt * units + u);
+        b0 = CS::load(sa, nslots, tt * units + u);
 #pragma unroll 1
       for (int j = 0; j < nsteps; j += 2) {
-        tt = (tt + 1 == Lt) ? 0 : tt + 1;
+        tt = min(tt + 1, NE - 1);
         if (active)
-          b1 = CS::load(set, nslots, tt * units + u);
+          b1 = CS::load(sa, nslots, tt * units + u);
         step(j, b0);
-        tt = (tt + 1 == Lt) ? 0 : tt + 1;
+        tt = min(tt + 1, NE - 1);
         if (active)
-          b0 = CS::load(set, nslots, tt * units + u);
+          b0 = CS::load(sa, nslots, tt * units + u);
         if (j + 1 < nsteps)
           step(j + 1, b1);
       }
@@ -350,18 +343,15 @@ __global__ void __launch_bounds__(256)
 #pragma unroll 1
       for (int k = 0; k < kt; k++) {
         const int t0 = row + k * rows;
-        // the cut this start slice's loops use
-        const unsigned char *set = (t0 < h) ? sa : sb;
-        const M a = active ? CS::load(set, nslots, t0 * units + u) : unit(M());
-        int tt = t0 + tmin;
-        tt = (tt >= Lt) ? tt - Lt : tt;
+        const M a = active ? CS::load(sa, nslots, t0 * units + u) : unit(M());
+        int tt = min(t0 + tmin, NE - 1);
 #pragma unroll 1
         for (int T = 0; T < nt; T++) {
           const Acc v =
-              (active && (!SLAB || t0 < tstarts)) ? gauge_trace<ADJ>(a, CS::load(set, nslots, tt * units + u), lane1) : Acc(0);
+              (active && (!SLAB || t0 < tstarts)) ? gauge_trace<ADJ>(a, CS::load(sa, nslots, tt * units + u), lane1) : Acc(0);
           Acc *r = red + (size_t)T * nthreads + tid;
           *r = (k == 0) ? v : *r + v;
-          tt = (tt + 1 == Lt) ? 0 : tt + 1;
+          tt = min(tt + 1, NE - 1);
         }
       }
     }
@@ -413,36 +403,34 @@ struct Rows01Set {
 };
 
 // The fundamental loops of the mixed SU(3) form with one column per thread
-// and KS consecutive start slices t0 = KS row + m (all of one cut: KS divides
-// the cut slice h) whose space lines stay in registers from one R to the
-// next. The trace sweep reads each top line once for the KS starts, as in
+// and KS consecutive start slices t0 = KS row + m whose space lines stay in
+// registers from one R to the next. The trace sweep reads each top line once for the KS starts, as in
 // wilson_gauge_kernel, but the lines are not lane-packed, so KS = 4 starts
 // fit in the registers: twice the loops per shared-memory byte of the
 // two-column, two-start form. Each R the thread extends its own starts' lines
-// in registers (and stores them for the other threads' sweeps) and the other
-// cut's lines of the same slices in shared memory. Lines are products of
+// in registers (and stores them for the other threads' sweeps) and its share
+// of the lines past slice KS rows - 1 in shared memory. Lines are products of
 // SU(3) links, so they are computed and kept in shared memory as rows 0 and 1
 // (48 bytes a line instead of 72; 72 instead of 108 multiply-adds a product),
 // and row 2 is rebuilt where a trace needs it. Compiled for 16 warps per SM
-// (128 registers, a few spilled): at SU(3) 32^4 that ran 2.45 ms against 2.98
-// ms at 175 registers (8 warps) and 3.01 ms for the two-column kernel.
+// (128 registers, a few spilled): 8 warps at 175 registers took a fifth more.
+// Bound by the FMA pipe's operands and the latency of the sweep (0.6
+// instructions per cycle and scheduler). With one set of Lt + T_max lines
+// instead of two cuts of Lt: 24^3 x 48, T <= 12, 1.42 -> 1.34 ms.
 // Partials, block sums and the per-thread FP32 loop sums as
 // wilson_gauge_kernel.
 template <int KS, bool SLAB>
 __global__ void __launch_bounds__(256, 2)
-    wilson_gauge_reg_kernel(const __grid_constant__ Geom g, const __grid_constant__ Fields4 UA,
-                            const __grid_constant__ Fields4 UB, int rmin, int rmax, int tmin,
-                            int tmax, int cols, int rows, double *partials, const int *flag, int split, int tstarts) {
+    wilson_gauge_reg_kernel(const __grid_constant__ Geom g, const __grid_constant__ Fields4 U,
+                            int NE, int rmin, int rmax, int tmin, int tmax, int cols, int rows,
+                            double *partials, const int *flag, int tstarts) {
   if (flag && *flag != 0)
     return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int Lt = g.L[3], h = split; // the first slice of cut B
   const int nt = tmax - tmin + 1;
   const int nthreads = blockDim.x;
-  const int nslots = Lt * cols;
   float *red = reinterpret_cast<float *>(smem_raw); // [nt][nthreads]
   unsigned char *sa = smem_raw + ((sizeof(float) * nt * nthreads + 15) & ~(size_t)15);
-  unsigned char *sb = sa + (size_t)Rows01Set::kBytes * nslots;
 
   const int tid = threadIdx.x;
   const int warp = tid >> 5, lane = tid & 31, nwarps = nthreads >> 5;
@@ -452,48 +440,44 @@ __global__ void __launch_bounds__(256, 2)
   const int s0 = column_base(g, blockIdx.x, cols, nu) + u;
   const bool active = (row < rows) && (s0 < g.Vs);
   const int t0 = KS * row;
-  // the cut of this thread's starts, and the other one
-  const bool cut_a = t0 < h;
-  unsigned char *own = cut_a ? sa : sb;
-  unsigned char *other = cut_a ? sb : sa;
-  const void *f_own = cut_a ? UA.f[nu] : UB.f[nu];
-  const void *f_other = cut_a ? UB.f[nu] : UA.f[nu];
+  const void *f = U.f[nu];
   const int Ln = sel4(g.L, nu), stn = sel4(g.stride, nu);
   const int xn = (s0 / stn) % Ln;
-  const size_t V = g.V;
+  const size_t VE = (size_t)NE * g.Vs;
   const int ne = (rmax - rmin + 1) * nt;
   double *part = partials + ((size_t)blockIdx.y * gridDim.x + blockIdx.x) * ne;
 
   SU3<float> a[KS];
 #pragma unroll 1
   for (int R = 1; R <= rmax; R++) {
-    // extend both cuts' lines of slices t0 .. t0 + KS - 1 by the link at
-    // x + (R-1) nu
+    // extend the lines by the link at x + (R-1) nu
     if (active) {
       const int l = s0 + ((xn + R - 1) % Ln - xn) * stn;
 #pragma unroll
       for (int m = 0; m < KS; m++) {
         const int t = t0 + m;
-        const int i = t * cols + u;
-        const SU3<float> lo = StoreF32SU3::load<float>(f_own, V, l + t * g.Vs);
-        const SU3<float> lx = StoreF32SU3::load<float>(f_other, V, l + t * g.Vs);
+        if (t >= NE)
+          break;
+        const SU3<float> lo = StoreF32SU3::load<float>(f, VE, l + t * g.Vs);
         if (R == 1) {
           a[m] = lo;
-          Rows01Set::store(other, i, lx);
         } else {
-          // rows 0 and 1 of the products; the own line's row 2 rebuilt for
-          // its traces
+          // rows 0 and 1 of the product; row 2 rebuilt for the traces
           a[m] = mul01(a[m], lo);
           rebuild_row2(a[m]);
-          Rows01Set::store(other, i, mul01(Rows01Set::load(other, i), lx));
         }
-        Rows01Set::store(own, i, a[m]);
+        Rows01Set::store(sa, t * cols + u, a[m]);
+      }
+#pragma unroll 1
+      for (int t = KS * rows + row; t < NE; t += rows) {
+        const int i = t * cols + u;
+        const SU3<float> lx = StoreF32SU3::load<float>(f, VE, l + t * g.Vs);
+        Rows01Set::store(sa, i, R == 1 ? lx : mul01(Rows01Set::load(sa, i), lx));
       }
     }
     __syncthreads();
     if (R >= rmin) {
-      int tt = t0 + tmin;
-      tt = (tt >= Lt) ? tt - Lt : tt;
+      int tt = min(t0 + tmin, NE - 1);
       float acc[KS]; // acc[m]: the sum for T index j - m
 #pragma unroll
       for (int m = 0; m < KS; m++)
@@ -514,22 +498,21 @@ __global__ void __launch_bounds__(256, 2)
           acc[m] = acc[m - 1];
         acc[0] = 0.f;
       };
-      // two top lines in flight (b0, b1 alternate); a slot one past the last
-      // step is still a slot of the column (in bounds, unused)
+      // two top lines in flight (b0, b1 alternate)
       const int nsteps = nt + KS - 1;
       SU3<float> b0, b1;
       if (active)
-        b0 = Rows01Set::load(own, tt * cols + u);
+        b0 = Rows01Set::load(sa, tt * cols + u);
 #pragma unroll 1
       for (int j = 0; j < nsteps; j += 2) {
-        tt = (tt + 1 == Lt) ? 0 : tt + 1;
+        tt = min(tt + 1, NE - 1);
         if (active)
-          b1 = Rows01Set::load(own, tt * cols + u);
+          b1 = Rows01Set::load(sa, tt * cols + u);
         rebuild_row2(b0);
         step(j, b0);
-        tt = (tt + 1 == Lt) ? 0 : tt + 1;
+        tt = min(tt + 1, NE - 1);
         if (active)
-          b0 = Rows01Set::load(own, tt * cols + u);
+          b0 = Rows01Set::load(sa, tt * cols + u);
         if (j + 1 < nsteps) {
           rebuild_row2(b1);
           step(j + 1, b1);
@@ -585,32 +568,26 @@ template <> struct QuatSet<double> {
 };
 
 // The fundamental SU(2) loops with one column per thread and KS consecutive
-// start slices of one cut whose space lines stay in registers (as
-// wilson_gauge_reg_kernel for SU(3)). A quaternion loop is a 4-term dot
-// product, so in the two-column kernel a step of the trace sweep spent more
-// instructions on its shared-memory loads, bounds checks, rolling sums and
-// index updates than on the loops themselves (0.87 instructions per cycle per
-// scheduler, issue-bound). Here the sweep runs over T: each step loads one
-// line into a register window and adds the KS loops of that T, with no checks
-// and no moves. Per-thread sums in the compute type (FP32 for the mixed
-// form), block and grid sums in FP64.
+// start slices whose space lines stay in registers. The sweep runs over T:
+// each step loads one line into a register window and adds the KS loops of
+// that T, with no checks and no moves. Per-thread sums in the compute type
+// (FP32 for the mixed form), block and grid sums in FP64. SLAB: starts are
+// checked (t0 < tstarts: a time slab, or 4 does not divide Lt).
 template <class Store, class CT, int KS, bool SLAB>
 __global__ void __launch_bounds__(256)
-    wilson_gauge_q_kernel(const __grid_constant__ Geom g, const __grid_constant__ Fields4 UA,
-                          const __grid_constant__ Fields4 UB, int rmin, int rmax, int tmin,
-                          int tmax, int cols, int rows, double *partials, const int *flag, int split, int tstarts) {
+    wilson_gauge_q_kernel(const __grid_constant__ Geom g, const __grid_constant__ Fields4 U,
+                          int NE, int rmin, int rmax, int tmin, int tmax, int cols, int rows,
+                          double *partials, const int *flag, int tstarts) {
   if (flag && *flag != 0)
     return;
   using Q = SU2<CT>;
   using QS = QuatSet<CT>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int Lt = g.L[3], h = split; // the first slice of cut B
   const int nt = tmax - tmin + 1;
   const int nthreads = blockDim.x;
-  const int nslots = Lt * cols;
+  const int nslots = NE * cols;
   CT *red = reinterpret_cast<CT *>(smem_raw); // [nt][nthreads]
   unsigned char *sa = smem_raw + ((sizeof(CT) * nt * nthreads + 15) & ~(size_t)15);
-  unsigned char *sb = sa + (size_t)QS::kBytes * nslots;
 
   const int tid = threadIdx.x;
   const int warp = tid >> 5, lane = tid & 31, nwarps = nthreads >> 5;
@@ -620,14 +597,10 @@ __global__ void __launch_bounds__(256)
   const int s0 = column_base(g, blockIdx.x, cols, nu) + u;
   const bool active = (row < rows) && (s0 < g.Vs);
   const int t0 = KS * row;
-  const bool cut_a = t0 < h;
-  unsigned char *own = cut_a ? sa : sb;
-  unsigned char *other = cut_a ? sb : sa;
-  const void *f_own = cut_a ? UA.f[nu] : UB.f[nu];
-  const void *f_other = cut_a ? UB.f[nu] : UA.f[nu];
+  const void *f = U.f[nu];
   const int Ln = sel4(g.L, nu), stn = sel4(g.stride, nu);
   const int xn = (s0 / stn) % Ln;
-  const size_t V = g.V;
+  const size_t VE = (size_t)NE * g.Vs;
   const int ne = (rmax - rmin + 1) * nt;
   double *part = partials + ((size_t)blockIdx.y * gridDim.x + blockIdx.x) * ne;
 
@@ -639,17 +612,17 @@ __global__ void __launch_bounds__(256)
 #pragma unroll
       for (int m = 0; m < KS; m++) {
         const int t = t0 + m;
+        if (SLAB && t >= NE)
+          break;
+        const Q lo = Store::template load<CT>(f, VE, l + t * g.Vs);
+        a[m] = R == 1 ? lo : mul(a[m], lo);
+        QS::store(sa, nslots, t * cols + u, a[m]);
+      }
+#pragma unroll 1
+      for (int t = KS * rows + row; t < NE; t += rows) {
         const int i = t * cols + u;
-        const Q lo = Store::template load<CT>(f_own, V, l + t * g.Vs);
-        const Q lx = Store::template load<CT>(f_other, V, l + t * g.Vs);
-        if (R == 1) {
-          a[m] = lo;
-          QS::store(other, nslots, i, lx);
-        } else {
-          a[m] = mul(a[m], lo);
-          QS::store(other, nslots, i, mul(QS::load(other, nslots, i), lx));
-        }
-        QS::store(own, nslots, i, a[m]);
+        const Q lx = Store::template load<CT>(f, VE, l + t * g.Vs);
+        QS::store(sa, nslots, i, R == 1 ? lx : mul(QS::load(sa, nslots, i), lx));
       }
     }
     __syncthreads();
@@ -668,20 +641,19 @@ __global__ void __launch_bounds__(256)
           a[m] = Q{CT(0), CT(0), CT(0), CT(0)};
       }
       Q w[W];
-      int tp = t0 + tmin; // slice of the next line to load
-      tp = (tp >= Lt) ? tp - Lt : tp;
+      int tp = min(t0 + tmin, NE - 1); // slice of the next line to load
 #pragma unroll
       for (int m = 0; m < KS; m++) {
-        w[m] = active ? QS::load(own, nslots, tp * cols + u) : a[0];
-        tp = (tp + 1 == Lt) ? 0 : tp + 1;
+        w[m] = active ? QS::load(sa, nslots, tp * cols + u) : a[0];
+        tp = min(tp + 1, NE - 1);
       }
 #pragma unroll 1
       for (int q0 = 0; q0 < nt; q0 += W) {
 #pragma unroll
         for (int r = 0; r < W; r++) {
           if (q0 + r < nt) {
-            w[(r + KS) % W] = active ? QS::load(own, nslots, tp * cols + u) : a[0];
-            tp = (tp + 1 == Lt) ? 0 : tp + 1;
+            w[(r + KS) % W] = active ? QS::load(sa, nslots, tp * cols + u) : a[0];
+            tp = min(tp + 1, NE - 1);
             CT d[KS];
 #pragma unroll
             for (int m = 0; m < KS; m++) {
@@ -737,23 +709,25 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-// The one-column kernel runs the fundamental loops of the mixed SU(3) form
-// when four consecutive start slices share a cut (8 divides Lt).
-bool gauge_reg_applies(int Lt, int nc, int ct_bytes, bool adjoint) {
-  return nc == 3 && ct_bytes == 4 && !adjoint && Lt % 8 == 0 && Lt / 4 <= 64;
+// Which fundamental loops take a one-column kernel (four starts per thread)
+// instead of the Gram matrix, whose tiles of 8 x 8 loops fill better with a
+// long T range (R <= L/2; whole W calls in us, one-column / Gram matrix):
+//   SU(3) mixed  16^4 T <= 8 158 / 163, 24^4 T <= 12 752 / 775, 32^4 T <= 4
+//                1488 / 2074, 32^4 T <= 16 2957 / 2703
+//   SU(2) FP64   20^4 T <= 10 138 / 162, 24^4 T <= 12 293 / 284, 32^4 T <= 16
+//                988 / 816, 48^4 T <= 24 9764 / 5743
+//   SU(2) mixed  48^4 T <= 24 5192 / 5855
+//   SU(3) FP64 has none: its lines of 18 doubles do not fit the registers
+//                (two starts per thread in a two-column kernel: 32^4 T <= 4
+//                3494, T <= 16 5930 against 2145 and 2971)
+// (q kernel: at most 32 threads per column, so that a block of 8 columns fits)
+constexpr int kStarts = 4;
+int start_rows(int Lt) { return (Lt + kStarts - 1) / kStarts; }
+bool gauge_q_applies(int Lt, int tmax, int nc, int ct_bytes) {
+  return nc == 2 && start_rows(Lt) <= 32 && (ct_bytes == 4 || tmax < 12);
 }
-
-// Start slices per thread of the SU(2) one-column kernel. Four in both
-// forms: at SU(2) 48^4 mixed, R,T <= 24, eight starts (122 registers, 15
-// warps per SM) took 5.68 ms against 5.15 ms for four (70 registers), which
-// keep twice the threads per column resident.
-constexpr int gauge_q_starts(int) { return 4; }
-// The SU(2) one-column kernel runs the fundamental loops when a thread's
-// consecutive start slices share a cut (2 x starts divides Lt).
-// (at most 32 threads per column, so that a block of 8 columns fits)
-bool gauge_q_applies(int Lt, int nc, int ct_bytes, bool adjoint) {
-  const int ks = gauge_q_starts(ct_bytes);
-  return nc == 2 && !adjoint && Lt % (2 * ks) == 0 && Lt / ks <= 32;
+bool gauge_reg_applies(int Lt, int tmax, int nc, int ct_bytes) {
+  return nc == 3 && ct_bytes == 4 && start_rows(Lt) <= 64 && tmax < 14;
 }
 
 int largest_divisor_upto_g(int n, int cap) {
@@ -765,43 +739,24 @@ int largest_divisor_upto_g(int n, int cap) {
 
 } // namespace
 
-// Block shape: every start slice of a column has a thread (rows = Lt up to
-// 64; beyond, the largest divisor of Lt up to 64 with Lt/rows slices each),
-// and about 128 threads per block.
-WilsonPlan wilson_gauge_plan(const Geom &g, int nt, int nc, int ct_bytes, int units_req,
-                             bool adjoint) {
+// The fundamental loops: wilson_gram_kernel's shape. The adjoint loops: every
+// start slice of a column has a thread (rows = Lt up to 64; beyond, the largest
+// divisor of Lt up to 64 with Lt/rows slices each), about 128 threads per block.
+WilsonPlan wilson_gauge_plan(const Geom &g, int tmin, int tmax, int nc, int ct_bytes,
+                             int units_req, bool adjoint, int tstarts) {
+  const int Lt = g.L[3], NE = Lt + wilson_gauge_ext(g, tmax, tstarts);
+  if (tstarts <= 0 || tstarts > Lt)
+    tstarts = Lt;
   WilsonPlan p{};
-  const int Lt = g.L[3];
-  const int ncomp = (nc == 3) ? 18 : 4;
-  if (gauge_reg_applies(Lt, nc, ct_bytes, adjoint)) {
-    // the one-column kernel: four starts per thread, columns of Lt/4 threads,
-    // by default the largest power of two of columns with at most 128 threads
-    // per block (SU(3) mixed, R,T <= L/2: 2.45 ms at 32^4 with 16 columns,
-    // 0.59 ms at 24^4 with 16, 1.11 ms at 24^3 x 48 with 8; 2-15% slower
-    // with twice or half the columns, 10-50% with a quarter)
-    p.kernel = 1;
-    p.starts = 4;
-    p.rows = Lt / 4;
-    int units = units_req;
-    if (units <= 0)
-      for (units = 1; 2 * units * p.rows <= 128;)
-        units *= 2;
-    p.cols_per_block = units;
-    p.threads = wilson_threads(units, p.rows, 1);
-    p.blocks = ((g.Vs + units - 1) / units) * 3;
-    p.smem = ((size_t)nt * p.threads * sizeof(float) + 15) / 16 * 16 +
-             2 * (size_t)Rows01Set::kBytes * Lt * units;
-    p.fits = p.threads <= 256 && p.smem <= 200 * 1024;
-    return p;
-  }
-  if (gauge_q_applies(Lt, nc, ct_bytes, adjoint)) {
-    // the SU(2) one-column kernel: four starts per thread, columns of Lt / 4
-    // threads, by default the largest power of two (at least 8) of columns
-    // with at most 192 threads per block (48^4 mixed: 5.15 ms with 16
-    // columns of 12 threads, 5.47 ms with 8)
+  const int nt = tmax - tmin + 1;
+  if (!adjoint && gauge_q_applies(Lt, tmax, nc, ct_bytes)) {
+    // the SU(2) one-column kernel: four starts per thread, by default the
+    // largest power of two (at least 8) of columns with at most 192 threads
+    // per block (48^4 mixed: 5.15 ms with 16 columns of 12 threads, 5.47 ms
+    // with 8)
     p.kernel = 2;
-    p.starts = gauge_q_starts(ct_bytes);
-    p.rows = Lt / p.starts;
+    p.starts = kStarts;
+    p.rows = start_rows(Lt);
     int units = units_req;
     if (units <= 0)
       for (units = 8; 2 * units * p.rows <= 192;)
@@ -810,17 +765,42 @@ WilsonPlan wilson_gauge_plan(const Geom &g, int nt, int nc, int ct_bytes, int un
     p.threads = wilson_threads(units, p.rows, 1);
     p.blocks = ((g.Vs + units - 1) / units) * 3;
     p.smem = ((size_t)nt * p.threads * ct_bytes + 15) / 16 * 16 +
-             2 * (size_t)(ct_bytes == 4 ? 16 : 32) * Lt * units;
+             (size_t)(ct_bytes == 4 ? 16 : 32) * NE * units;
     p.fits = p.threads <= 256 && p.smem <= 200 * 1024;
-    return p;
+    if (p.fits || units_req > 0)
+      return p;
   }
+  if (!adjoint && gauge_reg_applies(Lt, tmax, nc, ct_bytes)) {
+    // the mixed SU(3) one-column kernel: by default the largest power of two
+    // of columns with at most 128 threads per block (of 8, 16 and 32 columns
+    // 2-15% faster than twice or half, 10-50% than a quarter)
+    p.kernel = 3;
+    p.starts = kStarts;
+    p.rows = start_rows(Lt);
+    int units = units_req;
+    if (units <= 0)
+      for (units = 1; 2 * units * p.rows <= 128;)
+        units *= 2;
+    p.cols_per_block = units;
+    p.threads = wilson_threads(units, p.rows, 1);
+    p.blocks = ((g.Vs + units - 1) / units) * 3;
+    p.smem = ((size_t)nt * p.threads * sizeof(float) + 15) / 16 * 16 +
+             (size_t)Rows01Set::kBytes * NE * units;
+    p.fits = p.threads <= 256 && p.smem <= 200 * 1024;
+    if (p.fits || units_req > 0)
+      return p;
+  }
+  if (!adjoint)
+    return wilson_gram_plan(g, tstarts, tmax, nc, units_req, false);
+  p = WilsonPlan{};
+  const int ncomp = (nc == 3) ? 18 : 4;
   const int lanes = wilson_lanes(nc, ct_bytes);
-  // consecutive start slices per thread (a divisor of the cut slice h = Lt/2,
-  // so that a thread's starts share a cut): 2 for SU(3) (its registers hold
-  // two lane-packed matrices), 4 for SU(2) (quaternions are small)
+  // consecutive start slices per thread (a divisor of Lt): 2 for SU(3) (its
+  // registers hold two lane-packed matrices), 4 for SU(2) (quaternions are
+  // small)
   p.starts = 1;
   for (int ks : {nc == 2 ? 4 : 2, 2})
-    if (p.starts == 1 && Lt % (2 * ks) == 0 && Lt / ks <= 64)
+    if (p.starts == 1 && Lt % ks == 0 && Lt / ks <= 64)
       p.starts = ks;
   p.rows = p.starts > 1 ? Lt / p.starts : largest_divisor_upto_g(Lt, 64);
   // (about 128 threads: at SU(3) 32^4 the paired kernel took 5.5, 4.6, 3.8,
@@ -830,138 +810,135 @@ WilsonPlan wilson_gauge_plan(const Geom &g, int nt, int nc, int ct_bytes, int un
   p.cols_per_block = units * lanes;
   p.threads = wilson_threads(p.cols_per_block, p.rows, lanes);
   p.blocks = ((g.Vs + p.cols_per_block - 1) / p.cols_per_block) * 3;
-  const size_t sets = 2 * (size_t)ncomp * Lt * wilson_col_stride(p.cols_per_block, lanes) *
-                      ct_bytes;
-  // (the per-thread sums: GAcc, FP32 for the mixed form's fundamental loops)
-  const size_t acc = (!adjoint && ct_bytes == 4) ? 4 : 8;
-  p.smem = ((size_t)nt * p.threads * acc + 15) / 16 * 16 + sets;
+  p.smem = ((size_t)nt * p.threads * sizeof(double) + 15) / 16 * 16 +
+           (size_t)ncomp * NE * wilson_col_stride(p.cols_per_block, lanes) * ct_bytes;
   p.fits = p.threads <= 256 && p.smem <= 200 * 1024;
   return p;
 }
 
-bool wilson_gauge_applies(const Geom &g, int tmax, int nt, int nc, int ct_bytes, int tstarts) {
+int wilson_gauge_ext(const Geom &g, int tmax, int tstarts) {
+  return tstarts > 0 && tstarts < g.L[3] ? 0 : tmax;
+}
+
+bool wilson_gauge_applies(const Geom &g, int tmin, int tmax, int nc, int ct_bytes, bool adjoint,
+                          int tstarts) {
   const int Lt = g.L[3];
   const bool slab = tstarts > 0 && tstarts < Lt;
-  if (Lt < 2 || tmax > (slab ? Lt - tstarts : Lt / 2))
-    return false;
-  // (the fundamental and the adjoint loops may take different kernels)
-  return wilson_gauge_plan(g, nt, nc, ct_bytes, 0, true).fits &&
-         wilson_gauge_plan(g, nt, nc, ct_bytes, 0, false).fits;
+  return Lt >= 2 && tmax <= (slab ? Lt - tstarts : Lt / 2) &&
+         wilson_gauge_plan(g, tmin, tmax, nc, ct_bytes, 0, adjoint, tstarts).fits;
 }
 
 double wilson_gauge_tolerance(int ct_bytes) { return ct_bytes == 8 ? 1e-14 : 1e-6; }
 
-size_t wilson_gauge_line_bytes(const Geom &g, int nc) {
-  return ((size_t)(nc == 3 ? 144 : 32) * (size_t)g.V + 255) / 256 * 256;
+namespace {
+size_t align256(size_t n) { return (n + 255) / 256 * 256; }
+} // namespace
+
+size_t wilson_gauge_bytes(const Geom &g, int nc, int link_bytes, int ext) {
+  const size_t line = nc == 3 ? 144 : 32;
+  return align256(line * g.V) + align256(line * g.Vs) +
+         3 * align256((size_t)link_bytes * (g.L[3] + ext) * g.Vs);
+}
+
+GaugeLinks wilson_gauge_links(void *base, const Geom &g, int nc, int link_bytes, int ext) {
+  GaugeLinks l{};
+  const size_t line = nc == 3 ? 144 : 32;
+  char *p = static_cast<char *>(base);
+  l.G = p;
+  p += align256(line * g.V);
+  l.W = p;
+  p += align256(line * g.Vs);
+  l.NE = g.L[3] + ext;
+  for (int d = 0; d < 3; d++) {
+    l.U.f[d] = p;
+    p += align256((size_t)link_bytes * l.NE * g.Vs);
+  }
+  l.U.f[3] = nullptr;
+  return l;
 }
 
 template <class Store, class CT>
-int launch_wilson_gauge_prep(const Geom &g, const Fields4 &U, void *GA, void *GB,
-                             const Fields4 &UA, const Fields4 &UB, int *flag,
+int launch_wilson_gauge_prep(const Geom &g, const Fields4 &U, const GaugeLinks &l, int *flag,
                              cudaStream_t s) {
   cudaError_t e = cudaMemsetAsync(flag, 0, sizeof(int), s);
   if (e != cudaSuccess)
     return launch_check("gauge flag reset");
-  // (the two cuts' lines in separate blocks: blockIdx.y = 0 for cut A and
-  // the defect check, 1 for cut B)
-  gauge_lines_kernel<Store><<<dim3((g.Vs + 127) / 128, 2), 128, 0, s>>>(
-      g, U.f[3], GA, GB, g.L[3] / 2, wilson_gauge_tolerance((int)sizeof(CT)), flag);
+  const double tol = wilson_gauge_tolerance((int)sizeof(CT));
+  gauge_lines_kernel<Store><<<(g.Vs + kLinesBlock - 1) / kLinesBlock, kLinesBlock, 0, s>>>(
+      g, U.f[3], l.G, l.W, tol, flag);
   int rc = launch_check("gauge_lines_kernel");
   if (rc)
     return rc;
-  gauge_transform_kernel<Store><<<dim3((g.V + 127) / 128, 3), 128, 0, s>>>(
-      g, U, GA, GB, UA, UB, wilson_gauge_tolerance((int)sizeof(CT)), flag);
+  gauge_transform_kernel<Store><<<dim3((l.NE * g.Vs + 127) / 128, 3), 128, 0, s>>>(
+      g, U, l.G, l.W, l.U, l.NE, tol, flag);
   return launch_check("gauge_transform_kernel");
 }
 
 template <class Store, class CT>
-int launch_wilson_gauge_kernel(const Geom &g, const Fields4 &UA, const Fields4 &UB, int rmin,
-                               int rmax, int tmin, int tmax, bool adjoint, const int *flag,
-                               double *partials, int *blocks, cudaStream_t s, int units = 0,
-                               int tstarts = 0) {
+int launch_wilson_gauge_kernel(const Geom &g, const GaugeLinks &l, int rmin, int rmax, int tmin,
+                               int tmax, bool adjoint, const int *flag, double *partials,
+                               int *blocks, cudaStream_t s, int units = 0, int tstarts = 0) {
   const int nr = rmax - rmin + 1, nt = tmax - tmin + 1;
-  // every start slice in two cuts (A at slice 0, B at Lt/2), or the start
-  // slices [0, tstarts) of a time slab in cut A alone
+  // every start slice (on tmax further slices), or the start slices
+  // [0, tstarts) of a time slab
   const int Lt = g.L[3];
   const bool slab = tstarts > 0 && tstarts < Lt;
-  const int split = slab ? Lt : Lt / 2;
   if (!slab)
     tstarts = Lt;
   if (tmax > (slab ? Lt - tstarts : Lt / 2))
     return plan_error(slab ? "wilson_gauge_kernel: time_max above Lt - t_starts"
                            : "wilson_gauge_kernel: time_max above Lt/2");
-  const WilsonPlan p = wilson_gauge_plan(g, nt, Store::NC, (int)sizeof(CT), units, adjoint);
+  if (nr * nt > kWilsonMaxEntries)
+    return plan_error("wilson_gauge_kernel: too many (R,T) entries");
+  const WilsonPlan p =
+      wilson_gauge_plan(g, tmin, tmax, Store::NC, (int)sizeof(CT), units, adjoint, tstarts);
+  if (!adjoint && p.kernel == 1)
+    return launch_wilson_gram<Store, CT>(g, l, nullptr, rmin, rmax, tmin, tmax, flag, partials,
+                                         blocks, s, units, tstarts);
+  if (!p.fits || l.NE < tstarts + tmax)
+    return plan_error("wilson_gauge_kernel: block shape does not fit");
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   cudaStreamIsCapturing(s, &cap);
   const bool capturing = cap != cudaStreamCaptureStatusNone;
-  if (!p.fits || nr * nt > kWilsonMaxEntries)
-    return plan_error("wilson_gauge_kernel: block shape does not fit");
-  auto go = [&](auto kernel) {
+  auto go = [&](auto k_all, auto k_slab) {
+    // (the start-slice checks of a t-slab compiled in only where they are used)
+    auto kernel = slab ? k_slab : k_all;
     int r = allow_large_smem(kernel, p.smem, capturing);
     if (r)
       return r;
     kernel<<<dim3(p.blocks / 3, 3), p.threads, p.smem, s>>>(
-        g, UA, UB, rmin, rmax, tmin, tmax, p.cols_per_block, p.rows, partials, flag, split,
-        tstarts);
+        g, l.U, l.NE, rmin, rmax, tmin, tmax, p.cols_per_block, p.rows, partials, flag, tstarts);
     return GC_OK;
   };
-  int rc;
-  // (four starts per thread for SU(2), and in the one-column kernel for the
-  // mixed SU(3) form's fundamental loops, as the plan chooses)
-  constexpr int K4 = Store::NC == 2 ? 4 : 2;
   if constexpr (Store::NC == 2) {
     if (p.kernel == 2) {
-      constexpr int KS = gauge_q_starts((int)sizeof(CT));
-      rc = slab ? go(wilson_gauge_q_kernel<Store, CT, KS, true>)
-                : go(wilson_gauge_q_kernel<Store, CT, KS, false>);
-      if (rc)
-        return rc;
+      auto k_all = wilson_gauge_q_kernel<Store, CT, kStarts, false>;
+      auto k_some = wilson_gauge_q_kernel<Store, CT, kStarts, true>;
+      const int rc = go(Lt % kStarts ? k_some : k_all, k_some);
       *blocks = p.blocks;
-      return launch_check("wilson_gauge_q_kernel");
+      return rc ? rc : launch_check("wilson_gauge_q_kernel");
     }
   }
   if constexpr (std::is_same<Store, StoreF32SU3>::value) {
-    if (p.kernel == 1) {
-      rc = slab ? go(wilson_gauge_reg_kernel<4, true>) : go(wilson_gauge_reg_kernel<4, false>);
-      if (rc)
-        return rc;
+    if (p.kernel == 3) {
+      auto k_all = wilson_gauge_reg_kernel<kStarts, false>;
+      auto k_some = wilson_gauge_reg_kernel<kStarts, true>;
+      const int rc = go(Lt % kStarts ? k_some : k_all, k_some);
       *blocks = p.blocks;
-      return launch_check("wilson_gauge_reg_kernel");
+      return rc ? rc : launch_check("wilson_gauge_reg_kernel");
     }
   }
-  // (the start-slice checks of a t-slab compiled in only where they are used)
-  auto go2 = [&](auto k_all, auto k_slab) { return slab ? go(k_slab) : go(k_all); };
-  if (adjoint)
-    rc = p.starts == 4   ? go2(wilson_gauge_kernel<Store, CT, true, K4, false>,
-                               wilson_gauge_kernel<Store, CT, true, K4, true>)
-         : p.starts == 2 ? go2(wilson_gauge_kernel<Store, CT, true, 2, false>,
-                               wilson_gauge_kernel<Store, CT, true, 2, true>)
-                         : go2(wilson_gauge_kernel<Store, CT, true, 1, false>,
-                               wilson_gauge_kernel<Store, CT, true, 1, true>);
-  else
-    rc = p.starts == 4   ? go2(wilson_gauge_kernel<Store, CT, false, K4, false>,
-                               wilson_gauge_kernel<Store, CT, false, K4, true>)
-         : p.starts == 2 ? go2(wilson_gauge_kernel<Store, CT, false, 2, false>,
-                               wilson_gauge_kernel<Store, CT, false, 2, true>)
-                         : go2(wilson_gauge_kernel<Store, CT, false, 1, false>,
-                               wilson_gauge_kernel<Store, CT, false, 1, true>);
+  constexpr int K4 = Store::NC == 2 ? 4 : 2;
+  const int rc = p.starts == 4   ? go(wilson_gauge_kernel<Store, CT, true, K4, false>,
+                                      wilson_gauge_kernel<Store, CT, true, K4, true>)
+                 : p.starts == 2 ? go(wilson_gauge_kernel<Store, CT, true, 2, false>,
+                                      wilson_gauge_kernel<Store, CT, true, 2, true>)
+                                 : go(wilson_gauge_kernel<Store, CT, true, 1, false>,
+                                      wilson_gauge_kernel<Store, CT, true, 1, true>);
   if (rc)
     return rc;
   *blocks = p.blocks;
   return launch_check("wilson_gauge_kernel");
-}
-
-template <class Store, class CT>
-int launch_wilson_gauge(const Geom &g, const Fields4 &UA, const Fields4 &UB, int rmin,
-                        int rmax, int tmin, int tmax, bool adjoint, double *partials,
-                        double *out_dev, cudaStream_t s) {
-  int blocks = 0;
-  const int rc = launch_wilson_gauge_kernel<Store, CT>(g, UA, UB, rmin, rmax, tmin, tmax,
-                                                       adjoint, nullptr, partials, &blocks, s);
-  if (rc)
-    return rc;
-  return launch_reduce_wilson(partials, blocks, rmax - rmin + 1, tmax - tmin + 1,
-                              wilson_scale(g.V, Store::NC, adjoint), out_dev, s);
 }
 
 int launch_reduce_select(const double *partials, int blocks_exact, int blocks_gauge,
@@ -973,10 +950,9 @@ int launch_reduce_select(const double *partials, int blocks_exact, int blocks_ga
 }
 
 template <class Store, class CT>
-int launch_wilson_auto(const Geom &g, const Fields4 &U, const Fields4 &UA, const Fields4 &UB,
-                       int rmin, int rmax, int tmin, int tmax, bool adjoint, const int *flag,
-                       double *partials, double *out_dev, cudaStream_t s, int units,
-                       int tstarts) {
+int launch_wilson_auto(const Geom &g, const Fields4 &U, const GaugeLinks &l, int rmin, int rmax,
+                       int tmin, int tmax, bool adjoint, const int *flag, double *partials,
+                       double *out_dev, cudaStream_t s, int units, int tstarts) {
   if (tstarts <= 0 || tstarts > g.L[3])
     tstarts = g.L[3];
   int b_exact = 0, b_gauge = 0;
@@ -984,7 +960,7 @@ int launch_wilson_auto(const Geom &g, const Fields4 &U, const Fields4 &UA, const
                                                 partials, &b_exact, s, tstarts);
   if (rc)
     return rc;
-  rc = launch_wilson_gauge_kernel<Store, CT>(g, UA, UB, rmin, rmax, tmin, tmax, adjoint, flag,
+  rc = launch_wilson_gauge_kernel<Store, CT>(g, l, rmin, rmax, tmin, tmax, adjoint, flag,
                                              partials, &b_gauge, s, units, tstarts);
   if (rc)
     return rc;
@@ -995,11 +971,14 @@ int launch_wilson_auto(const Geom &g, const Fields4 &U, const Fields4 &UA, const
                               out_dev, s);
 }
 
-size_t wilson_auto_partials_count(const Geom &g, int nr, int nt, int nc, int units) {
+size_t wilson_auto_partials_count(const Geom &g, int nr, int tmin, int tmax, int nc, int units,
+                                  int tstarts) {
   int blocks = 0;
   for (int ct : {4, 8})
     for (bool adj : {false, true})
-      blocks = std::max(blocks, wilson_gauge_plan(g, nt, nc, ct, units, adj).blocks);
+      blocks = std::max(blocks,
+                        wilson_gauge_plan(g, tmin, tmax, nc, ct, units, adj, tstarts).blocks);
+  const int nt = tmax - tmin + 1;
   return std::max<size_t>(wilson_partials_count(g, nr, nt, nc), (size_t)blocks * nr * nt);
 }
 
@@ -1007,24 +986,22 @@ size_t wilson_auto_partials_count(const Geom &g, int nr, int nt, int nc, int uni
 // units per block (the autotuner's candidate), from prepared transformed
 // links; partials must hold wilson_auto_partials_count(.., units) doubles.
 template <class Store, class CT>
-int time_wilson_gauge(const Geom &g, const Fields4 &UA, const Fields4 &UB, int rmin, int rmax,
-                      int tmin, int tmax, int units, double *partials, cudaStream_t s,
-                      float *ms) {
-  const WilsonPlan p =
-      wilson_gauge_plan(g, tmax - tmin + 1, Store::NC, (int)sizeof(CT), units, false);
+int time_wilson_gauge(const Geom &g, const GaugeLinks &l, int rmin, int rmax, int tmin, int tmax,
+                      int units, double *partials, cudaStream_t s, float *ms) {
+  const WilsonPlan p = wilson_gauge_plan(g, tmin, tmax, Store::NC, (int)sizeof(CT), units);
   if (!p.fits)
     return GC_ERR_ARG;
   int blocks = 0;
-  int rc = launch_wilson_gauge_kernel<Store, CT>(g, UA, UB, rmin, rmax, tmin, tmax, false,
-                                                 nullptr, partials, &blocks, s, units);
+  int rc = launch_wilson_gauge_kernel<Store, CT>(g, l, rmin, rmax, tmin, tmax, false, nullptr,
+                                                 partials, &blocks, s, units);
   cudaEvent_t e0, e1;
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);
   float best = 1e30f;
   for (int rep = 0; rep < 3 && rc == GC_OK; rep++) {
     cudaEventRecord(e0, s);
-    rc = launch_wilson_gauge_kernel<Store, CT>(g, UA, UB, rmin, rmax, tmin, tmax, false,
-                                               nullptr, partials, &blocks, s, units);
+    rc = launch_wilson_gauge_kernel<Store, CT>(g, l, rmin, rmax, tmin, tmax, false, nullptr,
+                                               partials, &blocks, s, units);
     cudaEventRecord(e1, s);
     cudaEventSynchronize(e1);
     float t = 0;
@@ -1037,20 +1014,15 @@ int time_wilson_gauge(const Geom &g, const Fields4 &UA, const Fields4 &UB, int r
   return rc;
 }
 
-#define GC_INSTANTIATE_WG(STORE, CT)                                                        \
-  template int launch_wilson_gauge_prep<STORE, CT>(const Geom &, const Fields4 &, void *,   \
-                                                   void *, const Fields4 &, const Fields4 &, \
-                                                   int *, cudaStream_t);                    \
-  template int launch_wilson_gauge<STORE, CT>(const Geom &, const Fields4 &, const Fields4 &, \
-                                              int, int, int, int, bool, double *, double *,  \
-                                              cudaStream_t);                                 \
-  template int launch_wilson_auto<STORE, CT>(const Geom &, const Fields4 &, const Fields4 &,  \
-                                             const Fields4 &, int, int, int, int, bool,       \
-                                             const int *, double *, double *, cudaStream_t,   \
-                                             int, int);                                       \
-  template int time_wilson_gauge<STORE, CT>(const Geom &, const Fields4 &, const Fields4 &,   \
-                                            int, int, int, int, int, double *, cudaStream_t,  \
-                                            float *);
+#define GC_INSTANTIATE_WG(STORE, CT)                                                         \
+  template int launch_wilson_gauge_prep<STORE, CT>(const Geom &, const Fields4 &,            \
+                                                   const GaugeLinks &, int *, cudaStream_t); \
+  template int launch_wilson_auto<STORE, CT>(const Geom &, const Fields4 &,                  \
+                                             const GaugeLinks &, int, int, int, int, bool,   \
+                                             const int *, double *, double *, cudaStream_t,  \
+                                             int, int);                                      \
+  template int time_wilson_gauge<STORE, CT>(const Geom &, const GaugeLinks &, int, int, int, \
+                                            int, int, double *, cudaStream_t, float *);
 
 GC_INSTANTIATE_WG(StoreF64SU3, double)
 GC_INSTANTIATE_WG(StoreF64SU2, double)

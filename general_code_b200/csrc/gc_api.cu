@@ -708,9 +708,12 @@ int gc_hyp(gc_lattice *h, double a1, double a2, double a3, int steps) {
 // check of the links into *flag, a word of h->flag_dev. *use is cleared when
 // the scratch cannot hold them, or, with `optional`, when it cannot be
 // allocated (the caller has a form that does without it).
-enum { kFlagOnaxis = 0, kFlagOther = 1 }; // words of h->flag_dev
+enum { kFlagOnaxis = 0, kFlagOffaxis = 1 }; // words of h->flag_dev
+// second: a second configuration's links, whose spatial links go into
+// second_links in the same gauge.
 static int gauge_prepare(gc_lattice *h, int ext, GaugeLinks *links, bool *use, int **flag,
-                         int word = kFlagOnaxis, bool optional = false) {
+                         int word = kFlagOnaxis, bool optional = false,
+                         const Fields4 *second = nullptr, Fields4 *second_links = nullptr) {
   int rc = ensure_hyp(h);
   if (rc == GC_ERR_NOMEM && optional) {
     cudaGetLastError(); // (the failed allocation is not the next launch's error)
@@ -727,13 +730,22 @@ static int gauge_prepare(gc_lattice *h, int ext, GaugeLinks *links, bool *use, i
     }
   }
   const int link_bytes = (int)bytes_per_link(h->nc, h->prec);
-  if (wilson_gauge_bytes(h->g, h->nc, link_bytes, ext) > 15 * hyp_field_bytes(h)) {
+  const size_t main_bytes = wilson_gauge_bytes(h->g, h->nc, link_bytes, ext);
+  const size_t field = ((size_t)link_bytes * (h->g.L[3] + ext) * h->g.Vs + 255) / 256 * 256;
+  if (main_bytes + (second ? 3 * field : 0) > 15 * hyp_field_bytes(h)) {
     *use = false;
     return GC_OK;
   }
   *flag = h->flag_dev + word;
   *links = wilson_gauge_links(h->hyp, h->g, h->nc, link_bytes, ext);
   rc = GC_DISPATCH(h, launch_wilson_gauge_prep, h->g, h->cur, *links, *flag, h->stream);
+  if (!rc && second) {
+    for (int d = 0; d < 3; d++)
+      second_links->f[d] = (char *)h->hyp + main_bytes + d * field;
+    second_links->f[3] = nullptr;
+    rc = GC_DISPATCH(h, launch_wilson_gauge_second, h->g, *second, *links, *second_links, *flag,
+                     h->stream);
+  }
   if (rc)
     return launch_fail(h, rc);
   return GC_OK;
@@ -800,24 +812,43 @@ static int wilson_impl(gc_lattice *h, int rmin, int rmax, int tmin, int tmax,
     return rc;
   double *chunk_out = h->dev_out + (size_t)nr * nt;
   // The temporal-gauge form (gc_wilson_gauge.cu) for one configuration's
-  // on-axis or adjoint loops with T <= Lt/2, or, for the t-slab entry's start
-  // slices [0, t_starts), with T <= Lt - t_starts (no counted loop passes the
-  // slab lattice's last slice); it runs only where
-  // the device finds the temporal links unitary to the form's tolerance, and
-  // the exact recursion otherwise.
+  // on-axis or adjoint loops and the fundamental GEVP loops with T <= Lt/2, or,
+  // for the t-slab entry's start slices [0, t_starts), with T <= Lt - t_starts
+  // (no counted loop passes the slab lattice's last slice); it runs only where
+  // the device finds the links unitary to the form's tolerance, and the exact
+  // recursion otherwise. (GEVP: both configurations' links in the gauge of the
+  // first, from which the time lines are taken.)
   const int ct_bytes = h->prec == GC_PREC_FP64 ? 8 : 4;
-  bool gauge = h->wilson_method == GC_WILSON_AUTO && !second &&
+  bool gauge = h->wilson_method == GC_WILSON_AUTO && !(second && adjoint) &&
                wilson_gauge_applies(h->g, tmin, tmax, h->nc, ct_bytes, adjoint, tstarts);
+  WilsonPlan gevp_plan{};
+  if (gauge && second) {
+    // preparing the gauge costs what the exact walk of a few loops does: whole
+    // calls in us, exact / gauge, SU(3) FP64 16^4 R <= 4, T <= 2 159 / 176 and
+    // T <= 4 221 / 179, 24^4 R,T <= 6 1992 / 880; mixed 24^4 R,T <= 4 555 / 630
+    // and 6 1089 / 854; SU(2) FP64 16^4 R,T <= 4 86 / 102, mixed 16^4 R,T <= 6
+    // 109 / 105
+    const int loops = nr * tmax;
+    gauge = loops >= (h->nc == 3 && ct_bytes == 8 ? 12 : 25);
+  }
+  if (gauge && second) {
+    gevp_plan = wilson_gram_plan(h->g, h->g.L[3], tmax, h->nc, 0, true);
+    gauge = gevp_plan.fits;
+  }
   GaugeLinks links{};
+  Fields4 second_links{};
   int *flag = nullptr;
   if (gauge) {
-    rc = gauge_prepare(h, wilson_gauge_ext(h->g, tmax, tstarts), &links, &gauge, &flag);
+    rc = gauge_prepare(h, wilson_gauge_ext(h->g, tmax, tstarts), &links, &gauge, &flag,
+                       kFlagOnaxis, second != nullptr, u2, &second_links);
     if (rc)
       return rc;
   }
   if (gauge) {
-    rc = ensure_partials(h, wilson_auto_partials_count(h->g, std::min(rchunk, nr), tmin, tmax, h->nc, 0,
-                                                       tstarts));
+    const int ncr = std::min(rchunk, nr);
+    rc = ensure_partials(h, second ? (size_t)gevp_plan.blocks * ncr * nt
+                                   : wilson_auto_partials_count(h->g, ncr, tmin, tmax, h->nc, 0,
+                                                                tstarts));
     if (rc)
       return rc;
   }
@@ -828,7 +859,8 @@ static int wilson_impl(gc_lattice *h, int rmin, int rmax, int tmin, int tmax,
     const int ncr = r1 - r0 + 1;
     if (gauge)
       rc = GC_DISPATCH(h, launch_wilson_auto, h->g, h->cur, links, r0, r1, tmin, tmax,
-                       adjoint, flag, h->partials, chunk_out, h->stream, 0, tstarts);
+                       adjoint, flag, h->partials, chunk_out, h->stream, 0, tstarts, u2,
+                       second ? &second_links : nullptr);
     else
       rc = GC_DISPATCH(h, launch_wilson, h->g, h->cur, r0, r1, tmin, tmax,
                        h->partials, chunk_out, h->stream, adjoint, u2, tstarts);
@@ -1032,7 +1064,7 @@ static int offaxis_impl(gc_lattice *h, const std::vector<std::array<int, 3>> &di
   GaugeLinks links{};
   int *flag = nullptr;
   if (gauge) {
-    rc = gauge_prepare(h, tmax, &links, &gauge, &flag, kFlagOther, true);
+    rc = gauge_prepare(h, tmax, &links, &gauge, &flag, kFlagOffaxis, true);
     if (rc)
       return rc;
   }

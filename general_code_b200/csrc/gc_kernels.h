@@ -196,6 +196,12 @@ int launch_wilson_gram(const Geom &g, const GaugeLinks &l, const Fields4 *second
                        int rmax, int tmin, int tmax, const int *flag, double *partials,
                        int *blocks, cudaStream_t s, int cols, int tstarts);
 
+// The spatial links of a second configuration in the gauge of l (its time
+// lines), into out.f[0..2] as l.U; raises *flag as launch_wilson_gauge_prep.
+template <class Store, class CT>
+int launch_wilson_gauge_second(const Geom &g, const Fields4 &U2, const GaugeLinks &l,
+                               const Fields4 &out, int *flag, cudaStream_t s);
+
 // Both methods with the choice made on the device: the exact W kernel runs
 // (and the gauge one returns at once) when *flag != 0, else the other way
 // round; the fixed-order reduction then sums the partials of the method that
@@ -204,11 +210,13 @@ int launch_wilson_gram(const Geom &g, const GaugeLinks &l, const Fields4 *second
 // partials: wilson_auto_partials_count doubles. tstarts in (0, Lt): the
 // loops of the start slices [0, tstarts) only (a time slab's lattice of its
 // own slices and the ones above them); the caller guarantees time_max <=
-// Lt - tstarts (no loop passes the lattice's end).
+// Lt - tstarts (no loop passes the lattice's end). second, second_links: the
+// GEVP loops with a second configuration and its transformed links.
 template <class Store, class CT>
 int launch_wilson_auto(const Geom &g, const Fields4 &U, const GaugeLinks &l, int rmin, int rmax,
                        int tmin, int tmax, bool adjoint, const int *flag, double *partials,
-                       double *out_dev, cudaStream_t s, int units = 0, int tstarts = 0);
+                       double *out_dev, cudaStream_t s, int units = 0, int tstarts = 0,
+                       const Fields4 *second = nullptr, const Fields4 *second_links = nullptr);
 // out_dev[it * nr + ir] = scale * (fixed-order sum of the partials
 // [block][ir * nt + it]) over the blocks of the method that ran (*flag).
 int launch_reduce_select(const double *partials, int blocks_exact, int blocks_gauge,
@@ -220,12 +228,12 @@ template <class Store, class CT>
 int time_wilson_gauge(const Geom &g, const GaugeLinks &l, int rmin, int rmax, int tmin, int tmax,
                       int units, double *partials, cudaStream_t s, float *ms);
 // The exact W kernel, gated on *gate != 0, without the reduction; *blocks
-// receives the number of blocks (rows of partials). tstarts as for
-// launch_wilson_auto (0: every start slice).
+// receives the number of blocks (rows of partials). second: the GEVP loops
+// (fundamental). tstarts as for launch_wilson_auto (0: every start slice).
 template <class Store, class CT>
-int launch_wilson_exact_gated(const Geom &g, const Fields4 &U, int rmin, int rmax, int tmin,
-                              int tmax, bool adjoint, const int *gate, double *partials,
-                              int *blocks, cudaStream_t s, int tstarts = 0);
+int launch_wilson_exact_gated(const Geom &g, const Fields4 &U, const Fields4 *second, int rmin,
+                              int rmax, int tmin, int tmax, bool adjoint, const int *gate,
+                              double *partials, int *blocks, cudaStream_t s, int tstarts = 0);
 
 // An explicit block shape (rows must divide Lt, at most 256 threads).
 WilsonPlan wilson_plan_shape(const Geom &g, int nr, int nt, int nc, int ct_bytes, int rows,

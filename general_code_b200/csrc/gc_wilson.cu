@@ -181,21 +181,28 @@ __device__ __forceinline__ void wilson_block(const Geom &g, const Fields4 &U, co
   }
 }
 
+// gate: the temporal-gauge form's unitarity flag; that launch is the exact
+// fallback and computes nothing when the flag says the gauge form ran. Its
+// blocks then return at once, so it is launched with few of them, each taking
+// several of the `colblocks` x 3 work items (4 / 37 us of empty blocks at
+// 16^4 / 48^4 otherwise).
 template <class Store, class CT, bool ADJ, bool GEVP>
 __global__ void __launch_bounds__(256)
     wilson_kernel(const __grid_constant__ Geom g, const __grid_constant__ Fields4 U,
                   const __grid_constant__ Fields4 U2, int rmin, int rmax, int tmin, int tmax,
-                  int cols, int rows, double *partials, int tstarts,
+                  int cols, int rows, double *partials, int tstarts, int colblocks,
                   const int *gate = nullptr) {
-  // gate: the temporal-gauge form's unitarity flag; this launch is the exact
-  // fallback and computes nothing when the flag says the gauge form ran
   if (gate && *gate == 0)
     return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  const size_t blk = (size_t)blockIdx.y * gridDim.x + blockIdx.x;
   const int ne = (rmax - rmin + 1) * (tmax - tmin + 1);
-  wilson_block<Store, CT, ADJ, GEVP>(g, U, U2, rmin, rmax, tmin, tmax, cols, rows, blockIdx.x,
-                                     blockIdx.y, partials + blk * ne, smem_raw, tstarts);
+  for (int blk = blockIdx.x; blk < 3 * colblocks; blk += gridDim.x) {
+    wilson_block<Store, CT, ADJ, GEVP>(g, U, U2, rmin, rmax, tmin, tmax, cols, rows,
+                                       blk % colblocks, blk / colblocks,
+                                       partials + (size_t)blk * ne, smem_raw, tstarts);
+    if (gate)
+      __syncthreads(); // (the next item reuses the shared memory)
+  }
 }
 
 // Several lattices in one launch. A block finds its lattice by binary search
@@ -406,8 +413,9 @@ int launch_wilson_mode(const Geom &g, const Fields4 &U, const Fields4 &U2, int r
   int rc = allow_large_smem(wilson_kernel<Store, CT, ADJ, GEVP>, p.smem);
   if (rc)
     return rc;
-  wilson_kernel<Store, CT, ADJ, GEVP><<<dim3(p.blocks / 3, 3), p.threads, p.smem, s>>>(
-      g, U, U2, rmin, rmax, tmin, tmax, p.cols_per_block, p.rows, partials, tstarts);
+  wilson_kernel<Store, CT, ADJ, GEVP><<<p.blocks, p.threads, p.smem, s>>>(
+      g, U, U2, rmin, rmax, tmin, tmax, p.cols_per_block, p.rows, partials, tstarts,
+      p.blocks / 3);
   rc = launch_check("wilson_kernel");
   if (rc)
     return rc;
@@ -421,30 +429,31 @@ int launch_wilson_mode(const Geom &g, const Fields4 &U, const Fields4 &U2, int r
 }
 
 template <class Store, class CT>
-int launch_wilson_exact_gated(const Geom &g, const Fields4 &U, int rmin, int rmax, int tmin,
-                              int tmax, bool adjoint, const int *gate, double *partials,
-                              int *blocks, cudaStream_t s, int tstarts) {
+int launch_wilson_exact_gated(const Geom &g, const Fields4 &U, const Fields4 *second, int rmin,
+                              int rmax, int tmin, int tmax, bool adjoint, const int *gate,
+                              double *partials, int *blocks, cudaStream_t s, int tstarts) {
   const int nr = rmax - rmin + 1, nt = tmax - tmin + 1;
   if (tstarts <= 0 || tstarts > g.L[3])
     tstarts = g.L[3];
-  WilsonPlan p = wilson_plan(g, nr, nt, Store::NC, (int)sizeof(CT), 3);
+  WilsonPlan p = wilson_plan(g, nr, nt, Store::NC, (int)sizeof(CT), second ? 4 : 3);
   if (!p.fits || nr * nt > kWilsonMaxEntries)
     return plan_error("wilson_kernel: time extent or (R,T) range too large for "
                       "one block's shared memory");
-  int rc;
-  if (adjoint) {
-    rc = allow_large_smem(wilson_kernel<Store, CT, true, false>, p.smem);
-    if (rc)
-      return rc;
-    wilson_kernel<Store, CT, true, false><<<dim3(p.blocks / 3, 3), p.threads, p.smem, s>>>(
-        g, U, U, rmin, rmax, tmin, tmax, p.cols_per_block, p.rows, partials, tstarts, gate);
-  } else {
-    rc = allow_large_smem(wilson_kernel<Store, CT, false, false>, p.smem);
-    if (rc)
-      return rc;
-    wilson_kernel<Store, CT, false, false><<<dim3(p.blocks / 3, 3), p.threads, p.smem, s>>>(
-        g, U, U, rmin, rmax, tmin, tmax, p.cols_per_block, p.rows, partials, tstarts, gate);
-  }
+  if (second && adjoint)
+    return plan_error("wilson_kernel: no gated adjoint GEVP form");
+  auto go = [&](auto kernel) {
+    const int rc = allow_large_smem(kernel, p.smem);
+    if (!rc)
+      kernel<<<std::min(p.blocks, 4 * 148), p.threads, p.smem, s>>>(
+          g, U, second ? *second : U, rmin, rmax, tmin, tmax, p.cols_per_block, p.rows, partials,
+          tstarts, p.blocks / 3, gate);
+    return rc;
+  };
+  const int rc = second    ? go(wilson_kernel<Store, CT, false, true>)
+                 : adjoint ? go(wilson_kernel<Store, CT, true, false>)
+                           : go(wilson_kernel<Store, CT, false, false>);
+  if (rc)
+    return rc;
   *blocks = p.blocks;
   return launch_check("wilson_kernel");
 }
@@ -507,8 +516,8 @@ int launch_wilson_plan(const Geom &g, const Fields4 &U, int rmin, int rmax, int 
   int rc = allow_large_smem(wilson_kernel<Store, CT, false, false>, p.smem);
   if (rc)
     return rc;
-  wilson_kernel<Store, CT, false, false><<<dim3(p.blocks / 3, 3), p.threads, p.smem, s>>>(
-      g, U, U, rmin, rmax, tmin, tmax, p.cols_per_block, p.rows, partials, g.L[3]);
+  wilson_kernel<Store, CT, false, false><<<p.blocks, p.threads, p.smem, s>>>(
+      g, U, U, rmin, rmax, tmin, tmax, p.cols_per_block, p.rows, partials, g.L[3], p.blocks / 3);
   rc = launch_check("wilson_kernel");
   if (rc)
     return rc;
@@ -588,8 +597,8 @@ int launch_reduce_batch(const RJob *jobs, int njobs, int entries, cudaStream_t s
                                              const WilsonPlan &, double *,    \
                                              double *, cudaStream_t);         \
   template int launch_wilson_exact_gated<STORE, CT>(                          \
-      const Geom &, const Fields4 &, int, int, int, int, bool, const int *,   \
-      double *, int *, cudaStream_t, int);
+      const Geom &, const Fields4 &, const Fields4 *, int, int, int, int,     \
+      bool, const int *, double *, int *, cudaStream_t, int);
 
 GC_INSTANTIATE_W(StoreF64SU3, double)
 GC_INSTANTIATE_W(StoreF64SU2, double)

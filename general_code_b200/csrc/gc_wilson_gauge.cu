@@ -132,37 +132,85 @@ __device__ __forceinline__ typename Store::template M<double> gauge_time_link(
 __device__ __forceinline__ SU3<double> stored_line(const SU3<double> &G) { return polar_step(G); }
 __device__ __forceinline__ SU2<double> stored_line(const SU2<double> &G) { return G; }
 //
-// The chain over t is serial, so the next links are loaded two steps ahead of
-// the product that needs them, and blocks are small: a 16^3 slice has 4096
-// threads.
-constexpr int kLinesBlock = 32;
-template <class Store>
-__global__ void __launch_bounds__(kLinesBlock)
+// The chain over t is serial: the next two links are loaded ahead. Where the
+// columns alone leave most of the chip idle (a 16^3 slice has 4096) a column's
+// slices are split into kLinesSegs segments of warps: each multiplies its own
+// slices' links and keeps the partial lines, the segments' products meet in
+// shared memory, and each then puts the product of the earlier segments in
+// front of its partial lines. Four segments against one: 7.3 / 12.8 us at
+// SU(2) 16^4 FP64, 30.4 / 29.5 at SU(3) 24^4 FP64, 82 / 73 at SU(3) 32^4
+// mixed, so below 8192 columns only.
+constexpr int kLinesCols = 32;
+
+// Records of the line fields, read back by the thread that wrote them (not
+// through the read-only path of the link loads).
+__device__ __forceinline__ SU3<double> line_back(const void *f, size_t V, int site, SU3<double> *) {
+  const double2 *p = reinterpret_cast<const double2 *>(f) + site;
+  SU3<double> m;
+#pragma unroll
+  for (int k = 0; k < 9; k++) {
+    const double2 v = p[k * V];
+    m.e[k / 3][k % 3] = {v.x, v.y};
+  }
+  return m;
+}
+__device__ __forceinline__ SU2<double> line_back(const void *f, size_t V, int site, SU2<double> *) {
+  const double2 *p = reinterpret_cast<const double2 *>(f) + site;
+  const double2 a = p[0], b = p[V];
+  return {a.x, a.y, b.x, b.y};
+}
+
+template <class Store, int kLinesSegs>
+__global__ void __launch_bounds__(kLinesCols *kLinesSegs)
     gauge_lines_kernel(const __grid_constant__ Geom g, const void *Ut, void *GL, void *W,
                        double tol, int *flag) {
   using GS = typename F64Store<Store::NC>::type;
   using MD = typename Store::template M<double>;
-  const int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= g.Vs)
-    return;
+  __shared__ MD total[kLinesSegs][kLinesCols];
+  const int c = threadIdx.x % kLinesCols, seg = threadIdx.x / kLinesCols;
+  const int s = blockIdx.x * kLinesCols + c;
+  const bool active = s < g.Vs;
   const size_t V = g.V;
-  const int Lt = g.L[3];
+  const int Lt = g.L[3], len = (Lt + kLinesSegs - 1) / kLinesSegs;
+  const int t0 = min(Lt, seg * len), t1 = min(Lt, t0 + len);
   double dmax = 0.0;
   MD G = unit(MD());
-  MD u = Store::template load<double>(Ut, V, s);
-  MD next = Store::template load<double>(Ut, V, s + (Lt > 1 ? g.Vs : 0));
+  if (active && t0 < t1) {
+    auto link = [&](int t) {
+      return Store::template load<double>(Ut, V, s + min(t, t1 - 1) * g.Vs);
+    };
+    MD u = link(t0), next = link(t0 + 1);
 #pragma unroll 1
-  for (int t = 0; t < Lt; t++) {
-    const MD after = Store::template load<double>(Ut, V, s + min(t + 2, Lt - 1) * g.Vs);
-    GS::template store<double>(GL, V, s + t * g.Vs, stored_line(G));
-    dmax = fmax(dmax, unitarity_defect(u));
-    G = mul(G, gauge_time_link<Store>(u));
-    u = next;
-    next = after;
+    for (int t = t0; t < t1; t++) {
+      const MD after = link(t + 2);
+      GS::template store<double>(GL, V, s + t * g.Vs, seg ? G : stored_line(G));
+      dmax = fmax(dmax, unitarity_defect(u));
+      G = mul(G, gauge_time_link<Store>(u));
+      u = next;
+      next = after;
+    }
   }
-  GS::template store<double>(W, g.Vs, s, stored_line(G));
+  total[seg][c] = G;
+  __syncthreads();
+  if (!active)
+    return;
   if (!(dmax <= tol)) // (a NaN link counts as not unitary)
     *flag = 1;
+  if (kLinesSegs == 1)
+    GS::template store<double>(W, g.Vs, s, stored_line(G));
+  if (seg == 0)
+    return;
+  MD before = total[0][c];
+#pragma unroll 1
+  for (int q = 1; q < seg; q++)
+    before = mul(before, total[q][c]);
+#pragma unroll 2
+  for (int t = t0; t < t1; t++)
+    GS::template store<double>(
+        GL, V, s + t * g.Vs,
+        stored_line(mul(before, line_back(GL, V, s + t * g.Vs, (MD *)nullptr))));
+  if (seg == kLinesSegs - 1)
+    GS::template store<double>(W, g.Vs, s, stored_line(mul(before, G)));
 }
 
 // U'_nu(s,te) = G(s,te) U_nu(s,te mod Lt) G(s+nu,te)^dag on the slices te of
@@ -864,13 +912,26 @@ int launch_wilson_gauge_prep(const Geom &g, const Fields4 &U, const GaugeLinks &
   if (e != cudaSuccess)
     return launch_check("gauge flag reset");
   const double tol = wilson_gauge_tolerance((int)sizeof(CT));
-  gauge_lines_kernel<Store><<<(g.Vs + kLinesBlock - 1) / kLinesBlock, kLinesBlock, 0, s>>>(
-      g, U.f[3], l.G, l.W, tol, flag);
+  const int line_blocks = (g.Vs + kLinesCols - 1) / kLinesCols;
+  if (g.Vs < 8192)
+    gauge_lines_kernel<Store, 4>
+        <<<line_blocks, 4 * kLinesCols, 0, s>>>(g, U.f[3], l.G, l.W, tol, flag);
+  else
+    gauge_lines_kernel<Store, 1>
+        <<<line_blocks, kLinesCols, 0, s>>>(g, U.f[3], l.G, l.W, tol, flag);
   int rc = launch_check("gauge_lines_kernel");
   if (rc)
     return rc;
   gauge_transform_kernel<Store><<<dim3((l.NE * g.Vs + 127) / 128, 3), 128, 0, s>>>(
       g, U, l.G, l.W, l.U, l.NE, tol, flag);
+  return launch_check("gauge_transform_kernel");
+}
+
+template <class Store, class CT>
+int launch_wilson_gauge_second(const Geom &g, const Fields4 &U2, const GaugeLinks &l,
+                               const Fields4 &out, int *flag, cudaStream_t s) {
+  gauge_transform_kernel<Store><<<dim3((l.NE * g.Vs + 127) / 128, 3), 128, 0, s>>>(
+      g, U2, l.G, l.W, out, l.NE, wilson_gauge_tolerance((int)sizeof(CT)), flag);
   return launch_check("gauge_transform_kernel");
 }
 
@@ -952,22 +1013,27 @@ int launch_reduce_select(const double *partials, int blocks_exact, int blocks_ga
 template <class Store, class CT>
 int launch_wilson_auto(const Geom &g, const Fields4 &U, const GaugeLinks &l, int rmin, int rmax,
                        int tmin, int tmax, bool adjoint, const int *flag, double *partials,
-                       double *out_dev, cudaStream_t s, int units, int tstarts) {
+                       double *out_dev, cudaStream_t s, int units, int tstarts,
+                       const Fields4 *second, const Fields4 *second_links) {
   if (tstarts <= 0 || tstarts > g.L[3])
     tstarts = g.L[3];
   int b_exact = 0, b_gauge = 0;
-  int rc = launch_wilson_exact_gated<Store, CT>(g, U, rmin, rmax, tmin, tmax, adjoint, flag,
-                                                partials, &b_exact, s, tstarts);
+  int rc = launch_wilson_exact_gated<Store, CT>(g, U, second, rmin, rmax, tmin, tmax, adjoint,
+                                                flag, partials, &b_exact, s, tstarts);
   if (rc)
     return rc;
-  rc = launch_wilson_gauge_kernel<Store, CT>(g, l, rmin, rmax, tmin, tmax, adjoint, flag,
-                                             partials, &b_gauge, s, units, tstarts);
+  rc = second ? launch_wilson_gram<Store, CT>(g, l, second_links, rmin, rmax, tmin, tmax, flag,
+                                              partials, &b_gauge, s, units, tstarts)
+              : launch_wilson_gauge_kernel<Store, CT>(g, l, rmin, rmax, tmin, tmax, adjoint, flag,
+                                                      partials, &b_gauge, s, units, tstarts);
   if (rc)
     return rc;
   const int nr = rmax - rmin + 1, nt = tmax - tmin + 1;
-  // average over the loops counted: every site, or the tstarts slices
+  // average over the loops counted: every site, or the tstarts slices (GEVP
+  // counts every loop twice: the / (6 V) of wilson_loops.h:910)
   return launch_reduce_select(partials, b_exact, b_gauge, flag, nr, nt,
-                              wilson_scale((long long)g.Vs * tstarts, Store::NC, adjoint),
+                              wilson_scale((long long)g.Vs * tstarts, Store::NC, adjoint) /
+                                  (second ? 2.0 : 1.0),
                               out_dev, s);
 }
 
@@ -1020,7 +1086,10 @@ int time_wilson_gauge(const Geom &g, const GaugeLinks &l, int rmin, int rmax, in
   template int launch_wilson_auto<STORE, CT>(const Geom &, const Fields4 &,                  \
                                              const GaugeLinks &, int, int, int, int, bool,   \
                                              const int *, double *, double *, cudaStream_t,  \
-                                             int, int);                                      \
+                                             int, int, const Fields4 *, const Fields4 *);    \
+  template int launch_wilson_gauge_second<STORE, CT>(const Geom &, const Fields4 &,          \
+                                                     const GaugeLinks &, const Fields4 &,    \
+                                                     int *, cudaStream_t);                   \
   template int time_wilson_gauge<STORE, CT>(const Geom &, const GaugeLinks &, int, int, int, \
                                             int, int, double *, cudaStream_t, float *);
 

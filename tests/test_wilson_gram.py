@@ -72,3 +72,45 @@ def test_start_slices_of_a_slab(precision, nc, dims, t_starts, rng):
     with _smeared(dims, nc, precision) as lat:
         a, b = _both(lat, *rng, t_starts=t_starts)
         assert np.max(abs(a - b)) <= TOL[precision] * np.max(abs(b))
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("nc,dims,rng", [
+    (3, (4, 3, 5, 8), (1, 7, 1, 4)),
+    (3, (3, 2, 5, 13), (2, 6, 2, 6)),
+    (3, (3, 3, 2, 42), (1, 2, 1, 21)),
+    (2, (5, 4, 3, 10), (1, 5, 1, 5)),
+    (2, (3, 4, 3, 36), (1, 2, 5, 18)),
+    (2, (3, 4, 3, 9), (1, 4, 1, 7)),  # T > Lt/2: the exact product in both
+    (3, (4, 3, 5, 8), (1, 2, 1, 2)),  # few loops: the exact product in both
+])
+def test_two_configurations(precision, nc, dims, rng):
+    with _smeared(dims, nc, precision) as a, Lattice(dims, nc, precision) as b:
+        b.copy_from(a)
+        b.ape(0.5, 3)
+        got = a.wilson_gevp(b, *rng)
+        same = a.wilson_gevp(a, *rng)
+        table = a.wilson_loop(*rng)
+        a.set_wilson_method("exact")
+        want = a.wilson_gevp(b, *rng)
+        top = np.max(abs(want))
+        assert np.max(abs(got - want)) <= TOL[precision] * top
+        assert np.max(abs(same - table)) <= TOL[precision] * top
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_second_configuration_off_the_group(precision):
+    """The second configuration's links need be in SU(3) only where they are
+    stored as 12 reals; the first one's time links always."""
+    dims = (4, 3, 4, 6)
+    links = generate_config(dims, 3, 0.25, 43, 0)
+    bad = links.reshape(-1, 4, 18).copy()
+    bad[11, 2] *= 1.001
+    with Lattice(dims, 3, precision) as a, Lattice(dims, 3, precision) as b:
+        a.upload(links)
+        b.upload(bad.reshape(-1, 18))
+        got = a.wilson_gevp(b, 1, 9, 1, 3)
+        assert a.wilson_method_used() == ("gauge" if precision == "fp64" else "exact")
+        a.set_wilson_method("exact")
+        want = a.wilson_gevp(b, 1, 9, 1, 3)
+        assert np.max(abs(got - want)) <= TOL["fp64"] * np.max(abs(want))

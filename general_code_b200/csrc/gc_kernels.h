@@ -189,18 +189,42 @@ int launch_wilson_gauge_prep(const Geom &g, const Fields4 &U, const GaugeLinks &
 // The fundamental loops by FP64 matrix instructions (gc_wilson_gram.cu), or
 // with `second` (transformed links of a second configuration in the same
 // gauge) the GEVP loops: per-block partials [block][R][T], run when flag is
-// null or *flag == 0. tstarts start slices; cols 0 = the default.
+// null or *flag == 0. tstarts start slices; cols 0 = the default; the first
+// ndir directions.
 WilsonPlan wilson_gram_plan(const Geom &g, int tstarts, int tmax, int nc, int cols, bool gevp);
 template <class Store, class CT>
 int launch_wilson_gram(const Geom &g, const GaugeLinks &l, const Fields4 *second, int rmin,
                        int rmax, int tmin, int tmax, const int *flag, double *partials,
-                       int *blocks, cudaStream_t s, int cols, int tstarts);
+                       int *blocks, cudaStream_t s, int cols, int tstarts, int ndir = 3);
 
 // The spatial links of a second configuration in the gauge of l (its time
 // lines), into out.f[0..2] as l.U; raises *flag as launch_wilson_gauge_prep.
 template <class Store, class CT>
 int launch_wilson_gauge_second(const Geom &g, const Fields4 &U2, const GaugeLinks &l,
                                const Fields4 &out, int *flag, cudaStream_t s);
+
+// Loops whose time axis is a spatial axis mu (the spatial loops): g is the
+// lattice with its axes reordered, the two loop directions and t as the
+// columns' axes and mu as the slowest, and the links keep their own site
+// order, whose strides along g's axes map holds. Fills l (with slices past
+// the last one along mu): the time lines of Ut along mu, then for each pair of
+// direction fields F.f[0..1] the transformed links, then the loops of both
+// directions: out_dev[(T - tmin) nr + (R - rmin)] = scale * their sum. *flag
+// is raised, not reset; launch_axis_loops does nothing when it is.
+struct AxisMap {
+  int stride[4];
+};
+template <class Store, class CT>
+int launch_axis_gauge_lines(const Geom &g, const AxisMap &map, const void *Ut,
+                            const GaugeLinks &l, int *flag, cudaStream_t s);
+template <class Store, class CT>
+int launch_axis_gauge_links(const Geom &g, const AxisMap &map, const Fields4 &F,
+                            const GaugeLinks &l, int *flag, cudaStream_t s);
+size_t axis_loops_partials(const Geom &g, int nr, int tmin, int tmax, int nc, int ct_bytes);
+template <class Store, class CT>
+int launch_axis_loops(const Geom &g, const GaugeLinks &l, int rmin, int rmax, int tmin, int tmax,
+                      const int *flag, double *partials, double scale, double *out_dev,
+                      cudaStream_t s);
 
 // Both methods with the choice made on the device: the exact W kernel runs
 // (and the gauge one returns at once) when *flag != 0, else the other way

@@ -160,10 +160,24 @@ __device__ __forceinline__ SU2<double> line_back(const void *f, size_t V, int si
   return {a.x, a.y, b.x, b.y};
 }
 
-template <class Store, int kLinesSegs>
+//
+// MAPPED: the loops' time axis is a spatial axis of the lattice; g is the
+// lattice with its axes reordered (the columns' three, then the time axis),
+// which the lines and transformed links are stored on, and map gives the
+// strides of the links' own site order.
+template <bool MAPPED>
+__device__ __forceinline__ int own_site(const Geom &g, const AxisMap &map, int site) {
+  if (!MAPPED)
+    return site;
+  int x[4];
+  site_coords(g, site, x);
+  return x[0] * map.stride[0] + x[1] * map.stride[1] + x[2] * map.stride[2] + x[3] * map.stride[3];
+}
+
+template <class Store, int kLinesSegs, bool MAPPED>
 __global__ void __launch_bounds__(kLinesCols *kLinesSegs)
-    gauge_lines_kernel(const __grid_constant__ Geom g, const void *Ut, void *GL, void *W,
-                       double tol, int *flag) {
+    gauge_lines_kernel(const __grid_constant__ Geom g, const __grid_constant__ AxisMap map,
+                       const void *Ut, void *GL, void *W, double tol, int *flag) {
   using GS = typename F64Store<Store::NC>::type;
   using MD = typename Store::template M<double>;
   __shared__ MD total[kLinesSegs][kLinesCols];
@@ -176,8 +190,9 @@ __global__ void __launch_bounds__(kLinesCols *kLinesSegs)
   double dmax = 0.0;
   MD G = unit(MD());
   if (active && t0 < t1) {
+    const int base = own_site<MAPPED>(g, map, s), step = MAPPED ? map.stride[3] : g.Vs;
     auto link = [&](int t) {
-      return Store::template load<double>(Ut, V, s + min(t, t1 - 1) * g.Vs);
+      return Store::template load<double>(Ut, V, base + min(t, t1 - 1) * step);
     };
     MD u = link(t0), next = link(t0 + 1);
 #pragma unroll 1
@@ -216,11 +231,11 @@ __global__ void __launch_bounds__(kLinesCols *kLinesSegs)
 // U'_nu(s,te) = G(s,te) U_nu(s,te mod Lt) G(s+nu,te)^dag on the slices te of
 // the extended lattice (sites [0, NE Vs), plane stride NE Vs); thread per
 // (site, nu).
-template <class Store>
+template <class Store, bool MAPPED>
 __global__ void __launch_bounds__(128)
-    gauge_transform_kernel(const __grid_constant__ Geom g, const __grid_constant__ Fields4 U,
-                           const void *GL, const void *W, const __grid_constant__ Fields4 UE,
-                           int NE, double tol, int *flag) {
+    gauge_transform_kernel(const __grid_constant__ Geom g, const __grid_constant__ AxisMap map,
+                           const __grid_constant__ Fields4 U, const void *GL, const void *W,
+                           const __grid_constant__ Fields4 UE, int NE, double tol, int *flag) {
   using GS = typename F64Store<Store::NC>::type;
   using MD = typename Store::template M<double>;
   const int esite = blockIdx.x * blockDim.x + threadIdx.x;
@@ -234,7 +249,7 @@ __global__ void __launch_bounds__(128)
   site_coords(g, site, x);
   const int off = step_off(g, sel4(x, nu), nu, +1);
   const size_t V = g.V;
-  const MD u = Store::template load<double>(U.f[nu], V, site);
+  const MD u = Store::template load<double>(U.f[nu], V, own_site<MAPPED>(g, map, site));
   // 12-real links: the transformed link's third row is rebuilt from its first
   // two, which holds for links in SU(3) only
   if (Store::kBytes == 48 && !past && !(unitarity_defect(u) <= tol))
@@ -905,40 +920,65 @@ GaugeLinks wilson_gauge_links(void *base, const Geom &g, int nc, int link_bytes,
   return l;
 }
 
+namespace {
+
+template <class Store, class CT, bool MAPPED>
+int launch_gauge_lines(const Geom &g, const AxisMap &map, const void *Ut, const GaugeLinks &l,
+                       int *flag, cudaStream_t s) {
+  const double tol = wilson_gauge_tolerance((int)sizeof(CT));
+  const int blocks = (g.Vs + kLinesCols - 1) / kLinesCols;
+  if (g.Vs < 8192)
+    gauge_lines_kernel<Store, 4, MAPPED>
+        <<<blocks, 4 * kLinesCols, 0, s>>>(g, map, Ut, l.G, l.W, tol, flag);
+  else
+    gauge_lines_kernel<Store, 1, MAPPED>
+        <<<blocks, kLinesCols, 0, s>>>(g, map, Ut, l.G, l.W, tol, flag);
+  return launch_check("gauge_lines_kernel");
+}
+
+template <class Store, class CT, bool MAPPED>
+int launch_gauge_links(const Geom &g, const AxisMap &map, const Fields4 &U, const GaugeLinks &l,
+                       const Fields4 &out, int ndir, int *flag, cudaStream_t s) {
+  gauge_transform_kernel<Store, MAPPED><<<dim3((l.NE * g.Vs + 127) / 128, ndir), 128, 0, s>>>(
+      g, map, U, l.G, l.W, out, l.NE, wilson_gauge_tolerance((int)sizeof(CT)), flag);
+  return launch_check("gauge_transform_kernel");
+}
+
+} // namespace
+
 template <class Store, class CT>
 int launch_wilson_gauge_prep(const Geom &g, const Fields4 &U, const GaugeLinks &l, int *flag,
                              cudaStream_t s) {
   cudaError_t e = cudaMemsetAsync(flag, 0, sizeof(int), s);
   if (e != cudaSuccess)
     return launch_check("gauge flag reset");
-  const double tol = wilson_gauge_tolerance((int)sizeof(CT));
-  const int line_blocks = (g.Vs + kLinesCols - 1) / kLinesCols;
-  if (g.Vs < 8192)
-    gauge_lines_kernel<Store, 4>
-        <<<line_blocks, 4 * kLinesCols, 0, s>>>(g, U.f[3], l.G, l.W, tol, flag);
-  else
-    gauge_lines_kernel<Store, 1>
-        <<<line_blocks, kLinesCols, 0, s>>>(g, U.f[3], l.G, l.W, tol, flag);
-  int rc = launch_check("gauge_lines_kernel");
-  if (rc)
-    return rc;
-  gauge_transform_kernel<Store><<<dim3((l.NE * g.Vs + 127) / 128, 3), 128, 0, s>>>(
-      g, U, l.G, l.W, l.U, l.NE, tol, flag);
-  return launch_check("gauge_transform_kernel");
+  const int rc = launch_gauge_lines<Store, CT, false>(g, AxisMap{}, U.f[3], l, flag, s);
+  return rc ? rc : launch_gauge_links<Store, CT, false>(g, AxisMap{}, U, l, l.U, 3, flag, s);
 }
 
 template <class Store, class CT>
 int launch_wilson_gauge_second(const Geom &g, const Fields4 &U2, const GaugeLinks &l,
                                const Fields4 &out, int *flag, cudaStream_t s) {
-  gauge_transform_kernel<Store><<<dim3((l.NE * g.Vs + 127) / 128, 3), 128, 0, s>>>(
-      g, U2, l.G, l.W, out, l.NE, wilson_gauge_tolerance((int)sizeof(CT)), flag);
-  return launch_check("gauge_transform_kernel");
+  return launch_gauge_links<Store, CT, false>(g, AxisMap{}, U2, l, out, 3, flag, s);
+}
+
+template <class Store, class CT>
+int launch_axis_gauge_lines(const Geom &g, const AxisMap &map, const void *Ut,
+                            const GaugeLinks &l, int *flag, cudaStream_t s) {
+  return launch_gauge_lines<Store, CT, true>(g, map, Ut, l, flag, s);
+}
+
+template <class Store, class CT>
+int launch_axis_gauge_links(const Geom &g, const AxisMap &map, const Fields4 &F,
+                            const GaugeLinks &l, int *flag, cudaStream_t s) {
+  return launch_gauge_links<Store, CT, true>(g, map, F, l, l.U, 2, flag, s);
 }
 
 template <class Store, class CT>
 int launch_wilson_gauge_kernel(const Geom &g, const GaugeLinks &l, int rmin, int rmax, int tmin,
                                int tmax, bool adjoint, const int *flag, double *partials,
-                               int *blocks, cudaStream_t s, int units = 0, int tstarts = 0) {
+                               int *blocks, cudaStream_t s, int units = 0, int tstarts = 0,
+                               int ndir = 3) {
   const int nr = rmax - rmin + 1, nt = tmax - tmin + 1;
   // every start slice (on tmax further slices), or the start slices
   // [0, tstarts) of a time slab
@@ -955,7 +995,7 @@ int launch_wilson_gauge_kernel(const Geom &g, const GaugeLinks &l, int rmin, int
       wilson_gauge_plan(g, tmin, tmax, Store::NC, (int)sizeof(CT), units, adjoint, tstarts);
   if (!adjoint && p.kernel == 1)
     return launch_wilson_gram<Store, CT>(g, l, nullptr, rmin, rmax, tmin, tmax, flag, partials,
-                                         blocks, s, units, tstarts);
+                                         blocks, s, units, tstarts, ndir);
   if (!p.fits || l.NE < tstarts + tmax)
     return plan_error("wilson_gauge_kernel: block shape does not fit");
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
@@ -967,7 +1007,7 @@ int launch_wilson_gauge_kernel(const Geom &g, const GaugeLinks &l, int rmin, int
     int r = allow_large_smem(kernel, p.smem, capturing);
     if (r)
       return r;
-    kernel<<<dim3(p.blocks / 3, 3), p.threads, p.smem, s>>>(
+    kernel<<<dim3(p.blocks / 3, ndir), p.threads, p.smem, s>>>(
         g, l.U, l.NE, rmin, rmax, tmin, tmax, p.cols_per_block, p.rows, partials, flag, tstarts);
     return GC_OK;
   };
@@ -976,7 +1016,7 @@ int launch_wilson_gauge_kernel(const Geom &g, const GaugeLinks &l, int rmin, int
       auto k_all = wilson_gauge_q_kernel<Store, CT, kStarts, false>;
       auto k_some = wilson_gauge_q_kernel<Store, CT, kStarts, true>;
       const int rc = go(Lt % kStarts ? k_some : k_all, k_some);
-      *blocks = p.blocks;
+      *blocks = p.blocks / 3 * ndir;
       return rc ? rc : launch_check("wilson_gauge_q_kernel");
     }
   }
@@ -985,7 +1025,7 @@ int launch_wilson_gauge_kernel(const Geom &g, const GaugeLinks &l, int rmin, int
       auto k_all = wilson_gauge_reg_kernel<kStarts, false>;
       auto k_some = wilson_gauge_reg_kernel<kStarts, true>;
       const int rc = go(Lt % kStarts ? k_some : k_all, k_some);
-      *blocks = p.blocks;
+      *blocks = p.blocks / 3 * ndir;
       return rc ? rc : launch_check("wilson_gauge_reg_kernel");
     }
   }
@@ -998,7 +1038,7 @@ int launch_wilson_gauge_kernel(const Geom &g, const GaugeLinks &l, int rmin, int
                                       wilson_gauge_kernel<Store, CT, true, 1, true>);
   if (rc)
     return rc;
-  *blocks = p.blocks;
+  *blocks = p.blocks / 3 * ndir;
   return launch_check("wilson_gauge_kernel");
 }
 
@@ -1048,6 +1088,23 @@ size_t wilson_auto_partials_count(const Geom &g, int nr, int tmin, int tmax, int
   return std::max<size_t>(wilson_partials_count(g, nr, nt, nc), (size_t)blocks * nr * nt);
 }
 
+size_t axis_loops_partials(const Geom &g, int nr, int tmin, int tmax, int nc, int ct_bytes) {
+  return (size_t)wilson_gauge_plan(g, tmin, tmax, nc, ct_bytes).blocks / 3 * 2 * nr *
+         (tmax - tmin + 1);
+}
+
+template <class Store, class CT>
+int launch_axis_loops(const Geom &g, const GaugeLinks &l, int rmin, int rmax, int tmin, int tmax,
+                      const int *flag, double *partials, double scale, double *out_dev,
+                      cudaStream_t s) {
+  int blocks = 0;
+  const int rc = launch_wilson_gauge_kernel<Store, CT>(g, l, rmin, rmax, tmin, tmax, false, flag,
+                                                       partials, &blocks, s, 0, 0, 2);
+  return rc ? rc
+            : launch_reduce_wilson(partials, blocks, rmax - rmin + 1, tmax - tmin + 1, scale,
+                                   out_dev, s);
+}
+
 // Times one launch of the gauge W kernel of a lattice with `units` column
 // units per block (the autotuner's candidate), from prepared transformed
 // links; partials must hold wilson_auto_partials_count(.., units) doubles.
@@ -1090,6 +1147,14 @@ int time_wilson_gauge(const Geom &g, const GaugeLinks &l, int rmin, int rmax, in
   template int launch_wilson_gauge_second<STORE, CT>(const Geom &, const Fields4 &,          \
                                                      const GaugeLinks &, const Fields4 &,    \
                                                      int *, cudaStream_t);                   \
+  template int launch_axis_gauge_lines<STORE, CT>(const Geom &, const AxisMap &, const void *, \
+                                                  const GaugeLinks &, int *, cudaStream_t);  \
+  template int launch_axis_gauge_links<STORE, CT>(const Geom &, const AxisMap &,             \
+                                                  const Fields4 &, const GaugeLinks &,       \
+                                                  int *, cudaStream_t);                      \
+  template int launch_axis_loops<STORE, CT>(const Geom &, const GaugeLinks &, int, int, int,  \
+                                            int, const int *, double *, double, double *,     \
+                                            cudaStream_t);                                   \
   template int time_wilson_gauge<STORE, CT>(const Geom &, const GaugeLinks &, int, int, int, \
                                             int, int, double *, cudaStream_t, float *);
 

@@ -461,7 +461,7 @@ WilsonPlan wilson_gram_plan(const Geom &g, int tstarts, int tmax, int nc, int co
 template <class Store, class CT>
 int launch_wilson_gram(const Geom &g, const GaugeLinks &l, const Fields4 *second, int rmin,
                        int rmax, int tmin, int tmax, const int *flag, double *partials,
-                       int *blocks, cudaStream_t s, int cols, int tstarts) {
+                       int *blocks, cudaStream_t s, int cols, int tstarts, int ndir) {
   const WilsonPlan p = wilson_gram_plan(g, tstarts, tmax, Store::NC, cols, second != nullptr);
   if (!p.fits || l.NE < tstarts + tmax)
     return plan_error("wilson_gram_kernel: block shape does not fit");
@@ -470,21 +470,21 @@ int launch_wilson_gram(const Geom &g, const GaugeLinks &l, const Fields4 *second
   auto go = [&](auto kernel) {
     const int rc = allow_large_smem(kernel, p.smem, cap != cudaStreamCaptureStatusNone);
     if (!rc)
-      kernel<<<dim3(p.blocks / 3, 3), p.threads, p.smem, s>>>(
+      kernel<<<dim3(p.blocks / 3, ndir), p.threads, p.smem, s>>>(
           g, l.U, second ? *second : l.U, l.NE, rmin, rmax, tmin, tmax, p.cols_per_block,
           partials, flag, tstarts);
     return rc;
   };
   const int rc = second ? go(wilson_gram_kernel<Store, CT, true>)
                         : go(wilson_gram_kernel<Store, CT, false>);
-  *blocks = p.blocks;
+  *blocks = p.blocks / 3 * ndir;
   return rc ? rc : launch_check("wilson_gram_kernel");
 }
 
 #define GC_INSTANTIATE_GRAM(STORE, CT)                                                        \
   template int launch_wilson_gram<STORE, CT>(const Geom &, const GaugeLinks &,                \
                                              const Fields4 *, int, int, int, int, const int *, \
-                                             double *, int *, cudaStream_t, int, int);
+                                             double *, int *, cudaStream_t, int, int, int);
 
 GC_INSTANTIATE_GRAM(StoreF64SU3, double)
 GC_INSTANTIATE_GRAM(StoreF64SU2, double)

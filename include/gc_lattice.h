@@ -204,7 +204,8 @@ int gc_wilson_adjoint_onaxis(gc_lattice *h, int r_min, int r_max, int time_min,
                              int time_max, double *out);
 
 /* Selects the method of gc_wilson_onaxis, gc_wilson_adjoint_onaxis,
- * gc_wilson_gevp_onaxis (on its first handle) and the off-axis loops: GC_WILSON_AUTO (default) or GC_WILSON_EXACT.
+ * gc_wilson_gevp_onaxis (on its first handle), the off-axis and the spatial
+ * loops: GC_WILSON_AUTO (default) or GC_WILSON_EXACT.
  * No counterpart in the reference (which has one method, the exact product). */
 int gc_set_wilson_method(gc_lattice *h, int method);
 

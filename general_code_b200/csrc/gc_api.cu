@@ -1481,7 +1481,7 @@ static std::vector<int4> correlator_offsets(int D) {
 
 // Polyakov lines into h->aux (FP64 planes); optionally the loop average.
 static int polyakov_lines(gc_lattice *h, size_t extra_bytes, double *loop_dev) {
-  const size_t lines_bytes = (size_t)(h->nc == 3 ? 9 : 2) * h->g.Vs * sizeof(double2);
+  const size_t lines_bytes = (size_t)(h->nc == 3 ? 10 : 3) * h->g.Vs * sizeof(double2);
   int rc = ensure_aux(h, ((lines_bytes + 255) / 256) * 256 + extra_bytes);
   if (rc)
     return rc;
@@ -1528,13 +1528,55 @@ int gc_polyakov_correlator(gc_lattice *h, int d_max, int kind, double *out) {
     return fail(h, GC_ERR_ARG, "D_max too large");
   std::lock_guard<std::mutex> lk(h->mu);
   const std::vector<int4> offs = correlator_offsets(d_max);
+  const bool singlet = kind == GC_POLYAKOV_SINGLET;
+  const PolyakovRows plan = polyakov_rows_plan(h->g, h->nc, singlet, d_max);
+  const size_t per_dz = plan.entries;
+  bool rows = plan.fits;
+  if (rows) {
+    rc = ensure_partials(h, (size_t)plan.row_tiles * per_dz * plan.dz_per_launch);
+    if (rc == GC_ERR_NOMEM) { // (the other form needs none of it)
+      cudaGetLastError();
+      rows = false;
+    } else if (rc) {
+      return rc;
+    }
+  }
+  if (rows) {
+    rc = ensure_dev_out(h, per_dz * (2 * d_max + 1));
+    if (!rc)
+      rc = polyakov_lines(h, 0, nullptr);
+    if (rc)
+      return rc;
+    for (int k0 = 0; k0 < 2 * d_max + 1; k0 += plan.dz_per_launch) {
+      const int nz = std::min(plan.dz_per_launch, 2 * d_max + 1 - k0);
+      rc = launch_polyakov_rows(h->g, h->nc, singlet, (const double2 *)h->aux, d_max, plan,
+                                k0 - d_max, nz, h->partials, h->dev_out + k0 * per_dz, h->stream);
+      if (rc)
+        return launch_fail(h, rc);
+    }
+    std::vector<double> vals(per_dz * (2 * d_max + 1));
+    cudaError_t e = cudaMemcpyAsync(vals.data(), h->dev_out, vals.size() * sizeof(double),
+                                    cudaMemcpyDeviceToHost, h->stream);
+    if (e == cudaSuccess)
+      e = cudaStreamSynchronize(h->stream);
+    if (e != cudaSuccess)
+      return cuda_fail(h, "Polyakov correlator result", e);
+    std::fill(out, out + n, 0.0);
+    const size_t ndx = (size_t)plan.ndxt * plan.dxt;
+    for (const int4 &o : offs) {
+      const int sg = o.x < 0 ? -1 : 1; // C(-D) = C(D)
+      out[o.w] = vals[(size_t)(sg * o.z + d_max) * per_dz + (size_t)(sg * o.y + d_max) * ndx +
+                      sg * o.x];
+    }
+    return GC_OK;
+  }
   rc = ensure_dev_out(h, n);
   if (rc)
     return rc;
   rc = polyakov_lines(h, offs.size() * sizeof(int4), nullptr);
   if (rc)
     return rc;
-  const size_t lines_bytes = (size_t)(h->nc == 3 ? 9 : 2) * h->g.Vs * sizeof(double2);
+  const size_t lines_bytes = (size_t)(h->nc == 3 ? 10 : 3) * h->g.Vs * sizeof(double2);
   int4 *dev_offs = (int4 *)((char *)h->aux + ((lines_bytes + 255) / 256) * 256);
   cudaError_t e = cudaMemcpyAsync(dev_offs, offs.data(), offs.size() * sizeof(int4),
                                   cudaMemcpyHostToDevice, h->stream);
@@ -1543,8 +1585,7 @@ int gc_polyakov_correlator(gc_lattice *h, int d_max, int kind, double *out) {
   if (e != cudaSuccess)
     return cuda_fail(h, "Polyakov correlator setup", e);
   rc = launch_polyakov_correlator(h->g, h->nc, (const double2 *)h->aux, dev_offs,
-                                  (int)offs.size(), kind == GC_POLYAKOV_SINGLET, h->dev_out,
-                                  h->stream);
+                                  (int)offs.size(), singlet, h->dev_out, h->stream);
   if (rc)
     return launch_fail(h, rc);
   e = cudaMemcpyAsync(out, h->dev_out, n * sizeof(double), cudaMemcpyDeviceToHost, h->stream);

@@ -390,12 +390,25 @@ int launch_ape_plane(const Geom &g, const void *f1, const void *f2, void *o1, vo
                      int b, double alpha, cudaStream_t s);
 
 // Polyakov lines P(s) of every spatial site into `lines` (FP64 element
-// planes: 9 (SU(3)) or 2 (SU(2)) double2 planes of Vs entries), block sums of
+// planes: 9 (SU(3)) or 2 (SU(2)) double2 planes of Vs entries, and one of Tr P
+// / N), block sums of
 // Re Tr P / N into partials ((Vs + 255) / 256 of them) and, if out_dev is
 // given, the Polyakov loop (their mean) into out_dev[0].
 template <class Store, class CT>
 int launch_polyakov_lines(const Geom &g, const Fields4 &U, double2 *lines, double *partials,
                           double *out_dev, cudaStream_t s);
+// The correlators row by row: out_dev[dz - dz0][dy + D][dx] (entries per dz:
+// nch runs of dy, ndxt * dxt >= D + 1 values of dx; those outside the sphere
+// |(dx,dy,dz)| <= D are not defined) for dz in [dz0, dz0 + ndz), ndz <=
+// dz_per_launch. partials: row_tiles * ndz * entries doubles.
+struct PolyakovRows {
+  int ndxt, dxt, nch, row_tiles, entries, dz_per_launch;
+  bool fits;
+};
+PolyakovRows polyakov_rows_plan(const Geom &g, int nc, bool singlet, int D);
+int launch_polyakov_rows(const Geom &g, int nc, bool singlet, const double2 *lines, int D,
+                         const PolyakovRows &r, int dz0, int ndz, double *partials,
+                         double *out_dev, cudaStream_t s);
 // Correlator entries out_dev[offsets[i].w] for the offsets (x, y, z) of the
 // table; singlet: Re Tr(P P'^dag)/N, else Re(tr P conj(tr P')).
 int launch_polyakov_correlator(const Geom &g, int nc, const double2 *lines, const int4 *offsets,

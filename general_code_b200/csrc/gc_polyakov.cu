@@ -14,12 +14,24 @@
 // polyakov_lines_kernel: thread per spatial site, the Lt time links of the
 // site's column read in order (coalesced across threads), the product kept
 // in the compute type and stored in FP64 as element planes
-// (SU(3): 9 double2 planes, SU(2): 2 double2 planes, Vs entries each), with
+// (SU(3): 9 double2 planes, SU(2): 2 double2 planes, Vs entries each, and one
+// plane of normalised traces), with
 // fixed-order block sums of Re Tr P for the loop itself.
-// polyakov_correlator_kernel: one block per offset, each thread summing its
-// sites in a fixed order, then a fixed-order block tree: deterministic.
+// The correlators are sums over components k (double2 planes: 9 for SU(3)
+// singlets, 2 for SU(2), 1 for the traces) of products p_k(s) . p_k(s + D).
+// polyakov_rows_kernel: a block holds a few rows (y, z) of one slice and the
+// rows they meet for a run of dy at one dz in shared memory; a thread sums one
+// component and one dy over x for all dx of its tile, eight sites and the
+// tile's accumulators in registers, so that a load serves six
+// multiply-adds.
+// C(-D) = C(D), so only dx >= 0 is computed. polyakov_correlator_kernel, one
+// block per offset with every operand read from L2 for one multiply-add pair,
+// serves lattices whose rows do not fit. Fixed-order sums throughout.
 #include "gc_internal.cuh"
 #include "gc_kernels.h"
+
+#include <algorithm>
+#include <type_traits>
 
 namespace gc {
 
@@ -91,7 +103,9 @@ __global__ void __launch_bounds__(256)
       A = mul(A, Store::template load<CT>(Ut, V, s + t * g.Vs));
     const MD P = to_double(A);
     line_store(lines, g.Vs, s, P);
-    tr = norm_trace(P).x;
+    const double2 ntr = norm_trace(P);
+    lines[(size_t)(Store::NC == 3 ? 9 : 2) * g.Vs + s] = ntr; // the trace's own plane
+    tr = ntr.x;
   }
   const double b = block_sum(tr, sh);
   if (threadIdx.x == 0)
@@ -134,6 +148,133 @@ __global__ void __launch_bounds__(256)
     out[off.w] = sum * scale;
 }
 
+constexpr int kRowsY = 4;   // rows of a block
+constexpr int kRowsDy = 8;  // dy values of a block
+constexpr int kRowsX = 8;   // sites of a thread's tile
+
+// Shared rows: element (row, k, x) at row * NP * sx + k * sx + x, sx = 1 mod 8,
+// so that lanes (k fastest, then dy) read consecutive banks.
+__host__ __device__ inline int rows_sx(int Lx) { return (Lx + 6) / 8 * 8 + 1; }
+constexpr int rows_groups(int NP) { return NP == 9 ? 4 : 16; } // thread groups over (row, x tile)
+
+__device__ __forceinline__ void copy_async(double2 *smem, const double2 *global) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                   (unsigned)__cvta_generic_to_shared(smem)),
+               "l"(global)
+               : "memory");
+}
+
+// Bound by shared-memory loads: a tile of 8 sites makes 24 of them for DXT = 9
+// and they serve 144 FP64 fma; on 32^3, D = 8, SU(3) singlet, 280 us with the
+// load/store pipe 67% busy and the FP64 pipe 27% (the form with a block per
+// offset reads 18 operands from L2 for 18 fma). 6 or 9 dy a block, or 8 thread
+// groups, measured no better; so did copies without cp.async (worse).
+// partials[row tile][dz][dy][dx]: dz = dz0 + blockIdx.y / nch, dy = -D +
+// kRowsDy (blockIdx.y % nch) + i, dx = DXT blockIdx.z + j. p: NP planes.
+template <int NP, int DXT>
+__global__ void __launch_bounds__(NP * kRowsDy * rows_groups(NP))
+    polyakov_rows_kernel(const __grid_constant__ Geom g, const double2 *__restrict__ p, int D,
+                         int dz0, int nch, double *partials) {
+  extern __shared__ __align__(16) double2 rows[];
+  constexpr int NG = rows_groups(NP), nth = NP * kRowsDy * NG;
+  const int Lx = g.L[0], Ly = g.L[1], Lz = g.L[2], sx = rows_sx(Lx);
+  const int tid = threadIdx.x;
+  const int k = tid % NP, dyi = tid / NP % kRowsDy, group = tid / (NP * kRowsDy);
+  const int ny = (Ly + kRowsY - 1) / kRowsY;
+  const int y0 = blockIdx.x % ny * kRowsY, z = blockIdx.x / ny;
+  const int dz = dz0 + (int)blockIdx.y / nch, dy0 = -D + (int)blockIdx.y % nch * kRowsDy;
+  // the dy of this run nearest to 0 (nothing may lie within the sphere)
+  const int near = dy0 > 0 ? dy0 : dy0 + kRowsDy - 1 < 0 ? dy0 + kRowsDy - 1 : 0;
+  // and the dx of this tile that lie within it for the nearest dy
+  const int room = D * D - near * near - dz * dz;
+  int need = 0;
+  while (need < DXT && ((int)blockIdx.z * DXT + need) * ((int)blockIdx.z * DXT + need) <= room)
+    need++;
+  if (need == 0)
+    return;
+  const int yrows = min(kRowsY, Ly - y0);
+  // rows 0 .. kRowsY-1: y0 + r at z; then y0 + dy0 + r at z + dz
+  const int nb = kRowsY + kRowsDy - 1;
+  const int z2 = ((z + dz) % Lz + Lz) % Lz;
+  // (a warp per component and every kStep-th row, by asynchronous copies: all
+  // of a warp's rows are in flight, and no division per row)
+  constexpr int nwarps = nth / 32, kStep = nwarps / NP;
+  static_assert(nth % 32 == 0 && nwarps % NP == 0, "warps per component");
+  const int kk = (tid >> 5) % NP, first = (tid >> 5) / NP;
+  auto copy_rows = [&](int row0, int count, int y, int zz) {
+    const double2 *q = p + (size_t)kk * g.Vs + (size_t)Lx * Ly * zz;
+    y = ((y + first) % Ly + Ly) % Ly;
+    for (int r = first; r < count; r += kStep) {
+      double2 *dst = rows + ((row0 + r) * NP + kk) * sx;
+      for (int x = tid & 31; x < Lx; x += 32)
+        copy_async(dst + x, q + Lx * y + x);
+      for (y += kStep; y >= Ly;)
+        y -= Ly;
+    }
+  };
+  copy_rows(0, kRowsY, y0, z);
+  copy_rows(kRowsY, nb, y0 + dy0, z2);
+  asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
+  __syncthreads();
+  double acc[DXT];
+#pragma unroll
+  for (int j = 0; j < DXT; j++)
+    acc[j] = 0.0;
+  const int nx = (Lx + kRowsX - 1) / kRowsX;
+  const int dx0 = (int)blockIdx.z * DXT % Lx;
+#pragma unroll 1
+  for (int item = group; item < yrows * nx; item += NG) {
+    const int r = item / nx, x0 = item % nx * kRowsX;
+    const int a = (r * NP + k) * sx + x0, b = ((kRowsY + r + dyi) * NP + k) * sx;
+    double2 u[kRowsX];
+    if (x0 + kRowsX <= Lx) {
+#pragma unroll
+      for (int i = 0; i < kRowsX; i++)
+        u[i] = rows[a + i];
+    } else {
+#pragma unroll
+      for (int i = 0; i < kRowsX; i++)
+        u[i] = x0 + i < Lx ? rows[a + i] : make_double2(0.0, 0.0);
+    }
+    int x = x0 + dx0;
+    x = x >= Lx ? x - Lx : x;
+    int v = b + x;
+#pragma unroll
+    for (int w = 0; w < kRowsX + DXT - 1; w++) {
+      if (w >= kRowsX + need - 1)
+        break;
+      const double2 q = rows[v];
+      v = v + 1 == b + Lx ? b : v + 1;
+#pragma unroll
+      for (int i = 0; i < kRowsX; i++)
+        if (w - i >= 0 && w - i < DXT)
+          acc[w - i] = fma(u[i].y, q.y, fma(u[i].x, q.x, acc[w - i]));
+    }
+  }
+  __syncthreads();
+  // sum over components and groups, in order
+  double *red = reinterpret_cast<double *>(rows);
+#pragma unroll
+  for (int j = 0; j < DXT; j++)
+    red[j * nth + tid] = acc[j];
+  __syncthreads();
+  const int ndx = gridDim.z * DXT;
+  for (int e = tid; e < kRowsDy * DXT; e += nth) {
+    const int i = e / DXT, j = e % DXT;
+    double v = 0.0;
+    for (int q = 0; q < NG; q++)
+      for (int kk = 0; kk < NP; kk++)
+        v += red[j * nth + (q * kRowsDy + i) * NP + kk];
+    partials[((size_t)blockIdx.x * gridDim.y * kRowsDy + blockIdx.y * kRowsDy + i) * ndx +
+             blockIdx.z * DXT + j] = v;
+  }
+}
+
+size_t rows_smem(const Geom &g, int NP, int DXT) {
+  const size_t rows = (size_t)(2 * kRowsY + kRowsDy - 1) * NP * rows_sx(g.L[0]) * 16;
+  return std::max(rows, (size_t)NP * kRowsDy * rows_groups(NP) * DXT * 8);
+}
+
 } // namespace
 
 template <class Store, class CT>
@@ -170,6 +311,66 @@ int launch_polyakov_correlator(const Geom &g, int nc, const double2 *lines, cons
           <<<noffsets, 256, 0, s>>>(g, lines, offsets, scale, out_dev);
   }
   return launch_check("polyakov_correlator_kernel");
+}
+
+PolyakovRows polyakov_rows_plan(const Geom &g, int nc, bool singlet, int D) {
+  PolyakovRows r{};
+  const int NP = singlet ? (nc == 3 ? 9 : 2) : 1;
+  r.ndxt = (D + 1 + 8) / 9;
+  r.dxt = (D + 1 + r.ndxt - 1) / r.ndxt;
+  r.nch = (2 * D + 1 + kRowsDy - 1) / kRowsDy;
+  r.row_tiles = (g.L[1] + kRowsY - 1) / kRowsY * g.L[2];
+  r.entries = r.nch * kRowsDy * r.ndxt * r.dxt;
+  r.dz_per_launch = (int)std::min<size_t>(
+      2 * D + 1, std::max<size_t>(1, ((size_t)8 << 20) / ((size_t)r.row_tiles * r.entries)));
+  // SU(3) FP64, us per call, this form against a block per offset: 8^3 x 4,
+  // D = 2: 49 / 48; 12^3 x 4, D = 3: 52 / 62; 32^3 x 8, D = 8: 339 / 606, D =
+  // 16: 1850 / 3217; 48^3 x 8, D = 12: 3031 / 5678; SU(2) 32^3 x 8, D = 8: 149
+  // / 267. So it is taken wherever its rows fit the shared memory (SU(3): Lx
+  // up to 89) and its partial sums stay below 256 MB.
+  r.fits = rows_smem(g, NP, r.dxt) <= 200 * 1024 && (size_t)r.dz_per_launch * r.nch < 65536 &&
+           (size_t)r.row_tiles * r.entries <= (size_t)32 << 20;
+  return r;
+}
+
+int launch_polyakov_rows(const Geom &g, int nc, bool singlet, const double2 *lines, int D,
+                         const PolyakovRows &r, int dz0, int ndz, double *partials,
+                         double *out_dev, cudaStream_t s) {
+  // (the traces' plane follows the components')
+  const double2 *p = singlet ? lines : lines + (size_t)(nc == 3 ? 9 : 2) * g.Vs;
+  const dim3 grid(r.row_tiles, ndz * r.nch, r.ndxt);
+  auto go = [&](auto np, auto dxt) {
+    constexpr int NP = decltype(np)::value, DXT = decltype(dxt)::value;
+    const size_t smem = rows_smem(g, NP, DXT);
+    const int rc = allow_large_smem(polyakov_rows_kernel<NP, DXT>, smem);
+    if (!rc)
+      polyakov_rows_kernel<NP, DXT>
+          <<<grid, NP * kRowsDy * rows_groups(NP), smem, s>>>(g, p, D, dz0, r.nch, partials);
+    return rc;
+  };
+  using std::integral_constant;
+  auto tiles = [&](auto np) {
+    switch (r.dxt) {
+    case 1: return go(np, integral_constant<int, 1>());
+    case 2: return go(np, integral_constant<int, 2>());
+    case 3: return go(np, integral_constant<int, 3>());
+    case 4: return go(np, integral_constant<int, 4>());
+    case 5: return go(np, integral_constant<int, 5>());
+    case 6: return go(np, integral_constant<int, 6>());
+    case 7: return go(np, integral_constant<int, 7>());
+    case 8: return go(np, integral_constant<int, 8>());
+    default: return go(np, integral_constant<int, 9>());
+    }
+  };
+  int rc = singlet ? (nc == 3 ? tiles(integral_constant<int, 9>())
+                              : tiles(integral_constant<int, 2>()))
+                   : tiles(integral_constant<int, 1>());
+  if (!rc)
+    rc = launch_check("polyakov_rows_kernel");
+  if (rc)
+    return rc;
+  const double scale = 1.0 / ((double)g.Vs * (singlet && nc == 3 ? 3.0 : 1.0));
+  return launch_reduce_rows(partials, r.row_tiles, ndz * r.entries, scale, out_dev, s);
 }
 
 #define GC_INSTANTIATE_P(STORE, CT)                                                      \

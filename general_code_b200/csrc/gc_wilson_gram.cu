@@ -300,6 +300,8 @@ __global__ void __launch_bounds__(kGramThreads, 4)
   const int Ln = sel4(g.L, nu), stn = sel4(g.stride, nu);
   const int xn = (s / stn) % Ln;
   const size_t VE = (size_t)NE * g.Vs;
+  // slices the loops touch (a slab's lattice may have more than its tiles hold)
+  const int nslots = min(NE, tstarts + tmax);
   double *part = partials + ((size_t)blockIdx.y * gridDim.x + blockIdx.x) * (rmax - rmin + 1) * nt;
   // the warp's tasks: a group of start tiles and every nsub-th unit, or, with
   // more groups than warps, every nwarps-th group and all units
@@ -329,21 +331,21 @@ __global__ void __launch_bounds__(kGramThreads, 4)
     const int l = site(R);
 #pragma unroll
     for (int i = 0; i < kPre; i++)
-      if (trow + i * tstep < NE)
+      if (trow + i * tstep < nslots)
         pre[i].load(U.f[nu], VE, l + (trow + i * tstep) * g.Vs);
   };
   auto extend_from = [&](const void *f, int first, double2 *set, int R) {
     const int l = site(R);
 #pragma unroll 1
-    for (int t = trow + first * tstep; t < NE; t += kBatch * tstep) {
+    for (int t = trow + first * tstep; t < nslots; t += kBatch * tstep) {
       Raw x[kBatch];
 #pragma unroll
       for (int j = 0; j < kBatch; j++)
-        if (t + j * tstep < NE)
+        if (t + j * tstep < nslots)
           x[j].load(f, VE, l + (t + j * tstep) * g.Vs);
 #pragma unroll
       for (int j = 0; j < kBatch; j++)
-        if (t + j * tstep < NE)
+        if (t + j * tstep < nslots)
           apply(x[j], t + j * tstep, set, R);
     }
   };
@@ -359,7 +361,7 @@ __global__ void __launch_bounds__(kGramThreads, 4)
     if (active) {
 #pragma unroll
       for (int i = 0; i < kPre; i++)
-        if (trow + i * tstep < NE)
+        if (trow + i * tstep < nslots)
           apply(pre[i], trow + i * tstep, lines, R);
       if (GEVP)
         extend_from(U2.f[nu], 0, lines2, R);

@@ -99,7 +99,8 @@ struct WilsonPlan {
   size_t smem;        // dynamic shared memory bytes
   bool fits;          // false when even one column exceeds the budget
   int starts = 1;     // temporal-gauge form: consecutive start slices per thread
-  int kernel = 0;     // temporal-gauge form: 0 wilson_gauge_kernel, 1 wilson_gram_kernel
+  int kernel = 0;     // temporal-gauge form: 0 wilson_gauge_kernel, 1 wilson_gram_kernel,
+                      // 2 wilson_gauge_q_kernel, 3 wilson_gauge_reg_kernel, 4 wilson_corr_kernel
 };
 // Doubles of a W block's per-warp accumulators in shared memory, rounded up
 // to an even count so the 16-byte arrays placed after them stay aligned.
@@ -196,6 +197,15 @@ template <class Store, class CT>
 int launch_wilson_gram(const Geom &g, const GaugeLinks &l, const Fields4 *second, int rmin,
                        int rmax, int tmin, int tmax, const int *flag, double *partials,
                        int *blocks, cudaStream_t s, int cols, int tstarts, int ndir = 3);
+
+// The fundamental loops as correlations along time (gc_wilson_corr.cu), as
+// launch_wilson_gram.
+WilsonPlan wilson_corr_plan(const Geom &g, int tstarts, int tmin, int tmax, int nc, int ct_bytes,
+                            int cols);
+template <class Store, class CT>
+int launch_wilson_corr(const Geom &g, const GaugeLinks &l, int rmin, int rmax, int tmin, int tmax,
+                       const int *flag, double *partials, int *blocks, cudaStream_t s, int cols,
+                       int tstarts, int ndir);
 
 // The spatial links of a second configuration in the gauge of l (its time
 // lines), into out.f[0..2] as l.U; raises *flag as launch_wilson_gauge_prep.

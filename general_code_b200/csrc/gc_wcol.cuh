@@ -7,6 +7,7 @@
 #include "gc_internal.cuh"
 #include "gc_kernels.h"
 #include "gc_pair.cuh"
+#include "gc_rows01.cuh"
 
 #include <type_traits>
 
@@ -270,6 +271,63 @@ __device__ __forceinline__ GAcc<ADJ, T> gauge_trace(const SU2<T> &a, const SU2<T
     return dot4(a.a0, b.a0, a.a1, b.a1, a.a2, b.a2, a.a3, b.a3);
   return loop_value<ADJ>(a, b, lane1);
 }
+
+// First spatial site of a column block. When the block's columns tile the x
+// extent, consecutive blocks step along nu (for nu = y, z), so that the
+// blocks running at the same time extend their space lines with the same
+// transformed links (they hit L2 instead of each reading HBM); otherwise the
+// blocks take consecutive runs of sites.
+__device__ __forceinline__ int column_base(const Geom &g, int cb, int cols, int nu) {
+  if (nu == 0 || g.L[0] % cols != 0)
+    return cb * cols;
+  const int nxc = g.L[0] / cols;
+  int xc, y, z;
+  if (nu == 1) {
+    y = cb % g.L[1];
+    const int rest = cb / g.L[1];
+    xc = rest % nxc;
+    z = rest / nxc;
+  } else {
+    z = cb % g.L[2];
+    const int rest = cb / g.L[2];
+    xc = rest % nxc;
+    y = rest / nxc;
+  }
+  return xc * cols + g.L[0] * (y + g.L[1] * z);
+}
+
+// A link as it is loaded (12-real links: the third row is rebuilt when it is
+// used), and how many are in flight per thread: kPre across the matrix
+// instructions, kBatch in the extension.
+template <class Store, class CT> struct RawLink {
+  static constexpr int kPre = Store::NC == 3 ? 0 : 2, kBatch = Store::NC == 3 ? 1 : 4;
+  typename Store::template M<CT> m;
+  __device__ __forceinline__ void load(const void *f, size_t V, int site) {
+    m = Store::template load<CT>(f, V, site);
+  }
+  __device__ __forceinline__ typename Store::template M<CT> link() const { return m; }
+};
+template <> struct RawLink<StoreF32SU3, float> {
+  static constexpr int kPre = 0, kBatch = 3;
+  float4 a, b, c;
+  __device__ __forceinline__ void load(const void *f, size_t V, int site) {
+    const float4 *p = reinterpret_cast<const float4 *>(f) + site;
+    a = __ldg(p);
+    b = __ldg(p + V);
+    c = __ldg(p + 2 * V);
+  }
+  __device__ __forceinline__ SU3<float> link() const {
+    SU3<float> u;
+    u.e[0][0] = {a.x, a.y};
+    u.e[0][1] = {a.z, a.w};
+    u.e[0][2] = {b.x, b.y};
+    u.e[1][0] = {b.z, b.w};
+    u.e[1][1] = {c.x, c.y};
+    u.e[1][2] = {c.z, c.w};
+    rebuild_row2(u);
+    return u;
+  }
+};
 
 } // namespace
 

@@ -43,12 +43,15 @@
 //   gauge_transform_kernel  thread per (extended site, spatial nu): U'_nu,
 //                           computed in FP64, stored in the lattice's link
 //                           format
-//   wilson_gram_kernel      (gc_wilson_gram.cu) fundamental loops as FP64
-//                           matrix products
+//   wilson_corr_kernel      (gc_wilson_corr.cu) fundamental loops as
+//                           correlations of the lines' elements along t
+//   wilson_gram_kernel      (gc_wilson_gram.cu) FP64 fundamental loops of long
+//                           T ranges, and the GEVP loops, as FP64 matrix
+//                           products
 //   wilson_gauge_reg_kernel mixed SU(3), and
-//   wilson_gauge_q_kernel   SU(2) fundamental loops of shorter T ranges: one
+//   wilson_gauge_q_kernel   SU(2) fundamental loops of few slices and T: one
 //                           column per thread, the lines of its four start
-//                           slices in registers (gauge_*_applies has the line)
+//                           slices in registers (gauge_short_applies has the line)
 //   wilson_gauge_kernel     the adjoint loops (|Tr|^2 is no bilinear form of
 //                           the lines): block = `cols` columns (s, nu) over
 //                           all slices, the transformed space lines in shared
@@ -262,30 +265,6 @@ __global__ void __launch_bounds__(128)
     b = mul(GS::template load<double>(W, g.Vs, s + off), b);
   }
   Store::template store<double>(UE.f[nu], VE, esite, mul_ad(a, b));
-}
-
-// First spatial site of a column block. When the block's columns tile the x
-// extent, consecutive blocks step along nu (for nu = y, z), so that the
-// blocks running at the same time extend their space lines with the same
-// transformed links (they hit L2 instead of each reading HBM); otherwise the
-// blocks take consecutive runs of sites.
-__device__ __forceinline__ int column_base(const Geom &g, int cb, int cols, int nu) {
-  if (nu == 0 || g.L[0] % cols != 0)
-    return cb * cols;
-  const int nxc = g.L[0] / cols;
-  int xc, y, z;
-  if (nu == 1) {
-    y = cb % g.L[1];
-    const int rest = cb / g.L[1];
-    xc = rest % nxc;
-    z = rest / nxc;
-  } else {
-    z = cb % g.L[2];
-    const int rest = cb / g.L[2];
-    xc = rest % nxc;
-    y = rest / nxc;
-  }
-  return xc * cols + g.L[0] * (y + g.L[1] * z);
 }
 
 // Shared memory of one block: per-thread loop sums red[nt][threads] (GAcc),
@@ -772,26 +751,34 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-// Which fundamental loops take a one-column kernel (four starts per thread)
-// instead of the Gram matrix, whose tiles of 8 x 8 loops fill better with a
-// long T range (R <= L/2; whole W calls in us, one-column / Gram matrix):
-//   SU(3) mixed  16^4 T <= 8 158 / 163, 24^4 T <= 12 752 / 775, 32^4 T <= 4
-//                1488 / 2074, 32^4 T <= 16 2957 / 2703
-//   SU(2) FP64   20^4 T <= 10 138 / 162, 24^4 T <= 12 293 / 284, 32^4 T <= 16
-//                988 / 816, 48^4 T <= 24 9764 / 5743
-//   SU(2) mixed  48^4 T <= 24 5192 / 5855
-//   SU(3) FP64 has none: its lines of 18 doubles do not fit the registers
-//                (two starts per thread in a two-column kernel: 32^4 T <= 4
-//                3494, T <= 16 5930 against 2145 and 2971)
+// Which kernel takes the fundamental loops (whole W calls in us):
+// wilson_corr_kernel unless
+//   - the sequences are short, so that a thread's sums over its warp cost as
+//     much as its products: the one-column kernels (four starts per thread)
+//     take Lt x (T values) below a bound
+//       SU(3) mixed, one column / correlation: 32^3 x 6 T <= 3 260 / 346, 32^3
+//       x 8 T <= 4 316 / 371, 32^3 x 10 T <= 5 453 / 436, 24^4 T <= 2 407 /
+//       369; on small lattices the correlation's blocks fill more of the chip:
+//       12^3 x 8 87 / 71, 16^3 x 8 109 / 98, 24^3 x 8 134 / 144
+//       SU(2) mixed: 32^3 x 8 T <= 4 101 / 125, 24^4 T <= 5 127 / 135, T <= 6
+//       134 / 135, 32^4 T <= 6 370 / 346, 20^4 T <= 10 108 / 108
+//       SU(2) FP64: 16^4 T <= 2 65 / 76, T <= 8 78 / 80, 24^4 T <= 6 211 / 187
+//   - FP64 with a T range that one window does not cover (its 12 T values take
+//     48 registers; a second window reads the lines again): the Gram matrix
+//       SU(3), Gram matrix / correlation: 32^4 T <= 8 2248 / 2116, T <= 12
+//       2868 / 2613, T <= 13 2914 / 3340, T <= 16 2966 / 3370; SU(2) 24^4 T <=
+//       12 276 / 221, 32^4 T <= 12 812 / 629, T <= 16 802 / 792, 48^4 T <= 24
+//       5710 / 6557
 // (q kernel: at most 32 threads per column, so that a block of 8 columns fits)
 constexpr int kStarts = 4;
 int start_rows(int Lt) { return (Lt + kStarts - 1) / kStarts; }
-bool gauge_q_applies(int Lt, int tmax, int nc, int ct_bytes) {
-  return nc == 2 && start_rows(Lt) <= 32 && (ct_bytes == 4 || tmax < 12);
+bool gauge_short_applies(const Geom &g, int nt, int nc, int ct_bytes) {
+  const int work = g.L[3] * nt;
+  if (nc == 2)
+    return start_rows(g.L[3]) <= 32 && work < (ct_bytes == 4 ? 192 : 144);
+  return ct_bytes == 4 && start_rows(g.L[3]) <= 64 && work <= 40 && g.Vs > 8192;
 }
-bool gauge_reg_applies(int Lt, int tmax, int nc, int ct_bytes) {
-  return nc == 3 && ct_bytes == 4 && start_rows(Lt) <= 64 && tmax < 14;
-}
+bool gauge_corr_applies(int tmax, int ct_bytes) { return ct_bytes == 4 || tmax <= 12; }
 
 int largest_divisor_upto_g(int n, int cap) {
   for (int d = cap < n ? cap : n; d > 1; d--)
@@ -812,7 +799,13 @@ WilsonPlan wilson_gauge_plan(const Geom &g, int tmin, int tmax, int nc, int ct_b
     tstarts = Lt;
   WilsonPlan p{};
   const int nt = tmax - tmin + 1;
-  if (!adjoint && gauge_q_applies(Lt, tmax, nc, ct_bytes)) {
+  const bool few = gauge_short_applies(g, nt, nc, ct_bytes);
+  if (!adjoint && !few && gauge_corr_applies(tmax, ct_bytes)) {
+    p = wilson_corr_plan(g, tstarts, tmin, tmax, nc, ct_bytes, units_req);
+    if (p.fits || units_req > 0)
+      return p;
+  }
+  if (!adjoint && few && nc == 2) {
     // the SU(2) one-column kernel: four starts per thread, by default the
     // largest power of two (at least 8) of columns with at most 192 threads
     // per block (48^4 mixed: 5.15 ms with 16 columns of 12 threads, 5.47 ms
@@ -833,7 +826,7 @@ WilsonPlan wilson_gauge_plan(const Geom &g, int tmin, int tmax, int nc, int ct_b
     if (p.fits || units_req > 0)
       return p;
   }
-  if (!adjoint && gauge_reg_applies(Lt, tmax, nc, ct_bytes)) {
+  if (!adjoint && few && nc == 3) {
     // the mixed SU(3) one-column kernel: by default the largest power of two
     // of columns with at most 128 threads per block (of 8, 16 and 32 columns
     // 2-15% faster than twice or half, 10-50% than a quarter)
@@ -996,6 +989,9 @@ int launch_wilson_gauge_kernel(const Geom &g, const GaugeLinks &l, int rmin, int
   if (!adjoint && p.kernel == 1)
     return launch_wilson_gram<Store, CT>(g, l, nullptr, rmin, rmax, tmin, tmax, flag, partials,
                                          blocks, s, units, tstarts, ndir);
+  if (!adjoint && p.kernel == 4)
+    return launch_wilson_corr<Store, CT>(g, l, rmin, rmax, tmin, tmax, flag, partials, blocks, s,
+                                         units, tstarts, ndir);
   if (!p.fits || l.NE < tstarts + tmax)
     return plan_error("wilson_gauge_kernel: block shape does not fit");
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;

@@ -26,17 +26,19 @@
 //
 // Bound: the FP64 pipe, which the matrix instructions share with the FP64
 // form's products (64% busy at SU(3) 24^4 FP64, the matrix instructions alone
-// 46%; the mixed form 47%): the blocks' extension and multiplication phases
+// 46%): the blocks' extension and multiplication phases
 // overlap only between the four blocks of an SM, and of the computed tiles
-// T_max / (8 nd) lies within the band (0.5 at T <= 12, 0.67 at T <= 16). SU(3)
-// FP64, R,T <= L/2, whole W call: 32^4 5.93 -> 2.97 ms, 24^4 1.68 -> 0.80 ms;
-// SU(2) FP64 48^4 10.1 -> 5.74 ms; SU(3) mixed 32^4 2.88 -> 2.70 ms.
+// T_max / (8 nd) lies within the band (0.5 at T <= 12, 0.67 at T <= 16). FP64,
+// R,T <= L/2, whole W call: SU(3) 32^4 5.93 -> 2.97 ms, SU(2) 48^4 10.1 -> 5.74
+// ms. Where one window of T fits a thread's registers, gc_wilson_corr.cu is
+// faster (the rule is in gc_wilson_gauge.cu).
 //
 // GEVP (wilson_gevp_indexed, wilson_loops.h:1202-1233): a second set of
 // lines, C = S2 S1^T + S1 S2^T.
 #include "gc_internal.cuh"
 #include "gc_kernels.h"
 #include "gc_rows01.cuh"
+#include "gc_wcol.cuh"
 
 #include <algorithm>
 #include <type_traits>
@@ -114,39 +116,6 @@ template <class T> __device__ __forceinline__ void extend(double2 *p, const SU2<
   const double2 v = p[0], w = p[1];
   put(p, mul(SU2<T>{T(v.x), T(v.y), T(w.x), T(w.y)}, u));
 }
-
-// A link as it is loaded (12-real links: the third row is rebuilt when it is
-// used), and how many are in flight per thread: kPre across the matrix
-// instructions, kBatch in the extension.
-template <class Store, class CT> struct RawLink {
-  static constexpr int kPre = Store::NC == 3 ? 0 : 2, kBatch = Store::NC == 3 ? 1 : 4;
-  typename Store::template M<CT> m;
-  __device__ __forceinline__ void load(const void *f, size_t V, int site) {
-    m = Store::template load<CT>(f, V, site);
-  }
-  __device__ __forceinline__ typename Store::template M<CT> link() const { return m; }
-};
-template <> struct RawLink<StoreF32SU3, float> {
-  static constexpr int kPre = 0, kBatch = 3;
-  float4 a, b, c;
-  __device__ __forceinline__ void load(const void *f, size_t V, int site) {
-    const float4 *p = reinterpret_cast<const float4 *>(f) + site;
-    a = __ldg(p);
-    b = __ldg(p + V);
-    c = __ldg(p + 2 * V);
-  }
-  __device__ __forceinline__ SU3<float> link() const {
-    SU3<float> u;
-    u.e[0][0] = {a.x, a.y};
-    u.e[0][1] = {a.z, a.w};
-    u.e[0][2] = {b.x, b.y};
-    u.e[1][0] = {b.z, b.w};
-    u.e[1][1] = {c.x, c.y};
-    u.e[1][2] = {c.z, c.w};
-    rebuild_row2(u);
-    return u;
-  }
-};
 
 // Tiles of 8 slices: n0 of start slices, nd of end slices per start tile
 // (t1 - t0 up to tmax), and the slots of a column they touch.

@@ -25,17 +25,22 @@
 // shared memory and products.)
 //
 // The identity needs unitary temporal links. The lines kernel measures the
-// largest unitarity defect max |U_t U_t^dag - 1| of the lattice's temporal
-// links and raises a flag above the form's tolerance (FP64: 1e-14, a few
-// roundings; mixed: 1e-6, FP32 rounding of the 12-real links is 2.6e-7); for
-// 12-real links the transform kernel checks the spatial links as well.
+// unitarity defects d = max |U_t U_t^dag - 1| of the lattice's temporal links
+// and raises a flag when a block's links (32 columns) exceed the form's
+// tolerance in the mean (FP64: 1e-14, a few roundings) or one of them exceeds
+// 1e-12; mixed: when one exceeds 1e-6 (FP32 rounding of
+// the 12-real links is 2.6e-7); for 12-real links the transform kernel checks
+// the spatial links as well. (The mean, since W averages over all loops and every link enters as
+// many of them: one link past 1e-14 in a configuration, as an
+// orthonormalisation of nearly parallel rows leaves it, took the exact
+// product for all loops, 21 ms instead of 5.8 for the spatial loops of SU(3)
+// 24^4 FP64, for a difference below 1e-18.)
 // Both W kernels are launched and read the flag on the device: the exact
 // product (gc_wilson.cu) computes when it is raised, this form when it is
 // not, and the reduction sums the partials of the one that ran; no host
-// synchronisation, so the sequence can be captured in a graph. With defect
-// d per link a
-// loop differs from the reference's product of links by at most about
-// 2 T d (the two time lines), well inside the parity tolerances at these d.
+// synchronisation, so the sequence can be captured in a graph. With a
+// defect d per link a loop differs from the reference's product of links by at
+// most about 2 T d (the two time lines), well inside the parity tolerances.
 //
 // Kernels:
 //   gauge_lines_kernel      thread per spatial site: G(s,t), W(s) and the
@@ -107,6 +112,11 @@ __device__ __forceinline__ double unitarity_defect(const SU3<double> &u) {
 __device__ __forceinline__ double unitarity_defect(const SU2<double> &u) {
   return fabs(dot4(u.a0, u.a0, u.a1, u.a1, u.a2, u.a2, u.a3, u.a3) - 1.0);
 }
+
+__device__ __forceinline__ double row_sum(const SU3<double> &u) {
+  return (u.e[0][0].re + u.e[0][1].re) + u.e[0][2].re;
+}
+__device__ __forceinline__ double row_sum(const SU2<double> &u) { return u.a0; }
 
 // The temporal link the gauge lines are built from. FP64 links are unitary to
 // rounding. An FP32 link's last projection step leaves its singular values
@@ -180,17 +190,18 @@ __device__ __forceinline__ int own_site(const Geom &g, const AxisMap &map, int s
 template <class Store, int kLinesSegs, bool MAPPED>
 __global__ void __launch_bounds__(kLinesCols *kLinesSegs)
     gauge_lines_kernel(const __grid_constant__ Geom g, const __grid_constant__ AxisMap map,
-                       const void *Ut, void *GL, void *W, double tol, int *flag) {
+                       const void *Ut, void *GL, void *W, double tol, double most, int *flag) {
   using GS = typename F64Store<Store::NC>::type;
   using MD = typename Store::template M<double>;
   __shared__ MD total[kLinesSegs][kLinesCols];
+  __shared__ double defects[kLinesSegs];
   const int c = threadIdx.x % kLinesCols, seg = threadIdx.x / kLinesCols;
   const int s = blockIdx.x * kLinesCols + c;
   const bool active = s < g.Vs;
   const size_t V = g.V;
   const int Lt = g.L[3], len = (Lt + kLinesSegs - 1) / kLinesSegs;
   const int t0 = min(Lt, seg * len), t1 = min(Lt, t0 + len);
-  double dmax = 0.0;
+  double dmax = 0.0, dsum = 0.0;
   MD G = unit(MD());
   if (active && t0 < t1) {
     const int base = own_site<MAPPED>(g, map, s), step = MAPPED ? map.stride[3] : g.Vs;
@@ -202,18 +213,31 @@ __global__ void __launch_bounds__(kLinesCols *kLinesSegs)
     for (int t = t0; t < t1; t++) {
       const MD after = link(t + 2);
       GS::template store<double>(GL, V, s + t * g.Vs, seg ? G : stored_line(G));
-      dmax = fmax(dmax, unitarity_defect(u));
+      const double d = unitarity_defect(u);
+      dmax = fmax(dmax, d);
+      dsum += d;
       G = mul(G, gauge_time_link<Store>(u));
       u = next;
       next = after;
     }
   }
   total[seg][c] = G;
+  // (0 x G: NaN when a link was, whose defect's maximum may have dropped it)
+  const double sum = warp_sum(fma(0.0, row_sum(G), dsum));
+  if (c == 0)
+    defects[seg] = sum;
+  if (!(dmax <= most))
+    *flag = 1;
   __syncthreads();
+  if (threadIdx.x == 0) { // the mean over the block's links
+    double mean = 0.0;
+    for (int q = 0; q < kLinesSegs; q++)
+      mean += defects[q];
+    if (!(mean <= tol * min(kLinesCols, g.Vs - s) * Lt))
+      *flag = 1;
+  }
   if (!active)
     return;
-  if (!(dmax <= tol)) // (a NaN link counts as not unitary)
-    *flag = 1;
   if (kLinesSegs == 1)
     GS::template store<double>(W, g.Vs, s, stored_line(G));
   if (seg == 0)
@@ -919,13 +943,14 @@ template <class Store, class CT, bool MAPPED>
 int launch_gauge_lines(const Geom &g, const AxisMap &map, const void *Ut, const GaugeLinks &l,
                        int *flag, cudaStream_t s) {
   const double tol = wilson_gauge_tolerance((int)sizeof(CT));
+  const double most = sizeof(CT) == 8 ? 100 * tol : tol;
   const int blocks = (g.Vs + kLinesCols - 1) / kLinesCols;
   if (g.Vs < 8192)
     gauge_lines_kernel<Store, 4, MAPPED>
-        <<<blocks, 4 * kLinesCols, 0, s>>>(g, map, Ut, l.G, l.W, tol, flag);
+        <<<blocks, 4 * kLinesCols, 0, s>>>(g, map, Ut, l.G, l.W, tol, most, flag);
   else
     gauge_lines_kernel<Store, 1, MAPPED>
-        <<<blocks, kLinesCols, 0, s>>>(g, map, Ut, l.G, l.W, tol, flag);
+        <<<blocks, kLinesCols, 0, s>>>(g, map, Ut, l.G, l.W, tol, most, flag);
   return launch_check("gauge_lines_kernel");
 }
 

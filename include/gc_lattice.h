@@ -183,10 +183,10 @@ int gc_set_hyp_method(gc_lattice *h, int method);
  * the reference's std::map keyed (T,R), in the map's iteration order.
  * Two methods give the same table: the exact product of links (walked in T
  * for every corner), and, for T <= Lt/2 when the temporal links are unitary
- * (checked on the device for every call: defect max |U U^dag - 1| at most
- * 1e-14 in FP64, 1e-6 in the mixed form, there for the spatial SU(3) links as
- * well), the same loops in the temporal
- * gauge (one trace per loop instead of two matrix products); see
+ * (checked on the device for every call: defect max |U U^dag - 1| in FP64 at
+ * most 1e-14 in the mean over 32 columns and 1e-12 for any link, in the mixed
+ * form at most 1e-6, there for the spatial SU(3) links as well), the same loops
+ * in the temporal gauge (one trace per loop instead of two matrix products); see
  * gc_set_wilson_method. A block keeps one column's lines of all Lt slices in
  * shared memory: GC_ERR_ARG when they do not fit (SU(3): Lt > 246).
  * Replaces: wilson_loop(conf, r_min, r_max, time_min, time_max)

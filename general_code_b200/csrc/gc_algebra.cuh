@@ -661,7 +661,7 @@ template <bool ROW2> GC_HD SU3<float> polar_finish(const SU3<float> &U) {
         re = GC_FMA(V.e[i][j].im, V.e[k][j].im, re);
       }
       if (i == k) {
-        c[i][i] = {float(-0.5 * re), 0.f};
+        c[i][i] = {-0.5f * float(re), 0.f};
         continue;
       }
       double im = V.e[i][0].im * V.e[k][0].re;
@@ -671,7 +671,7 @@ template <bool ROW2> GC_HD SU3<float> polar_finish(const SU3<float> &U) {
         im = GC_FMA(V.e[i][j].im, V.e[k][j].re, im);
         im = GC_FMA(-V.e[i][j].re, V.e[k][j].im, im);
       }
-      c[i][k] = {float(-0.5 * re), float(-0.5 * im)};
+      c[i][k] = {-0.5f * float(re), -0.5f * float(im)};
       c[k][i] = {c[i][k].re, -c[i][k].im};
     }
   // Im det = Im sum_j (row0 x row1)_j row2_j

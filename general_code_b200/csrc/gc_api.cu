@@ -340,6 +340,7 @@ static int create_impl(const int dims[4], int nc, int precision, cudaStream_t or
   h->g.stride[3] = dims[0] * dims[1] * dims[2];
   h->g.V = (int)V;
   h->g.Vs = dims[0] * dims[1] * dims[2];
+  set_reciprocals(h->g);
   // 256-byte aligned fields
   h->field_bytes = ((bytes_per_link(nc, precision) * (size_t)V + 255) / 256) * 256;
   cudaError_t e;
@@ -1280,6 +1281,7 @@ int gc_wilson_spatial_3d(gc_lattice *h, int r_min, int r_max, int time_min, int 
       map[p].stride[d] = h->g.stride[order[d]];
     }
     pg[p].Vs = pg[p].stride[3];
+    set_reciprocals(pg[p]);
     gauge = gauge && wilson_gauge_applies(pg[p], 1, time_max, h->nc, ct_bytes, false) &&
             wilson_gauge_bytes(pg[p], h->nc, link_bytes, time_max) <= 15 * hyp_field_bytes(h);
     if (gauge)
@@ -1743,6 +1745,7 @@ long long gc_job_device_bytes(const int dims[4], int nc, int precision,
     g.L[d] = dims[d];
   g.V = (int)V;
   g.Vs = dims[0] * dims[1] * dims[2];
+  set_reciprocals(g);
   const int nr = std::max(1, rmax), nt = std::max(1, tmax);
   const long long partials =
       (long long)wilson_auto_partials_count(g, std::min(nr, std::max(1, 1024 / nt)), 1, nt, nc) *

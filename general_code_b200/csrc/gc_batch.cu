@@ -686,6 +686,7 @@ int gc_batch_create(const gc_job *jobs, int njobs, int precision, gc_batch **out
     j.g.stride[3] = j.g.L[0] * j.g.L[1] * j.g.L[2];
     j.g.V = j.g.stride[3] * j.g.L[3];
     j.g.Vs = j.g.stride[3];
+    set_reciprocals(j.g);
     j.field_bytes = align256(link_bytes(j.desc.nc, precision) * (size_t)j.g.V);
     const bool w = !(j.desc.r_max == 0 && j.desc.time_max == 0);
     j.nr = w ? j.desc.r_max - j.desc.r_min + 1 : 0;

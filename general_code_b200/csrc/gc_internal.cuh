@@ -25,15 +25,37 @@ struct Geom {
   int stride[4]; // 1, Lx, Lx*Ly, Lx*Ly*Lz
   int V;         // sites
   int Vs;        // spatial sites (Lx*Ly*Lz)
+  unsigned inv[3]; // reciprocals of L[0..2] (set_reciprocals)
 };
 
+// floor(2^32 / L): umulhi(n, inv) is n / L or one less for every n < 2^32
+// (L = 1: 2^32 - 1, the same), so that the divisions of site_coords by run-time
+// extents take five instructions each instead of about 25 and three
+// conversions.
+inline void set_reciprocals(Geom &g) {
+  for (int d = 0; d < 3; d++)
+    g.inv[d] = g.L[d] > 1 ? (unsigned)((1ull << 32) / (unsigned)g.L[d]) : 0xffffffffu;
+}
+
+// n / d and n % d for 0 <= n, inv = floor(2^32 / d)
+__host__ __device__ __forceinline__ int div_rem(int n, int d, unsigned inv, int *rem) {
+#if defined(__CUDA_ARCH__)
+  int q = (int)__umulhi((unsigned)n, inv);
+#else
+  int q = (int)(((unsigned long long)(unsigned)n * inv) >> 32);
+#endif
+  int r = n - q * d;
+  if (r >= d) {
+    q++;
+    r -= d;
+  }
+  *rem = r;
+  return q;
+}
+
 __host__ __device__ inline void site_coords(const Geom &g, int site, int x[4]) {
-  x[0] = site % g.L[0];
-  int r = site / g.L[0];
-  x[1] = r % g.L[1];
-  r /= g.L[1];
-  x[2] = r % g.L[2];
-  x[3] = r / g.L[2];
+  const int r = div_rem(site, g.L[0], g.inv[0], &x[0]);
+  x[3] = div_rem(div_rem(r, g.L[1], g.inv[1], &x[1]), g.L[2], g.inv[2], &x[2]);
 }
 
 // a[d] for a direction d known only at run time, as selects (a dynamically

@@ -146,6 +146,7 @@ extern "C" int gc_wilson_onaxis_noalloc(const int dims[4], int nc, int precision
   g.stride[3] = dims[0] * dims[1] * dims[2];
   g.V = (int)V;
   g.Vs = dims[0] * dims[1] * dims[2];
+  set_reciprocals(g);
 
   const size_t blocks = (size_t)wilson_max_blocks(g, nc);
   const size_t per_r = blocks * nt + nt;

@@ -129,6 +129,25 @@ __device__ __forceinline__ void proj_store(void *out, size_t V, int site, const 
   }
 }
 
+// A site's coordinates. By reciprocals, except in the FP64 SU(3) kernels, which
+// the FP64 pipe bounds and which took 1-2% longer with them (per step, us,
+// division / reciprocals: HYP SU(2) mixed 48^4 1160 / 1050, SU(3) mixed 32^4
+// 1246 / 1213, SU(2) FP64 32^4 388 / 377, SU(3) FP64 24^4 654 / 669; APE SU(2)
+// mixed 48^4 171 / 159, SU(3) FP64 32^4 384 / 387).
+template <class Store>
+__device__ __forceinline__ void smear_coords(const Geom &g, int site, int x[4]) {
+  if constexpr (Store::NC == 3 && Store::kBytes == 144) {
+    x[0] = site % g.L[0];
+    int r = site / g.L[0];
+    x[1] = r % g.L[1];
+    r /= g.L[1];
+    x[2] = r % g.L[2];
+    x[3] = r / g.L[2];
+  } else {
+    site_coords(g, site, x);
+  }
+}
+
 struct Nbr {
   int pnu, pmu, mnu, mnu_pmu;
 };
@@ -221,7 +240,7 @@ __device__ __forceinline__ void ape_site_mixed_su3(const Geom &g, const Fields4 
                                                    const Fields4 &out, double alpha,
                                                    int site, int mu) {
   int x[4];
-  site_coords(g, site, x);
+  smear_coords<StoreF32SU3>(g, site, x);
   const size_t V = g.V;
   const float c = float(alpha / 4);
   SU3<float> S = scale(StoreF32SU3::load<float>(in.f[mu], V, site), float(1 - alpha));
@@ -246,7 +265,7 @@ __device__ __forceinline__ void ape_site(const Geom &g, const Fields4 &in,
   }
   using M = typename Store::template M<CT>;
   int x[4];
-  site_coords(g, site, x);
+  smear_coords<Store>(g, site, x);
   const size_t V = g.V;
   M S = scale(Store::template load<CT>(in.f[mu], V, site), CT(1 - alpha));
   const CT c = CT(alpha / 4);
@@ -290,7 +309,7 @@ __device__ __forceinline__ void hyp_l1_site(const Geom &g, const Fields4 &U,
     // the mixed form's staples of stored (SU(3)) links, in two rows as in
     // ape_site_mixed_su3
     int x[4];
-    site_coords(g, site, x);
+    smear_coords<Store>(g, site, x);
     const size_t V = g.V;
     const int mu = kL1Mu[f], eta = kL1Eta[f];
     SU3<float> S = scale(StoreF32SU3::load<float>(U.f[mu], V, site), float(1 - alpha3));
@@ -302,7 +321,7 @@ __device__ __forceinline__ void hyp_l1_site(const Geom &g, const Fields4 &U,
   }
   using M = typename Store::template M<CT>;
   int x[4];
-  site_coords(g, site, x);
+  smear_coords<Store>(g, site, x);
   const size_t V = g.V;
   const int mu = kL1Mu[f], eta = kL1Eta[f];
   M S = scale(Store::template load<CT>(U.f[mu], V, site), CT(1 - alpha3));
@@ -333,7 +352,7 @@ __device__ __forceinline__ void hyp_l2_site(const Geom &g, const Fields4 &U,
   using M = typename Store::template M<CT>;
   using I = typename InterStore<Store>::type;
   int x[4];
-  site_coords(g, site, x);
+  smear_coords<Store>(g, site, x);
   const size_t V = g.V;
   const bool temporal = f < 3;
   const int nu = temporal ? f : f - 3;
@@ -367,7 +386,7 @@ __device__ __forceinline__ void hyp_l3_site(const Geom &g, const void *Ut,
                                             double alpha1, int site, const DecAddr &d) {
   using M = typename Store::template M<CT>;
   int x[4];
-  site_coords(g, site, x);
+  smear_coords<Store>(g, site, x);
   const size_t V = g.V;
   M S = scale(Store::template load<CT>(Ut, V, site), CT(1 - alpha1));
   const CT c = CT(alpha1 / 6);
@@ -392,7 +411,7 @@ __device__ __forceinline__ void ape_site_su2(const Geom &g, const Fields4 &in,
                                              const Fields4 &out, double alpha, int site) {
   using M = SU2<CT>;
   int x[4];
-  site_coords(g, site, x);
+  smear_coords<Store>(g, site, x);
   const size_t V = g.V;
   int fwd[3], bwd[3];
 #pragma unroll
@@ -642,7 +661,7 @@ __global__ void __launch_bounds__(128, ape_min_blocks<Store, CT>())
       return;
     const int mu = second ? b : a, nu = second ? a : b;
     int x[4];
-    site_coords(g, site, x);
+    smear_coords<Store>(g, site, x);
     const Nbr n = neighbours(g, site, x, mu, nu);
     M S = scale(Store::template load<CT>(in.f[mu], V, site), CT(1 - alpha));
     if constexpr (std::is_same<Store, StoreF32SU3>::value)
@@ -658,7 +677,7 @@ __global__ void __launch_bounds__(128, ape_min_blocks<Store, CT>())
   if (site >= g.V)
     return;
   int x[4];
-  site_coords(g, site, x);
+  smear_coords<Store>(g, site, x);
   const int pa = site + step_off(g, sel4(x, a), a, +1);
   const int pb = site + step_off(g, sel4(x, b), b, +1);
   const int mb = site + step_off(g, sel4(x, b), b, -1);

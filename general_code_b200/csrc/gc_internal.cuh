@@ -252,4 +252,33 @@ int launch_check(const char *what);
 // Records a launch-planning error (returned by the launcher as GC_ERR_ARG).
 int plan_error(const char *what);
 
+// Launches of one chain on a stream. A kernel launched by launch_chained is
+// set up while the memory of the one before it drains: its blocks start when
+// that kernel's have exited and wait (wait_previous, the first statement of
+// every kernel launched this way) until its writes are visible. Saves about 2.4 us of
+// each launch's 4 us gap (an APE step, us: SU(2) mixed 16^4 6.4 -> 3.9, SU(3)
+// mixed 16^4 18.8 -> 16.1, 32^4 215 -> 212.6). Letting the next kernel start
+// earlier (a trigger at the blocks' start) measured the same. Under stream
+// capture the launch is an ordinary one.
+__device__ __forceinline__ void wait_previous() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+template <class... P, class... A>
+inline void launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem,
+                           cudaStream_t s, A &&...args) {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  cudaStreamIsCapturing(s, &cap);
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = attr;
+  cfg.numAttrs = cap == cudaStreamCaptureStatusNone ? 1 : 0;
+  cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...); // (errors: launch_check)
+}
+
 } // namespace gc

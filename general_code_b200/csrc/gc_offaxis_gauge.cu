@@ -164,6 +164,7 @@ __global__ void __launch_bounds__(512)
                          int NE, const OffaxisNode *__restrict__ nodes,
                          const int *__restrict__ chunk_nodes, int line0, int nlines, int tmin,
                          int tmax, int cols, double *partials, const int *flag) {
+  wait_previous();
   if (*flag != 0)
     return;
   using M = typename Store::template M<CT>;
@@ -293,8 +294,8 @@ int launch_offaxis_gauge(const Geom &g, const GaugeLinks &l, const OffaxisNode *
   auto go = [&](auto kernel) {
     const int rc = allow_large_smem(kernel, f.smem);
     if (!rc)
-      kernel<<<grid, f.threads, f.smem, s>>>(g, l.U, l.NE, nodes, chunk_nodes + chunk0, line0,
-                                             nlines, tmin, tmax, f.cols, partials, flag);
+      launch_chained(kernel, grid, f.threads, f.smem, s, g, l.U, l.NE, nodes, chunk_nodes + chunk0,
+                     line0, nlines, tmin, tmax, f.cols, partials, flag);
     return rc;
   };
   const int rc = adjoint ? go(offaxis_gauge_kernel<Store, CT, true>)

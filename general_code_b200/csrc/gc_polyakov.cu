@@ -90,6 +90,7 @@ template <class Store, class CT>
 __global__ void __launch_bounds__(256)
     polyakov_lines_kernel(const __grid_constant__ Geom g, const void *Ut, double2 *lines,
                           double *partials) {
+  wait_previous();
   using M = typename Store::template M<CT>;
   using MD = typename Store::template M<double>;
   __shared__ double sh[256];
@@ -175,6 +176,7 @@ template <int NP, int DXT>
 __global__ void __launch_bounds__(NP * kRowsDy * rows_groups(NP))
     polyakov_rows_kernel(const __grid_constant__ Geom g, const double2 *__restrict__ p, int D,
                          int dz0, int nch, double *partials) {
+  wait_previous();
   extern __shared__ __align__(16) double2 rows[];
   constexpr int NG = rows_groups(NP), nth = NP * kRowsDy * NG;
   const int Lx = g.L[0], Ly = g.L[1], Lz = g.L[2], sx = rows_sx(Lx);
@@ -281,7 +283,7 @@ template <class Store, class CT>
 int launch_polyakov_lines(const Geom &g, const Fields4 &U, double2 *lines, double *partials,
                           double *out_dev, cudaStream_t s) {
   const int nb = (g.Vs + 255) / 256;
-  polyakov_lines_kernel<Store, CT><<<nb, 256, 0, s>>>(g, U.f[3], lines, partials);
+  launch_chained(polyakov_lines_kernel<Store, CT>, nb, 256, 0, s, g, U.f[3], lines, partials);
   int rc = launch_check("polyakov_lines_kernel");
   if (rc)
     return rc;
@@ -344,8 +346,8 @@ int launch_polyakov_rows(const Geom &g, int nc, bool singlet, const double2 *lin
     const size_t smem = rows_smem(g, NP, DXT);
     const int rc = allow_large_smem(polyakov_rows_kernel<NP, DXT>, smem);
     if (!rc)
-      polyakov_rows_kernel<NP, DXT>
-          <<<grid, NP * kRowsDy * rows_groups(NP), smem, s>>>(g, p, D, dz0, r.nch, partials);
+      launch_chained(polyakov_rows_kernel<NP, DXT>, grid, NP * kRowsDy * rows_groups(NP), smem, s,
+                     g, p, D, dz0, r.nch, partials);
     return rc;
   };
   using std::integral_constant;

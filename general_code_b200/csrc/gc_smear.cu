@@ -470,6 +470,7 @@ template <class Store, class CT>
 __global__ void __launch_bounds__(128, ape_min_blocks<Store, CT>())
     ape_kernel(Geom g, const __grid_constant__ Fields4 in,
                const __grid_constant__ Fields4 out, double alpha) {
+  wait_previous();
   if constexpr (Store::NC == 2) {
     const int site = blockIdx.x * blockDim.x + threadIdx.x;
     if (site < g.V)
@@ -486,6 +487,7 @@ template <class Store, class CT>
 __global__ void __launch_bounds__(128, 4)
     hyp_level1_kernel(Geom g, const __grid_constant__ Fields4 U,
                       const __grid_constant__ HypL1 out, double alpha3) {
+  wait_previous();
   const int f = blockIdx.x % 9;
   const int site = (blockIdx.x / 9) * blockDim.x + threadIdx.x;
   if (site < g.V)
@@ -497,6 +499,7 @@ __global__ void __launch_bounds__(128, 4)
     hyp_level2_kernel(Geom g, const __grid_constant__ Fields4 U,
                       const __grid_constant__ HypL1 l1,
                       const __grid_constant__ HypL2 out, double alpha2) {
+  wait_previous();
   const int f = blockIdx.x % 6;
   const int site = (blockIdx.x / 6) * blockDim.x + threadIdx.x;
   if (site < g.V)
@@ -507,6 +510,7 @@ template <class Store, class CT>
 __global__ void __launch_bounds__(128)
     hyp_level3_kernel(Geom g, const void *Ut, const __grid_constant__ HypL2 l2,
                       void *out_t, double alpha1) {
+  wait_previous();
   const int site = blockIdx.x * blockDim.x + threadIdx.x;
   if (site < g.V)
     hyp_l3_site<Store, CT>(g, Ut, l2, out_t, alpha1, site, whole_lattice(g));
@@ -542,6 +546,7 @@ __global__ void __launch_bounds__(128, 4)
                       const __grid_constant__ HypL1 l1, const __grid_constant__ HypL2 l2,
                       void *out_t, double a1, double a2, double a3,
                       const __grid_constant__ HypStage st) {
+  wait_previous();
   const int b = blockIdx.x;
   const int p = b < st.start[1] ? 0 : b < st.start[2] ? 1 : b < st.start[3] ? 2
               : b < st.start[4] ? 3 : 4;
@@ -648,6 +653,7 @@ template <class Store, class CT>
 __global__ void __launch_bounds__(128, ape_min_blocks<Store, CT>())
     ape_plane_kernel(const __grid_constant__ Geom g, const __grid_constant__ Fields4 in,
                      const __grid_constant__ Fields4 out, int a, int b, double alpha) {
+  wait_previous();
   using M = typename Store::template M<CT>;
   const size_t V = g.V;
   if constexpr (Store::NC == 3) {
@@ -705,7 +711,8 @@ template <class Store, class CT>
 int launch_ape(const Geom &g, const Fields4 &in, const Fields4 &out,
                double alpha, cudaStream_t s) {
   const unsigned nb = (g.V + kSmearBlock - 1) / kSmearBlock;
-  ape_kernel<Store, CT><<<nb * ape_items<Store>(), kSmearBlock, 0, s>>>(g, in, out, alpha);
+  launch_chained(ape_kernel<Store, CT>, nb * ape_items<Store>(), kSmearBlock, 0, s, g, in, out,
+                 alpha);
   return launch_check("ape_kernel");
 }
 
@@ -714,15 +721,15 @@ int launch_hyp(const Geom &g, const Fields4 &U, const HypL1 &l1,
                const HypL2 &l2, void *out_t, double a1, double a2, double a3,
                cudaStream_t s) {
   const int nb = (g.V + kSmearBlock - 1) / kSmearBlock;
-  hyp_level1_kernel<Store, CT><<<nb * 9, kSmearBlock, 0, s>>>(g, U, l1, a3);
+  launch_chained(hyp_level1_kernel<Store, CT>, nb * 9, kSmearBlock, 0, s, g, U, l1, a3);
   int rc = launch_check("hyp_level1_kernel");
   if (rc)
     return rc;
-  hyp_level2_kernel<Store, CT><<<nb * 6, kSmearBlock, 0, s>>>(g, U, l1, l2, a2);
+  launch_chained(hyp_level2_kernel<Store, CT>, nb * 6, kSmearBlock, 0, s, g, U, l1, l2, a2);
   rc = launch_check("hyp_level2_kernel");
   if (rc)
     return rc;
-  hyp_level3_kernel<Store, CT><<<nb, kSmearBlock, 0, s>>>(g, U.f[3], l2, out_t, a1);
+  launch_chained(hyp_level3_kernel<Store, CT>, nb, kSmearBlock, 0, s, g, U.f[3], l2, out_t, a1);
   return launch_check("hyp_level3_kernel");
 }
 
@@ -749,8 +756,8 @@ int launch_hyp_slices(const Geom &g, const Fields4 &U, const HypL1 &l1, const Hy
         blocks += kFields[p] * nbs;
     }
     st.start[5] = blocks;
-    hyp_slices_kernel<Store, CT><<<blocks, kSmearBlock, 0, s>>>(g, U, l1, l2, out_t, a1, a2,
-                                                                 a3, st);
+    launch_chained(hyp_slices_kernel<Store, CT>, blocks, kSmearBlock, 0, s, g, U, l1, l2, out_t, a1,
+                   a2, a3, st);
     const int rc = launch_check("hyp_slices_kernel");
     if (rc)
       return rc;
@@ -794,8 +801,8 @@ int launch_ape_plane(const Geom &g, const void *f1, const void *f2, void *o1, vo
   out.f[a] = o1;
   out.f[b] = o2;
   const unsigned nb = (g.V + kSmearBlock - 1) / kSmearBlock;
-  ape_plane_kernel<Store, CT>
-      <<<Store::NC == 3 ? 2 * nb : nb, kSmearBlock, 0, s>>>(g, in, out, a, b, alpha);
+  launch_chained(ape_plane_kernel<Store, CT>, Store::NC == 3 ? 2 * nb : nb, kSmearBlock, 0, s, g,
+                 in, out, a, b, alpha);
   return launch_check("ape_plane_kernel");
 }
 

@@ -191,7 +191,8 @@ __global__ void __launch_bounds__(256)
     wilson_kernel(const __grid_constant__ Geom g, const __grid_constant__ Fields4 U,
                   const __grid_constant__ Fields4 U2, int rmin, int rmax, int tmin, int tmax,
                   int cols, int rows, double *partials, int tstarts, int colblocks,
-                  const int *gate = nullptr) {
+                  const int *gate) {
+  wait_previous();
   if (gate && *gate == 0)
     return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -275,6 +276,7 @@ __global__ void __launch_bounds__(256)
 __global__ void __launch_bounds__(256)
     reduce_partials_kernel(const double *partials, int nblocks, int nentries,
                            int nr, int nt, double scale, double *out) {
+  wait_previous();
   __shared__ double sh[256];
   const int e = blockIdx.x;
   double s = 0.0;
@@ -301,6 +303,7 @@ template <class Store, class CT>
 __global__ void __launch_bounds__(256)
     plaquette_kernel(const __grid_constant__ Geom g, const __grid_constant__ Fields4 U,
                      double *partials) {
+  wait_previous();
   using M = typename Store::template M<CT>;
   __shared__ double sh[2][256];
   const int site = blockIdx.x * blockDim.x + threadIdx.x;
@@ -413,9 +416,9 @@ int launch_wilson_mode(const Geom &g, const Fields4 &U, const Fields4 &U2, int r
   int rc = allow_large_smem(wilson_kernel<Store, CT, ADJ, GEVP>, p.smem);
   if (rc)
     return rc;
-  wilson_kernel<Store, CT, ADJ, GEVP><<<p.blocks, p.threads, p.smem, s>>>(
-      g, U, U2, rmin, rmax, tmin, tmax, p.cols_per_block, p.rows, partials, tstarts,
-      p.blocks / 3);
+  launch_chained(wilson_kernel<Store, CT, ADJ, GEVP>, p.blocks, p.threads, p.smem, s, g, U, U2,
+                 rmin, rmax, tmin, tmax, p.cols_per_block, p.rows, partials, tstarts, p.blocks / 3,
+                 (const int *)nullptr);
   rc = launch_check("wilson_kernel");
   if (rc)
     return rc;
@@ -423,8 +426,8 @@ int launch_wilson_mode(const Geom &g, const Fields4 &U, const Fields4 &U2, int r
   // GEVP counts every loop twice (the / (6 V) of wilson_loops.h:910, 954)
   const double scale =
       wilson_scale((long long)g.Vs * tstarts, Store::NC, ADJ) / (GEVP ? 2.0 : 1.0);
-  reduce_partials_kernel<<<nr * nt, 256, 0, s>>>(partials, p.blocks, nr * nt, nr, nt, scale,
-                                                 out_dev);
+  launch_chained(reduce_partials_kernel, nr * nt, 256, 0, s, partials, p.blocks, nr * nt, nr, nt,
+                 scale, out_dev);
   return launch_check("reduce_partials_kernel");
 }
 
@@ -444,9 +447,9 @@ int launch_wilson_exact_gated(const Geom &g, const Fields4 &U, const Fields4 *se
   auto go = [&](auto kernel) {
     const int rc = allow_large_smem(kernel, p.smem);
     if (!rc)
-      kernel<<<std::min(p.blocks, 4 * 148), p.threads, p.smem, s>>>(
-          g, U, second ? *second : U, rmin, rmax, tmin, tmax, p.cols_per_block, p.rows, partials,
-          tstarts, p.blocks / 3, gate);
+      launch_chained(kernel, std::min(p.blocks, 4 * 148), p.threads, p.smem, s, g, U,
+                     second ? *second : U, rmin, rmax, tmin, tmax, p.cols_per_block, p.rows,
+                     partials, tstarts, p.blocks / 3, gate);
     return rc;
   };
   const int rc = second    ? go(wilson_kernel<Store, CT, false, true>)
@@ -479,14 +482,12 @@ template <class Store, class CT>
 int launch_plaquette(const Geom &g, const Fields4 &U, double *partials,
                      double *out_dev, cudaStream_t s) {
   const int nb = (g.V + 255) / 256;
-  plaquette_kernel<Store, CT><<<nb, 256, 0, s>>>(g, U, partials);
+  launch_chained(plaquette_kernel<Store, CT>, nb, 256, 0, s, g, U, partials);
   int rc = launch_check("plaquette_kernel");
   if (rc)
     return rc;
-  reduce_partials_kernel<<<2, 256, 0, s>>>(partials, nb, 2, 2, 1,
-                                           1.0 / (3.0 * (double)g.V *
-                                                  wilson_trace_norm(Store::NC)),
-                                           out_dev);
+  launch_chained(reduce_partials_kernel, 2, 256, 0, s, partials, nb, 2, 2, 1,
+                 1.0 / (3.0 * (double)g.V * wilson_trace_norm(Store::NC)), out_dev);
   return launch_check("reduce_partials_kernel");
 }
 
@@ -516,15 +517,16 @@ int launch_wilson_plan(const Geom &g, const Fields4 &U, int rmin, int rmax, int 
   int rc = allow_large_smem(wilson_kernel<Store, CT, false, false>, p.smem);
   if (rc)
     return rc;
-  wilson_kernel<Store, CT, false, false><<<p.blocks, p.threads, p.smem, s>>>(
-      g, U, U, rmin, rmax, tmin, tmax, p.cols_per_block, p.rows, partials, g.L[3], p.blocks / 3);
+  launch_chained(wilson_kernel<Store, CT, false, false>, p.blocks, p.threads, p.smem, s, g, U, U,
+                 rmin, rmax, tmin, tmax, p.cols_per_block, p.rows, partials, g.L[3], p.blocks / 3,
+                 (const int *)nullptr);
   rc = launch_check("wilson_kernel");
   if (rc)
     return rc;
   if (!out_dev)
     return GC_OK;
-  reduce_partials_kernel<<<nr * nt, 256, 0, s>>>(
-      partials, p.blocks, nr * nt, nr, nt, wilson_scale(g.V, Store::NC, false), out_dev);
+  launch_chained(reduce_partials_kernel, nr * nt, 256, 0, s, partials, p.blocks, nr * nt, nr, nt,
+                 wilson_scale(g.V, Store::NC, false), out_dev);
   return launch_check("reduce_partials_kernel");
 }
 
@@ -559,20 +561,20 @@ int launch_wilson_batch(const WJob *jobs, int njobs, int blocks, int threads, si
 
 int launch_reduce_sum(const double *partials, int n, double scale, double *out_dev,
                       cudaStream_t s) {
-  reduce_partials_kernel<<<1, 256, 0, s>>>(partials, n, 1, 1, 1, scale, out_dev);
+  launch_chained(reduce_partials_kernel, 1, 256, 0, s, partials, n, 1, 1, 1, scale, out_dev);
   return launch_check("reduce_partials_kernel");
 }
 
 int launch_reduce_rows(const double *partials, int blocks, int n, double scale,
                        double *out_dev, cudaStream_t s) {
-  reduce_partials_kernel<<<n, 256, 0, s>>>(partials, blocks, n, 1, n, scale, out_dev);
+  launch_chained(reduce_partials_kernel, n, 256, 0, s, partials, blocks, n, 1, n, scale, out_dev);
   return launch_check("reduce_partials_kernel");
 }
 
 int launch_reduce_wilson(const double *partials, int blocks, int nr, int nt, double scale,
                          double *out_dev, cudaStream_t s) {
-  reduce_partials_kernel<<<nr * nt, 256, 0, s>>>(partials, blocks, nr * nt, nr, nt, scale,
-                                                 out_dev);
+  launch_chained(reduce_partials_kernel, nr * nt, 256, 0, s, partials, blocks, nr * nt, nr, nt,
+                 scale, out_dev);
   return launch_check("reduce_partials_kernel");
 }
 

@@ -89,6 +89,7 @@ __global__ void __launch_bounds__(Store::NC == 3 ? 160 : 128, Store::NC == 2 || 
     wilson_corr_kernel(const __grid_constant__ Geom g, const __grid_constant__ Fields4 U, int NE,
                        int rmin, int rmax, int tmin, int tmax, int cols, double *partials,
                        const int *flag, int tstarts) {
+  wait_previous();
   // the exact product runs instead when a link failed the check
   if (flag && *flag != 0)
     return;
@@ -238,8 +239,8 @@ int launch_wilson_corr(const Geom &g, const GaugeLinks &l, int rmin, int rmax, i
                             cap != cudaStreamCaptureStatusNone);
   if (rc)
     return rc;
-  wilson_corr_kernel<Store, CT><<<dim3(p.blocks / 3, ndir), p.threads, p.smem, s>>>(
-      g, l.U, l.NE, rmin, rmax, tmin, tmax, p.cols_per_block, partials, flag, tstarts);
+  launch_chained(wilson_corr_kernel<Store, CT>, dim3(p.blocks / 3, ndir), p.threads, p.smem, s, g,
+                 l.U, l.NE, rmin, rmax, tmin, tmax, p.cols_per_block, partials, flag, tstarts);
   *blocks = p.blocks / 3 * ndir;
   return launch_check("wilson_corr_kernel");
 }

@@ -191,6 +191,7 @@ template <class Store, int kLinesSegs, bool MAPPED>
 __global__ void __launch_bounds__(kLinesCols *kLinesSegs)
     gauge_lines_kernel(const __grid_constant__ Geom g, const __grid_constant__ AxisMap map,
                        const void *Ut, void *GL, void *W, double tol, double most, int *flag) {
+  wait_previous();
   using GS = typename F64Store<Store::NC>::type;
   using MD = typename Store::template M<double>;
   __shared__ MD total[kLinesSegs][kLinesCols];
@@ -263,6 +264,7 @@ __global__ void __launch_bounds__(128)
     gauge_transform_kernel(const __grid_constant__ Geom g, const __grid_constant__ AxisMap map,
                            const __grid_constant__ Fields4 U, const void *GL, const void *W,
                            const __grid_constant__ Fields4 UE, int NE, double tol, int *flag) {
+  wait_previous();
   using GS = typename F64Store<Store::NC>::type;
   using MD = typename Store::template M<double>;
   const int esite = blockIdx.x * blockDim.x + threadIdx.x;
@@ -307,6 +309,7 @@ __global__ void __launch_bounds__(256)
     wilson_gauge_kernel(const __grid_constant__ Geom g, const __grid_constant__ Fields4 U,
                         int NE, int rmin, int rmax, int tmin, int tmax, int cols, int rows,
                         double *partials, const int *flag, int tstarts) {
+  wait_previous();
   // the exact product runs instead when a temporal link failed the check
   if (flag && *flag != 0)
     return;
@@ -490,6 +493,7 @@ __global__ void __launch_bounds__(256, 2)
     wilson_gauge_reg_kernel(const __grid_constant__ Geom g, const __grid_constant__ Fields4 U,
                             int NE, int rmin, int rmax, int tmin, int tmax, int cols, int rows,
                             double *partials, const int *flag, int tstarts) {
+  wait_previous();
   if (flag && *flag != 0)
     return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -644,6 +648,7 @@ __global__ void __launch_bounds__(256)
     wilson_gauge_q_kernel(const __grid_constant__ Geom g, const __grid_constant__ Fields4 U,
                           int NE, int rmin, int rmax, int tmin, int tmax, int cols, int rows,
                           double *partials, const int *flag, int tstarts) {
+  wait_previous();
   if (flag && *flag != 0)
     return;
   using Q = SU2<CT>;
@@ -755,6 +760,7 @@ __global__ void __launch_bounds__(256)
 __global__ void __launch_bounds__(256)
     reduce_select_kernel(const double *partials, int blocks_exact, int blocks_gauge,
                          const int *flag, int nr, int nt, double scale, double *out) {
+  wait_previous();
   __shared__ double sh[256];
   const int e = blockIdx.x;
   const int nblocks = *flag ? blocks_exact : blocks_gauge;
@@ -946,19 +952,20 @@ int launch_gauge_lines(const Geom &g, const AxisMap &map, const void *Ut, const 
   const double most = sizeof(CT) == 8 ? 100 * tol : tol;
   const int blocks = (g.Vs + kLinesCols - 1) / kLinesCols;
   if (g.Vs < 8192)
-    gauge_lines_kernel<Store, 4, MAPPED>
-        <<<blocks, 4 * kLinesCols, 0, s>>>(g, map, Ut, l.G, l.W, tol, most, flag);
+    launch_chained(gauge_lines_kernel<Store, 4, MAPPED>, blocks, 4 * kLinesCols, 0, s, g, map, Ut,
+                   l.G, l.W, tol, most, flag);
   else
-    gauge_lines_kernel<Store, 1, MAPPED>
-        <<<blocks, kLinesCols, 0, s>>>(g, map, Ut, l.G, l.W, tol, most, flag);
+    launch_chained(gauge_lines_kernel<Store, 1, MAPPED>, blocks, kLinesCols, 0, s, g, map, Ut, l.G,
+                   l.W, tol, most, flag);
   return launch_check("gauge_lines_kernel");
 }
 
 template <class Store, class CT, bool MAPPED>
 int launch_gauge_links(const Geom &g, const AxisMap &map, const Fields4 &U, const GaugeLinks &l,
                        const Fields4 &out, int ndir, int *flag, cudaStream_t s) {
-  gauge_transform_kernel<Store, MAPPED><<<dim3((l.NE * g.Vs + 127) / 128, ndir), 128, 0, s>>>(
-      g, map, U, l.G, l.W, out, l.NE, wilson_gauge_tolerance((int)sizeof(CT)), flag);
+  launch_chained(gauge_transform_kernel<Store, MAPPED>, dim3((l.NE * g.Vs + 127) / 128, ndir), 128,
+                 0, s, g, map, U, l.G, l.W, out, l.NE, wilson_gauge_tolerance((int)sizeof(CT)),
+                 flag);
   return launch_check("gauge_transform_kernel");
 }
 
@@ -1028,8 +1035,8 @@ int launch_wilson_gauge_kernel(const Geom &g, const GaugeLinks &l, int rmin, int
     int r = allow_large_smem(kernel, p.smem, capturing);
     if (r)
       return r;
-    kernel<<<dim3(p.blocks / 3, ndir), p.threads, p.smem, s>>>(
-        g, l.U, l.NE, rmin, rmax, tmin, tmax, p.cols_per_block, p.rows, partials, flag, tstarts);
+    launch_chained(kernel, dim3(p.blocks / 3, ndir), p.threads, p.smem, s, g, l.U, l.NE, rmin, rmax,
+                   tmin, tmax, p.cols_per_block, p.rows, partials, flag, tstarts);
     return GC_OK;
   };
   if constexpr (Store::NC == 2) {
@@ -1066,8 +1073,8 @@ int launch_wilson_gauge_kernel(const Geom &g, const GaugeLinks &l, int rmin, int
 int launch_reduce_select(const double *partials, int blocks_exact, int blocks_gauge,
                          const int *flag, int nr, int nt, double scale, double *out_dev,
                          cudaStream_t s) {
-  reduce_select_kernel<<<nr * nt, 256, 0, s>>>(partials, blocks_exact, blocks_gauge, flag, nr,
-                                               nt, scale, out_dev);
+  launch_chained(reduce_select_kernel, nr * nt, 256, 0, s, partials, blocks_exact, blocks_gauge,
+                 flag, nr, nt, scale, out_dev);
   return launch_check("reduce_select_kernel");
 }
 

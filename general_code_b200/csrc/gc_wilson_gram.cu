@@ -247,6 +247,7 @@ __global__ void __launch_bounds__(kGramThreads, 4)
     wilson_gram_kernel(const __grid_constant__ Geom g, const __grid_constant__ Fields4 U,
                        const __grid_constant__ Fields4 U2, int NE, int rmin, int rmax, int tmin,
                        int tmax, int cols, double *partials, const int *flag, int tstarts) {
+  wait_previous();
   // the exact product runs instead when a link failed the check
   if (flag && *flag != 0)
     return;
@@ -441,9 +442,9 @@ int launch_wilson_gram(const Geom &g, const GaugeLinks &l, const Fields4 *second
   auto go = [&](auto kernel) {
     const int rc = allow_large_smem(kernel, p.smem, cap != cudaStreamCaptureStatusNone);
     if (!rc)
-      kernel<<<dim3(p.blocks / 3, ndir), p.threads, p.smem, s>>>(
-          g, l.U, second ? *second : l.U, l.NE, rmin, rmax, tmin, tmax, p.cols_per_block,
-          partials, flag, tstarts);
+      launch_chained(kernel, dim3(p.blocks / 3, ndir), p.threads, p.smem, s, g, l.U,
+                     second ? *second : l.U, l.NE, rmin, rmax, tmin, tmax, p.cols_per_block,
+                     partials, flag, tstarts);
     return rc;
   };
   const int rc = second ? go(wilson_gram_kernel<Store, CT, true>)

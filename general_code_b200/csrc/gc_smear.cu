@@ -167,6 +167,90 @@ __device__ __forceinline__ Nbr neighbours(const Geom &g, int site,
 
 constexpr int kSmearBlock = 128;
 
+// ------------------------------------------------------ FP64 SU(3) staples
+// A thread of the FP64 SU(3) kernels holds the sum, a product and an operand
+// (108 registers), so that no register is left to load the next links ahead,
+// and at 16 warps on an SM the loads' latency shows. The ring keeps three links
+// per thread in shared memory, each copied there asynchronously one product
+// before it is used; a thread reads its own links only, so no barrier is
+// needed, and the product reads its operands from there as it goes. HYP levels
+// 2 and 3, which find 9-14% of their links in L1: at 24^4 317 -> 290 and 114 ->
+// 77 us (FP64 pipe 54 -> 62% and 34 -> 53%). The copies pass L1 by (through it:
+// a third slower), so APE and level 1, which find 22-31% there, lose by it
+// (APE 130 -> 139 us, level 1 265 -> 280) and keep plain loads.
+constexpr int kRingBlock = 96; // 41 KB: five blocks on an SM
+struct LinkRing {
+  double2 *own; // the thread's first element: element k of slot i at (9 i + k) kRingBlock
+  size_t V;
+  // starts the copy of a link into a slot (one group)
+  __device__ __forceinline__ void fetch(int slot, const void *f, int site) const {
+    const double2 *p = reinterpret_cast<const double2 *>(f) + site;
+    const unsigned d = (unsigned)__cvta_generic_to_shared(own + 9 * slot * kRingBlock);
+#pragma unroll
+    for (int k = 0; k < 9; k++)
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d + 16 * kRingBlock * k),
+                   "l"(p + k * V)
+                   : "memory");
+    commit();
+  }
+  __device__ __forceinline__ static void commit() {
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  }
+  // until at most `pending` of the copies are in flight
+  template <int pending> __device__ __forceinline__ static void wait() {
+    asm volatile("cp.async.wait_group %0;" ::"n"(pending) : "memory");
+  }
+  __device__ __forceinline__ SU3<double> get(int slot) const {
+    SU3<double> u;
+#pragma unroll
+    for (int k = 0; k < 9; k++) {
+      const double2 v = own[(9 * slot + k) * kRingBlock];
+      u.e[k / 3][k % 3] = {v.x, v.y};
+    }
+    return u;
+  }
+};
+// The links of one staple pair, as add_staples2 takes them.
+struct StapleLinks {
+  const void *fmu, *fnu;
+  int nu_x, mu_pnu, nu_pmu, nu_mnu, mu_mnu, nu_mnu_pmu;
+};
+// add_staples2 of the pairs links(0), links(1), ... links(n - 1) (the same
+// operations in the same order).
+template <class F>
+__device__ __forceinline__ void add_staples_ring(SU3<double> &S, const LinkRing &ring, int n,
+                                                 double c, F links) {
+  StapleLinks l = links(0);
+  ring.fetch(0, l.fnu, l.nu_x);
+  ring.fetch(1, l.fmu, l.mu_pnu);
+#pragma unroll 1
+  for (int j = 0; j < n; j++) {
+    ring.fetch(2, l.fnu, l.nu_pmu);
+    ring.wait<1>();
+    SU3<double> a = scale(mul(ring.get(0), ring.get(1)), c);
+    ring.fetch(0, l.fnu, l.nu_mnu);
+    ring.fetch(1, l.fmu, l.mu_mnu);
+    ring.wait<2>();
+    S = add(S, mul_ad(a, ring.get(2)));
+    ring.fetch(2, l.fnu, l.nu_mnu_pmu);
+    ring.wait<1>();
+    a = scale(mul_da(ring.get(0), ring.get(1)), c);
+    if (j + 1 < n) {
+      l = links(j + 1);
+      ring.fetch(0, l.fnu, l.nu_x);
+      ring.fetch(1, l.fmu, l.mu_pnu);
+    } else {
+      ring.commit();
+      ring.commit();
+    }
+    ring.wait<2>();
+    S = add(S, mul(a, ring.get(2)));
+  }
+}
+template <class Store> struct UsesRing {
+  static constexpr bool value = std::is_same<Store, StoreF64SU3>::value;
+};
+
 // ---------------------------------------------------- mixed SU(3) staples
 // The mixed form stores two rows of an SU(3) link and rebuilds the third as
 // conj(row0 x row1); a product of such links is again in SU(3), so a staple
@@ -377,6 +461,25 @@ __device__ __forceinline__ void hyp_l2_site(const Geom &g, const Fields4 &U,
   proj_store<I>(out.f[f], d.VR, site + (temporal ? d.q0 : d.o0), S);
 }
 
+__device__ __forceinline__ void hyp_l2_site_ring(const Geom &g, const Fields4 &U, const HypL1 &l1,
+                                                 const HypL2 &out, double alpha2, int site, int f,
+                                                 const LinkRing &ring) {
+  int x[4];
+  smear_coords<StoreF64SU3>(g, site, x);
+  const bool temporal = f < 3;
+  const int nu = temporal ? f : f - 3;
+  const int mu = temporal ? 3 : nu;
+  SU3<double> S = scale(StoreF64SU3::load<double>(U.f[mu], g.V, site), 1 - alpha2);
+  add_staples_ring(S, ring, 2, alpha2 / 4, [&](int j) {
+    const int rho = j + (j >= nu);
+    const Nbr n = neighbours(g, site, x, mu, rho);
+    return StapleLinks{temporal ? l1.f[l1_temporal(nu, rho)] : l1.f[l1_spatial(nu, rho)],
+                       l1.f[l1_spatial(rho, nu)],
+                       site, n.pnu, n.pmu, n.mnu, n.mnu, n.mnu_pmu};
+  });
+  proj_store<StoreF64SU3>(out.f[f], g.V, site, S);
+}
+
 // Level 3: the new temporal link (smearing.h:484-503). Reads the level-2
 // temporal links on the site's slice and the level-2 spatial links on it and
 // on the slice above.
@@ -398,6 +501,19 @@ __device__ __forceinline__ void hyp_l3_site(const Geom &g, const void *Ut,
         n.mnu + d.o0, n.mnu + d.q0, n.mnu_pmu + d.o1, c);
   }
   proj_store<Store>(out_t, V, site, S);
+}
+
+__device__ __forceinline__ void hyp_l3_site_ring(const Geom &g, const void *Ut, const HypL2 &l2,
+                                                 void *out_t, double alpha1, int site,
+                                                 const LinkRing &ring) {
+  int x[4];
+  smear_coords<StoreF64SU3>(g, site, x);
+  SU3<double> S = scale(StoreF64SU3::load<double>(Ut, g.V, site), 1 - alpha1);
+  add_staples_ring(S, ring, 3, alpha1 / 6, [&](int nu) {
+    const Nbr n = neighbours(g, site, x, 3, nu);
+    return StapleLinks{l2.f[nu], l2.f[3 + nu], site, n.pnu, n.pmu, n.mnu, n.mnu, n.mnu_pmu};
+  });
+  proj_store<StoreF64SU3>(out_t, g.V, site, S);
 }
 
 // One APE step of SU(2) at a site, all three spatial links: the staples of
@@ -495,25 +611,37 @@ __global__ void __launch_bounds__(128, 4)
 }
 
 template <class Store, class CT>
-__global__ void __launch_bounds__(128, 4)
+__global__ void __launch_bounds__(UsesRing<Store>::value ? kRingBlock : 128,
+                                  UsesRing<Store>::value ? 5 : 4)
     hyp_level2_kernel(Geom g, const __grid_constant__ Fields4 U,
                       const __grid_constant__ HypL1 l1,
                       const __grid_constant__ HypL2 out, double alpha2) {
   wait_previous();
   const int f = blockIdx.x % 6;
   const int site = (blockIdx.x / 6) * blockDim.x + threadIdx.x;
-  if (site < g.V)
+  if constexpr (UsesRing<Store>::value) {
+    __shared__ __align__(16) double2 links[27 * kRingBlock];
+    if (site < g.V)
+      hyp_l2_site_ring(g, U, l1, out, alpha2, site, f, LinkRing{links + threadIdx.x, (size_t)g.V});
+  } else if (site < g.V) {
     hyp_l2_site<Store, CT>(g, U, l1, out, alpha2, site, f, whole_lattice(g));
+  }
 }
 
 template <class Store, class CT>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(UsesRing<Store>::value ? kRingBlock : 128,
+                                  UsesRing<Store>::value ? 5 : 1)
     hyp_level3_kernel(Geom g, const void *Ut, const __grid_constant__ HypL2 l2,
                       void *out_t, double alpha1) {
   wait_previous();
   const int site = blockIdx.x * blockDim.x + threadIdx.x;
-  if (site < g.V)
+  if constexpr (UsesRing<Store>::value) {
+    __shared__ __align__(16) double2 links[27 * kRingBlock];
+    if (site < g.V)
+      hyp_l3_site_ring(g, Ut, l2, out_t, alpha1, site, LinkRing{links + threadIdx.x, (size_t)g.V});
+  } else if (site < g.V) {
     hyp_l3_site<Store, CT>(g, Ut, l2, out_t, alpha1, site, whole_lattice(g));
+  }
 }
 
 // ------------------------------------------------------ HYP slice pipeline
@@ -721,15 +849,18 @@ int launch_hyp(const Geom &g, const Fields4 &U, const HypL1 &l1,
                const HypL2 &l2, void *out_t, double a1, double a2, double a3,
                cudaStream_t s) {
   const int nb = (g.V + kSmearBlock - 1) / kSmearBlock;
+  // (levels 2 and 3: the block of the kernels with a ring)
+  constexpr int block = UsesRing<Store>::value ? kRingBlock : kSmearBlock;
+  const int nb2 = (g.V + block - 1) / block;
   launch_chained(hyp_level1_kernel<Store, CT>, nb * 9, kSmearBlock, 0, s, g, U, l1, a3);
   int rc = launch_check("hyp_level1_kernel");
   if (rc)
     return rc;
-  launch_chained(hyp_level2_kernel<Store, CT>, nb * 6, kSmearBlock, 0, s, g, U, l1, l2, a2);
+  launch_chained(hyp_level2_kernel<Store, CT>, nb2 * 6, block, 0, s, g, U, l1, l2, a2);
   rc = launch_check("hyp_level2_kernel");
   if (rc)
     return rc;
-  launch_chained(hyp_level3_kernel<Store, CT>, nb, kSmearBlock, 0, s, g, U.f[3], l2, out_t, a1);
+  launch_chained(hyp_level3_kernel<Store, CT>, nb2, block, 0, s, g, U.f[3], l2, out_t, a1);
   return launch_check("hyp_level3_kernel");
 }
 

@@ -94,8 +94,9 @@ def algorithmic(wl, form, w_method="exact"):
     """Algorithmic bytes and FP flops per site for each kernel family. W's
     flops are those of the method that ran: the exact product (two products
     and a dot per (x, nu, R, T)) or the temporal-gauge form (per site: the
-    gauge lines of two cuts, the six transformed links, per (nu, R) one
-    product per cut for the space lines, per (nu, R, T) one dot)."""
+    gauge line; on the Lt + T_max slices of the extended lattice the three
+    transformed links and per (nu, R) one product for the space lines; per
+    (nu, R, T) one dot)."""
     nc = wl["nc"]
     b = link_bytes(nc, form)
     mm = 198 if nc == 3 else 28          # one matrix product
@@ -104,7 +105,8 @@ def algorithmic(wl, form, w_method="exact"):
     nr = wl["r"][1] - wl["r"][0] + 1
     nt = wl["t"][1] - wl["t"][0] + 1
     if w_method == "gauge":
-        w_flops = 2 * mm + 3 * 2 * 2 * mm + 3 * (2 * wl["r"][1] * mm + nr * nt * dot)
+        ext = 1 + wl["t"][1] / wl["dims"][3]
+        w_flops = mm + 3 * ext * (2 + wl["r"][1]) * mm + 3 * nr * nt * dot
     else:
         w_flops = 3 * nr * nt * (2 * mm + dot)
     return {

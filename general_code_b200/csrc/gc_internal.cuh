@@ -255,9 +255,9 @@ int plan_error(const char *what);
 // Launches of one chain on a stream. A kernel launched by launch_chained is
 // set up while the memory of the one before it drains: its blocks start when
 // that kernel's have exited and wait (wait_previous, the first statement of
-// every kernel launched this way) until its writes are visible. Saves about 2.4 us of
-// each launch's 4 us gap (an APE step, us: SU(2) mixed 16^4 6.4 -> 3.9, SU(3)
-// mixed 16^4 18.8 -> 16.1, 32^4 215 -> 212.6). Letting the next kernel start
+// every kernel launched this way) until its writes are visible. Saves about 2.4 us a
+// launch (an APE step, us: SU(2) mixed 16^4 6.4 -> 3.9, SU(3) mixed 16^4 18.8 ->
+// 16.1, 32^4 215 -> 212.6). Letting the next kernel start
 // earlier (a trigger at the blocks' start) measured the same. Under stream
 // capture the launch is an ordinary one.
 __device__ __forceinline__ void wait_previous() {

@@ -485,7 +485,8 @@ struct Rows01Set {
 // (128 registers, a few spilled): 8 warps at 175 registers took a fifth more.
 // Bound by the FMA pipe's operands and the latency of the sweep (0.6
 // instructions per cycle and scheduler). With one set of Lt + T_max lines
-// instead of two cuts of Lt: 24^3 x 48, T <= 12, 1.42 -> 1.34 ms.
+// instead of two cuts of Lt: 24^3 x 48, T <= 12, 1.42 -> 1.34 ms (a size that
+// wilson_corr_kernel has now, 1.04 ms at T <= 24).
 // Partials, block sums and the per-thread FP32 loop sums as
 // wilson_gauge_kernel.
 template <int KS, bool SLAB>

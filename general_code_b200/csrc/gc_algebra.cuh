@@ -439,7 +439,13 @@ template <class T> GC_HD SU2<T> proj(const SU2<T> &A, T) { return proj(A); }
 // true) only inside a region where the six steps end within 1e-14 of the
 // limit: 0.25 <= m <= 1.001, p m >= 0.24 with p = det(1 - E), and a phase
 // below 0.7 (checked over 30 million singular values and phases up to the
-// region's edge: 4e-15). Sums of SU(3) matrices with weights that add to one
+// region's edge: 4e-15). Inside it the polynomial's own loops may not converge
+// either: where one singular value is 1.52 to 1.535 times the rms and the others
+// are equal, E reaches -1.36, the series starts near its zero at -1.366, and
+// eight Newton steps (a factor 1.5 each from there) do not reach the root. A
+// loop that ends at its cap answers false as well (3 million matrices with a
+// singular value from 1 to 1.535 times the rms: 2.3e-15 in FP64, 1.4e-6 in
+// FP32; at the cap the error was 0.45). Sums of SU(3) matrices with weights that add to one
 // have m <= 1; of HYP's level-1 sums on a rough field (plaquette 0.6) less
 // than 1% lie outside, of APE sums none. Elsewhere U is left unset and the
 // caller takes the reference's steps.
@@ -530,6 +536,7 @@ template <class T> GC_HD bool polar_su3(const SU3<T> &A, SU3<T> &U) {
   T x1 = GC_FMA(T(35.0 / 128.0), d, GC_FMA(GC_FMA(c5, q, T(0.3125)), q, T(0.5)));
   T x2 = GC_FMA(c5, d, GC_FMA(T(35.0 / 128.0), q, T(0.375)));
   // (the series' error is 0.23 |E|^6: below T's rounding it needs no step)
+  T rn = T(0);
 #pragma unroll 1
   for (int it = 0; it < 8 && q > PolarTol<T>::series; it++) {
     // s = x^2, r = 1 - s + E s
@@ -540,7 +547,7 @@ template <class T> GC_HD bool polar_su3(const SU3<T> &A, SU3<T> &U) {
     const T r0 = GC_FMA(d, s2, T(1) - s0);
     const T r1 = GC_FMA(q, s2, s0 - s1);
     const T r2 = s1 - s2;
-    const T rn = fabs(r0) + (fabs(r1) + fabs(r2));
+    rn = fabs(r0) + (fabs(r1) + fabs(r2));
     // x += x r / 2
     const T p3 = GC_FMA(x1, r2, x2 * r1), p4 = x2 * r2;
     const T p0 = GC_FMA(d, p3, x0 * r0);
@@ -561,15 +568,20 @@ template <class T> GC_HD bool polar_su3(const SU3<T> &A, SU3<T> &U) {
   cx<T> z = cmul(t, w1);
   z.re += T(1);
   // (error 0.17 |w1|^3)
+  T gn = T(0);
 #pragma unroll 1
   for (int it = 0; it < 8 && fabs(w1.re) + fabs(w1.im) > PolarTol<T>::cube; it++) {
     const cx<T> r = cmul(cmul(cmul(z, z), z), w);
     const cx<T> g = {T(1) - r.re, -r.im}; // 1 - z^3 w
     const cx<T> u = {GC_FMA(T(1.0 / 3.0), g.re, T(1)), T(1.0 / 3.0) * g.im};
     z = cmul(z, u);
-    if (!(fabs(g.re) + fabs(g.im) > PolarTol<T>::value))
+    gn = fabs(g.re) + fabs(g.im);
+    if (!(gn > PolarTol<T>::value))
       break;
   }
+  // a loop ended at its cap (see above)
+  if (rn > PolarTol<T>::value || gn > PolarTol<T>::value)
+    return false;
   // X = rs (x0 + x1 E + x2 F); F off the diagonal: -e2 a + b conj(c),
   // -e1 b + a c, -e0 c + conj(a) b
   x0 *= rs;

@@ -7,6 +7,7 @@
 
 #include "../../include/gc_lattice.h"
 #include "gc_internal.cuh"
+#include "gc_offaxis_tree.h"
 
 #include <array>
 #include <vector>
@@ -301,13 +302,6 @@ int launch_reduce_rows(const double *partials, int blocks, int n, double scale,
 
 // ------------------------------------------------------------ off-axis loops
 constexpr int kOffaxisMaxSteps = 256;
-// A space line's links, in order (OffaxisLine::pattern, OffaxisLineDesc::s):
-// +a steps forward along axis a-1 (1..3), -a steps back and takes the
-// link's adjoint.
-struct OffaxisLine {
-  std::vector<int> pattern;
-  int disp[3];
-};
 // Device table entry of one line for the fused kernel: its steps and the
 // displacement of its end as non-negative residues.
 struct OffaxisLineDesc {
@@ -348,30 +342,8 @@ int launch_offaxis_fused(const Geom &g, const Fields4 &U, const OffaxisLineDesc 
 // Column blocks of the fused launch (rows of its partials) for a lattice.
 int offaxis_fused_blocks(const Geom &g, int nc, int ct_bytes);
 
-// The same loops in the temporal gauge (gc_offaxis_gauge.cu). The lines with
-// equal step patterns are one line, and lines that begin alike share the
-// product of the common steps: the patterns form a tree, one node per step.
-struct OffaxisNode {
-  int d[3];          // site of the node's link, as a residue displacement from the start
-  int line;          // distinct line that ends here, or -1
-  signed char axis;  // the link's axis
-  signed char back;  // 1: a step back (the link's adjoint)
-  signed char from;  // product extended: -1 the previous node's, >= 0 that stack level's,
-                     // -2 none (first step)
-  signed char push;  // stack level that keeps this node's product, or -1
-  int pad[3];
-};
-struct OffaxisTree {
-  std::vector<int> distinct;       // plan line -> distinct line
-  std::vector<int> first;          // distinct line -> a plan line
-  std::vector<OffaxisNode> nodes;  // chunk after chunk
-  std::vector<int> chunk_nodes;    // first node of each chunk, and the end
-  std::vector<int> chunk_lines;    // first distinct line of each chunk, and the end
-};
-// Distinct lines are numbered in tree order; each chunk of at most
-// lines_per_chunk of them walks its own part of the tree. Empty nodes: a line
-// needs more stack levels than the kernel keeps.
-OffaxisTree offaxis_tree(const Geom &g, const OffaxisPlan &plan, int lines_per_chunk);
+// The same loops in the temporal gauge (gc_offaxis_gauge.cu), over the tree of
+// gc_offaxis_tree.h.
 // Blocks of columns (rows of partials) of the gauge launch, 0 when its block
 // does not fit (long time extents).
 int offaxis_gauge_blocks(const Geom &g, int nc, int ct_bytes, int tmin, int tmax, bool adjoint);

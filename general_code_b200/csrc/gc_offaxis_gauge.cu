@@ -37,14 +37,11 @@
 #include "gc_wcol.cuh"
 
 #include <algorithm>
-#include <map>
 #include <type_traits>
 
 namespace gc {
 
 namespace {
-
-constexpr int kTreeStack = 12;
 
 // A line slot's matrix in shared memory: planes of 16-byte vectors (and one
 // of 8 bytes for the 18 reals of an FP32 SU(3) matrix) over the block's slots.
@@ -312,131 +309,5 @@ GC_INSTANTIATE_OG(StoreF64SU3, double)
 GC_INSTANTIATE_OG(StoreF64SU2, double)
 GC_INSTANTIATE_OG(StoreF32SU3, float)
 GC_INSTANTIATE_OG(StoreF32SU2, float)
-
-// ------------------------------------------------------------------ host tree
-namespace {
-
-struct TreeNode {
-  int step = 0, line = -1, weight = 0; // weight: nodes of the subtree
-  std::vector<int> children;
-};
-
-// Children in walking order: the largest subtree last (its products need no
-// stack level below it), the others by size, equal sizes by step.
-void order_children(std::vector<TreeNode> &t, int n) {
-  t[n].weight = 1;
-  for (int c : t[n].children) {
-    order_children(t, c);
-    t[n].weight += t[c].weight;
-  }
-  std::sort(t[n].children.begin(), t[n].children.end(), [&](int a, int b) {
-    return t[a].weight != t[b].weight ? t[a].weight < t[b].weight : t[a].step < t[b].step;
-  });
-}
-
-int add_line(std::vector<TreeNode> &t, const std::vector<int> &steps) {
-  int n = 0;
-  for (int e : steps) {
-    int next = -1;
-    for (int c : t[n].children)
-      if (t[c].step == e)
-        next = c;
-    if (next < 0) {
-      next = (int)t.size();
-      t[n].children.push_back(next);
-      t.emplace_back();
-      t[next].step = e;
-    }
-    n = next;
-  }
-  return n;
-}
-
-} // namespace
-
-OffaxisTree offaxis_tree(const Geom &g, const OffaxisPlan &plan, int lines_per_chunk) {
-  OffaxisTree out;
-  // all distinct lines, numbered in the order of a walk of their tree
-  std::vector<TreeNode> all(1);
-  std::vector<int> end(plan.lines.size()), first_of;
-  for (size_t i = 0; i < plan.lines.size(); i++) {
-    end[i] = add_line(all, plan.lines[i].pattern);
-    if (all[end[i]].line < 0)
-      all[end[i]].line = (int)i; // (a plan line with this pattern)
-  }
-  order_children(all, 0);
-  std::vector<int> number(all.size(), -1), todo{0};
-  while (!todo.empty()) {
-    const int n = todo.back();
-    todo.pop_back();
-    if (all[n].line >= 0) {
-      number[n] = (int)out.first.size();
-      out.first.push_back(all[n].line);
-    }
-    for (size_t k = all[n].children.size(); k-- > 0;)
-      todo.push_back(all[n].children[k]);
-  }
-  for (size_t i = 0; i < plan.lines.size(); i++)
-    out.distinct.push_back(number[end[i]]);
-  // each chunk of consecutive lines as a walk of its own tree
-  const int total = (int)out.first.size();
-  for (int l0 = 0; l0 < total; l0 += lines_per_chunk) {
-    const int l1 = std::min(total, l0 + lines_per_chunk);
-    std::vector<TreeNode> t(1);
-    for (int l = l0; l < l1; l++)
-      t[add_line(t, plan.lines[out.first[l]].pattern)].line = l;
-    order_children(t, 0);
-    out.chunk_nodes.push_back((int)out.nodes.size());
-    out.chunk_lines.push_back(l0);
-    struct Visit {
-      int node, parent_level; // stack level of the parent's product, -1: in registers
-      int level;              // first free stack level
-      int pos[3];             // displacement of the parent's end
-    };
-    // depth first; a node with several children keeps its product on a level
-    // until the last of them, which continues from the stack as well
-    std::vector<Visit> visits;
-    for (size_t k = t[0].children.size(); k-- > 0;)
-      visits.push_back({t[0].children[k], -2, 0, {0, 0, 0}});
-    while (!visits.empty()) {
-      const Visit v = visits.back();
-      visits.pop_back();
-      const TreeNode &tn = t[v.node];
-      OffaxisNode q{};
-      const int axis = std::abs(tn.step) - 1;
-      int at[3] = {v.pos[0], v.pos[1], v.pos[2]}, to[3] = {v.pos[0], v.pos[1], v.pos[2]};
-      if (tn.step > 0)
-        to[axis] += 1;
-      else
-        at[axis] -= 1, to[axis] -= 1;
-      for (int k = 0; k < 3; k++)
-        q.d[k] = ((at[k] % g.L[k]) + g.L[k]) % g.L[k];
-      q.line = tn.line;
-      q.axis = (signed char)axis;
-      q.back = tn.step < 0;
-      q.from = (signed char)v.parent_level;
-      const size_t nch = tn.children.size();
-      q.push = -1;
-      if (nch > 1) {
-        if (v.level >= kTreeStack) {
-          out.nodes.clear();
-          return out;
-        }
-        q.push = (signed char)v.level;
-      }
-      out.nodes.push_back(q);
-      for (size_t k = nch; k-- > 0;) {
-        // the first child follows at once (registers); the others find the
-        // product on the stack, and the last one frees its level
-        Visit w{tn.children[k], k == 0 ? -1 : (int)q.push, 0, {to[0], to[1], to[2]}};
-        w.level = nch > 1 && k + 1 < nch ? v.level + 1 : v.level;
-        visits.push_back(w);
-      }
-    }
-  }
-  out.chunk_nodes.push_back((int)out.nodes.size());
-  out.chunk_lines.push_back(total);
-  return out;
-}
 
 } // namespace gc

@@ -435,8 +435,8 @@ template <class T> GC_HD SU2<T> proj(const SU2<T> &A, T) { return proj(A); }
 // The reference takes exactly six matrix steps, which reach the limit only
 // for sums not too far from a multiple of an SU(3) matrix. The steps act on
 // the three singular values and the determinant's phase alone, so where they
-// converge is a property of four numbers, and polar_su3 answers (returns
-// true) only inside a region where the six steps end within 1e-14 of the
+// converge is a property of four numbers, and polar_parts (U = z Y) answers
+// (returns true) only inside a region where the six steps end within 1e-14 of the
 // limit: 0.25 <= m <= 1.001, p m >= 0.24 with p = det(1 - E), and a phase
 // below 0.7 (checked over 30 million singular values and phases up to the
 // region's edge: 4e-15). Inside it the polynomial's own loops may not converge
@@ -447,8 +447,8 @@ template <class T> GC_HD SU2<T> proj(const SU2<T> &A, T) { return proj(A); }
 // singular value from 1 to 1.535 times the rms: 2.3e-15 in FP64, 1.4e-6 in
 // FP32; at the cap the error was 0.45). Sums of SU(3) matrices with weights that add to one
 // have m <= 1; of HYP's level-1 sums on a rough field (plaquette 0.6) less
-// than 1% lie outside, of APE sums none. Elsewhere U is left unset and the
-// caller takes the reference's steps.
+// than 1% lie outside, of APE sums none. Elsewhere the result is not set and
+// the caller takes the reference's steps.
 GC_HD double gc_rsqrt(double x) {
 #if defined(__CUDA_ARCH__)
   return rsqrt(x);
@@ -475,7 +475,7 @@ template <> struct PolarTol<float> {
   static constexpr float value = 2e-4f, series = 2e-3f, cube = 4e-3f;
 };
 
-template <class T> GC_HD bool polar_su3(const SU3<T> &A, SU3<T> &U) {
+template <class T> GC_HD bool polar_parts(const SU3<T> &A, SU3<T> &Y, cx<T> &z) {
   // H = A^dag A: diagonal h, off-diagonal (0,1), (0,2), (1,2)
   T h[3];
   cx<T> o[3];
@@ -565,7 +565,7 @@ template <class T> GC_HD bool polar_su3(const SU3<T> &A, SU3<T> &U) {
   const cx<T> w1 = {GC_FMA(D.re, wn, T(-1)), w.im};
   // (1 + t)^(-1/3) = 1 - t/3 + 2/9 t^2
   const cx<T> t = {GC_FMA(T(2.0 / 9.0), w1.re, T(-1.0 / 3.0)), T(2.0 / 9.0) * w1.im};
-  cx<T> z = cmul(t, w1);
+  z = cmul(t, w1);
   z.re += T(1);
   // (error 0.17 |w1|^3)
   T gn = T(0);
@@ -583,10 +583,23 @@ template <class T> GC_HD bool polar_su3(const SU3<T> &A, SU3<T> &U) {
   if (rn > PolarTol<T>::value || gn > PolarTol<T>::value)
     return false;
   // X = rs (x0 + x1 E + x2 F); F off the diagonal: -e2 a + b conj(c),
-  // -e1 b + a c, -e0 c + conj(a) b
-  x0 *= rs;
-  x1 *= rs;
-  x2 *= rs;
+  // -e1 b + a c, -e0 c + conj(a) b. FP32: the factor rs x0 goes to z, so that
+  // polar_finish (FP64) multiplies Y by a number that is not 1. With z = 1 on a
+  // smooth field U would be Y, on the grid of FP32, where an update below half a
+  // rounding has no effect, and the common error of Y's scalars would stay in
+  // every link (mean of U U^dag - 1 after 20 APE steps 1e-9, against 5e-11).
+  if constexpr (sizeof(T) == 4) {
+    const T ix = T(1) / x0, scale = rs * x0;
+    x0 = T(1);
+    x1 *= ix;
+    x2 *= ix;
+    z.re *= scale;
+    z.im *= scale;
+  } else {
+    x0 *= rs;
+    x1 *= rs;
+    x2 *= rs;
+  }
   const cx<T> bc = cmul_c(b, c), ab = cmulc(a, b);
   const T X0 = GC_FMA(x2, f0, GC_FMA(x1, e0, x0)), X1 = GC_FMA(x2, f1, GC_FMA(x1, e1, x0)),
           X2 = GC_FMA(x2, f2, GC_FMA(x1, e2, x0));
@@ -596,21 +609,30 @@ template <class T> GC_HD bool polar_su3(const SU3<T> &A, SU3<T> &U) {
   const cx<T> Xc = {GC_FMA(x2, ab.re, kc * c.re), GC_FMA(x2, ab.im, kc * c.im)};
 #pragma unroll
   for (int i = 0; i < 3; i++) {
-    // row i of A X, times z
+    // row i of A X: the small terms first, so that one product and sum is
+    // rounded at full size
     const cx<T> r0 = A.e[i][0], r1 = A.e[i][1], r2 = A.e[i][2];
-    cx<T> y0 = {r0.re * X0, r0.im * X0};
-    y0 = cmadd(y0, r1, {Xa.re, -Xa.im});
-    y0 = cmadd(y0, r2, {Xb.re, -Xb.im});
-    cx<T> y1 = {r1.re * X1, r1.im * X1};
-    y1 = cmadd(y1, r0, Xa);
-    y1 = cmadd(y1, r2, {Xc.re, -Xc.im});
-    cx<T> y2 = {r2.re * X2, r2.im * X2};
-    y2 = cmadd(y2, r0, Xb);
-    y2 = cmadd(y2, r1, Xc);
-    U.e[i][0] = cmul(z, y0);
-    U.e[i][1] = cmul(z, y1);
-    U.e[i][2] = cmul(z, y2);
+    const cx<T> y0 = cmadd(cmul_c(r1, Xa), r2, {Xb.re, -Xb.im});
+    const cx<T> y1 = cmadd(cmul(r0, Xa), r2, {Xc.re, -Xc.im});
+    const cx<T> y2 = cmadd(cmul(r0, Xb), r1, Xc);
+    Y.e[i][0] = {GC_FMA(r0.re, X0, y0.re), GC_FMA(r0.im, X0, y0.im)};
+    Y.e[i][1] = {GC_FMA(r1.re, X1, y1.re), GC_FMA(r1.im, X1, y1.im)};
+    Y.e[i][2] = {GC_FMA(r2.re, X2, y2.re), GC_FMA(r2.im, X2, y2.im)};
   }
+  return true;
+}
+
+// z y, rounded once at full size where z is nearly real
+template <class T> GC_HD cx<T> cphase(cx<T> z, cx<T> y) {
+  return {GC_FMA(z.re, y.re, -z.im * y.im), GC_FMA(z.re, y.im, z.im * y.re)};
+}
+template <class T> GC_HD bool polar_su3(const SU3<T> &A, SU3<T> &U) {
+  cx<T> z;
+  if (!polar_parts(A, U, z))
+    return false;
+#pragma unroll
+  for (int k = 0; k < 9; k++)
+    U.e[k / 3][k % 3] = cphase(z, U.e[k / 3][k % 3]);
   return true;
 }
 
@@ -646,44 +668,43 @@ template <class T> GC_HD SU3<T> ns_until(SU3<T> B, T tol, int max_steps, int *st
   return B;
 }
 
-// The FP32 result of polar_su3 made unitary with determinant 1 to FP64
-// accuracy, rounded to FP32 once: with G = U U^dag (FP64, of the FP32 values)
-// and the determinant's phase, U += (-(G - 1)/2 - i Im(det U)/3) U to first
-// order; the defect is a few 1e-7, so the second order is below 1e-12 and the
-// update itself can be formed in FP32. Rows 0 and 1, and row 2 with ROW2 (the
-// 12-real links rebuild it). Without this step the FP32 rounding left in G
-// enters every loop.
-template <bool ROW2> GC_HD SU3<float> polar_finish(const SU3<float> &U) {
-  SU3<double> V;
+// The FP32 parts of polar_parts, U = z Y, made unitary with determinant 1 to FP64
+// accuracy and rounded to FP32 once: with G = U U^dag and the determinant's
+// phase, U += (-(G - 1)/2 - i Im(det U)/3) U to first order; the defect is a few
+// 1e-7, so the second order is below 1e-12. Rows 0 and 1, and row 2 with ROW2
+// (the 12-real links rebuild it).
+template <bool ROW2> GC_HD SU3<float> polar_finish(const SU3<float> &Y, cx<float> z) {
+  const cx<double> zd = {double(z.re), double(z.im)};
+  SU3<double> U;
 #pragma unroll
   for (int k = 0; k < 9; k++)
-    V.e[k / 3][k % 3] = {double(U.e[k / 3][k % 3].re), double(U.e[k / 3][k % 3].im)};
-  cx<float> c[3][3];
+    U.e[k / 3][k % 3] = cphase(zd, {double(Y.e[k / 3][k % 3].re), double(Y.e[k / 3][k % 3].im)});
+  cx<double> c[3][3];
 #pragma unroll
   for (int i = 0; i < 3; i++)
 #pragma unroll
     for (int k = i; k < 3; k++) {
       if (i == 2 && !ROW2)
         continue;
-      double re = i == k ? GC_FMA(V.e[i][0].re, V.e[k][0].re, -1.0) : V.e[i][0].re * V.e[k][0].re;
-      re = GC_FMA(V.e[i][0].im, V.e[k][0].im, re);
+      double re = i == k ? GC_FMA(U.e[i][0].re, U.e[k][0].re, -1.0) : U.e[i][0].re * U.e[k][0].re;
+      re = GC_FMA(U.e[i][0].im, U.e[k][0].im, re);
 #pragma unroll
       for (int j = 1; j < 3; j++) {
-        re = GC_FMA(V.e[i][j].re, V.e[k][j].re, re);
-        re = GC_FMA(V.e[i][j].im, V.e[k][j].im, re);
+        re = GC_FMA(U.e[i][j].re, U.e[k][j].re, re);
+        re = GC_FMA(U.e[i][j].im, U.e[k][j].im, re);
       }
       if (i == k) {
-        c[i][i] = {-0.5f * float(re), 0.f};
+        c[i][i] = {-0.5 * re, 0.0};
         continue;
       }
-      double im = V.e[i][0].im * V.e[k][0].re;
-      im = GC_FMA(-V.e[i][0].re, V.e[k][0].im, im);
+      double im = U.e[i][0].im * U.e[k][0].re;
+      im = GC_FMA(-U.e[i][0].re, U.e[k][0].im, im);
 #pragma unroll
       for (int j = 1; j < 3; j++) {
-        im = GC_FMA(V.e[i][j].im, V.e[k][j].re, im);
-        im = GC_FMA(-V.e[i][j].re, V.e[k][j].im, im);
+        im = GC_FMA(U.e[i][j].im, U.e[k][j].re, im);
+        im = GC_FMA(-U.e[i][j].re, U.e[k][j].im, im);
       }
-      c[i][k] = {-0.5f * float(re), -0.5f * float(im)};
+      c[i][k] = {-0.5 * re, -0.5 * im};
       c[k][i] = {c[i][k].re, -c[i][k].im};
     }
   // Im det = Im sum_j (row0 x row1)_j row2_j
@@ -691,21 +712,21 @@ template <bool ROW2> GC_HD SU3<float> polar_finish(const SU3<float> &U) {
 #pragma unroll
   for (int j = 0; j < 3; j++) {
     const int a = (j + 1) % 3, b = (j + 2) % 3;
-    const cx<double> x = cmul_sub(V.e[0][a], V.e[1][b], V.e[0][b], V.e[1][a]);
-    di = GC_FMA(x.re, V.e[2][j].im, di);
-    di = GC_FMA(x.im, V.e[2][j].re, di);
+    const cx<double> x = cmul_sub(U.e[0][a], U.e[1][b], U.e[0][b], U.e[1][a]);
+    di = GC_FMA(x.re, U.e[2][j].im, di);
+    di = GC_FMA(x.im, U.e[2][j].re, di);
   }
-  const float ph = float(di * (-1.0 / 3.0));
+  const double ph = di * (-1.0 / 3.0);
   SU3<float> R;
 #pragma unroll
   for (int i = 0; i < (ROW2 ? 3 : 2); i++) {
     c[i][i].im = ph;
 #pragma unroll
     for (int j = 0; j < 3; j++) {
-      cx<float> s = cmul(c[i][0], U.e[0][j]);
+      cx<double> s = cmadd(U.e[i][j], c[i][0], U.e[0][j]);
       s = cmadd(s, c[i][1], U.e[1][j]);
       s = cmadd(s, c[i][2], U.e[2][j]);
-      R.e[i][j] = {U.e[i][j].re + s.re, U.e[i][j].im + s.im};
+      R.e[i][j] = {float(s.re), float(s.im)};
     }
   }
   return R;

@@ -101,8 +101,9 @@ __device__ __forceinline__ void proj_store(void *out, size_t V, int site, const 
   using MD = typename Store::template M<double>;
   if constexpr (MixedSU3<Store>::value) {
     SU3<float> U;
-    if (polar_su3(S, U)) {
-      U = polar_finish<Store::kBytes == 72>(U);
+    cx<float> z;
+    if (polar_parts(S, U, z)) {
+      U = polar_finish<Store::kBytes == 72>(U, z);
     } else {
       U = S;
       proj_steps<NORM>(U);

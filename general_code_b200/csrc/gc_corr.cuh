@@ -41,11 +41,13 @@ template <> struct CorrVec<double> {
 // acc[j] += sum_{t < tstarts} s[t] s[t + T + j], j < J (a multiple of V). s is
 // 16-byte aligned, T = 1 modulo V; reads s up to the vector of index
 // tstarts - 1 + T + J - 1 (finite values there). OWN (T = 1): the starts are
-// the window's first vector.
+// the window's first vector. FP32 sums the products of eight starts (two
+// vectors) at a time and adds those sums.
 template <class CT, int J, bool OWN>
 __device__ __forceinline__ void correlate(const CT *s, int T, int tstarts, CT (&acc)[J]) {
   using CV = CorrVec<CT>;
   constexpr int V = CV::V, N = J / V + 1;
+  constexpr bool kGroups = sizeof(CT) == 4;
   static_assert(J % V == 0, "whole vectors");
   const CT *b = s + (T - 1);
   CT w[N][V];
@@ -53,12 +55,18 @@ __device__ __forceinline__ void correlate(const CT *s, int T, int tstarts, CT (&
   for (int i = 0; i < N - 1; i++)
     CV::load(b + i * V, w[i]);
   const int full = tstarts / V;
+  CT part[J];
 #pragma unroll 1
   for (int q = 0; q < full; q += N) {
 #pragma unroll
     for (int r = 0; r < N; r++) {
-      if (q + r >= full)
+      if (q + r >= full) {
+        if (kGroups && r % 2 == 1)
+#pragma unroll
+          for (int j = 0; j < J; j++)
+            acc[j] += part[j];
         break;
+      }
       CV::load(b + (q + r + N - 1) * V, w[(r + N - 1) % N]);
       CT a[V];
       if (OWN) {
@@ -71,8 +79,17 @@ __device__ __forceinline__ void correlate(const CT *s, int T, int tstarts, CT (&
 #pragma unroll
       for (int m = 0; m < V; m++)
 #pragma unroll
+        for (int j = 0; j < J; j++) {
+          const CT x = w[(r + (m + 1 + j) / V) % N][(m + 1 + j) % V];
+          if (!kGroups)
+            acc[j] = GC_FMA(a[m], x, acc[j]);
+          else
+            part[j] = r % 2 == 0 && m == 0 ? a[m] * x : GC_FMA(a[m], x, part[j]);
+        }
+      if (kGroups && (r % 2 == 1 || r == N - 1))
+#pragma unroll
         for (int j = 0; j < J; j++)
-          acc[j] = GC_FMA(a[m], w[(r + (m + 1 + j) / V) % N][(m + 1 + j) % V], acc[j]);
+          acc[j] += part[j];
     }
   }
   if (tstarts % V) { // the starts that do not fill a vector
@@ -103,10 +120,11 @@ __device__ __forceinline__ void corr_halve(const T (&v)[N], T (&h)[N / 2], int l
 }
 
 // Sum of acc over the warp in a fixed order, into out[0 .. J - 1] (written
-// by the lanes that hold them): two halvings in the compute type (a
+// by the lanes that hold them; added to what they wrote before with `more`): two halvings in the compute type (a
 // sum of four lanes' values), the other eight in FP64.
 template <class CT, int J>
-__device__ __forceinline__ void corr_warp_sum(const CT (&acc)[J], int lane, double *out) {
+__device__ __forceinline__ void corr_warp_sum(const CT (&acc)[J], int lane, double *out,
+                                              bool more) {
   static_assert(J % 4 == 0, "quarters");
   CT h[J / 2], q[J / 4];
   corr_halve<J>(acc, h, lane, 16);
@@ -125,7 +143,7 @@ __device__ __forceinline__ void corr_warp_sum(const CT (&acc)[J], int lane, doub
       e[j] += __shfl_xor_sync(0xffffffffu, e[j], 2);
       e[j] += __shfl_xor_sync(0xffffffffu, e[j], 1);
       if ((lane & 3) == 0)
-        out[j] = e[j];
+        out[j] = more ? out[j] + e[j] : e[j];
     }
   } else {
 #pragma unroll
@@ -134,10 +152,19 @@ __device__ __forceinline__ void corr_warp_sum(const CT (&acc)[J], int lane, doub
       for (int o = 4; o > 0; o >>= 1)
         d[j] += __shfl_xor_sync(0xffffffffu, d[j], o);
       if ((lane & 7) == 0)
-        out[j] = d[j];
+        out[j] = more ? out[j] + d[j] : d[j];
     }
   }
 }
+
+// Starts that the FP32 sums of one pass take, at most; FP64 adds the passes. With
+// the groups of eight in correlate the FP32 sums stay short however long the
+// time extent is. On links of constant phase, whose products all round alike, W
+// misses the exact value by 7e-8 (rms over the phase, Lt = 48 and 240; one chain
+// over all starts 2e-7 and 1.7e-6, sums of four loops in FP32 3e-8). W calls,
+// one chain / this / one pass of 32 / of 16 starts, us: SU(3) 32^4 T <= 16 1755
+// / 1900 / 1830 / 2015, SU(2) 48^4 T <= 24 2930 / 3570 / 3300 / 3590.
+constexpr int kCorrPass = 64;
 
 // A range of T in chunks of J: T = first + i J, i < n (first = 1 modulo V,
 // first <= tmin).

@@ -190,14 +190,15 @@ template <> struct LaneLoad<StoreF32SU3, float, 2> {
   }
 };
 
-// The loop value from Tr[a b^dag] as loop_value (gc_wcol.cuh) computes it,
+// The loop value from Tr[a b^dag] as loop_value above computes it,
 // with the sum split into one fused chain per row and the three rows added at
 // the end: three independent chains instead of one of 18 dependent FMAs,
-// which the trace loop below (a few warps per scheduler, shared-memory
-// operands) needs to keep the FMA pipe fed.
+// which the trace loops (a few warps per scheduler, shared-memory
+// operands) need to keep the FMA pipe fed.
 // Per-thread sums of the loop values: FP32 for the fundamental loops of the
-// mixed form (a thread adds at most a few loops; every loop value is an FP32
-// dot product), FP64 otherwise; the block and the grid sum them in FP64.
+// mixed form (every loop value is an FP32 dot product, and a thread of the
+// kernels that take their values from here adds at most four), FP64 otherwise;
+// the block and the grid sum them in FP64.
 template <bool ADJ, class CT>
 using GAcc = typename std::conditional<!ADJ && std::is_same<CT, float>::value, float,
                                        double>::type;

@@ -18,8 +18,10 @@
 // Bound: instruction issue (SU(3) mixed 32^4: 74% of the slots, FMA pipe 49%,
 // 24 warps on an SM; SU(2) 48^4 77% and 51%; SU(3) FP64 24^4 shared-memory
 // wavefronts 66%, FP64 pipe 49%). R,T <= L/2, whole W calls: SU(3) mixed 32^4
-// 2.70 -> 1.78 ms, 24^4 0.75 -> 0.49, 18 x 20 x 22 x 26 0.48 -> 0.30; SU(2)
-// mixed 48^4 5.16 -> 2.95; SU(3) FP64 24^4 0.80 -> 0.74.
+// 2.70 -> 1.90 ms, 24^4 0.75 -> 0.51, 18 x 20 x 22 x 26 0.48 -> 0.29; SU(2)
+// mixed 48^4 5.16 -> 3.58; SU(3) FP64 24^4 0.80 -> 0.74. (The mixed figures with
+// the short FP32 sums of gc_corr.cuh; with one chain over all starts, 7-20%
+// faster, the shares above were taken.)
 //
 // 8 SU(3) columns a block (144 sequences, five warps, five blocks on an SM): 16
 // with nine warps took 1.86 ms at 32^4. A warp stays on 8 columns, four slices
@@ -40,9 +42,16 @@ namespace gc {
 
 namespace {
 
-// T values of a thread's window: their accumulators and the window take 2 J
-// registers (FP64 4 J).
-template <class CT> constexpr int corr_jmax() { return sizeof(CT) == 4 ? 24 : 12; }
+// T values of a thread's window: their sums (FP32 two sets) and the window take
+// 3 J registers (FP64 4 J). More spill: 24 for SU(2) 48^4, T <= 24, 3.86 ms
+// against 3.57 in two windows of 12; 20 for SU(3) 32^4, T <= 16, 1.95 ms against
+// 1.90.
+constexpr int corr_jmax(int nc, size_t ct_bytes) { return ct_bytes == 8 ? 12 : nc == 2 ? 20 : 16; }
+// Starts of one pass: equal shares of tstarts, whole vectors.
+__device__ __forceinline__ int corr_pass(int tstarts, int V) {
+  const int n = (tstarts + kCorrPass - 1) / kCorrPass;
+  return ((tstarts + n - 1) / n + V - 1) / V * V;
+}
 template <class Store> constexpr int corr_elems() { return Store::NC == 3 ? 18 : 4; }
 
 // A line's elements as sequences: element k of column c at (k cols + c) st.
@@ -94,12 +103,14 @@ __global__ void __launch_bounds__(Store::NC == 3 ? 160 : 128, Store::NC == 2 || 
   if (flag && *flag != 0)
     return;
   constexpr int K = corr_elems<Store>(), V = CorrVec<CT>::V, kBatch = corr_batch<Store, CT>();
+  constexpr int JMAX = corr_jmax(Store::NC, sizeof(CT));
   using Raw = RawLink<Store, CT>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
   const int nt = tmax - tmin + 1;
   const int nslots = min(NE, tstarts + tmax); // slices the loops touch
-  const CorrRange cr = corr_range(tmin, tmax, V, corr_jmax<CT>());
+  const CorrRange cr = corr_range(tmin, tmax, V, JMAX);
+  const int pass = corr_pass(tstarts, V);
   const int st = corr_stride(cr, nslots, tstarts, V), es = cols * st, nred = cr.n * cr.J;
   CT *seq = reinterpret_cast<CT *>(smem_raw);                 // [K][cols][st]
   double *red = reinterpret_cast<double *>(seq + (size_t)K * es); // [nwarps][nred]
@@ -158,17 +169,25 @@ __global__ void __launch_bounds__(Store::NC == 3 ? 160 : 128, Store::NC == 2 || 
         const int T = cr.first + ch * cr.J;
         auto run = [&](auto jj) {
           constexpr int J = decltype(jj)::value;
-          CT acc[J];
+          auto part = [&](int t, int n, bool more) {
+            CT acc[J];
 #pragma unroll
-          for (int j = 0; j < J; j++)
-            acc[j] = CT(0);
-          if (valid) {
-            if (T == 1)
-              correlate<CT, J, true>(mine, T, tstarts, acc);
-            else
-              correlate<CT, J, false>(mine, T, tstarts, acc);
-          }
-          corr_warp_sum<CT, J>(acc, lane, red + warp * nred + ch * J);
+            for (int j = 0; j < J; j++)
+              acc[j] = CT(0);
+            if (valid) {
+              if (T == 1)
+                correlate<CT, J, true>(mine + t, T, n, acc);
+              else
+                correlate<CT, J, false>(mine + t, T, n, acc);
+            }
+            corr_warp_sum<CT, J>(acc, lane, red + warp * nred + ch * J, more);
+          };
+          if constexpr (sizeof(CT) == 8)
+            part(0, tstarts, false);
+          else
+#pragma unroll 1
+            for (int t = 0; t < tstarts; t += pass)
+              part(t, min(pass, tstarts - t), t > 0);
         };
         using std::integral_constant;
         switch (cr.J) {
@@ -176,16 +195,12 @@ __global__ void __launch_bounds__(Store::NC == 3 ? 160 : 128, Store::NC == 2 || 
         case 8: run(integral_constant<int, 8>()); break;
         case 12: run(integral_constant<int, 12>()); break;
         case 16:
-          if constexpr (corr_jmax<CT>() >= 16)
+          if constexpr (JMAX >= 16)
             run(integral_constant<int, 16>());
           break;
         case 20:
-          if constexpr (corr_jmax<CT>() >= 20)
+          if constexpr (JMAX >= 20)
             run(integral_constant<int, 20>());
-          break;
-        default:
-          if constexpr (corr_jmax<CT>() >= 24)
-            run(integral_constant<int, 24>());
         }
       }
     }
@@ -206,7 +221,7 @@ WilsonPlan wilson_corr_plan(const Geom &g, int tstarts, int tmin, int tmax, int 
                             int cols_req) {
   WilsonPlan p{};
   const int V = 16 / ct_bytes, K = nc == 3 ? 18 : 4;
-  const CorrRange cr = corr_range(tmin, tmax, V, ct_bytes == 4 ? 24 : 12);
+  const CorrRange cr = corr_range(tmin, tmax, V, corr_jmax(nc, ct_bytes));
   const int st = corr_stride(cr, tstarts + tmax, tstarts, V);
   auto shape = [&](int cols) {
     p.cols_per_block = cols;

@@ -1265,13 +1265,18 @@ int gc_wilson_spatial_3d(gc_lattice *h, int r_min, int r_max, int time_min, int 
   // reduction, against 2 R_max loop and line launches that walk the exact
   // product through L2: R,T <= 6 with 4 measurements at SU(3) 24^4 20.9 -> 5.7
   // ms FP64, 11.0 -> 4.4 ms mixed, SU(2) 5.2 -> 1.6 and 4.3 -> 1.1 ms.
+  // The mixed SU(3) form keeps the transformed links with all 18 reals: a planar
+  // sum that six steps do not bring onto the group (a few in a million at
+  // plaquette 0.5) is no reason for the exact product then, and what is left to
+  // check are the links along mu, which no planar step changes. They are checked
+  // first, and a plane with one off the group goes to the exact product at once.
   const int ct_bytes = h->prec == GC_PREC_FP64 ? 8 : 4;
-  const int link_bytes = (int)bytes_per_link(h->nc, h->prec);
+  const int link_bytes = (int)inter_link_bytes(h->nc, h->prec);
   bool gauge = h->wilson_method == GC_WILSON_AUTO && r_min == 1 && time_min == 1 &&
                nr * nt <= kWilsonMaxEntries;
   Geom pg[3];
   AxisMap map[3];
-  size_t axis_partials = 0;
+  size_t axis_partials = 0, lines_bytes = 0, links_bytes = 0;
   for (int p = 0; p < 3; p++) {
     const int order[4] = {planes[p][0], planes[p][1], 3, 3 - planes[p][0] - planes[p][1]};
     pg[p] = h->g;
@@ -1282,12 +1287,16 @@ int gc_wilson_spatial_3d(gc_lattice *h, int r_min, int r_max, int time_min, int 
     }
     pg[p].Vs = pg[p].stride[3];
     set_reciprocals(pg[p]);
-    gauge = gauge && wilson_gauge_applies(pg[p], 1, time_max, h->nc, ct_bytes, false) &&
-            wilson_gauge_bytes(pg[p], h->nc, link_bytes, time_max) <= 15 * hyp_field_bytes(h);
+    gauge = gauge && axis_loops_apply(pg[p], time_max, h->nc, ct_bytes);
     if (gauge)
       axis_partials = std::max(axis_partials,
                                axis_loops_partials(pg[p], nr, 1, time_max, h->nc, ct_bytes));
+    const size_t lines = wilson_gauge_lines_bytes(pg[p], h->nc);
+    lines_bytes += lines;
+    links_bytes = std::max(links_bytes,
+                           wilson_gauge_bytes(pg[p], h->nc, link_bytes, time_max) - lines);
   }
+  gauge = gauge && lines_bytes + links_bytes <= 15 * hyp_field_bytes(h);
   if (gauge) {
     rc = ensure_hyp(h);
     if (rc == GC_ERR_NOMEM) {
@@ -1337,51 +1346,43 @@ int gc_wilson_spatial_3d(gc_lattice *h, int r_min, int r_max, int time_min, int 
     }
   };
   bool exact[3] = {true, true, true};
-  std::vector<double> vals(3 * per_plane);
-  auto read_back = [&]() {
-    cudaError_t e = cudaMemcpyAsync(vals.data(), h->dev_out, vals.size() * sizeof(double),
+  const double scale = line_loop_scale(h->g, h->nc, false);
+  if (gauge) {
+    GaugeLinks links[3];
+    size_t off = 0;
+    for (int p = 0; p < 3; p++) {
+      links[p] = wilson_gauge_links((char *)h->hyp + off, pg[p], h->nc, link_bytes, time_max,
+                                    (char *)h->hyp + lines_bytes);
+      off += wilson_gauge_lines_bytes(pg[p], h->nc);
+      rc = GC_DISPATCH(h, launch_axis_gauge_lines, pg[p], map[p],
+                       h->cur.f[3 - planes[p][0] - planes[p][1]], links[p],
+                       h->flag_dev + kFlagSpatial + p, h->stream);
+      if (rc)
+        return launch_fail(h, rc);
+    }
+    int flags[3] = {0, 0, 0};
+    cudaError_t e = cudaMemcpyAsync(flags, h->flag_dev + kFlagSpatial, sizeof flags,
                                     cudaMemcpyDeviceToHost, h->stream);
     if (e == cudaSuccess)
       e = cudaStreamSynchronize(h->stream);
-    return e;
-  };
-  // sums per (smearing, T, R), then / 6
-  std::map<std::tuple<int, int, int>, double> acc;
-  const double scale = line_loop_scale(h->g, h->nc, false);
-  if (gauge) {
-    int flags[3] = {0, 0, 0};
+    if (e != cudaSuccess)
+      return cuda_fail(h, "unitarity of the axis links", e);
     for (int p = 0; p < 3; p++) {
-      const GaugeLinks links = wilson_gauge_links(h->hyp, pg[p], h->nc, link_bytes, time_max);
+      exact[p] = flags[p] != 0;
+      if (exact[p])
+        continue;
       int *flag = h->flag_dev + kFlagSpatial + p;
-      rc = GC_DISPATCH(h, launch_axis_gauge_lines, pg[p], map[p],
-                       h->cur.f[3 - planes[p][0] - planes[p][1]], links, flag, h->stream);
-      if (rc)
-        return launch_fail(h, rc);
       rc = run_plane(p, [&](int mi) {
         const Fields4 dir{{F[0], F[1], nullptr, nullptr}};
-        const int r = GC_DISPATCH(h, launch_axis_gauge_links, pg[p], map[p], dir, links, flag,
+        const int r = GC_DISPATCH(h, launch_axis_gauge_links, pg[p], map[p], dir, links[p], flag,
                                   h->stream);
         return r ? r
-                 : GC_DISPATCH(h, launch_axis_loops, pg[p], links, 1, r_max, 1, time_max, flag,
+                 : GC_DISPATCH(h, launch_axis_loops, pg[p], links[p], 1, r_max, 1, time_max, flag,
                                h->partials, scale,
                                h->dev_out + p * per_plane + (size_t)mi * nr * 2 * nt, h->stream);
       });
       if (rc)
         return rc;
-    }
-    cudaError_t e = cudaMemcpyAsync(flags, h->flag_dev + kFlagSpatial, sizeof flags,
-                                    cudaMemcpyDeviceToHost, h->stream);
-    if (e == cudaSuccess)
-      e = read_back();
-    if (e != cudaSuccess)
-      return cuda_fail(h, "spatial loop results", e);
-    for (int p = 0; p < 3; p++) {
-      exact[p] = flags[p] != 0;
-      for (int mi = 0; mi < nm && !exact[p]; mi++)
-        for (int t = 0; t < nt; t++)
-          for (int r = 0; r < nr; r++)
-            acc[std::make_tuple(measured[mi], 1 + t, 1 + r)] +=
-                vals[p * per_plane + (size_t)mi * nr * 2 * nt + (size_t)t * nr + r];
     }
   }
   if (exact[0] || exact[1] || exact[2]) {
@@ -1437,19 +1438,29 @@ int gc_wilson_spatial_3d(gc_lattice *h, int r_min, int r_max, int time_min, int 
       if (rc)
         return rc;
     }
-    cudaError_t e = read_back();
-    if (e != cudaSuccess)
-      return cuda_fail(h, "spatial loop results", e);
-    // in the reference's order: planes, then r, t, the nu axis before the eta axis
-    for (int p = 0; p < 3; p++)
-      for (int mi = 0; mi < nm && exact[p]; mi++)
-        for (int r = r_min; r <= r_max; r++)
-          for (int t = time_min; t <= time_max; t++)
-            for (int k = 0; k < 2; k++)
-              acc[std::make_tuple(measured[mi], t, r)] +=
-                  vals[p * per_plane + (((size_t)mi * nr + (r - r_min)) * 2 + k) * nt +
-                       (t - time_min)];
   }
+  std::vector<double> vals(3 * per_plane);
+  cudaError_t e = cudaMemcpyAsync(vals.data(), h->dev_out, vals.size() * sizeof(double),
+                                  cudaMemcpyDeviceToHost, h->stream);
+  if (e == cudaSuccess)
+    e = cudaStreamSynchronize(h->stream);
+  if (e != cudaSuccess)
+    return cuda_fail(h, "spatial loop results", e);
+  // sums per (smearing, T, R), then / 6; exact planes in the reference's order:
+  // r, t, the nu axis before the eta axis
+  std::map<std::tuple<int, int, int>, double> acc;
+  for (int p = 0; p < 3; p++)
+    for (int mi = 0; mi < nm; mi++)
+      for (int r = r_min; r <= r_max; r++)
+        for (int t = time_min; t <= time_max; t++) {
+          double &sum = acc[std::make_tuple(measured[mi], t, r)];
+          const double *v = vals.data() + p * per_plane + (size_t)mi * nr * 2 * nt;
+          if (!exact[p])
+            sum += v[(size_t)(t - time_min) * nr + (r - r_min)];
+          else
+            for (int k = 0; k < 2; k++)
+              sum += v[((size_t)(r - r_min) * 2 + k) * nt + (t - time_min)];
+        }
   *count = (int)acc.size();
   if (*count > capacity)
     return fail(h, GC_ERR_ARG, "output capacity too small (*count holds the size needed)");

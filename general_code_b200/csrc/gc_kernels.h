@@ -182,7 +182,10 @@ struct GaugeLinks {
   int NE;
 };
 size_t wilson_gauge_bytes(const Geom &g, int nc, int link_bytes, int ext);
-GaugeLinks wilson_gauge_links(void *base, const Geom &g, int nc, int link_bytes, int ext);
+size_t wilson_gauge_lines_bytes(const Geom &g, int nc); // of G and W
+// links: where the links go; null: behind the lines.
+GaugeLinks wilson_gauge_links(void *base, const Geom &g, int nc, int link_bytes, int ext,
+                              void *links = nullptr);
 // Fills them; *flag (a device int) is set to 1 when a link's defect exceeds
 // the tolerance, else left 0.
 template <class Store, class CT>
@@ -233,6 +236,7 @@ template <class Store, class CT>
 int launch_axis_gauge_links(const Geom &g, const AxisMap &map, const Fields4 &F,
                             const GaugeLinks &l, int *flag, cudaStream_t s);
 size_t axis_loops_partials(const Geom &g, int nr, int tmin, int tmax, int nc, int ct_bytes);
+bool axis_loops_apply(const Geom &g, int tmax, int nc, int ct_bytes);
 template <class Store, class CT>
 int launch_axis_loops(const Geom &g, const GaugeLinks &l, int rmin, int rmax, int tmin, int tmax,
                       const int *flag, double *partials, double scale, double *out_dev,

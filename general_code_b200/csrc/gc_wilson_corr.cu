@@ -68,25 +68,30 @@ template <class T> __device__ __forceinline__ void put_seq(T *p, int es, const S
   p[2 * es] = q.a2;
   p[3 * es] = q.a3;
 }
-__device__ __forceinline__ void extend_seq(double *p, int es, const SU3<double> &u) {
-  SU3<double> a;
+template <class T> __device__ __forceinline__ SU3<T> get_seq(const T *p, int es, SU3<T> *) {
+  SU3<T> a;
 #pragma unroll
   for (int k = 0; k < 9; k++)
     a.e[k / 3][k % 3] = {p[(2 * k) * es], p[(2 * k + 1) * es]};
-  put_seq(p, es, mul(a, u));
+  return a;
 }
-__device__ __forceinline__ void extend_seq(float *p, int es, const SU3<float> &u) {
-  // products of SU(3) links: rows 0 and 1, row 2 rebuilt
-  SU3<float> a;
+template <class T> __device__ __forceinline__ SU2<T> get_seq(const T *p, int es, SU2<T> *) {
+  return {p[0], p[es], p[2 * es], p[3 * es]};
+}
+template <class Store, class T, class M>
+__device__ __forceinline__ void extend_seq(T *p, int es, const M &u) {
+  if constexpr (Store::kBytes == 48) {
+    // products of SU(3) links: rows 0 and 1, row 2 rebuilt
+    SU3<float> a;
 #pragma unroll
-  for (int k = 0; k < 6; k++)
-    a.e[k / 3][k % 3] = {p[(2 * k) * es], p[(2 * k + 1) * es]};
-  a = mul01(a, u);
-  rebuild_row2(a);
-  put_seq(p, es, a);
-}
-template <class T> __device__ __forceinline__ void extend_seq(T *p, int es, const SU2<T> &u) {
-  put_seq(p, es, mul(SU2<T>{p[0], p[es], p[2 * es], p[3 * es]}, u));
+    for (int k = 0; k < 6; k++)
+      a.e[k / 3][k % 3] = {p[(2 * k) * es], p[(2 * k + 1) * es]};
+    a = mul01(a, u);
+    rebuild_row2(a);
+    put_seq(p, es, a);
+  } else {
+    put_seq(p, es, mul(get_seq(p, es, (M *)nullptr), u));
+  }
 }
 
 template <class Store, class CT> constexpr int corr_batch() {
@@ -152,7 +157,7 @@ __global__ void __launch_bounds__(Store::NC == 3 ? 160 : 128, Store::NC == 2 || 
           if (R == 1)
             put_seq(p, es, x[j].link());
           else
-            extend_seq(p, es, x[j].link());
+            extend_seq<Store>(p, es, x[j].link());
         }
     }
     l += stn;
@@ -268,6 +273,7 @@ int launch_wilson_corr(const Geom &g, const GaugeLinks &l, int rmin, int rmax, i
 GC_INSTANTIATE_CORR(StoreF64SU3, double)
 GC_INSTANTIATE_CORR(StoreF64SU2, double)
 GC_INSTANTIATE_CORR(StoreF32SU3, float)
+GC_INSTANTIATE_CORR(StoreF32SU3Full, float)
 GC_INSTANTIATE_CORR(StoreF32SU2, float)
 
 } // namespace gc

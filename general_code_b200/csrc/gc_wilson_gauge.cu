@@ -257,14 +257,17 @@ __global__ void __launch_bounds__(kLinesCols *kLinesSegs)
 }
 
 // U'_nu(s,te) = G(s,te) U_nu(s,te mod Lt) G(s+nu,te)^dag on the slices te of
-// the extended lattice (sites [0, NE Vs), plane stride NE Vs); thread per
-// (site, nu).
-template <class Store, bool MAPPED>
+// the extended lattice (sites [0, NE Vs), plane stride NE Vs), stored as Out;
+// thread per (site, nu). Nothing where the lines raised the flag (the loops are
+// not computed from these links then).
+template <class Store, class Out, bool MAPPED>
 __global__ void __launch_bounds__(128)
     gauge_transform_kernel(const __grid_constant__ Geom g, const __grid_constant__ AxisMap map,
                            const __grid_constant__ Fields4 U, const void *GL, const void *W,
                            const __grid_constant__ Fields4 UE, int NE, double tol, int *flag) {
   wait_previous();
+  if (*flag != 0)
+    return;
   using GS = typename F64Store<Store::NC>::type;
   using MD = typename Store::template M<double>;
   const int esite = blockIdx.x * blockDim.x + threadIdx.x;
@@ -281,7 +284,7 @@ __global__ void __launch_bounds__(128)
   const MD u = Store::template load<double>(U.f[nu], V, own_site<MAPPED>(g, map, site));
   // 12-real links: the transformed link's third row is rebuilt from its first
   // two, which holds for links in SU(3) only
-  if (Store::kBytes == 48 && !past && !(unitarity_defect(u) <= tol))
+  if (Out::kBytes == 48 && !past && !(unitarity_defect(u) <= tol))
     *flag = 1;
   MD a = mul(GS::template load<double>(GL, V, site), u);
   MD b = GS::template load<double>(GL, V, site + off);
@@ -290,7 +293,7 @@ __global__ void __launch_bounds__(128)
     a = mul(GS::template load<double>(W, g.Vs, s), a);
     b = mul(GS::template load<double>(W, g.Vs, s + off), b);
   }
-  Store::template store<double>(UE.f[nu], VE, esite, mul_ad(a, b));
+  Out::template store<double>(UE.f[nu], VE, esite, mul_ad(a, b));
 }
 
 // Shared memory of one block: per-thread loop sums red[nt][threads] (GAcc),
@@ -921,20 +924,25 @@ namespace {
 size_t align256(size_t n) { return (n + 255) / 256 * 256; }
 } // namespace
 
-size_t wilson_gauge_bytes(const Geom &g, int nc, int link_bytes, int ext) {
+size_t wilson_gauge_lines_bytes(const Geom &g, int nc) {
   const size_t line = nc == 3 ? 144 : 32;
-  return align256(line * g.V) + align256(line * g.Vs) +
+  return align256(line * g.V) + align256(line * g.Vs);
+}
+
+size_t wilson_gauge_bytes(const Geom &g, int nc, int link_bytes, int ext) {
+  return wilson_gauge_lines_bytes(g, nc) +
          3 * align256((size_t)link_bytes * (g.L[3] + ext) * g.Vs);
 }
 
-GaugeLinks wilson_gauge_links(void *base, const Geom &g, int nc, int link_bytes, int ext) {
+GaugeLinks wilson_gauge_links(void *base, const Geom &g, int nc, int link_bytes, int ext,
+                              void *links) {
   GaugeLinks l{};
   const size_t line = nc == 3 ? 144 : 32;
   char *p = static_cast<char *>(base);
   l.G = p;
   p += align256(line * g.V);
   l.W = p;
-  p += align256(line * g.Vs);
+  p = links ? static_cast<char *>(links) : p + align256(line * g.Vs);
   l.NE = g.L[3] + ext;
   for (int d = 0; d < 3; d++) {
     l.U.f[d] = p;
@@ -961,11 +969,11 @@ int launch_gauge_lines(const Geom &g, const AxisMap &map, const void *Ut, const 
   return launch_check("gauge_lines_kernel");
 }
 
-template <class Store, class CT, bool MAPPED>
+template <class Store, class Out, class CT, bool MAPPED>
 int launch_gauge_links(const Geom &g, const AxisMap &map, const Fields4 &U, const GaugeLinks &l,
                        const Fields4 &out, int ndir, int *flag, cudaStream_t s) {
-  launch_chained(gauge_transform_kernel<Store, MAPPED>, dim3((l.NE * g.Vs + 127) / 128, ndir), 128,
-                 0, s, g, map, U, l.G, l.W, out, l.NE, wilson_gauge_tolerance((int)sizeof(CT)),
+  launch_chained(gauge_transform_kernel<Store, Out, MAPPED>,
+                 dim3((l.NE * g.Vs + 127) / 128, ndir), 128, 0, s, g, map, U, l.G, l.W, out, l.NE, wilson_gauge_tolerance((int)sizeof(CT)),
                  flag);
   return launch_check("gauge_transform_kernel");
 }
@@ -979,13 +987,13 @@ int launch_wilson_gauge_prep(const Geom &g, const Fields4 &U, const GaugeLinks &
   if (e != cudaSuccess)
     return launch_check("gauge flag reset");
   const int rc = launch_gauge_lines<Store, CT, false>(g, AxisMap{}, U.f[3], l, flag, s);
-  return rc ? rc : launch_gauge_links<Store, CT, false>(g, AxisMap{}, U, l, l.U, 3, flag, s);
+  return rc ? rc : launch_gauge_links<Store, Store, CT, false>(g, AxisMap{}, U, l, l.U, 3, flag, s);
 }
 
 template <class Store, class CT>
 int launch_wilson_gauge_second(const Geom &g, const Fields4 &U2, const GaugeLinks &l,
                                const Fields4 &out, int *flag, cudaStream_t s) {
-  return launch_gauge_links<Store, CT, false>(g, AxisMap{}, U2, l, out, 3, flag, s);
+  return launch_gauge_links<Store, Store, CT, false>(g, AxisMap{}, U2, l, out, 3, flag, s);
 }
 
 template <class Store, class CT>
@@ -997,7 +1005,8 @@ int launch_axis_gauge_lines(const Geom &g, const AxisMap &map, const void *Ut,
 template <class Store, class CT>
 int launch_axis_gauge_links(const Geom &g, const AxisMap &map, const Fields4 &F,
                             const GaugeLinks &l, int *flag, cudaStream_t s) {
-  return launch_gauge_links<Store, CT, true>(g, map, F, l, l.U, 2, flag, s);
+  return launch_gauge_links<Store, typename InterStore<Store>::type, CT, true>(g, map, F, l, l.U, 2,
+                                                                              flag, s);
 }
 
 template <class Store, class CT>
@@ -1117,18 +1126,43 @@ size_t wilson_auto_partials_count(const Geom &g, int nr, int tmin, int tmax, int
   return std::max<size_t>(wilson_partials_count(g, nr, nt, nc), (size_t)blocks * nr * nt);
 }
 
+// Kernels of the axis loops. Mixed SU(3) lines are full products there (planar
+// APE sums need not project onto the group), which the one-column kernel of few
+// slices does not have.
+static WilsonPlan axis_loops_plan(const Geom &g, int tmin, int tmax, int nc, int ct_bytes) {
+  WilsonPlan p = wilson_gauge_plan(g, tmin, tmax, nc, ct_bytes);
+  if (p.kernel != 3)
+    return p;
+  p = wilson_corr_plan(g, g.L[3], tmin, tmax, nc, ct_bytes, 0);
+  return p.fits ? p : wilson_gram_plan(g, g.L[3], tmax, nc, 0, false);
+}
+
 size_t axis_loops_partials(const Geom &g, int nr, int tmin, int tmax, int nc, int ct_bytes) {
-  return (size_t)wilson_gauge_plan(g, tmin, tmax, nc, ct_bytes).blocks / 3 * 2 * nr *
+  return (size_t)axis_loops_plan(g, tmin, tmax, nc, ct_bytes).blocks / 3 * 2 * nr *
          (tmax - tmin + 1);
+}
+
+bool axis_loops_apply(const Geom &g, int tmax, int nc, int ct_bytes) {
+  return g.L[3] >= 2 && tmax <= g.L[3] / 2 && axis_loops_plan(g, 1, tmax, nc, ct_bytes).fits;
 }
 
 template <class Store, class CT>
 int launch_axis_loops(const Geom &g, const GaugeLinks &l, int rmin, int rmax, int tmin, int tmax,
                       const int *flag, double *partials, double scale, double *out_dev,
                       cudaStream_t s) {
-  int blocks = 0;
-  const int rc = launch_wilson_gauge_kernel<Store, CT>(g, l, rmin, rmax, tmin, tmax, false, flag,
-                                                       partials, &blocks, s, 0, 0, 2);
+  int blocks = 0, rc;
+  if constexpr (std::is_same<Store, StoreF32SU3>::value) {
+    const WilsonPlan p = axis_loops_plan(g, tmin, tmax, 3, 4);
+    rc = p.kernel == 4
+             ? launch_wilson_corr<StoreF32SU3Full, float>(g, l, rmin, rmax, tmin, tmax, flag,
+                                                          partials, &blocks, s, 0, g.L[3], 2)
+             : launch_wilson_gram<StoreF32SU3Full, float>(g, l, nullptr, rmin, rmax, tmin, tmax,
+                                                          flag, partials, &blocks, s, 0, g.L[3],
+                                                          2);
+  } else {
+    rc = launch_wilson_gauge_kernel<Store, CT>(g, l, rmin, rmax, tmin, tmax, false, flag, partials,
+                                               &blocks, s, 0, 0, 2);
+  }
   return rc ? rc
             : launch_reduce_wilson(partials, blocks, rmax - rmin + 1, tmax - tmin + 1, scale,
                                    out_dev, s);

@@ -95,24 +95,24 @@ template <class T> __device__ __forceinline__ void put(double2 *p, const SU2<T> 
   p[1] = make_double2(double(q.a2), double(q.a3));
 }
 // line <- line u
-__device__ __forceinline__ void extend(double2 *p, const SU3<double> &u) {
-  SU3<double> a;
+template <class Store, class T> __device__ __forceinline__ void extend(double2 *p, const SU3<T> &u) {
+  SU3<T> a;
+  if constexpr (Store::kBytes == 48) {
+    // products of SU(3) links: rows 0 and 1, row 2 rebuilt
 #pragma unroll
-  for (int k = 0; k < 9; k++)
-    a.e[k / 3][k % 3] = {p[k].x, p[k].y};
-  put(p, mul(a, u));
-}
-__device__ __forceinline__ void extend(double2 *p, const SU3<float> &u) {
-  // products of SU(3) links: rows 0 and 1, row 2 rebuilt
-  SU3<float> a;
+    for (int k = 0; k < 6; k++)
+      a.e[k / 3][k % 3] = {T(p[k].x), T(p[k].y)};
+    a = mul01(a, u);
+    rebuild_row2(a);
+    put(p, a);
+  } else {
 #pragma unroll
-  for (int k = 0; k < 6; k++)
-    a.e[k / 3][k % 3] = {float(p[k].x), float(p[k].y)};
-  a = mul01(a, u);
-  rebuild_row2(a);
-  put(p, a);
+    for (int k = 0; k < 9; k++)
+      a.e[k / 3][k % 3] = {T(p[k].x), T(p[k].y)};
+    put(p, mul(a, u));
+  }
 }
-template <class T> __device__ __forceinline__ void extend(double2 *p, const SU2<T> &u) {
+template <class Store, class T> __device__ __forceinline__ void extend(double2 *p, const SU2<T> &u) {
   const double2 v = p[0], w = p[1];
   put(p, mul(SU2<T>{T(v.x), T(v.y), T(w.x), T(w.y)}, u));
 }
@@ -293,7 +293,7 @@ __global__ void __launch_bounds__(kGramThreads, 4)
     if (R == 1)
       put(p, x.link());
     else
-      extend(p, x.link());
+      extend<Store>(p, x.link());
   };
   auto fetch = [&](int R) {
     if (!active)
@@ -447,8 +447,12 @@ int launch_wilson_gram(const Geom &g, const GaugeLinks &l, const Fields4 *second
                      partials, flag, tstarts);
     return rc;
   };
-  const int rc = second ? go(wilson_gram_kernel<Store, CT, true>)
-                        : go(wilson_gram_kernel<Store, CT, false>);
+  int rc;
+  if constexpr (Store::kBytes == 72) // (the spatial loops' links: no GEVP)
+    rc = go(wilson_gram_kernel<Store, CT, false>);
+  else
+    rc = second ? go(wilson_gram_kernel<Store, CT, true>)
+                : go(wilson_gram_kernel<Store, CT, false>);
   *blocks = p.blocks / 3 * ndir;
   return rc ? rc : launch_check("wilson_gram_kernel");
 }
@@ -461,6 +465,7 @@ int launch_wilson_gram(const Geom &g, const GaugeLinks &l, const Fields4 *second
 GC_INSTANTIATE_GRAM(StoreF64SU3, double)
 GC_INSTANTIATE_GRAM(StoreF64SU2, double)
 GC_INSTANTIATE_GRAM(StoreF32SU3, float)
+GC_INSTANTIATE_GRAM(StoreF32SU3Full, float)
 GC_INSTANTIATE_GRAM(StoreF32SU2, float)
 
 } // namespace gc

@@ -831,13 +831,24 @@ static int wilson_impl(gc_lattice *h, int rmin, int rmax, int tmin, int tmax,
                wilson_gauge_applies(h->g, tmin, tmax, h->nc, ct_bytes, adjoint, tstarts);
   WilsonPlan gevp_plan{};
   if (gauge && second) {
-    // preparing the gauge costs what the exact walk of a few loops does: whole
-    // calls in us, exact / gauge, SU(3) FP64 16^4 R <= 4, T <= 2 159 / 176 and
-    // T <= 4 221 / 179, 24^4 R,T <= 6 1992 / 880; mixed 24^4 R,T <= 4 555 / 630
-    // and 6 1089 / 854; SU(2) FP64 16^4 R,T <= 4 86 / 102, mixed 16^4 R,T <= 6
-    // 109 / 105
-    const int loops = nr * tmax;
-    gauge = loops >= (h->nc == 3 && ct_bytes == 8 ? 12 : 25);
+    // Preparing the gauge costs what the exact walk of a few loops does, and the
+    // 8 x 8 tiles of the loop kernel stay empty at small T and Lt: whole calls in
+    // us, exact / gauge.
+    //   SU(3) FP64: R,T <= 3,4 16^4 160 / 139, 24^3 x 8 256 / 215, but 10^4 54 /
+    //   61 and 8^3 x 32 67 / 73 (4,4 81 / 78); Lt = 4, 16^3 R,T <= 6,2 74 / 105
+    //   SU(3) mixed: 5,5 12^4 87 / 103, 20^4 386 / 421, 24^4 780 / 719; 8,4 16^3 x
+    //   32 406 / 456, 32^4 2869 / 3015; 6,6 12^4 110 / 114, 14^4 183 / 159, 24^4
+    //   1052 / 834; 4,8 8^3 x 32 98 / 84
+    //   SU(2) FP64: 5,5 12^4 59 / 65, 14^4 75 / 71, 24^4 345 / 222, 12^3 x 24 79 /
+    //   68; 8,4 24^3 x 8 160 / 172, 24^3 x 12 236 / 210; mixed 5,5 12^4 50 / 54,
+    //   14^4 62 / 58; 8,4 32^3 x 8 254 / 268
+    const int loops = nr * tmax, Lt = h->g.L[3];
+    if (h->nc == 2)
+      gauge = Lt >= 12 && h->g.V >= 30000 && loops >= 25;
+    else if (ct_bytes == 8)
+      gauge = (Lt >= 8 || tmax >= 3) && loops >= (h->g.Vs < 1728 ? 16 : 12);
+    else
+      gauge = Lt > 12 && tmax >= 6 && loops >= 25;
   }
   if (gauge && second) {
     gevp_plan = wilson_gram_plan(h->g, h->g.L[3], tmax, h->nc, 0, true);

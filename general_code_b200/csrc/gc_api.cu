@@ -1075,7 +1075,8 @@ static int offaxis_impl(gc_lattice *h, const std::vector<std::array<int, 3>> &di
   const size_t fill = std::max<size_t>(1, 12 * 148 / (size_t)std::max(1, gauge_blocks));
   const OffaxisTree tree = offaxis_tree(
       h->g.L, plan.lines,
-      (int)std::min(most, std::max<size_t>(8, std::min<size_t>(48, plan.lines.size() / fill))));
+      (int)std::min(most, std::max<size_t>(8, std::min<size_t>(48, plan.lines.size() / fill))),
+      gauge_blocks > 0 ? kTreeStack : -1);
   const size_t nlines = tree.first.size();
   if (tree.nodes.empty())
     gauge_blocks = 0;

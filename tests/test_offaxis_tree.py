@@ -113,7 +113,7 @@ def test_walk_gives_every_line(tree, per_chunk):
     assert found == {k: lines[i] for k, i in enumerate(t["first"])}
 
 
-@pytest.mark.parametrize("levels", [0, 1])
+@pytest.mark.parametrize("levels", [-1, 0, 1])
 def test_lines_and_chunks_are_complete_without_room_on_the_stack(tree, levels):
     lines = _lines(90, 7)
     t = tree(lines, 30, levels)

@@ -1078,7 +1078,11 @@ static int offaxis_impl(gc_lattice *h, const std::vector<std::array<int, 3>> &di
       (int)std::min(most, std::max<size_t>(8, std::min<size_t>(48, plan.lines.size() / fill))),
       gauge_blocks > 0 ? kTreeStack : -1);
   const size_t nlines = tree.first.size();
-  if (tree.nodes.empty())
+  // (a few lines cost less than the gauge: whole calls in us, exact / gauge, the
+  // three lines of r = 1, T = 1 SU(3) mixed 24^4 99 / 184, FP64 16^4 74 / 91, SU(2)
+  // 24^4 75 / 99, T = 6 SU(3) mixed 24^4 1.21 times; six lines 1.1 to 1.8 times;
+  // eighteen, r <= 6 along the axes, T <= 3, 16^4 126 / 113, 8^4 63 / 60)
+  if (tree.nodes.empty() || nlines < 16)
     gauge_blocks = 0;
   bool gauge = gauge_blocks > 0;
   GaugeLinks links{};

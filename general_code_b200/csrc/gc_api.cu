@@ -1290,6 +1290,13 @@ int gc_wilson_spatial_3d(gc_lattice *h, int r_min, int r_max, int time_min, int 
   const int link_bytes = (int)inter_link_bytes(h->nc, h->prec);
   bool gauge = h->wilson_method == GC_WILSON_AUTO && r_min == 1 && time_min == 1 &&
                nr * nt <= kWilsonMaxEntries;
+  // Preparing the gauge costs what the exact walk of the first loops does: whole
+  // calls in us, exact / gauge, without smearing, R,T <= 1,2 SU(3) FP64 24^4 464 /
+  // 542, SU(2) 32^4 332 / 385; 2,1 724 / 592 and 521 / 416. SU(3) mixed 24^4 2,1
+  // 354 / 446, 2,2 417 / 458 (32^3 x 8 341 / 397), with two smearing steps measured
+  // 1330 / 1188, 3,3 with one 1732 / 1242.
+  gauge = gauge && nr >= 2 &&
+          (h->nc == 2 || ct_bytes == 8 || nr * nt * std::min(nm, 2) >= 6);
   Geom pg[3];
   AxisMap map[3];
   size_t axis_partials = 0, lines_bytes = 0, links_bytes = 0;

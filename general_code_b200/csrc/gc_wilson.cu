@@ -181,10 +181,15 @@ __device__ __forceinline__ void wilson_block(const Geom &g, const Fields4 &U, co
   }
 }
 
+// As many blocks as an SM may hold of the smallest shapes (16 x 148), so that the
+// exact product is as fast as in a launch of its own: with 4 x 148 GEVP R,T <= 5
+// of SU(3) FP64 24^3 x 8 took 496 us against 395. Empty they take 2 us.
+constexpr int kGatedBlocks = 16 * 148;
+
 // gate: the temporal-gauge form's unitarity flag; that launch is the exact
 // fallback and computes nothing when the flag says the gauge form ran. Its
-// blocks then return at once, so it is launched with few of them, each taking
-// several of the `colblocks` x 3 work items (4 / 37 us of empty blocks at
+// blocks then return at once, so it is launched with at most kGatedBlocks, each
+// taking several of the `colblocks` x 3 work items (4 / 37 us of empty blocks at
 // 16^4 / 48^4 otherwise).
 template <class Store, class CT, bool ADJ, bool GEVP>
 __global__ void __launch_bounds__(256)
@@ -447,7 +452,7 @@ int launch_wilson_exact_gated(const Geom &g, const Fields4 &U, const Fields4 *se
   auto go = [&](auto kernel) {
     const int rc = allow_large_smem(kernel, p.smem);
     if (!rc)
-      launch_chained(kernel, std::min(p.blocks, 4 * 148), p.threads, p.smem, s, g, U,
+      launch_chained(kernel, std::min(p.blocks, kGatedBlocks), p.threads, p.smem, s, g, U,
                      second ? *second : U, rmin, rmax, tmin, tmax, p.cols_per_block, p.rows,
                      partials, tstarts, p.blocks / 3, gate);
     return rc;

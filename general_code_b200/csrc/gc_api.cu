@@ -65,7 +65,10 @@ struct gc_lattice {
   size_t field_bytes = 0;   // one direction's field
   void *links = nullptr;    // 8 fields: two sets of 4 directions
   gc::Fields4 cur{}, alt{}; // current / spare buffer of each direction
-  void *hyp = nullptr;      // 15 decorated-link fields (allocated on first HYP)
+  void *hyp = nullptr;      // scratch: HYP's 15 decorated-link fields, or the gauge form's lines
+  size_t hyp_cap = 0;       // and links (bytes)
+  bool hyp_optional = false; // only a form that the caller can do without has asked for it
+  bool hyp_in_use = false;   // by the call under way
   double *staging = nullptr; // host-layout staging buffer (device)
   double *partials = nullptr;
   size_t partials_cap = 0;  // doubles
@@ -114,11 +117,6 @@ int launch_fail(gc_lattice *h, int rc) {
 
 // Device allocations of a handle: ordinary, or stream-ordered on the handle's
 // stream (no device-wide synchronisation when freed).
-cudaError_t dev_alloc(gc_lattice *h, void **p, size_t n) {
-  if (h->stream_ordered)
-    return cudaMallocAsync(p, n, h->stream);
-  return cudaMalloc(p, n);
-}
 void dev_free(gc_lattice *h, void *p) {
   if (!p)
     return;
@@ -126,6 +124,21 @@ void dev_free(gc_lattice *h, void *p) {
     cudaFreeAsync(p, h->stream);
   else
     cudaFree(p);
+}
+cudaError_t dev_alloc(gc_lattice *h, void **p, size_t n) {
+  auto alloc = [&] {
+    return h->stream_ordered ? cudaMallocAsync(p, n, h->stream) : cudaMalloc(p, n);
+  };
+  cudaError_t e = alloc();
+  if (e == cudaErrorMemoryAllocation && h->hyp && h->hyp_optional && !h->hyp_in_use) {
+    // scratch that no form needs makes room
+    cudaGetLastError();
+    dev_free(h, h->hyp);
+    h->hyp = nullptr;
+    h->hyp_cap = 0;
+    e = alloc();
+  }
+  return e;
 }
 
 size_t bytes_per_link(int nc, int prec) {
@@ -239,16 +252,40 @@ size_t hyp_field_bytes(const gc_lattice *h) {
   return ((inter_link_bytes(h->nc, h->prec) * (size_t)h->g.V + 255) / 256) * 256;
 }
 
-int ensure_hyp(gc_lattice *h) {
-  if (h->hyp)
+// Scratch of at least `bytes`. optional: for a form that the caller can do
+// without (GC_ERR_NOMEM then means to do without it); taken only where three
+// quarters of the free memory stay free, and given back when another allocation
+// of the handle needs the room.
+int ensure_scratch(gc_lattice *h, size_t bytes, bool optional) {
+  if (h->hyp_cap >= bytes) {
+    h->hyp_optional = h->hyp_optional && optional;
     return GC_OK;
-  cudaError_t e = dev_alloc(h, &h->hyp, 15 * hyp_field_bytes(h));
+  }
+  size_t free_bytes = 0, total = 0;
+  if (optional && (cudaMemGetInfo(&free_bytes, &total) != cudaSuccess || bytes > free_bytes / 4))
+    return GC_ERR_NOMEM;
+  h->hyp_optional = optional && (!h->hyp || h->hyp_optional);
+  dev_free(h, h->hyp);
+  h->hyp = nullptr;
+  h->hyp_cap = 0;
+  cudaError_t e = dev_alloc(h, &h->hyp, bytes);
   if (e != cudaSuccess) {
     h->hyp = nullptr;
+    if (optional)
+      cudaGetLastError(); // (not the next launch's error)
     return cuda_fail(h, "cudaMalloc(HYP decorated links)", e);
   }
+  h->hyp_cap = bytes;
   return GC_OK;
 }
+int ensure_hyp(gc_lattice *h) { return ensure_scratch(h, 15 * hyp_field_bytes(h), false); }
+
+// A call's hold on the scratch.
+struct ScratchUse {
+  gc_lattice *h;
+  explicit ScratchUse(gc_lattice *lat) : h(lat) {}
+  ~ScratchUse() { h->hyp_in_use = false; }
+};
 
 int ensure_flag(gc_lattice *h) {
   if (h->flag_dev)
@@ -713,37 +750,42 @@ int gc_hyp(gc_lattice *h, double a1, double a2, double a3, int steps) {
   return GC_OK;
 }
 
-// Prepares the temporal-gauge form: the gauge time lines and the transformed
-// spatial links (with `ext` slices past the last one) in the HYP
-// decorated-link scratch, which holds them (FP64 SU(3): at most 144 (1 + 1/Lt)
-// + 3 x 1.5 x 144 bytes per site against 15 x 144), and the device's unitarity
-// check of the links into *flag, a word of h->flag_dev. *use is cleared when
-// the scratch cannot hold them, or, with `optional`, when it cannot be
-// allocated (the caller has a form that does without it).
 enum { kFlagOnaxis = 0, kFlagOffaxis = 1, kFlagSpatial = 2 }; // words of h->flag_dev (spatial: three)
-// second: a second configuration's links, whose spatial links go into
-// second_links in the same gauge.
+
+// Prepares the temporal-gauge form: the gauge time lines and the transformed
+// spatial links (with `ext` slices past the last one) in the scratch, which
+// HYP's decorated links (15 fields) leave room for (FP64 SU(3): at most 144 (1 +
+// 1/Lt) + 3 x 1.5 x 144 bytes per site against 15 x 144), and the device's
+// unitarity check of the links into *flag, a word of h->flag_dev. *use is
+// cleared when that scratch cannot hold them, or, with `optional`, when it cannot
+// be had (the caller has a form that does without it). second: a second
+// configuration's links, whose spatial links go into second_links in the same
+// gauge.
 static int gauge_prepare(gc_lattice *h, int ext, GaugeLinks *links, bool *use, int **flag,
                          int word = kFlagOnaxis, bool optional = false,
                          const Fields4 *second = nullptr, Fields4 *second_links = nullptr) {
-  int rc = ensure_hyp(h);
-  if (rc == GC_ERR_NOMEM && optional) {
-    cudaGetLastError(); // (the failed allocation is not the next launch's error)
-    *use = false;
-    return GC_OK;
-  }
-  if (rc)
-    return rc;
-  rc = ensure_flag(h);
-  if (rc)
-    return rc;
   const int link_bytes = (int)bytes_per_link(h->nc, h->prec);
   const size_t main_bytes = wilson_gauge_bytes(h->g, h->nc, link_bytes, ext);
   const size_t field = ((size_t)link_bytes * (h->g.L[3] + ext) * h->g.Vs + 255) / 256 * 256;
-  if (main_bytes + (second ? 3 * field : 0) > 15 * hyp_field_bytes(h)) {
+  const size_t bytes = main_bytes + (second ? 3 * field : 0);
+  int rc = GC_OK;
+  if (!optional)
+    rc = ensure_hyp(h);
+  if (!rc && bytes > 15 * hyp_field_bytes(h)) {
     *use = false;
     return GC_OK;
   }
+  if (optional)
+    rc = ensure_scratch(h, bytes, true);
+  if (rc == GC_ERR_NOMEM && optional) {
+    *use = false;
+    return GC_OK;
+  }
+  if (!rc)
+    rc = ensure_flag(h);
+  if (rc)
+    return rc;
+  h->hyp_in_use = true;
   *flag = h->flag_dev + word;
   *links = wilson_gauge_links(h->hyp, h->g, h->nc, link_bytes, ext);
   rc = GC_DISPATCH(h, launch_wilson_gauge_prep, h->g, h->cur, *links, *flag, h->stream);
@@ -814,8 +856,9 @@ static int wilson_impl(gc_lattice *h, int rmin, int rmax, int tmin, int tmax,
   rc = ensure_dev_out(h, (size_t)nr * nt + (size_t)rchunk * nt);
   if (rc)
     return rc;
-  rc = ensure_partials(h, wilson_partials_count(h->g, std::min(rchunk, nr), nt, h->nc,
-                                                second ? 4 : 3));
+  const size_t exact_partials =
+      wilson_partials_count(h->g, std::min(rchunk, nr), nt, h->nc, second ? 4 : 3);
+  rc = ensure_partials(h, exact_partials);
   if (rc)
     return rc;
   double *chunk_out = h->dev_out + (size_t)nr * nt;
@@ -857,6 +900,7 @@ static int wilson_impl(gc_lattice *h, int rmin, int rmax, int tmin, int tmax,
   GaugeLinks links{};
   Fields4 second_links{};
   int *flag = nullptr;
+  const ScratchUse use(h);
   if (gauge) {
     rc = gauge_prepare(h, wilson_gauge_ext(h->g, tmax, tstarts), &links, &gauge, &flag,
                        kFlagOnaxis, second != nullptr, u2, &second_links);
@@ -868,6 +912,12 @@ static int wilson_impl(gc_lattice *h, int rmin, int rmax, int tmin, int tmax,
     rc = ensure_partials(h, second ? (size_t)gevp_plan.blocks * ncr * nt
                                    : wilson_auto_partials_count(h->g, ncr, tmin, tmax, h->nc, 0,
                                                                 tstarts));
+    if (rc == GC_ERR_NOMEM) { // (the exact form needs fewer)
+      cudaGetLastError();
+      gauge = false;
+      h->hyp_in_use = false;
+      rc = ensure_partials(h, exact_partials);
+    }
     if (rc)
       return rc;
   }
@@ -1084,9 +1134,26 @@ static int offaxis_impl(gc_lattice *h, const std::vector<std::array<int, 3>> &di
   // eighteen, r <= 6 along the axes, T <= 3, 16^4 126 / 113, 8^4 63 / 60)
   if (tree.nodes.empty() || nlines < 16)
     gauge_blocks = 0;
+  // what every form needs, then what the gauge form needs
+  rc = ensure_dev_out(h, nlines * (size_t)nt);
+  if (!rc)
+    rc = ensure_aux(h, tree.nodes.size() * sizeof(OffaxisNode) +
+                           tree.chunk_nodes.size() * sizeof(int) + 16 +
+                           nlines * sizeof(OffaxisLineDesc));
+  if (rc)
+    return rc;
+  rc = ensure_partials(h, per_line * std::min(most, nlines));
+  if (rc == GC_ERR_NOMEM && gauge_blocks > exact_blocks) {
+    cudaGetLastError();
+    gauge_blocks = 0;
+    rc = ensure_partials(h, (size_t)exact_blocks * nt * std::min(most, nlines));
+  }
+  if (rc)
+    return rc;
   bool gauge = gauge_blocks > 0;
   GaugeLinks links{};
   int *flag = nullptr;
+  const ScratchUse use(h);
   if (gauge) {
     rc = gauge_prepare(h, tmax, &links, &gauge, &flag, kFlagOffaxis, true);
     if (rc)
@@ -1114,20 +1181,11 @@ static int offaxis_impl(gc_lattice *h, const std::vector<std::array<int, 3>> &di
     std::memcpy(host.data() + node_bytes, tree.chunk_nodes.data(), chunk_bytes);
   }
   std::memcpy(host.data() + table_off, table.data(), nlines * sizeof(OffaxisLineDesc));
-  rc = ensure_aux(h, host.size());
-  if (rc)
-    return rc;
   // (from pageable memory: returns once the table is staged, so `host` may go)
   cudaError_t ce = cudaMemcpyAsync(h->aux, host.data(), host.size(), cudaMemcpyHostToDevice,
                                    h->stream);
   if (ce != cudaSuccess)
     return cuda_fail(h, "cudaMemcpyAsync(off-axis lines)", ce);
-  rc = ensure_partials(h, per_line * std::min(most, nlines));
-  if (rc)
-    return rc;
-  rc = ensure_dev_out(h, nlines * (size_t)nt);
-  if (rc)
-    return rc;
   const unsigned char *aux = static_cast<const unsigned char *>(h->aux);
   const OffaxisNode *dev_nodes = reinterpret_cast<const OffaxisNode *>(aux);
   const int *dev_chunks = reinterpret_cast<const int *>(aux + node_bytes);
@@ -1320,9 +1378,14 @@ int gc_wilson_spatial_3d(gc_lattice *h, int r_min, int r_max, int time_min, int 
                            wilson_gauge_bytes(pg[p], h->nc, link_bytes, time_max) - lines);
   }
   gauge = gauge && lines_bytes + links_bytes <= 15 * hyp_field_bytes(h);
+  const ScratchUse use(h);
   if (gauge) {
-    rc = ensure_hyp(h);
-    if (rc == GC_ERR_NOMEM) {
+    rc = ensure_flag(h);
+    if (!rc)
+      rc = ensure_partials(h, axis_partials);
+    if (!rc)
+      rc = ensure_scratch(h, lines_bytes + links_bytes, true);
+    if (rc == GC_ERR_NOMEM) { // (the exact product needs none of it)
       cudaGetLastError();
       gauge = false;
     } else if (rc) {
@@ -1330,11 +1393,7 @@ int gc_wilson_spatial_3d(gc_lattice *h, int r_min, int r_max, int time_min, int 
     }
   }
   if (gauge) {
-    rc = ensure_flag(h);
-    if (!rc)
-      rc = ensure_partials(h, axis_partials);
-    if (rc)
-      return rc;
+    h->hyp_in_use = true;
     cudaError_t e = cudaMemsetAsync(h->flag_dev + kFlagSpatial, 0, 3 * sizeof(int), h->stream);
     if (e != cudaSuccess)
       return cuda_fail(h, "cudaMemsetAsync(flags)", e);
@@ -1408,6 +1467,7 @@ int gc_wilson_spatial_3d(gc_lattice *h, int r_min, int r_max, int time_min, int 
         return rc;
     }
   }
+  h->hyp_in_use = false;
   if (exact[0] || exact[1] || exact[2]) {
     // the 2 nr lines of one (plane, measurement) share a partials buffer,
     // [block][(r, axis)][T], and one reduction launch when it stays within 32 MB

@@ -170,7 +170,7 @@ bool wilson_gauge_applies(const Geom &g, int tmin, int tmax, int nc, int ct_byte
 int wilson_gauge_ext(const Geom &g, int tmax, int tstarts = 0);
 // Unitarity defect max |U U^dag - 1| of the temporal links for which the form
 // is used: FP64 (ct_bytes 8) the mean over 32 columns, with no link
-// beyond a hundred times it; mixed (4) the largest.
+// beyond a hundred times it (a time slab: beyond it); mixed (4) the largest.
 double wilson_gauge_tolerance(int ct_bytes);
 // The form's scratch: gauge time lines G (V matrices, FP64) and W (the lines
 // over the whole extent, Vs matrices), and the transformed spatial links

@@ -152,7 +152,7 @@ int gc_copy_slices(gc_lattice *dst, int dst_t0, gc_lattice *src, int src_t0, int
  * (wilson_loops.h:1047-1074). Methods as gc_wilson_onaxis: for
  * time_max <= Lt - t_starts (no counted loop passes slice Lt - 1) the
  * temporal gauge on the slab's own slices where the device finds the temporal
- * links unitary, else the exact product. */
+ * links unitary (in FP64 every one of them to 1e-14), else the exact product. */
 int gc_wilson_onaxis_tslab(gc_lattice *h, int t_starts, int r_min, int r_max, int time_min,
                            int time_max, int adjoint, double *out);
 

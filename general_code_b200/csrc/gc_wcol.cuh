@@ -230,32 +230,27 @@ __device__ __forceinline__ GAcc<ADJ, T> gauge_trace(const SU3<T> &a, const SU3<T
   const double m = double((im[0] + im[1]) + im[2]);
   return fma(r, r, fma(m, m, -1.0));
 }
+// (two columns per thread: the adjoint loops only)
 template <bool ADJ>
-__device__ __forceinline__ GAcc<ADJ, float> gauge_trace(const SU3<f2> &a, const SU3<f2> &b,
-                                                        bool lane1) {
+__device__ __forceinline__ double gauge_trace(const SU3<f2> &a, const SU3<f2> &b, bool lane1) {
+  static_assert(ADJ, "adjoint loops");
   f2 re[3], im[3];
 #pragma unroll
   for (int i = 0; i < 3; i++) {
     re[i] = a.e[i][0].re * b.e[i][0].re;
     re[i] = fma(a.e[i][0].im, b.e[i][0].im, re[i]);
-    if (ADJ) {
-      im[i] = a.e[i][0].im * b.e[i][0].re;
-      im[i] = fma(-a.e[i][0].re, b.e[i][0].im, im[i]);
-    }
+    im[i] = a.e[i][0].im * b.e[i][0].re;
+    im[i] = fma(-a.e[i][0].re, b.e[i][0].im, im[i]);
 #pragma unroll
     for (int j = 1; j < 3; j++) {
       re[i] = fma(a.e[i][j].re, b.e[i][j].re, re[i]);
       re[i] = fma(a.e[i][j].im, b.e[i][j].im, re[i]);
-      if (ADJ) {
-        im[i] = fma(a.e[i][j].im, b.e[i][j].re, im[i]);
-        im[i] = fma(-a.e[i][j].re, b.e[i][j].im, im[i]);
-      }
+      im[i] = fma(a.e[i][j].im, b.e[i][j].re, im[i]);
+      im[i] = fma(-a.e[i][j].re, b.e[i][j].im, im[i]);
     }
   }
   const float2 r = make_float2((re[0].v.x + re[1].v.x) + re[2].v.x,
                                (re[0].v.y + re[1].v.y) + re[2].v.y);
-  if (!ADJ)
-    return lane1 ? r.x + r.y : r.x;
   const float2 m = make_float2((im[0].v.x + im[1].v.x) + im[2].v.x,
                                (im[0].v.y + im[1].v.y) + im[2].v.y);
   const double r0 = double(r.x), i0 = double(m.x);

@@ -296,7 +296,8 @@ __global__ void __launch_bounds__(128)
   Out::template store<double>(UE.f[nu], VE, esite, mul_ad(a, b));
 }
 
-// Shared memory of one block: per-thread loop sums red[nt][threads] (GAcc),
+// The adjoint loops. Shared memory of one block: per-thread loop sums
+// red[nt][threads] (FP64),
 // then the space lines, one slot per (slice, column unit) over the NE slices.
 // KS > 1: a thread owns KS consecutive start slices t0 = KS row + m, m < KS
 // (KS divides Lt), and one shared-memory load of
@@ -307,7 +308,7 @@ __global__ void __launch_bounds__(128)
 // SLAB compiles in the check that a start is counted (t0 < tstarts, a time
 // slab). A top line past the last slice belongs to an uncounted loop: its slot
 // is clamped.
-template <class Store, class CT, bool ADJ, int KS, bool SLAB>
+template <class Store, class CT, int KS, bool SLAB>
 __global__ void __launch_bounds__(256)
     wilson_gauge_kernel(const __grid_constant__ Geom g, const __grid_constant__ Fields4 U,
                         int NE, int rmin, int rmax, int tmin, int tmax, int cols, int rows,
@@ -327,7 +328,7 @@ __global__ void __launch_bounds__(256)
   const int cs = wilson_col_stride(cols, LANES);
   const int units = cs / LANES;
   const int nslots = NE * units;
-  using Acc = GAcc<ADJ, CT>;
+  using Acc = double;
   Acc *red = reinterpret_cast<Acc *>(smem_raw); // [nt][nthreads]
   unsigned char *sa = smem_raw + ((sizeof(Acc) * nt * nthreads + 15) & ~(size_t)15);
 
@@ -383,7 +384,7 @@ __global__ void __launch_bounds__(256)
 #pragma unroll
           for (int m = 0; m < KS; m++)
             if (j - m >= 0 && j - m < nt && (!SLAB || t0 + m < tstarts)) // T = tmin + j - m
-              acc[m] += gauge_trace<ADJ>(a[m], b, lane1);
+              acc[m] += gauge_trace<true>(a[m], b, lane1);
         }
         if (j - (KS - 1) >= 0) // T index j - KS + 1 has all KS starts
           red[(size_t)(j - (KS - 1)) * nthreads + tid] = acc[KS - 1];
@@ -420,7 +421,7 @@ __global__ void __launch_bounds__(256)
 #pragma unroll 1
         for (int T = 0; T < nt; T++) {
           const Acc v =
-              (active && (!SLAB || t0 < tstarts)) ? gauge_trace<ADJ>(a, CS::load(sa, nslots, tt * units + u), lane1) : Acc(0);
+              (active && (!SLAB || t0 < tstarts)) ? gauge_trace<true>(a, CS::load(sa, nslots, tt * units + u), lane1) : Acc(0);
           Acc *r = red + (size_t)T * nthreads + tid;
           *r = (k == 0) ? v : *r + v;
           tt = min(tt + 1, NE - 1);
@@ -1071,12 +1072,12 @@ int launch_wilson_gauge_kernel(const Geom &g, const GaugeLinks &l, int rmin, int
     }
   }
   constexpr int K4 = Store::NC == 2 ? 4 : 2;
-  const int rc = p.starts == 4   ? go(wilson_gauge_kernel<Store, CT, true, K4, false>,
-                                      wilson_gauge_kernel<Store, CT, true, K4, true>)
-                 : p.starts == 2 ? go(wilson_gauge_kernel<Store, CT, true, 2, false>,
-                                      wilson_gauge_kernel<Store, CT, true, 2, true>)
-                                 : go(wilson_gauge_kernel<Store, CT, true, 1, false>,
-                                      wilson_gauge_kernel<Store, CT, true, 1, true>);
+  const int rc = p.starts == 4   ? go(wilson_gauge_kernel<Store, CT, K4, false>,
+                                      wilson_gauge_kernel<Store, CT, K4, true>)
+                 : p.starts == 2 ? go(wilson_gauge_kernel<Store, CT, 2, false>,
+                                      wilson_gauge_kernel<Store, CT, 2, true>)
+                                 : go(wilson_gauge_kernel<Store, CT, 1, false>,
+                                      wilson_gauge_kernel<Store, CT, 1, true>);
   if (rc)
     return rc;
   *blocks = p.blocks / 3 * ndir;

@@ -131,19 +131,6 @@ __host__ __device__ inline GramTiles gram_tiles(int tstarts, int tmax) {
   return t;
 }
 
-// First spatial site of a column block: consecutive blocks step along nu (for
-// nu = y, z) where the columns tile the x extent, so that blocks running at
-// the same time extend with the same links (see gc_wilson_gauge.cu).
-__device__ __forceinline__ int gram_base(const Geom &g, int cb, int cols, int nu) {
-  if (nu == 0 || g.L[0] % cols != 0)
-    return cb * cols;
-  const int nxc = g.L[0] / cols;
-  const int Ln = nu == 1 ? g.L[1] : g.L[2];
-  const int n = cb % Ln, rest = cb / Ln;
-  const int xc = rest % nxc, other = rest / nxc;
-  return xc * cols + g.L[0] * (nu == 1 ? n + g.L[1] * other : other + g.L[1] * n);
-}
-
 // One warp task: the tiles (i0 + m, i0 + m + d0 + d), m < MT, d < ND, summed
 // over the units sub, sub + nsub, ... and over the start tiles, into E.
 // f1 / f2: the lane's first fragment element of unit 0 (slice 8 i0 + lane / 4,
@@ -265,7 +252,7 @@ __global__ void __launch_bounds__(kGramThreads, 4)
 
   const int nu = blockIdx.y;
   const int c = tid % cols, trow = tid / cols, tstep = kGramThreads / cols;
-  const int s = gram_base(g, blockIdx.x, cols, nu) + c;
+  const int s = column_base(g, blockIdx.x, cols, nu) + c;
   const bool active = s < g.Vs;
   const int Ln = sel4(g.L, nu), stn = sel4(g.stride, nu);
   const int xn = (s / stn) % Ln;

@@ -18,10 +18,10 @@
 // Bound: instruction issue (SU(3) mixed 32^4: 74% of the slots, FMA pipe 49%,
 // 24 warps on an SM; SU(2) 48^4 77% and 51%; SU(3) FP64 24^4 shared-memory
 // wavefronts 66%, FP64 pipe 49%). R,T <= L/2, whole W calls: SU(3) mixed 32^4
-// 2.70 -> 1.90 ms, 24^4 0.75 -> 0.51, 18 x 20 x 22 x 26 0.48 -> 0.29; SU(2)
-// mixed 48^4 5.16 -> 3.58; SU(3) FP64 24^4 0.80 -> 0.74. (The mixed figures with
-// the short FP32 sums of gc_corr.cuh; with one chain over all starts, 7-20%
-// faster, the shares above were taken.)
+// 2.70 -> 1.84 ms, 24^4 0.75 -> 0.50, 18 x 20 x 22 x 26 0.48 -> 0.29; SU(2)
+// mixed 48^4 5.16 -> 3.52; SU(3) FP64 24^4 0.80 -> 0.74. (The mixed figures with
+// the short FP32 sums of gc_corr.cuh; the shares were taken with one chain over
+// all starts, 5-17% faster.)
 //
 // 8 SU(3) columns a block (144 sequences, five warps, five blocks on an SM): 16
 // with nine warps took 1.86 ms at 32^4. A warp stays on 8 columns, four slices
@@ -45,7 +45,8 @@ namespace {
 // T values of a thread's window: their sums (FP32 two sets) and the window take
 // 3 J registers (FP64 4 J). More spill: 24 for SU(2) 48^4, T <= 24, 3.86 ms
 // against 3.57 in two windows of 12; 20 for SU(3) 32^4, T <= 16, 1.95 ms against
-// 1.90.
+// 1.90. (24 with four blocks on an SM does not, and takes 3.43 ms, but 32^3 x 40,
+// T <= 20, 0.64 ms against 0.60.)
 constexpr int corr_jmax(int nc, size_t ct_bytes) { return ct_bytes == 8 ? 12 : nc == 2 ? 20 : 16; }
 // Starts of one pass: equal shares of tstarts, whole vectors.
 __device__ __forceinline__ int corr_pass(int tstarts, int V) {

@@ -804,6 +804,10 @@ __global__ void __launch_bounds__(256)
 //       2868 / 2613, T <= 13 2914 / 3340, T <= 16 2966 / 3370; SU(2) 24^4 T <=
 //       12 276 / 221, 32^4 T <= 12 812 / 629, T <= 16 802 / 792, 48^4 T <= 24
 //       5710 / 6557
+//     (these with one FP32 chain of the correlation's mixed form; with its short
+//     sums, 5 to 17% slower, calls on either side of the line still meet: SU(3)
+//     32^3 x 10 T <= 4 / 5 686 / 702, 24^3 x 8 T <= 3 / 4 212 / 230, SU(2) 24^4 T
+//     <= 7 / 8 128 / 122)
 // (q kernel: at most 32 threads per column, so that a block of 8 columns fits)
 constexpr int kStarts = 4;
 int start_rows(int Lt) { return (Lt + kStarts - 1) / kStarts; }

@@ -445,10 +445,10 @@ template <class T> GC_HD SU2<T> proj(const SU2<T> &A, T) { return proj(A); }
 // eight Newton steps (a factor 1.5 each from there) do not reach the root. A
 // loop that ends at its cap answers false as well (3 million matrices with a
 // singular value from 1 to 1.535 times the rms: 2.3e-15 in FP64, 1.4e-6 in
-// FP32; at the cap the error was 0.45). Sums of SU(3) matrices with weights that add to one
-// have m <= 1; of HYP's level-1 sums on a rough field (plaquette 0.6) less
-// than 1% lie outside, of APE sums none. Elsewhere the result is not set and
-// the caller takes the reference's steps.
+// FP32; at the cap the error was 0.45). Sums of SU(3) matrices with weights that
+// add to one have m <= 1; of HYP's level-1 sums at plaquette 0.6 less than 1% lie outside,
+// of APE sums none (of sums of random matrices 82% and 74%). Elsewhere the result
+// is not set and the caller takes the reference's steps.
 GC_HD double gc_rsqrt(double x) {
 #if defined(__CUDA_ARCH__)
   return rsqrt(x);

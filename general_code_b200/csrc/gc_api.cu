@@ -1338,7 +1338,7 @@ int gc_wilson_spatial_3d(gc_lattice *h, int r_min, int r_max, int time_min, int 
   // one transform, one launch for all loops of both directions and one
   // reduction, against 2 R_max loop and line launches that walk the exact
   // product through L2: R,T <= 6 with 4 measurements at SU(3) 24^4 20.9 -> 5.7
-  // ms FP64, 11.0 -> 4.4 ms mixed, SU(2) 5.2 -> 1.6 and 4.3 -> 1.1 ms.
+  // ms FP64, 11.0 -> 3.9 ms mixed, SU(2) 5.2 -> 1.6 and 4.3 -> 1.1 ms.
   // The mixed SU(3) form keeps the transformed links with all 18 reals: a planar
   // sum that six steps do not bring onto the group (a few in a million at
   // plaquette 0.5) is no reason for the exact product then, and what is left to

@@ -259,7 +259,9 @@ int plan_error(const char *what);
 // launch (an APE step, us: SU(2) mixed 16^4 6.4 -> 3.9, SU(3) mixed 16^4 18.8 ->
 // 16.1, 32^4 215 -> 212.6). Letting the next kernel start
 // earlier (a trigger at the blocks' start) measured the same. Under stream
-// capture the launch is an ordinary one.
+// capture the launch is an ordinary one: the batch, which captures its chains,
+// puts multi-job kernels between these that do not wait this way, and such edges
+// of a graph have not been measured.
 __device__ __forceinline__ void wait_previous() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
 }

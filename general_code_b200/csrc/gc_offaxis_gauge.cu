@@ -13,9 +13,10 @@
 // per line at r, T <= 6). Many are equal step for step (the reference counts
 // an orientation twice, and permutations repeat symmetric patterns), and many
 // begin alike: as a tree with a node per step the 678 lines of r <= 6 (4473
-// links) are 550 distinct lines and 1140 products. A block walks a part of
+// links) are 550 distinct lines and 1140 products (gc_offaxis_tree.h builds the
+// tree). A block walks a part of
 // the tree in depth-first order for its columns: a thread owns one line slot
-// (column, slice, cut), keeps the current product in registers and the
+// (column, slice), keeps the current product in registers and the
 // products that a later branch continues on a short private stack (the
 // largest branch is walked last, so the stack holds at most log2 of the nodes).
 // The link of the next node is loaded while the current one is multiplied

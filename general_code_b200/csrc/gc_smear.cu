@@ -61,15 +61,20 @@ template <class Store> struct MixedSU3 {
   static constexpr bool value = Store::NC == 3 && (Store::kBytes == 48 || Store::kBytes == 72);
 };
 
-// Projection of a sum and its store. SU(3): polar_su3 (gc_algebra.cuh), and
+// Projection of a sum and its store. SU(3): polar_parts (gc_algebra.cuh), and
 // outside its region the reference's matrix steps (out of line: one sum in a
-// hundred of HYP's level 1, none of APE's). What bounds it: the FP64 pipe in
-// the FP64 form, the FMA pipe's operand bandwidth in the mixed form, so what
-// counts is the number of multiply-adds. Against the matrix iteration for
-// every sum (3 to 6 steps): HYP at SU(3) 32^4 3.18 -> 2.05 ms FP64 and 1.60
-// -> 1.25 ms mixed, an APE step 0.498 -> 0.384 ms FP64; a mixed APE step
-// 0.251 -> 0.236 ms on the first ten after HYP and unchanged (0.215 ms) on a
-// field so smooth that one FP32 matrix step had been enough.
+// hundred of HYP's level 1 at plaquette 0.6, none of APE's). What bounds it: the
+// FP64 pipe in the FP64 form, the FMA pipe's operand bandwidth in the mixed form,
+// so what counts is the number of multiply-adds. A warp with one sum outside
+// takes both, so on a field rougher than plaquette 0.4 the matrix steps for
+// every sum (3 to 6 of them) would be faster. us at SU(3) 24^4, matrix steps /
+// this, by plaquette:
+//   FP64   HYP  0.78  998 / 586   0.50 1026 / 768   0.37 1030 / 1021   0.15 1028 / 1236
+//          APE        216 / 137         215 / 146         218 / 195          220 / 257
+//   mixed  HYP        504 / 430         552 / 523         569 / 667          584 / 766
+//          APE         98 / 75          100 / 78          105 / 101          109 / 136
+// (Deciding before the Gram matrix's other elements, so that warps with all sums
+// outside pass the rest by, changed none of these.)
 //
 // Steps: FP64 the iteration with the early exit of proj(A, tol); FP32 steps
 // while the unitarity defect exceeds 2e-5 (at most five), then one FP64 step.

@@ -46,8 +46,11 @@ extern "C" {
 #define GC_ERR_BUSY 8      /* admission refused (no free slot or memory)      */
 
 #define GC_PREC_FP64 0     /* links stored and computed in FP64               */
-#define GC_PREC_MIXED 1    /* FP32 links (SU(3): 12 reals, third row rebuilt),
-                              FP64 projection and FP64 trace accumulation     */
+#define GC_PREC_MIXED 1    /* FP32 links (SU(3): 12 reals, third row rebuilt) and
+                              products; SU(3) projection in FP32 with its last
+                              correction in FP64 (SU(2): FP64); loops summed in
+                              FP32 over at most 64 time slices of a line element
+                              or four loops, in FP64 beyond                  */
 
 /* Methods of the on-axis Wilson loops (gc_set_wilson_method). */
 #define GC_WILSON_AUTO 0   /* temporal gauge where it applies, else exact     */

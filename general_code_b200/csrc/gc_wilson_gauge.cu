@@ -891,10 +891,14 @@ WilsonPlan wilson_gauge_plan(const Geom &g, int tmin, int tmax, int nc, int ct_b
   const int ncomp = (nc == 3) ? 18 : 4;
   const int lanes = wilson_lanes(nc, ct_bytes);
   // consecutive start slices per thread (a divisor of Lt): 2 for SU(3) (its
-  // registers hold two lane-packed matrices), 4 for SU(2) (quaternions are
-  // small)
+  // registers hold two lane-packed matrices) and on SU(2) lattices that leave the
+  // chip idle otherwise, 4 on larger SU(2) lattices (quaternions are small). SU(2)
+  // calls in us with 2 / 4 starts: FP64 12^4 R,T <= 6 56 / 69, 16^3 x 4 54 / 67,
+  // 16^4 R,T <= 8 75 / 90, 20^4 117 / 138, 16^3 x 32 102 / 102, 24^4 R,T <= 6 179 /
+  // 165; mixed 16^4 70 / 79, 10^3 x 48 60 / 65, 16^3 x 32 101 / 90, 20^4 105 / 96
   p.starts = 1;
-  for (int ks : {nc == 2 ? 4 : 2, 2})
+  const bool four = nc == 2 && g.V > (ct_bytes == 8 ? 160000 : 65536);
+  for (int ks : {four ? 4 : 2, 2})
     if (p.starts == 1 && Lt % ks == 0 && Lt / ks <= 64)
       p.starts = ks;
   p.rows = p.starts > 1 ? Lt / p.starts : largest_divisor_upto_g(Lt, 64);
